@@ -448,22 +448,60 @@ __global__ void kb_carry_undo(const BatchCtl* ctl, const int* slot_mesh, BatchMe
 }
 
 // ---------------------------------------------------------------- job set-up and results
-__global__ void kb_offset_faces(int4* tri, const long long* foff, const long long* voff, int n_meshes, int n_faces) {
+// mesh m with off[m] <= i < off[m + 1] (empty meshes own nothing)
+__device__ __forceinline__ int mesh_of(const long long* __restrict__ off, int n_meshes, long long i) {
+    int lo = 0, hi = n_meshes - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (off[mid] <= i) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+// every mesh's faces with their indices checked against the mesh (launch_load_tris over the whole batch)
+__global__ void kb_load_tris(const int* __restrict__ tris, const long long* __restrict__ foff,
+                             const long long* __restrict__ voff, int n_meshes, int n_faces, int4* out, RoundCounters* rc) {
     for (int f = gtid(); f < n_faces; f += gstride()) {
-        int lo = 0, hi = n_meshes - 1;  // the mesh m with foff[m] <= f < foff[m + 1]
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (foff[mid] <= f) lo = mid;
-            else hi = mid - 1;
-        }
-        int4 t = tri[f];
+        const int m = mesh_of(foff, n_meshes, f);
+        const int n_pts = (int)(voff[m + 1] - voff[m]);
+        const int a = tris[3 * (size_t)f], b = tris[3 * (size_t)f + 1], c = tris[3 * (size_t)f + 2];
+        const bool dead = (a == -1 && b == -1 && c == -1);
+        const bool ok = dead || (a >= 0 && a < n_pts && b >= 0 && b < n_pts && c >= 0 && c < n_pts);
+        if (!ok) atomicOr(&rc->status, kErrBadIndex);
+        out[f] = ok ? make_int4(a, b, c, 0) : make_int4(-1, -1, -1, 0);
+    }
+}
+
+// The first round's shuffle of every mesh in one pass: mesh m owns 2^bits flags from goff[m] (its bijection's domain;
+// the keys are the same for all sizes), one scan runs over all of them, and because the meshes before m flag exactly
+// their face counts the scan gives the place in the batch's face numbering. The faces leave in the batch's vertex
+// numbering. (64 meshes: 192 launches of 4 to 6 us one after the other before, three now.)
+__global__ void kb_shuffle_flags(Feistel fb, const long long* __restrict__ goff, const long long* __restrict__ foff,
+                                 int n_meshes, int n_flags, int* flags) {
+    for (int i = gtid(); i < n_flags; i += gstride()) {
+        const int m = mesh_of(goff, n_meshes, i);
+        const unsigned long long nf = (unsigned long long)(foff[m + 1] - foff[m]);
+        flags[i] = feistel(fb, feistel_size(nf), (unsigned long long)(i - goff[m])) < nf ? 1 : 0;
+    }
+    if (gtid() == 0) flags[n_flags] = 0;
+}
+
+__global__ void kb_shuffle_gather(Feistel fb, const long long* __restrict__ goff, const long long* __restrict__ foff,
+                                  const long long* __restrict__ voff, int n_meshes, int n_flags,
+                                  const int* __restrict__ scan, const int4* __restrict__ src, int4* dst) {
+    for (int i = gtid(); i < n_flags; i += gstride()) {
+        if (scan[i + 1] == scan[i]) continue;
+        const int m = mesh_of(goff, n_meshes, i);
+        const FeistelSize z = feistel_size((unsigned long long)(foff[m + 1] - foff[m]));
+        int4 t = src[foff[m] + (long long)feistel(fb, z, (unsigned long long)(i - goff[m]))];
         if (t.x >= 0) {
-            const int o = (int)voff[lo];
+            const int o = (int)voff[m];
             t.x += o;
             t.y += o;
             t.z += o;
         }
-        tri[f] = t;
+        dst[scan[i]] = t;
     }
 }
 
@@ -539,7 +577,9 @@ struct pamo_csr {
     Buf<int> slot_mesh, slot_v0, slot_np, slot_f0, slot_nf, slot_stuck, mesh_root;
     Buf<float> slot_scale, mesh_scale, centre;
     Buf<float4> mean;
-    Buf<long long> dev_voff, dev_foff, dev_out_voff, dev_out_foff;
+    Buf<long long> dev_voff, dev_foff, dev_goff, dev_out_voff, dev_out_foff;
+    Buf<CenterJob> center_jobs;
+    Buf<unsigned char> center_scratch;
     RoundCounters* rc = nullptr;
     BatchCtl* ctl = nullptr;
     BatchCtl* h_ctl = nullptr;
@@ -615,7 +655,7 @@ struct pamo_csr {
         release(invalid_reg); release(ecost_reg); release(mesh); release(slot_mesh); release(slot_v0);
         release(slot_np); release(slot_f0); release(slot_nf); release(slot_stuck); release(mesh_root);
         release(slot_scale); release(mesh_scale); release(centre); release(mean); release(dev_voff);
-        release(dev_foff); release(dev_out_voff); release(dev_out_foff);
+        release(dev_foff); release(dev_goff); release(center_jobs); release(center_scratch); release(dev_out_voff); release(dev_out_foff);
         if (bvh_mem) cudaFree(bvh_mem);
         bvh_mem = nullptr;
         if (rc) cudaFree(rc);
@@ -638,7 +678,7 @@ struct pamo_csr {
         if ((r = grow(tri, fc)) || (r = grow(orig_tri, fc)) || (r = grow(tri_in, fc)) || (r = grow(tri_next, fc)) ||
             (r = grow(res_tri, fc)) || (r = grow(tri_load, fc)) || (r = grow(ecount, fc + 1)) ||
             (r = grow(qflag, fc + 1)) || (r = grow(qlist, fc)) || (r = grow(fflags, fc + 1)) || (r = grow(nt, 3 * fc)) ||
-            (r = grow(nxt, 3 * fc)) || (r = grow(spc, 3 * fc)) || (r = grow(fmesh, fc)) || (r = grow(shuffle_flags, 2 * fc + 40)) ||
+            (r = grow(nxt, 3 * fc)) || (r = grow(spc, 3 * fc)) || (r = grow(fmesh, fc)) ||
             (r = grow(fgeo, 6 * fc)) || (r = grow(face_mean, 3 * fc)) || (r = grow(fkey, fc)) || (r = grow(hit, fc + 1)))
             return r;
         if ((r = grow(edges, ec)) || (r = grow(eorder, ec)) || (r = grow(win, ec + 1)) || (r = grow(winners, ec)) ||
@@ -830,22 +870,50 @@ struct pamo_csr {
         cudaMemcpyAsync(dev_voff.p, voff, (M + 1) * sizeof(long long), cudaMemcpyHostToDevice, s);
         cudaMemcpyAsync(dev_foff.p, foff, (M + 1) * sizeof(long long), cudaMemcpyHostToDevice, s);
         cudaMemsetAsync(rc, 0, sizeof(RoundCounters), s);
-        // per mesh: centring and scale (numpy's order), validation, the first round's shuffle
+        // centring and scale (numpy's order), validation, the first round's shuffle, each over all meshes at once
+        std::vector<CenterJob> jobs;
+        std::vector<long long> goff(M + 1);
+        long long flags = 0, chunks = 0, faces = 0;
+        int max_nf = 0, max_nv = 0;
         for (int m = 0; m < M; ++m) {
             const int nv = (int)(voff[m + 1] - voff[m]), nf = (int)(foff[m + 1] - foff[m]);
-            if (nv > 0 && nf > 0)
-                launch_center(points + 3 * voff[m], triangles + 3 * foff[m], nv, nf, face_mean.p, centre.p + 16 * m,
-                              mesh_scale.p + m, pos_in.p + voff[m], s, true);
-            else
-                cudaMemsetAsync(centre.p + 16 * m, 0, 16 * sizeof(float), s);
-            if (nf > 0) {
-                launch_load_tris(triangles + 3 * foff[m], nf, nv, tri_load.p + foff[m], rc, s);
-                Feistel fb = make_feistel((unsigned long long)nf);
-                launch_shuffle_tris(fb, shuffle_flags.p, scan_scratch, tri_load.p + foff[m], tri_in.p + foff[m], nf, s,
-                                    &rc->status);
-            }
+            goff[m] = flags;
+            if (nf > 0) flags += (long long)make_feistel((unsigned long long)nf).n;
+            if (nv < 1 || nf < 1) continue;
+            CenterJob J{points + 3 * voff[m], triangles + 3 * foff[m], nv, nf, faces, (int)chunks, centre.p + 16 * m,
+                        mesh_scale.p + m, pos_in.p + voff[m]};
+            jobs.push_back(J);
+            chunks += center_chunks(nf);
+            faces += nf;
+            max_nf = std::max(max_nf, nf);
+            max_nv = std::max(max_nv, nv);
         }
-        kb_offset_faces<<<grid_for(F, kT), kT, 0, s>>>(tri_in.p, dev_foff.p, dev_voff.p, M, (int)F); note_launch();
+        goff[M] = flags;
+        if ((r = grow(shuffle_flags, (size_t)flags + 1)) || (r = grow(dev_goff, (size_t)M + 1)) ||
+            (r = grow(center_jobs, std::max<size_t>(jobs.size(), 1))) ||
+            (r = grow(center_scratch, center_scratch_bytes(chunks) + 16)))
+            return r;
+        cudaMemsetAsync(centre.p, 0, (size_t)M * 16 * sizeof(float), s);
+        cudaMemcpyAsync(dev_goff.p, goff.data(), (M + 1) * sizeof(long long), cudaMemcpyHostToDevice, s);
+        if (!jobs.empty()) {
+            cudaMemcpyAsync(center_jobs.p, jobs.data(), jobs.size() * sizeof(CenterJob), cudaMemcpyHostToDevice, s);
+            CenterJobs J{};
+            J.many = center_jobs.p;
+            J.n = (int)jobs.size();
+            J.n_chunks = (int)chunks;
+            launch_center_jobs(J, face_mean.p, center_scratch.p, max_nf, max_nv, s, true);
+        }
+        if (F > 0) {
+            kb_load_tris<<<grid_for(F, kT), kT, 0, s>>>(triangles, dev_foff.p, dev_voff.p, M, (int)F, tri_load.p, rc);
+            note_launch();
+            const Feistel fb = make_feistel(1);
+            const int g = grid_for(flags, kT);
+            kb_shuffle_flags<<<g, kT, 0, s>>>(fb, dev_goff.p, dev_foff.p, M, (int)flags, shuffle_flags.p); note_launch();
+            exclusive_scan(shuffle_flags.p, shuffle_flags.p, nullptr, (int)flags + 1, nullptr, scan_scratch, s,
+                           &rc->status, flags);
+            kb_shuffle_gather<<<g, kT, 0, s>>>(fb, dev_goff.p, dev_foff.p, dev_voff.p, M, (int)flags, shuffle_flags.p,
+                                               tri_load.p, tri_in.p); note_launch();
+        }
         kb_mean_table<<<grid_for(M, kT), kT, 0, s>>>(centre.p, M, mean.p); note_launch();
         {
             int st = 0;

@@ -1022,7 +1022,8 @@ int simplify_loop_on(pamo_ctx* ctx, const float* points, const int32_t* triangle
 
     // centring and scale on the device, with numpy's float32 summation order
     ctx->prof.begin(kPhCenter, s);
-    launch_center(points, triangles, n_points, n_triangles, ctx->face_mean.p, ctx->d_center, ctx->d_scale,
+    // the chunk records go to the ring records' buffer (96 bytes a face, free until the first round)
+    launch_center(points, triangles, n_points, n_triangles, ctx->face_mean.p, ctx->fgeo.p, ctx->d_center, ctx->d_scale,
                   ctx->pos_in.p, s, opt.centre);
     ctx->prof.end(kPhCenter, s);
 
@@ -1231,7 +1232,7 @@ int pamo_tris_mean(pamo_ctx* ctx, const float* points, const int32_t* triangles,
     ctx->stream = (cudaStream_t)stream;
     int r;
     if ((r = ctx->ensure_vertex_buffers(n_points)) || (r = ctx->ensure_face_buffers(n_triangles))) return r;
-    launch_center(points, triangles, n_points, n_triangles, ctx->face_mean.p, ctx->d_center, ctx->d_scale,
+    launch_center(points, triangles, n_points, n_triangles, ctx->face_mean.p, ctx->fgeo.p, ctx->d_center, ctx->d_scale,
                   ctx->pos_out.p, ctx->stream, true);
     cudaMemcpyAsync(ctx->h_pinned_f, ctx->d_center, 3 * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream);
     if ((r = ctx->check(cudaStreamSynchronize(ctx->stream), "tris_mean"))) return r;

@@ -75,30 +75,16 @@ __global__ void k_copy4(const int4* __restrict__ src, int4* dst, int n) {
     for (int f = gtid(); f < n; f += gstride()) dst[f] = src[f];
 }
 
-__device__ __forceinline__ unsigned long long feistel(const Feistel& fb, unsigned long long idx) {
-    uint32_t s0 = (uint32_t)(idx >> fb.rbits), s1 = (uint32_t)(idx & fb.rmask);
-#pragma unroll 4
-    for (int r = 0; r < 24; ++r) {
-        const unsigned long long prod = 0xD2B74407B1CE6E93ull * (unsigned long long)s0;
-        const uint32_t hi = (uint32_t)(prod >> 32);
-        uint32_t lo = (uint32_t)prod;
-        lo = (lo << (fb.rbits - fb.lbits)) | (s1 >> fb.lbits);
-        s0 = ((hi ^ fb.key[r]) ^ s1) & fb.lmask;
-        s1 = lo & fb.rmask;
-    }
-    return ((unsigned long long)s0 << fb.rbits) | (unsigned long long)s1;
-}
-
 __global__ void k_shuffle_flags(Feistel fb, int* flags) {
     const long long n = (long long)fb.n;
-    for (long long i = gtid(); i < n; i += gstride()) flags[i] = feistel(fb, (unsigned long long)i) < fb.m ? 1 : 0;
+    for (long long i = gtid(); i < n; i += gstride()) flags[i] = feistel(fb, fb.size, (unsigned long long)i) < fb.m ? 1 : 0;
     if (gtid() == 0) flags[n] = 0;
 }
 
 __global__ void k_shuffle_gather(Feistel fb, const int* __restrict__ scan, const int4* __restrict__ src, int4* dst) {
     const long long n = (long long)fb.n;
     for (long long i = gtid(); i < n; i += gstride()) {
-        const unsigned long long g = feistel(fb, (unsigned long long)i);
+        const unsigned long long g = feistel(fb, fb.size, (unsigned long long)i);
         if (g < fb.m) dst[scan[i]] = src[g];
     }
 }
@@ -975,233 +961,6 @@ __global__ void k_export_mesh(int np, int nf, const float4* __restrict__ pos, co
     }
 }
 
-// ------------------------------------------------------------------ centring (pamo/__init__.py:60-72, 117, 126)
-// numpy float32 semantics: per-face ((a + b) + c) / 3, then a sequential float32 sum over faces / F.
-// Face means are written per coordinate (SoA) so that the sequential pass can stage them through shared
-// memory with coalesced loads; three lanes of one warp then run the three dependent add chains while the
-// other warps fetch the next tile.
-__global__ void k_face_means(const float* __restrict__ pts, const int* __restrict__ tris, int nf, float* fm) {
-    for (int f = gtid(); f < nf; f += gstride()) {
-        const int a = tris[3 * f], b = tris[3 * f + 1], c = tris[3 * f + 2];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) fm[(size_t)d * nf + f] = ((pts[3 * a + d] + pts[3 * b + d]) + pts[3 * c + d]) / 3.0f;
-    }
-}
-
-
-// The sequential float32 sum s_k = fl(s_(k-1) + x_k) of numpy's axis-0 reduction, exact, with window
-// parallelism (one block per coordinate). While the running sum stays inside one binade [2^e, 2^(e+1)) (float
-// spacing u = 2^(e-23)) and off its end points, fl(s + x) = s + u * round(x / u): the rounded increments are
-// integers, so a window's running sums are s + u * (prefix sums of the increments), exact in int64. Each element
-// is checked (its running sum inside [2^23 + 1, 2^24 - 1] units of u, its increment not a half-way tie, whose
-// rounding would depend on the sum's parity); the first element that fails is added with a float add and the
-// next window starts after it. Where failures are dense (a sum near zero, or crossing binades quickly), a
-// stretch is summed in order by one thread.
-constexpr int kSumThreads = 1024;
-constexpr int kSumPer = 16;
-constexpr int kSumWindow = kSumThreads * kSumPer;
-
-__global__ void __launch_bounds__(kSumThreads) k_exact_sequential_sum(const float* __restrict__ fm, int nf,
-                                                                      float* center) {
-    const float* x = fm + (size_t)blockIdx.x * nf;
-    constexpr int kStage = 4096;
-    __shared__ long long wsum[32];
-    __shared__ int wmin[32];
-    __shared__ float stage[kStage];
-    __shared__ float s_sh;
-    __shared__ int k_sh, burst_sh, fail_sh, short_sh;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) {
-        s_sh = 0.0f;
-        k_sh = 0;
-        burst_sh = 0;
-        short_sh = 0;
-    }
-    __syncthreads();
-    while (true) {
-        const float s = s_sh;
-        const int k = k_sh;
-        const int burst = burst_sh;
-        __syncthreads();  // everyone has read the state
-        if (k >= nf) break;
-        int e = 0;
-        bool par = burst == 0 && s != 0.0f && isfinite(s);
-        if (par) {
-            e = ilogbf(s);
-            par = e >= -125 && e <= 126;
-        }
-        if (!par) {
-            // in order, staged through shared memory: a burst after dense failures, 64 elements while the sum is
-            // zero or subnormal, the rest when it is not finite (every later sum stays so)
-            const int n = min(burst > 0 ? burst : (isfinite(s) ? 64 : nf - k), nf - k);
-            float t = s;
-            for (int c = 0; c < n; c += kStage) {
-                const int m = min(kStage, n - c);
-                for (int i = threadIdx.x; i < m; i += kSumThreads) stage[i] = x[k + c + i];
-                __syncthreads();
-                if (threadIdx.x == 0)
-                    for (int i = 0; i < m; ++i) t += stage[i];
-                __syncthreads();
-            }
-            if (threadIdx.x == 0) {
-                s_sh = t;
-                k_sh = k + n;
-                burst_sh = 0;
-            }
-            __syncthreads();
-            continue;
-        }
-        // integer arithmetic on the float bits (the fp64 pipe is too slow for this): s = S * u with u = 2^(e-23),
-        // x / u = +-m * 2^(ex - e) for x's 24-bit significand m
-        const unsigned sb = __float_as_uint(s);
-        const long long S = (sb >> 31) ? -(long long)((sb & 0x7FFFFFu) | 0x800000u) : (long long)((sb & 0x7FFFFFu) | 0x800000u);
-        const int base = k + threadIdx.x * kSumPer;
-        const int wend = min(k + kSumWindow, nf);
-        long long q[kSumPer];
-        unsigned badm = 0;
-        long long tsum = 0;
-#pragma unroll
-        for (int i = 0; i < kSumPer; ++i) {
-            const int idx = base + i;
-            q[i] = 0;
-            if (idx < wend) {
-                const unsigned b = __float_as_uint(x[idx]);
-                const int bex = (int)((b >> 23) & 0xFFu);
-                if (bex == 0xFF) {
-                    badm |= 1u << i;  // inf or nan
-                } else if ((b & 0x7FFFFFFFu) != 0u) {
-                    const long long m = bex ? (long long)((b & 0x7FFFFFu) | 0x800000u) : (long long)(b & 0x7FFFFFu);
-                    const int sh = (bex ? bex - 127 : -126) - e;  // x / u = m * 2^sh
-                    long long mag;
-                    if (sh >= 0) {
-                        if (sh > 16) badm |= 1u << i;  // |x / u| >= 2^40: leaves the binade anyway
-                        mag = sh > 16 ? 0 : m << sh;
-                    } else if (-sh >= 25) {
-                        mag = 0;  // |x / u| < 1/2
-                    } else {
-                        const int kk = -sh;
-                        const long long rem = m & ((1ll << kk) - 1), half = 1ll << (kk - 1);
-                        if (rem == half) badm |= 1u << i;  // a tie: rounds by the sum's parity
-                        mag = (m >> kk) + (rem > half ? 1 : 0);
-                    }
-                    q[i] = (b >> 31) ? -mag : mag;
-                }
-            }
-            tsum += q[i];
-        }
-        // block exclusive scan of the per-thread sums
-        long long inc = tsum;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const long long t = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += t;
-        }
-        if (lane == 31) wsum[warp] = inc;
-        __syncthreads();
-        if (warp == 0) {
-            long long w = wsum[lane];
-            long long wi = w;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const long long t = __shfl_up_sync(0xffffffffu, wi, o);
-                if (lane >= o) wi += t;
-            }
-            wsum[lane] = wi - w;
-        }
-        __syncthreads();
-        long long R = S + wsum[warp] + inc - tsum;
-        const long long lo = s > 0.0f ? (1ll << 23) + 1 : -((1ll << 24) - 1);
-        const long long hi = s > 0.0f ? (1ll << 24) - 1 : -((1ll << 23) + 1);
-        int first = nf;
-#pragma unroll
-        for (int i = 0; i < kSumPer; ++i) {
-            const int idx = base + i;
-            if (idx < wend && first == nf) {
-                R += q[i];
-                if ((badm >> i & 1u) || R < lo || R > hi) first = idx;
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) first = min(first, __shfl_xor_sync(0xffffffffu, first, o));
-        if (lane == 0) wmin[warp] = first;
-        __syncthreads();
-        if (warp == 0) {
-            int m = wmin[lane];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) m = min(m, __shfl_xor_sync(0xffffffffu, m, o));
-            if (lane == 0) fail_sh = m;
-        }
-        __syncthreads();
-        const int f = min(fail_sh, wend);  // elements [k, f) are exact; f fails (or ends the window)
-        // the owner of element f - 1 publishes the sum after it
-        if (f > k && (f - 1 - k) / kSumPer == (int)threadIdx.x) {
-            long long r = S + wsum[warp] + inc - tsum;
-            for (int i = 0; i <= (f - 1 - k) % kSumPer; ++i) r += q[i];
-            // r * u with 2^23 < |r| < 2^24: the float with r's significand and s's exponent
-            s_sh = __uint_as_float((r < 0 ? 0x80000000u : 0u) | ((unsigned)(e + 127) << 23) |
-                                   ((unsigned)(r < 0 ? -r : r) & 0x7FFFFFu));
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            if (f < wend) {  // the failing element: a float add in order
-                s_sh = s_sh + x[f];
-                k_sh = f + 1;
-                // four windows in a row that advanced less than 32 elements: sum the next 1024 in order
-                short_sh = (f - k < 32) ? short_sh + 1 : 0;
-                if (short_sh >= 4) {
-                    burst_sh = 1024;
-                    short_sh = 0;
-                }
-            } else {
-                k_sh = wend;
-                short_sh = 0;
-            }
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) center[blockIdx.x] = s_sh / (float)nf;
-}
-
-__global__ void k_center_points(const float* __restrict__ pts, int np, const float* __restrict__ center, float4* out,
-                                unsigned* ext) {
-    const float cx = center[0], cy = center[1], cz = center[2];
-    float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (int v = gtid(); v < np; v += gstride()) {
-        const float x = pts[3 * v] - cx, y = pts[3 * v + 1] - cy, z = pts[3 * v + 2] - cz;
-        out[v] = make_float4(x, y, z, 0.f);
-        mn[0] = fminf(mn[0], x); mn[1] = fminf(mn[1], y); mn[2] = fminf(mn[2], z);
-        mx[0] = fmaxf(mx[0], x); mx[1] = fmaxf(mx[1], y); mx[2] = fmaxf(mx[2], z);
-    }
-#pragma unroll
-    for (int d = 0; d < 3; ++d)
-        for (int o = 16; o > 0; o >>= 1) {
-            mn[d] = fminf(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], o));
-            mx[d] = fmaxf(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], o));
-        }
-    if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            unsigned a = __float_as_uint(mn[d]), b = __float_as_uint(mx[d]);
-            a = (a & 0x80000000u) ? ~a : (a | 0x80000000u);
-            b = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-            atomicMin(&ext[d], a);
-            atomicMax(&ext[3 + d], b);
-        }
-    }
-}
-
-__device__ __forceinline__ float ord_dec(unsigned u) { return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u); }
-
-// scale = max(max(ex, ey), ez) of the centred points (pamo/__init__.py:126)
-__global__ void k_extents(const unsigned* ext, float* scale) {
-    if (threadIdx.x != 0) return;
-    const float ex = ord_dec(ext[3]) - ord_dec(ext[0]);
-    const float ey = ord_dec(ext[4]) - ord_dec(ext[1]);
-    const float ez = ord_dec(ext[5]) - ord_dec(ext[2]);
-    const float m = (ey > ex) ? ey : ex;
-    *scale = (ez > m) ? ez : m;
-}
-
 // ================================================================== device-driven rounds
 // The same steps as the host-sized launchers, with every size read from the device (LoopState, RoundCounters),
 // so that one captured graph serves every round of a size class.
@@ -1313,27 +1072,13 @@ __global__ void k_copy_undo_dev(const RoundCounters* rc, const int* __restrict__
 // ================================================================== host launchers
 Feistel make_feistel(unsigned long long m) {
     Feistel fb{};
-    unsigned long long bits;
-    if (m <= 16) {
-        bits = 4;
-    } else {
-        bits = 0;
-        unsigned long long t = m - 1;
-        while (t) {
-            ++bits;
-            t >>= 1;
-        }
-    }
-    fb.lbits = (uint32_t)(bits / 2);
-    fb.rbits = (uint32_t)(bits - bits / 2);
-    fb.lmask = (uint32_t)((1ull << fb.lbits) - 1);
-    fb.rmask = (uint32_t)((1ull << fb.rbits) - 1);
+    fb.size = feistel_size(m);
     unsigned long long x = 1;  // minstd_rand, default seed
     for (int r = 0; r < 24; ++r) {
         x = (x * 48271ull) % 2147483647ull;
         fb.key[r] = (uint32_t)x;
     }
-    fb.n = 1ull << bits;
+    fb.n = 1ull << (fb.size.lbits + fb.size.rbits);
     fb.m = m;
     return fb;
 }
@@ -1549,22 +1294,6 @@ void launch_export_mesh(int n_pts, int n_tris, const float4* pos, const int4* tr
                         int* tris, cudaStream_t s) {
     const int n = n_pts > n_tris ? n_pts : n_tris;
     k_export_mesh<<<grid_for(n, kT), kT, 0, s>>>(n_pts, n_tris, pos, tri, add, verts, tris); note_launch();
-}
-
-void launch_center(const float* pts, const int* tris, int n_pts, int n_tris, float* face_mean, float* center,
-                   float* d_scale, float4* pos_out, cudaStream_t s, bool centre) {
-    // center[0..2] = tris_mean (zero when not centring); center[4..9] scratch (order-preserving extents)
-    if (centre) {
-        k_face_means<<<grid_for(n_tris, kT), kT, 0, s>>>(pts, tris, n_tris, face_mean); note_launch();
-        k_exact_sequential_sum<<<3, kSumThreads, 0, s>>>(face_mean, n_tris, center); note_launch();
-    } else {
-        cudaMemsetAsync(center, 0, 4 * sizeof(float), s);
-    }
-    unsigned* ext = (unsigned*)(center + 4);
-    cudaMemsetAsync(ext, 0xFF, 3 * sizeof(unsigned), s);
-    cudaMemsetAsync(ext + 3, 0x00, 3 * sizeof(unsigned), s);
-    k_center_points<<<grid_for(n_pts, kT), kT, 0, s>>>(pts, n_pts, center, pos_out, ext); note_launch();
-    k_extents<<<1, 32, 0, s>>>(ext, d_scale); note_launch();
 }
 
 // ---- device-driven rounds ----

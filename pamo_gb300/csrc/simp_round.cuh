@@ -7,13 +7,43 @@
 
 namespace pamo {
 
-struct Feistel {  // thrust::shuffle's bijection parameters for m elements
-    uint32_t key[24];
+// thrust::shuffle's bijection on [0, 2^bits), 2^bits >= m elements (at least 2^4)
+struct FeistelSize {
     uint32_t lbits, rbits, lmask, rmask;
+};
+__host__ __device__ inline FeistelSize feistel_size(unsigned long long m) {
+    uint32_t bits = 4;
+    if (m > 16) {
+        bits = 0;
+        for (unsigned long long t = m - 1; t; t >>= 1) ++bits;
+    }
+    FeistelSize z;
+    z.lbits = bits / 2;
+    z.rbits = bits - bits / 2;
+    z.lmask = (uint32_t)((1ull << z.lbits) - 1);
+    z.rmask = (uint32_t)((1ull << z.rbits) - 1);
+    return z;
+}
+struct Feistel {
+    uint32_t key[24];  // the same for every size
+    FeistelSize size;
     unsigned long long n;  // 2^bits
     unsigned long long m;
 };
 Feistel make_feistel(unsigned long long m);
+__device__ __forceinline__ unsigned long long feistel(const Feistel& fb, const FeistelSize& z, unsigned long long idx) {
+    uint32_t s0 = (uint32_t)(idx >> z.rbits), s1 = (uint32_t)(idx & z.rmask);
+#pragma unroll 4
+    for (int r = 0; r < 24; ++r) {
+        const unsigned long long prod = 0xD2B74407B1CE6E93ull * (unsigned long long)s0;
+        const uint32_t hi = (uint32_t)(prod >> 32);
+        uint32_t lo = (uint32_t)prod;
+        lo = (lo << (z.rbits - z.lbits)) | (s1 >> z.lbits);
+        s0 = ((hi ^ fb.key[r]) ^ s1) & z.lmask;
+        s1 = lo & z.rmask;
+    }
+    return ((unsigned long long)s0 << z.rbits) | (unsigned long long)s1;
+}
 
 // ---- set-up of a round ----
 void launch_undo_bookkeeping(const int* verts_undo, int n_verts_undo, int is_stuck, int* tmp_undo, int* undo_list,
@@ -99,9 +129,30 @@ void launch_export_mesh(int n_pts, int n_tris, const float4* pos, const int4* tr
                         int* tris, cudaStream_t s);
 
 // ---- whole-loop helpers ----
-void launch_center(const float* pts, const int* tris, int n_pts, int n_tris, float* face_mean, float* center,
-                   float* d_scale, float4* pos_out, cudaStream_t s,
-                   bool centre = true);
+// One mesh's centring: center[0..2] = tris_mean (zero when not centring), center[4..9] scratch (order-preserving
+// extents), *scale = the largest extent of the centred points, pos_out = the centred points.
+struct CenterJob {
+    const float* pts;
+    const int* tris;
+    int n_pts, n_tris;   // at least one each
+    long long face0;     // the job's first face in the face means (the sum of the earlier jobs' n_tris)
+    int chunk0;          // its first chunk (the sum of the earlier jobs' center_chunks)
+    float* center;
+    float* scale;
+    float4* pos_out;
+};
+struct CenterJobs {
+    CenterJob one;          // the job, where many is null
+    const CenterJob* many;  // device array of n jobs
+    int n, n_chunks;        // jobs and the sum of their center_chunks
+};
+int center_chunks(int n_tris);
+size_t center_scratch_bytes(long long chunks);
+// face_mean: three floats per face; scratch: center_scratch_bytes, 16-byte aligned; max_*: the largest job's sizes
+void launch_center_jobs(const CenterJobs& J, float* face_mean, void* scratch, int max_tris, int max_pts, cudaStream_t s,
+                        bool centre);
+void launch_center(const float* pts, const int* tris, int n_pts, int n_tris, float* face_mean, void* scratch,
+                   float* center, float* d_scale, float4* pos_out, cudaStream_t s, bool centre = true);
 void launch_after_check(RoundCounters* rc, cudaStream_t s);
 
 // ---- device-driven rounds: sizes from LoopState / RoundCounters, host values only bound the grids ----
