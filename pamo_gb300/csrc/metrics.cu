@@ -3,10 +3,11 @@
 // Chamfer and Hausdorff distances) and the per-face minimum angles behind compute_min_angle and
 // compute_bad_tri_ratio. Off the simplification path; inputs are float64 like the metrics' NumPy arrays.
 //
-// Point-to-mesh distance: the stage-2 LBVH built over float copies of the vertices, each box widened by a
-// relative 2^-20 of its coordinates so that it bounds the float64 triangle; a branch-and-bound walk per point
-// (nearest child first) with the exact float64 point-triangle distance at the leaves (Ericson, Real-Time
-// Collision Detection, 5.1.5).
+// Point-to-mesh distance: two walks per point through the packed stage-2 LBVH over float copies of the vertices. The
+// first, all in float, gives an upper bound of the distance; the second collects the triangles that may be as near, and
+// those few take the exact float64 point-triangle distance (Ericson, Real-Time Collision Detection, 5.1.5), the lanes
+// of a warp together. The nearest triangle and the smallest index of equally near ones are the same as by trying every
+// triangle in float64; the margins below hold what float adds.
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -20,8 +21,9 @@ namespace {
 using namespace pamo;
 
 constexpr int kT = 256;
-constexpr int kQT = 128;
+constexpr int kQT = 64;
 constexpr int kStack = 64;
+constexpr int kList = 8;  // triangles a lane collects before the warp evaluates them
 
 struct D3 {
     double x, y, z;
@@ -71,93 +73,188 @@ __global__ void k_to_int4(const int* __restrict__ f, int n, int nv, int4* out, i
     }
 }
 
-// squared distance from p to a box widened by a relative 2^-20 (so that it bounds the float64 geometry the
-// float box was rounded from), as a lower bound for pruning
-__device__ __forceinline__ double box_lower_bound(D3 p, float4 lo, float4 hi) {
-    const double e = 9.5367431640625e-07;  // 2^-20
-    auto axis = [&](double x, float l, float h) {
-        const double dl = (double)l - e * fabs((double)l) - 1e-30, dh = (double)h + e * fabs((double)h) + 1e-30;
-        return x < dl ? dl - x : (x > dh ? x - dh : 0.0);
-    };
-    const double dx = axis(p.x, lo.x, hi.x), dy = axis(p.y, lo.y, hi.y), dz = axis(p.z, lo.z, hi.z);
-    return dx * dx + dy * dy + dz * dz;
+struct F3 {
+    float x, y, z;
+};
+__device__ __forceinline__ F3 fsub(F3 a, F3 b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
+__device__ __forceinline__ float fdot(F3 a, F3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+__device__ __forceinline__ F3 f3(float4 v) { return {v.x, v.y, v.z}; }
+
+__device__ __forceinline__ float unit(float x) { return fminf(fmaxf(x, 0.f), 1.f); }  // a NaN counts as 0
+
+// Distance in float from p to the triangle, and its scale: the largest of |ab|, |ac| and the distance. The point that it
+// is taken to lies in the triangle whatever the rounding did (the parameters are clamped), so the distance is an upper
+// bound of the true one up to the rounding of that point. slim: it is no lower bound to rely on. The parameters come from
+// differences of products of size (side * scale)^2, rounded to about 1e-6 of that and divided by n2 = |ab x ac|^2, so the
+// point is off by up to 1e-6 side^3 scale^2 / n2, within kLower * scale (with a factor of 4) if side^3 scale <= 25 n2.
+__device__ __forceinline__ float tri_distance(F3 p, F3 a, F3 b, F3 c, float& scale, bool& slim) {
+    const F3 ab = fsub(b, a), ac = fsub(c, a), ap = fsub(p, a);
+    const float d1 = fdot(ab, ap), d2 = fdot(ac, ap);
+    const float bb = fdot(ab, ab), cc = fdot(ac, ac), bc = fdot(ab, ac);
+    float v = 0.f, w = 0.f;
+    if (!(d1 <= 0.f && d2 <= 0.f)) {
+        const F3 bp = fsub(p, b), cp = fsub(p, c);
+        const float d3 = fdot(ab, bp), d4 = fdot(ac, bp), d5 = fdot(ab, cp), d6 = fdot(ac, cp);
+        const float vc = d1 * d4 - d3 * d2, vb = d5 * d2 - d1 * d6, va = d3 * d6 - d5 * d4;
+        if (d3 >= 0.f && d4 <= d3) v = 1.f;
+        else if (vc <= 0.f && d1 >= 0.f && d3 <= 0.f) v = unit(d1 / (d1 - d3));
+        else if (d6 >= 0.f && d5 <= d6) w = 1.f;
+        else if (vb <= 0.f && d2 >= 0.f && d6 <= 0.f) w = unit(d2 / (d2 - d6));
+        else if (va <= 0.f && (d4 - d3) >= 0.f && (d5 - d6) >= 0.f) {
+            w = unit((d4 - d3) / ((d4 - d3) + (d5 - d6)));
+            v = 1.f - w;
+        } else {
+            const float den = 1.f / (va + vb + vc);
+            v = unit(vb * den);
+            w = fminf(unit(vc * den), 1.f - v);
+        }
+    }
+    const F3 r = {ab.x * v + ac.x * w - ap.x, ab.y * v + ac.y * w - ap.y, ab.z * v + ac.z * w - ap.z};
+    const float d = sqrtf(fdot(r, r));
+    const float side = sqrtf(fmaxf(bb, cc)), n2 = bb * cc - bc * bc;
+    scale = fmaxf(side, d);
+    slim = !(n2 > 1e-30f && n2 < 1e30f && side * side * side * scale <= 25.f * n2);
+    return d;
 }
 
+// The margins. kCoord of the largest coordinate covers the float copies of a vertex and of the point (2^-24 of it for
+// each of three coordinates, twice) and kTiny squares that underflow; a distance to a point of a triangle is computed
+// within kUpper of the triangle's scale, and the nearest point of a triangle that is not slim is found within kLower of
+// it.
+constexpr float kCoord = 5e-7f, kTiny = 1e-18f, kUpper = 2e-6f, kLower = 1e-4f;
+
+__device__ __forceinline__ float box_sq(F3 p, float4 lo, float4 hi) {
+    const float dx = fmaxf(fmaxf(lo.x - p.x, 0.f), p.x - hi.x), dy = fmaxf(fmaxf(lo.y - p.y, 0.f), p.y - hi.y),
+                dz = fmaxf(fmaxf(lo.z - p.z, 0.f), p.z - hi.z);
+    return dx * dx + dy * dy + dz * dz;
+}
+// squared distances above this are above `upper` for certain
+__device__ __forceinline__ float above(float upper, float margin) {
+    const float u = upper + margin;
+    return u * u * 1.00001f;
+}
+
+// One walk per point in float64 with a float64 box bound took 1.97 ms for 20,000 points and 327,680 faces: the float64
+// pipes (1/64 of the float32 rate) and three dependent loads a node set its time. The whole call, with its copies from and
+// to NumPy arrays, went from 2.94 to 1.16 ms.
 __global__ void __launch_bounds__(kQT) k_point_mesh(const double* __restrict__ pts, int np, const double* __restrict__ V,
-                                                    const int4* __restrict__ tri, const int2* __restrict__ child,
-                                                    const float4* __restrict__ nlo, const float4* __restrict__ nhi,
-                                                    const float4* __restrict__ llo, const float4* __restrict__ lhi,
+                                                    const float4* __restrict__ pos, const int4* __restrict__ tri,
+                                                    const float4* __restrict__ packed, const unsigned* __restrict__ scene,
                                                     const int* __restrict__ leaf_face, const RoundCounters* rc,
                                                     double* out_d2, int* out_face, int* status) {
-    __shared__ int stack[kStack][kQT];
-    const int nl = rc->n_live;
-    for (int i = gtid(); i < np; i += gstride()) {
-        const D3 p = dload(pts, i);
+    __shared__ int s_node[kStack][kQT];
+    __shared__ float s_dist[kStack][kQT];
+    __shared__ int s_list[kList][kQT];
+    const int nl = rc->n_live, me = threadIdx.x;
+    float extent = 0.f;
+    for (int d = 0; d < 6; ++d) {
+        const unsigned u = scene[d];
+        extent = fmaxf(extent, fabsf(__uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u)));
+    }
+    // all lanes of a warp make the same number of rounds (the walks end in warp votes)
+    for (int i0 = gtid() & ~31; i0 < np; i0 += gstride()) {
+        const int i = i0 + (me & 31);
+        const bool on = i < np;
+        const D3 pd = on ? dload(pts, i) : D3{0.0, 0.0, 0.0};
+        const F3 p = {(float)pd.x, (float)pd.y, (float)pd.z};
+        const float margin = kCoord * fmaxf(extent, fmaxf(fabsf(p.x), fmaxf(fabsf(p.y), fabsf(p.z)))) + kTiny;
+        float upper = INFINITY;
         double best = INFINITY;
         int bf = -1;
-        auto leaf = [&](int li) {
-            const int f = leaf_face[li];
-            const int4 t = tri[f];
-            const D3 c = closest_point_triangle(p, dload(V, t.x), dload(V, t.y), dload(V, t.z));
-            const D3 d = dsub(c, p);
-            const double d2 = ddot(d, d);
-            if (d2 < best || (d2 == best && f < bf)) {
-                best = d2;
-                bf = f;
+        auto evaluate = [&](int count) {
+            for (int k = 0; __any_sync(0xffffffffu, k < count); ++k) {
+                if (k >= count) continue;
+                const int f = s_list[k][me];
+                const int4 t = tri[f];
+                const D3 c = closest_point_triangle(pd, dload(V, t.x), dload(V, t.y), dload(V, t.z));
+                const D3 d = dsub(c, pd);
+                const double d2 = ddot(d, d);
+                if (d2 < best || (d2 == best && f < bf)) {
+                    best = d2;
+                    bf = f;
+                }
             }
         };
-        if (nl == 1) leaf(0);
+        if (nl == 1) {
+            if (on) s_list[0][me] = leaf_face[0];
+            evaluate(on ? 1 : 0);
+        }
         if (nl >= 2) {
-            int sp = 0, node = 0, guard = 0;
-            while (true) {
-                if (++guard > (1 << 22)) {
-                    atomicOr(status, kErrIterLimit);
-                    break;
-                }
-                const int2 c = child[node];
-                int nxt[2];
-                double nd[2];
-                int nn = 0;
-                for (int side = 0; side < 2; ++side) {
-                    const int x = side ? c.y : c.x;
-                    const double d = x < 0 ? box_lower_bound(p, llo[~x], lhi[~x]) : box_lower_bound(p, nlo[x], nhi[x]);
-                    if (d > best) continue;
-                    if (x < 0) leaf(~x);
-                    else {
-                        nxt[nn] = x;
-                        nd[nn] = d;
-                        ++nn;
+            // pass 0: the upper bound; pass 1: the triangles that may be nearest
+            for (int pass = 0; pass < 2; ++pass) {
+                int sp = 0, node = on ? 0 : -1, guard = 0, count = 0;
+                float limit = above(upper, margin);
+                while (__any_sync(0xffffffffu, node >= 0)) {
+                    if (node >= 0 && ++guard > (1 << 22)) {
+                        atomicOr(status, kErrIterLimit);
+                        node = -1;
                     }
-                }
-                if (nn == 2) {
-                    if (nd[1] < nd[0]) {
-                        const int t = nxt[0];
-                        nxt[0] = nxt[1];
-                        nxt[1] = t;
-                    }
-                    if (sp >= kStack) {
-                        atomicOr(status, kErrStackOverflow);
-                        break;
-                    }
-                    stack[sp++][threadIdx.x] = nxt[1];
-                    node = nxt[0];
-                } else if (nn == 1) {
-                    node = nxt[0];
-                } else {
-                    bool found = false;
-                    while (sp > 0) {
-                        node = stack[--sp][threadIdx.x];
-                        if (box_lower_bound(p, nlo[node], nhi[node]) <= best) {
-                            found = true;
-                            break;
+                    if (node >= 0) {
+                        const float4* rec = packed + 4 * (size_t)node;
+                        const float4 lo0 = __ldg(rec), hi0 = __ldg(rec + 1), lo1 = __ldg(rec + 2), hi1 = __ldg(rec + 3);
+                        float b0 = box_sq(p, lo0, hi0), b1 = box_sq(p, lo1, hi1);
+                        int c0 = __float_as_int(lo0.w), c1 = __float_as_int(lo1.w);
+                        int g0 = __float_as_int(hi0.w), g1 = __float_as_int(hi1.w);
+                        if (b1 < b0) {  // the nearer child first
+                            const float tb = b0; b0 = b1; b1 = tb;
+                            const int tc = c0; c0 = c1; c1 = tc;
+                            const int tg = g0; g0 = g1; g1 = tg;
+                        }
+                        int n0 = -1, n1 = -1;
+#pragma unroll
+                        for (int side = 0; side < 2; ++side) {
+                            const float bd = side ? b1 : b0;
+                            if (bd > limit) continue;
+                            const int x = side ? c1 : c0, f = side ? g1 : g0;
+                            if (x >= 0) {
+                                if (side) n1 = x;
+                                else n0 = x;
+                                continue;
+                            }
+                            const int4 t = tri[f];
+                            float scale;
+                            bool slim;
+                            const float d = tri_distance(p, f3(pos[t.x]), f3(pos[t.y]), f3(pos[t.z]), scale, slim);
+                            if (pass == 0) {
+                                const float u = d + (kUpper * scale + margin);
+                                if (u < upper) {
+                                    upper = u;
+                                    limit = above(upper, margin);
+                                }
+                            } else if (slim || !(d - (kLower * scale + margin) > upper)) {
+                                s_list[count++][me] = f;
+                            }
+                        }
+                        if (n0 >= 0 && n1 >= 0) {
+                            if (sp >= kStack) {
+                                atomicOr(status, kErrStackOverflow);
+                                node = -1;
+                                sp = 0;
+                            } else {
+                                s_node[sp][me] = n1;
+                                s_dist[sp++][me] = b1;
+                                node = n0;
+                            }
+                        } else {
+                            node = n0 >= 0 ? n0 : n1;
+                        }
+                        while (node < 0 && sp > 0) {
+                            --sp;
+                            if (!(s_dist[sp][me] > limit)) node = s_node[sp][me];
                         }
                     }
-                    if (!found) break;
+                    if (__any_sync(0xffffffffu, count > kList - 2)) {
+                        evaluate(count);
+                        count = 0;
+                    }
                 }
+                evaluate(count);
             }
         }
-        out_d2[i] = best;
-        if (out_face) out_face[i] = bf;
+        if (on) {
+            out_d2[i] = best;
+            if (out_face) out_face[i] = bf;
+        }
     }
 }
 
@@ -239,10 +336,9 @@ int pamo_point_mesh_sqdist(const double* points, int32_t n_points, const double*
         k_to_float4<<<grid_for(n_vertices, kT), kT, 0, s>>>(vertices, n_vertices, pos);
         k_to_int4<<<grid_for(n_triangles, kT), kT, 0, s>>>(triangles, n_triangles, n_vertices, tri, &rc->status);
         note_launches(2);
-        bvh_build(b, tri, pos, rc, n_triangles, s);
-        k_point_mesh<<<grid_for(n_points, kQT, 16), kQT, 0, s>>>(points, n_points, vertices, tri, b.child, b.nlo, b.nhi,
-                                                                b.llo, b.lhi, b.vals[0], rc, out_sqdist, out_face,
-                                                                &rc->status);
+        bvh_build(b, tri, pos, rc, n_triangles, s, false, nullptr, false);
+        k_point_mesh<<<grid_for(n_points, kQT, 16), kQT, 0, s>>>(points, n_points, vertices, pos, tri, b.packed, b.scene,
+                                                                b.vals[0], rc, out_sqdist, out_face, &rc->status);
         note_launch();
         r = cuda_status(cudaStreamSynchronize(s));
         if (r == PAMO_OK) {

@@ -44,6 +44,27 @@ def test_point_mesh_sqdist_matches_brute_force():
         assert _point_tri_sqdist(P[i:i + 1], V[f[0]], V[f[1]], V[f[2]])[0] == pytest.approx(d2[i], rel=1e-9, abs=1e-20)
 
 
+@pytest.mark.parametrize("scale, shift, thin, far", [(1.0, 0.0, 1.0, 1.0), (1.0, 300.0, 1.0, 1.0), (1e-12, 0.0, 1.0, 1.0),
+                                                     (1e15, 0.0, 1.0, 1.0), (1.0, 0.0, 1e-5, 1.0), (1.0, 2.0, 1.0, 500.0)])
+@pytest.mark.parametrize("faces", [1, 2, 33, None])
+def test_point_mesh_sqdist_over_scales_and_shapes(scale, shift, thin, far, faces):
+    """The float bounds must not lose the nearest triangle: small and large coordinates, away from the origin, slivers,
+    points far from the mesh. 1e-9 of the value (as above), or what float64 itself loses where coordinates are larger
+    than the distance."""
+    V, F = meshes.tangled(n=6, seed=8)
+    F = F[:faces]
+    V = V.astype(np.float64) * [1.0, thin, 1.0]
+    rng = np.random.default_rng(3)
+    P = np.vstack([far * rng.normal(0, 1.0, (200, 3)), V[:40], V[:60] * (1 + 1e-7), metrics.sample_surface(V, F, 70, seed=5)])
+    V, P = scale * (V + shift), scale * (P + shift)
+    d2, fi = metrics.point_mesh_sqdist(P, V, F)
+    all_d2 = np.stack([_point_tri_sqdist(P, V[f[0]], V[f[1]], V[f[2]]) for f in F])
+    want, size = all_d2.min(0), np.abs(P).max(1) + np.abs(V).max()
+    bound = 1e-9 * want + (1e-13 / min(thin, 1.0) * size) * np.sqrt(want) + (1e-13 / min(thin, 1.0) * size) ** 2
+    assert (np.abs(d2 - want) <= bound).all()
+    assert (np.abs(all_d2[fi, np.arange(len(P))] - want) <= bound).all()
+
+
 def test_face_min_angles_match_the_reference_formulas():
     V, F = meshes.with_degenerate_face()
     V = V.astype(np.float64)
