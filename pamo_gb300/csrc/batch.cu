@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "../../include/pamo_gb300.h"
+#include "pamo_common.cuh"
 
 namespace {
 
@@ -38,6 +39,7 @@ using Clock = std::chrono::steady_clock;
 // float32 -> float64, on the device (the request's input points, already there for stage 2, become the stage-3
 // target without a host round trip)
 __global__ void k_widen(const float* __restrict__ in, long long n, double* out) {
+    pamo::pdl_wait();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         out[i] = (double)in[i];
 }
@@ -399,7 +401,7 @@ struct pamo_server {
             (r = ensure_dev(st, cst, 3 * std::max<size_t>(nfm, 1), w.stream)))
             return r;
         const long long ng = 3 * (long long)ngp;
-        k_widen<<<(unsigned)std::min<long long>((ng + 255) / 256, 1024), 256, 0, w.stream>>>(d_gt_points, ng, gp);
+        pamo::pdl(k_widen, (unsigned)std::min<long long>((ng + 255) / 256, 1024), 256, 0, w.stream)(d_gt_points, ng, gp);
         cudaMemcpyAsync(sp, vm.data(), vm.size() * sizeof(double), cudaMemcpyHostToDevice, w.stream);
         cudaMemcpyAsync(st, fm.data(), fm.size() * sizeof(int32_t), cudaMemcpyHostToDevice, w.stream);
         double* out = sp + 3 * nm;

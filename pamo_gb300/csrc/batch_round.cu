@@ -81,6 +81,7 @@ __global__ void __launch_bounds__(kCtlThreads) kb_round_begin(BatchMesh* mesh, i
                                                               int* slot_stuck, float* slot_scale,
                                                               const float* mesh_scale, RoundCounters* rc,
                                                               BatchCtl* ctl) {
+    pdl_wait();
     __shared__ int sm[33];
     int lo;
     const int cnt = bx_chunk(n_meshes, threadIdx.x, lo);
@@ -129,6 +130,7 @@ __global__ void __launch_bounds__(kCtlThreads) kb_round_begin(BatchMesh* mesh, i
 // vertex and face -> slot
 __global__ void kb_fill_slots(const BatchCtl* ctl, const int* slot_v0, const int* slot_np, const int* slot_f0,
                               const int* slot_nf, int* vmesh, int* fmesh) {
+    pdl_wait();
     for (int k = blockIdx.x; k < ctl->n_slots; k += gridDim.x) {
         const int v0 = slot_v0[k], np = slot_np[k], f0 = slot_f0[k], nf = slot_nf[k];
         for (int i = threadIdx.x; i < np; i += blockDim.x) vmesh[v0 + i] = k;
@@ -141,6 +143,7 @@ __global__ void kb_fill_slots(const BatchCtl* ctl, const int* slot_v0, const int
 // map; then the carried vertices are marked invalid
 __global__ void kb_undo_book(const BatchCtl* ctl, const int* slot_mesh, const BatchMesh* mesh, const int* undo_in,
                              int* tmp_undo, int* undo_list, const int* map, unsigned char* invalid) {
+    pdl_wait();
     for (int k = blockIdx.x; k < ctl->n_slots; k += gridDim.x) {
         const BatchMesh& M = mesh[slot_mesh[k]];
         const long long r = M.vreg;
@@ -162,6 +165,7 @@ __global__ void kb_undo_book(const BatchCtl* ctl, const int* slot_mesh, const Ba
 // each mesh's edges: [e0, e0 + ne) of the round's edge numbering (from the scanned per-face edge counts)
 __global__ void kb_slot_edges(const BatchCtl* ctl, const int* slot_mesh, BatchMesh* mesh, const int* ecount_scan,
                               RoundCounters* rc) {
+    pdl_wait();
     for (int k = gtid(); k < ctl->n_slots; k += gstride()) {
         BatchMesh& M = mesh[slot_mesh[k]];
         M.e0 = ecount_scan[M.f0];
@@ -174,6 +178,7 @@ __global__ void kb_slot_edges(const BatchCtl* ctl, const int* slot_mesh, BatchMe
 __global__ void kb_gather(const RoundCounters* rc, const int* slot_mesh, const BatchMesh* mesh, const int* vmesh,
                           const int2* edges, const uint32_t* ecost_reg, const unsigned char* invalid_reg,
                           uint32_t* cost, unsigned char* invalid) {
+    pdl_wait();
     const int ne = rc->n_edges, np = rc->n_pts;
     const int n = max(ne, np);
     for (int i = gtid(); i < n; i += gstride()) {
@@ -192,6 +197,7 @@ __global__ void kb_gather(const RoundCounters* rc, const int* slot_mesh, const B
 
 __global__ void kb_scatter_costs(const RoundCounters* rc, const int* slot_mesh, const BatchMesh* mesh, const int* vmesh,
                                  const int2* edges, const uint32_t* cost, uint32_t* ecost_reg) {
+    pdl_wait();
     const int ne = rc->n_edges;
     for (int i = gtid(); i < ne; i += gstride()) {
         const BatchMesh& M = mesh[slot_mesh[vmesh[edges[i].x]]];
@@ -205,6 +211,7 @@ __global__ void kb_scatter_costs(const RoundCounters* rc, const int* slot_mesh, 
 __global__ void kb_line_apply(RoundCounters* rc, BatchCtl* ctl, const int* slot_mesh, BatchMesh* mesh,
                               const int* vmesh, const int2* __restrict__ edges, const int* __restrict__ nt_off,
                               const int* __restrict__ nt, int4* tri, float4* pos, int* occ, int* lines, int cap) {
+    pdl_wait();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     int k = 0;
     if (rc->n_line > 0) {
@@ -232,6 +239,7 @@ __global__ void kb_line_apply(RoundCounters* rc, BatchCtl* ctl, const int* slot_
 // line collapses (the check's grid is sized from h before the line collapses are appended, :1007-1016)
 __global__ void __launch_bounds__(kCtlThreads) kb_considered(const BatchCtl* ctl, const int* slot_mesh,
                                                              BatchMesh* mesh, const int* win_scan, RoundCounters* rc) {
+    pdl_wait();
     __shared__ int sm[33];
     const int n = ctl->n_slots;
     int lo;
@@ -262,6 +270,7 @@ __global__ void __launch_bounds__(kCtlThreads) kb_considered(const BatchCtl* ctl
 
 __global__ void kb_considered_fill(const BatchCtl* ctl, const int* slot_mesh, const BatchMesh* mesh,
                                    const int* winners, const int* lines, int* considered) {
+    pdl_wait();
     for (int k = blockIdx.x; k < ctl->n_slots; k += gridDim.x) {
         const BatchMesh& M = mesh[slot_mesh[k]];
         for (int i = threadIdx.x; i < M.ncons; i += blockDim.x)
@@ -272,6 +281,7 @@ __global__ void kb_considered_fill(const BatchCtl* ctl, const int* slot_mesh, co
 // after an intersection check, per mesh that was checked: its undo edges, the undo-vertex count, and whether it
 // takes another pass (fewer than five extra passes so far, :1024-1040)
 __global__ void kb_after_check(BatchCtl* ctl, const int* slot_mesh, BatchMesh* mesh, const int* uscan) {
+    pdl_wait();
     int any = 0;
     for (int k = gtid(); k < ctl->n_slots; k += gstride()) {
         BatchMesh& M = mesh[slot_mesh[k]];
@@ -297,6 +307,7 @@ __global__ void kb_undo_apply(const RoundCounters* rc, const int* slot_mesh, con
                               const int* __restrict__ nt, int4* tri, const int4* __restrict__ orig_tri, float4* pos,
                               const float4* __restrict__ orig_pos, int* occ, int* tmp_undo, int* undo_list,
                               const int* __restrict__ map, int* status) {
+    pdl_wait();
     const int n = rc->n_considered;
     for (int c = gtid(); c < n; c += gstride()) {
         if (uscan[c + 1] == uscan[c]) continue;
@@ -323,6 +334,7 @@ __global__ void kb_undo_apply(const RoundCounters* rc, const int* slot_mesh, con
 }
 
 __global__ void kb_after_apply(BatchCtl* ctl, const int* slot_mesh, BatchMesh* mesh) {
+    pdl_wait();
     for (int k = gtid(); k < ctl->n_slots; k += gstride()) {
         BatchMesh& M = mesh[slot_mesh[k]];
         M.checking = M.apply;
@@ -338,6 +350,7 @@ __global__ void kb_after_apply(BatchCtl* ctl, const int* slot_mesh, BatchMesh* m
 // go on get the next round's offsets (prefix sums in mesh order)
 __global__ void __launch_bounds__(kCtlThreads) kb_round_end(BatchCtl* ctl, const int* slot_mesh, BatchMesh* mesh,
                                                             const int* vscan, const int* fscan, RoundCounters* rc) {
+    pdl_wait();
     __shared__ int sm[33];
     const int n = ctl->n_slots;
     int lo;
@@ -398,6 +411,7 @@ __global__ void kb_compact(const RoundCounters* rc, const int* slot_mesh, BatchM
                            const int* __restrict__ vscan, const int4* __restrict__ tri, const int* __restrict__ fscan,
                            int* map, const float4* __restrict__ mean, float4* next_pos, int4* next_tri, float4* res_pos,
                            int4* res_tri) {
+    pdl_wait();
     const int np = rc->n_pts, nf = rc->n_tris;
     const int n = max(np, nf);
     for (int i = gtid(); i < n; i += gstride()) {
@@ -434,6 +448,7 @@ __global__ void kb_compact(const RoundCounters* rc, const int* slot_mesh, BatchM
 // the undo vertices each mesh carries into its next round (the host loop's verts_undo)
 __global__ void kb_carry_undo(const BatchCtl* ctl, const int* slot_mesh, BatchMesh* mesh, const int* undo_list,
                               int* undo_in) {
+    pdl_wait();
     for (int k = blockIdx.x; k < ctl->n_slots; k += gridDim.x) {
         BatchMesh& M = mesh[slot_mesh[k]];
         const int nu = min(M.n_vertices_undo, M.lp);
@@ -462,6 +477,7 @@ __device__ __forceinline__ int mesh_of(const long long* __restrict__ off, int n_
 // every mesh's faces with their indices checked against the mesh (launch_load_tris over the whole batch)
 __global__ void kb_load_tris(const int* __restrict__ tris, const long long* __restrict__ foff,
                              const long long* __restrict__ voff, int n_meshes, int n_faces, int4* out, RoundCounters* rc) {
+    pdl_wait();
     for (int f = gtid(); f < n_faces; f += gstride()) {
         const int m = mesh_of(foff, n_meshes, f);
         const int n_pts = (int)(voff[m + 1] - voff[m]);
@@ -479,6 +495,7 @@ __global__ void kb_load_tris(const int* __restrict__ tris, const long long* __re
 // numbering. (64 meshes: 192 launches of 4 to 6 us one after the other before, three now.)
 __global__ void kb_shuffle_flags(Feistel fb, const long long* __restrict__ goff, const long long* __restrict__ foff,
                                  int n_meshes, int n_flags, int* flags) {
+    pdl_wait();
     for (int i = gtid(); i < n_flags; i += gstride()) {
         const int m = mesh_of(goff, n_meshes, i);
         const unsigned long long nf = (unsigned long long)(foff[m + 1] - foff[m]);
@@ -490,6 +507,7 @@ __global__ void kb_shuffle_flags(Feistel fb, const long long* __restrict__ goff,
 __global__ void kb_shuffle_gather(Feistel fb, const long long* __restrict__ goff, const long long* __restrict__ foff,
                                   const long long* __restrict__ voff, int n_meshes, int n_flags,
                                   const int* __restrict__ scan, const int4* __restrict__ src, int4* dst) {
+    pdl_wait();
     for (int i = gtid(); i < n_flags; i += gstride()) {
         if (scan[i + 1] == scan[i]) continue;
         const int m = mesh_of(goff, n_meshes, i);
@@ -508,6 +526,7 @@ __global__ void kb_shuffle_gather(Feistel fb, const long long* __restrict__ goff
 __global__ void kb_pack_results(const BatchMesh* mesh, int n_meshes, const long long* out_voff,
                                 const long long* out_foff, const float4* __restrict__ res_pos,
                                 const int4* __restrict__ res_tri, float* out_points, int* out_tris) {
+    pdl_wait();
     for (int m = blockIdx.x; m < n_meshes; m += gridDim.x) {
         const BatchMesh& M = mesh[m];
         const int nv = (int)(out_voff[m + 1] - out_voff[m]), nf = (int)(out_foff[m + 1] - out_foff[m]);
@@ -529,6 +548,7 @@ __global__ void kb_pack_results(const BatchMesh* mesh, int n_meshes, const long 
 }
 
 __global__ void kb_mean_table(const float* centre16, int n_meshes, float4* mean) {
+    pdl_wait();
     for (int m = gtid(); m < n_meshes; m += gstride())
         mean[m] = make_float4(centre16[16 * m], centre16[16 * m + 1], centre16[16 * m + 2], 0.f);
 }
@@ -734,7 +754,7 @@ struct pamo_csr {
                   fmesh.p, mesh_root.p);
         launch_undo_check(rc, Eb, considered.p, edges.p, valence.p, nt.p, hit.p, uflag.p, s);
         exclusive_scan(uflag.p, uflag.p, &rc->n_considered, 1, &rc->n_undo, scan_scratch, s, &rc->status, Eb);
-        kb_after_check<<<1, kCtlThreads, 0, s>>>(ctl, slot_mesh.p, mesh.p, uflag.p); note_launch();
+        pdl(kb_after_check, 1, kCtlThreads, 0, s)(ctl, slot_mesh.p, mesh.p, uflag.p); note_launch();
         (void)Vb;
         (void)M;
     }
@@ -745,10 +765,10 @@ struct pamo_csr {
         const int Eb = 3 * Fb;
         const uint32_t collapse_t = collapse_threshold(threshold);
         const int gM = std::max(1, std::min(M, 4096));
-        kb_round_begin<<<1, kCtlThreads, 0, s>>>(mesh.p, M, slot_mesh.p, slot_v0.p, slot_np.p, slot_f0.p, slot_nf.p,
+        pdl(kb_round_begin, 1, kCtlThreads, 0, s)(mesh.p, M, slot_mesh.p, slot_v0.p, slot_np.p, slot_f0.p, slot_nf.p,
                                                  slot_stuck.p, slot_scale.p, mesh_scale.p, rc, ctl); note_launch();
-        kb_fill_slots<<<gM, kT, 0, s>>>(ctl, slot_v0.p, slot_np.p, slot_f0.p, slot_nf.p, vmesh.p, fmesh.p); note_launch();
-        kb_undo_book<<<gM, kT, 0, s>>>(ctl, slot_mesh.p, mesh.p, undo_in_reg.p, tmp_undo_reg.p, undo_list_reg.p,
+        pdl(kb_fill_slots, gM, kT, 0, s)(ctl, slot_v0.p, slot_np.p, slot_f0.p, slot_nf.p, vmesh.p, fmesh.p); note_launch();
+        pdl(kb_undo_book, gM, kT, 0, s)(ctl, slot_mesh.p, mesh.p, undo_in_reg.p, tmp_undo_reg.p, undo_list_reg.p,
                                        map_reg.p, invalid_reg.p); note_launch();
         launch_round_prologue_dev(zero_ls, rc, Vb, Fb, nullptr, nullptr, pos_in.p, pos.p, orig_pos.p, occ.p, tri_in.p,
                                   tri.p, orig_tri.p, valence.p, cursor.p, vedges.p, vcursor.p, qflag.p, s);
@@ -767,13 +787,13 @@ struct pamo_csr {
         const int* nt_off = valence.p;
         launch_quadrics(rc, Vb, nt_off, nt.p, tri.p, fgeo.p, quad.p, nxt.p, spc.p, s);
         // cost with each mesh's stale costs and invalid table, then the costs back to the meshes' regions
-        kb_slot_edges<<<gM, kT, 0, s>>>(ctl, slot_mesh.p, mesh.p, ecount.p, rc); note_launch();
-        kb_gather<<<grid_for(std::max(Eb, Vb), kT), kT, 0, s>>>(rc, slot_mesh.p, mesh.p, vmesh.p, edges.p, ecost_reg.p,
+        pdl(kb_slot_edges, gM, kT, 0, s)(ctl, slot_mesh.p, mesh.p, ecount.p, rc); note_launch();
+        pdl(kb_gather, grid_for(std::max(Eb, Vb), kT), kT, 0, s)(rc, slot_mesh.p, mesh.p, vmesh.p, edges.p, ecost_reg.p,
                                                                invalid_reg.p, cost.p, invalid.p); note_launch();
         launch_fill_u64_dev(rc, Vb, vmin.p, ~0ull, s);
         launch_edge_cost_batch(rc, Eb, eorder.p, edges.p, nt_off, nt.p, tri.p, pos.p, quad.p, fgeo.p, nxt.p, spc.p, invalid.p,
                                cost.p, vmin.p, slot_scale.p, slot_stuck.p, vmesh.p, threshold, s, skinny_pow);
-        kb_scatter_costs<<<grid_for(Eb, kT), kT, 0, s>>>(rc, slot_mesh.p, mesh.p, vmesh.p, edges.p, cost.p, ecost_reg.p);
+        pdl(kb_scatter_costs, grid_for(Eb, kT), kT, 0, s)(rc, slot_mesh.p, mesh.p, vmesh.p, edges.p, cost.p, ecost_reg.p);
         note_launch();
         // selection and collapse
         launch_face_keys(rc, Fb, tri.p, vmin.p, fkey.p, s);
@@ -783,10 +803,10 @@ struct pamo_csr {
         launch_compact_winners(rc, Eb, win.p, winners.p, s);
         launch_remove_invalid(rc, Fb, tri.p, s);
         launch_line_detect(rc, Eb, edges.p, pos.p, s);
-        kb_line_apply<<<1, 32, 0, s>>>(rc, ctl, slot_mesh.p, mesh.p, vmesh.p, edges.p, nt_off, nt.p, tri.p, pos.p, occ.p,
+        pdl(kb_line_apply, 1, 32, 0, s)(rc, ctl, slot_mesh.p, mesh.p, vmesh.p, edges.p, nt_off, nt.p, tri.p, pos.p, occ.p,
                                        lines.p, (int)lines.n); note_launch();
-        kb_considered<<<1, kCtlThreads, 0, s>>>(ctl, slot_mesh.p, mesh.p, win.p, rc); note_launch();
-        kb_considered_fill<<<gM, kT, 0, s>>>(ctl, slot_mesh.p, mesh.p, winners.p, lines.p, considered.p); note_launch();
+        pdl(kb_considered, 1, kCtlThreads, 0, s)(ctl, slot_mesh.p, mesh.p, win.p, rc); note_launch();
+        pdl(kb_considered_fill, gM, kT, 0, s)(ctl, slot_mesh.p, mesh.p, winners.p, lines.p, considered.p); note_launch();
         // faces whose intersections decide the undo: rings of the considered collapsed edges
         launch_mark_query(rc, Eb, considered.p, edges.p, nt_off, nt.p, qflag.p, s);
         exclusive_scan(qflag.p, qflag.p, &rc->n_tris, 1, &rc->n_query, scan_scratch, s, &rc->status, Fb);
@@ -806,11 +826,11 @@ struct pamo_csr {
         int r;
         if ((r = read_ctl())) return r;
         while (h_ctl->any_apply) {
-            kb_undo_apply<<<grid_for(Eb, kT), kT, 0, s>>>(rc, slot_mesh.p, mesh.p, vmesh.p, considered.p, uflag.p,
+            pdl(kb_undo_apply, grid_for(Eb, kT), kT, 0, s)(rc, slot_mesh.p, mesh.p, vmesh.p, considered.p, uflag.p,
                                                           edges.p, nt_off, nt.p, tri.p, orig_tri.p, pos.p, orig_pos.p,
                                                           occ.p, tmp_undo_reg.p, undo_list_reg.p, map_reg.p, &rc->status);
             note_launch();
-            kb_after_apply<<<1, kCtlThreads, 0, s>>>(ctl, slot_mesh.p, mesh.p); note_launch();
+            pdl(kb_after_apply, 1, kCtlThreads, 0, s)(ctl, slot_mesh.p, mesh.p); note_launch();
             check_pass(Vb, Fb, Eb, M, bm);
             if ((r = read_ctl())) return r;
         }
@@ -822,12 +842,12 @@ struct pamo_csr {
                                      {fflags.p, fflags.p, &rc->n_tris, 1, nullptr, scan_scratch + sz}};
             exclusive_scans(jobs, 2, s, &rc->status, std::max(Vb, Fb));
         }
-        kb_round_end<<<1, kCtlThreads, 0, s>>>(ctl, slot_mesh.p, mesh.p, vscan.p, fflags.p, rc); note_launch();
-        kb_compact<<<grid_for(std::max(Vb, Fb), kT), kT, 0, s>>>(rc, slot_mesh.p, mesh.p, vmesh.p, fmesh.p, pos.p, occ.p,
+        pdl(kb_round_end, 1, kCtlThreads, 0, s)(ctl, slot_mesh.p, mesh.p, vscan.p, fflags.p, rc); note_launch();
+        pdl(kb_compact, grid_for(std::max(Vb, Fb), kT), kT, 0, s)(rc, slot_mesh.p, mesh.p, vmesh.p, fmesh.p, pos.p, occ.p,
                                                                  vscan.p, tri.p, fflags.p, map_reg.p, mean.p,
                                                                  pos_next.p, tri_next.p, res_pos.p, res_tri.p);
         note_launch();
-        kb_carry_undo<<<gM, kT, 0, s>>>(ctl, slot_mesh.p, mesh.p, undo_list_reg.p, undo_in_reg.p); note_launch();
+        pdl(kb_carry_undo, gM, kT, 0, s)(ctl, slot_mesh.p, mesh.p, undo_list_reg.p, undo_in_reg.p); note_launch();
         if ((r = read_ctl())) return r;
         if ((r = status_error(h_ctl->status))) return r;
         std::swap(pos_in, pos_next);
@@ -904,17 +924,17 @@ struct pamo_csr {
             launch_center_jobs(J, face_mean.p, center_scratch.p, max_nf, max_nv, s, true);
         }
         if (F > 0) {
-            kb_load_tris<<<grid_for(F, kT), kT, 0, s>>>(triangles, dev_foff.p, dev_voff.p, M, (int)F, tri_load.p, rc);
+            pdl(kb_load_tris, grid_for(F, kT), kT, 0, s)(triangles, dev_foff.p, dev_voff.p, M, (int)F, tri_load.p, rc);
             note_launch();
             const Feistel fb = make_feistel(1);
             const int g = grid_for(flags, kT);
-            kb_shuffle_flags<<<g, kT, 0, s>>>(fb, dev_goff.p, dev_foff.p, M, (int)flags, shuffle_flags.p); note_launch();
+            pdl(kb_shuffle_flags, g, kT, 0, s)(fb, dev_goff.p, dev_foff.p, M, (int)flags, shuffle_flags.p); note_launch();
             exclusive_scan(shuffle_flags.p, shuffle_flags.p, nullptr, (int)flags + 1, nullptr, scan_scratch, s,
                            &rc->status, flags);
-            kb_shuffle_gather<<<g, kT, 0, s>>>(fb, dev_goff.p, dev_foff.p, dev_voff.p, M, (int)flags, shuffle_flags.p,
+            pdl(kb_shuffle_gather, g, kT, 0, s)(fb, dev_goff.p, dev_foff.p, dev_voff.p, M, (int)flags, shuffle_flags.p,
                                                tri_load.p, tri_in.p); note_launch();
         }
-        kb_mean_table<<<grid_for(M, kT), kT, 0, s>>>(centre.p, M, mean.p); note_launch();
+        pdl(kb_mean_table, grid_for(M, kT), kT, 0, s)(centre.p, M, mean.p); note_launch();
         {
             int st = 0;
             cudaMemcpyAsync(&st, &rc->status, sizeof(int), cudaMemcpyDeviceToHost, s);
@@ -947,7 +967,7 @@ struct pamo_csr {
         }
         cudaMemcpyAsync(dev_out_voff.p, out_voff, (M + 1) * sizeof(long long), cudaMemcpyHostToDevice, s);
         cudaMemcpyAsync(dev_out_foff.p, out_foff, (M + 1) * sizeof(long long), cudaMemcpyHostToDevice, s);
-        kb_pack_results<<<std::max(1, std::min(M, 4096)), kT, 0, s>>>(mesh.p, M, dev_out_voff.p, dev_out_foff.p,
+        pdl(kb_pack_results, std::max(1, std::min(M, 4096)), kT, 0, s)(mesh.p, M, dev_out_voff.p, dev_out_foff.p,
                                                                        res_pos.p, res_tri.p, out_points, out_tris);
         note_launch();
         return check(cudaStreamSynchronize(s), "batch results");

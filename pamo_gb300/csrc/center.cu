@@ -87,6 +87,7 @@ __device__ __forceinline__ int chunks_of(int nf) { return (nf + kChunk - 1) / kC
 
 // face means (per coordinate, so that the chunks read them in order) and each chunk's plain sum
 __global__ void __launch_bounds__(kChunkThreads) k_center_means(CenterJobs J, float* fm_all, float* csum) {
+    pdl_wait();
     __shared__ float part[3][kChunkThreads / 32];
     for (int j = blockIdx.y; j < J.n; j += gridDim.y) {
         const CenterJob job = J.many ? J.many[j] : J.one;
@@ -130,6 +131,7 @@ __global__ void __launch_bounds__(kChunkThreads) k_center_means(CenterJobs J, fl
 // the running sum that plain prefix sums predict at each chunk's start (block x = coordinate), in place of the chunk
 // sums; a wrong prediction only sends a chunk to the walk's element loop. Also clears the extents.
 __global__ void __launch_bounds__(kPredThreads) k_center_predict(CenterJobs J, float* csum) {
+    pdl_wait();
     __shared__ double wsum[32];
     __shared__ double carry;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -168,6 +170,7 @@ __global__ void __launch_bounds__(kPredThreads) k_center_predict(CenterJobs J, f
 
 __global__ void __launch_bounds__(kChunkThreads) k_center_incs(CenterJobs J, const float* __restrict__ fm_all,
                                                                const float* __restrict__ pred, ChunkInfo* info) {
+    pdl_wait();
     constexpr int W = kChunkThreads / 32;
     __shared__ Inc2 wtot[W];
     __shared__ int red[4][W];
@@ -259,6 +262,7 @@ __global__ void __launch_bounds__(kChunkThreads) k_center_incs(CenterJobs J, con
 // One warp per coordinate (block x) walks the chunks; all lanes hold the same running sum.
 __global__ void __launch_bounds__(32) k_center_walk(CenterJobs J, const float* __restrict__ fm_all,
                                                     const ChunkInfo* __restrict__ info) {
+    pdl_wait();
     __shared__ __align__(16) float stage[kChunk];
     const int lane = threadIdx.x, d = blockIdx.x;
     for (int j = blockIdx.y; j < J.n; j += gridDim.y) {
@@ -332,6 +336,7 @@ __device__ __forceinline__ float ord_dec(unsigned u) { return __uint_as_float((u
 constexpr int kPtThreads = 256;
 
 __global__ void __launch_bounds__(kPtThreads) k_center_points(CenterJobs J) {
+    pdl_wait();
     __shared__ float red[6][kPtThreads / 32];
     for (int j = blockIdx.y; j < J.n; j += gridDim.y) {
         const CenterJob job = J.many ? J.many[j] : J.one;
@@ -373,6 +378,7 @@ __global__ void __launch_bounds__(kPtThreads) k_center_points(CenterJobs J) {
 
 // scale = max(max(ex, ey), ez) of the centred points (pamo/__init__.py:126)
 __global__ void k_center_scale(CenterJobs J) {
+    pdl_wait();
     for (int j = gtid(); j < J.n; j += gstride()) {
         const CenterJob job = J.many ? J.many[j] : J.one;
         const unsigned* ext = reinterpret_cast<const unsigned*>(job.center + 4);
@@ -386,6 +392,7 @@ __global__ void k_center_scale(CenterJobs J) {
 
 // not centring: zero mean, cleared extents
 __global__ void k_center_zero(CenterJobs J) {
+    pdl_wait();
     for (int j = gtid(); j < J.n; j += gstride()) {
         const CenterJob job = J.many ? J.many[j] : J.one;
         unsigned* ext = reinterpret_cast<unsigned*>(job.center + 4);
@@ -412,17 +419,17 @@ void launch_center_jobs(const CenterJobs& J, float* face_mean, void* scratch, in
         float* csum = reinterpret_cast<float*>(info + 3 * (size_t)J.n_chunks);
         const int nch = center_chunks(max_tris);
         const int gx = nch < per_job ? (nch < 1 ? 1 : nch) : per_job;
-        k_center_means<<<dim3(gx, gy), kChunkThreads, 0, s>>>(J, face_mean, csum); note_launch();
-        k_center_predict<<<dim3(3, gy), kPredThreads, 0, s>>>(J, csum); note_launch();
-        k_center_incs<<<dim3(gx, gy, 3), kChunkThreads, 0, s>>>(J, face_mean, csum, info); note_launch();
-        k_center_walk<<<dim3(3, gy), 32, 0, s>>>(J, face_mean, info); note_launch();
+        pdl(k_center_means, dim3(gx, gy), kChunkThreads, 0, s)(J, face_mean, csum); note_launch();
+        pdl(k_center_predict, dim3(3, gy), kPredThreads, 0, s)(J, csum); note_launch();
+        pdl(k_center_incs, dim3(gx, gy, 3), kChunkThreads, 0, s)(J, face_mean, csum, info); note_launch();
+        pdl(k_center_walk, dim3(3, gy), 32, 0, s)(J, face_mean, info); note_launch();
     } else {
-        k_center_zero<<<grid_for(J.n, 256), 256, 0, s>>>(J); note_launch();
+        pdl(k_center_zero, grid_for(J.n, 256), 256, 0, s)(J); note_launch();
     }
     const int pt = (max_pts + kPtThreads - 1) / kPtThreads;
     const int px = pt < per_job ? (pt < 1 ? 1 : pt) : (per_job < 8 * kNumSM ? per_job : 8 * kNumSM);
-    k_center_points<<<dim3(px, gy), kPtThreads, 0, s>>>(J); note_launch();
-    k_center_scale<<<grid_for(J.n, 256), 256, 0, s>>>(J); note_launch();
+    pdl(k_center_points, dim3(px, gy), kPtThreads, 0, s)(J); note_launch();
+    pdl(k_center_scale, grid_for(J.n, 256), 256, 0, s)(J); note_launch();
 }
 
 void launch_center(const float* pts, const int* tris, int n_pts, int n_tris, float* face_mean, void* scratch,

@@ -44,6 +44,7 @@ __device__ __forceinline__ unsigned expand10(unsigned v) {
 __global__ void __launch_bounds__(256) k_boxes(const int4* __restrict__ tri, const float4* __restrict__ pos,
                                                 const RoundCounters* rc, float4* box_lo, float4* box_hi, int* live,
                                                 unsigned* scene, int all_faces) {
+    pdl_wait();
     const int n = rc->n_tris;
     float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
     for (int f = gtid(); f < n; f += gstride()) {
@@ -90,6 +91,7 @@ __global__ void __launch_bounds__(256) k_boxes(const int4* __restrict__ tri, con
 __global__ void __launch_bounds__(256) k_morton(const RoundCounters* rc, const int* live_scan, const float4* box_lo,
                                                  const float4* box_hi, const unsigned* scene, unsigned* keys, int* vals,
                                                  const int* __restrict__ fmesh, int mesh_bits) {
+    pdl_wait();
     const int n = rc->n_tris;
     float lo[3], ext[3];
 #pragma unroll
@@ -131,6 +133,7 @@ __device__ __forceinline__ void sort_chunk(int n, int& lo, int& hi) {
 
 __global__ void __launch_bounds__(kSortThreads) k_rs_hist(const unsigned* __restrict__ keys, const int* d_n, int shift,
                                                           int* hist) {
+    pdl_wait();
     __shared__ int h[256];
     h[threadIdx.x] = 0;
     __syncthreads();
@@ -146,6 +149,7 @@ __global__ void __launch_bounds__(kSortThreads) k_rs_hist(const unsigned* __rest
 __global__ void __launch_bounds__(kSortThreads) k_rs_scatter(const unsigned* __restrict__ kin, const int* __restrict__ vin,
                                                              unsigned* kout, int* vout, const int* d_n, int shift,
                                                              const int* hist) {
+    pdl_wait();
     constexpr int W = kSortThreads / 32;
     __shared__ int base[256];
     __shared__ int wcnt[W][256];
@@ -198,6 +202,7 @@ __device__ __forceinline__ int delta(const unsigned* k, int n, int i, int j) {
 
 __global__ void __launch_bounds__(256) k_leaves(const RoundCounters* rc, const int* vals, const float4* box_lo,
                                                  const float4* box_hi, float4* llo, float4* lhi, int* visit, int* lparent) {
+    pdl_wait();
     const int n = rc->n_live;
     for (int i = gtid(); i < n; i += gstride()) {
         int f = vals[i];
@@ -210,6 +215,7 @@ __global__ void __launch_bounds__(256) k_leaves(const RoundCounters* rc, const i
 
 __global__ void __launch_bounds__(256) k_karras(const RoundCounters* rc, const unsigned* keys, int2* child, int* iparent,
                                                  int* lparent, int2* range) {
+    pdl_wait();
     const int n = rc->n_live;
     for (int i = gtid(); i < n - 1; i += gstride()) {
         const int d = (delta(keys, n, i, i + 1) - delta(keys, n, i, i - 1)) >= 0 ? 1 : -1;
@@ -342,6 +348,7 @@ __global__ void __launch_bounds__(kTileThreads, 3) k_bottom_up_tiles(RoundCounte
                                                                   const float4* lhi, float4* nlo, float4* nhi, int* visit,
                                                                   const int* leaf_face, const int* qscan, float4* packed,
                                                                   int* meta_out, const int* active, int* upq) {
+    pdl_wait();
     __shared__ int svisit[kTileLeaves];
     __shared__ float4 slo[kTileLeaves], shi[kTileLeaves];    // internal nodes a .. b-2
     __shared__ float4 sllo[kTileLeaves], slhi[kTileLeaves];  // leaves a .. b-1
@@ -424,6 +431,7 @@ __global__ void __launch_bounds__(256) k_bottom_up_upper(RoundCounters* rc, cons
                                                          float4* nhi, int* visit, const int* leaf_face,
                                                          const int* qscan, float4* packed, const int* upq,
                                                          const int* active) {
+    pdl_wait();
     if (active && *active == 0) return;
     const int nq = upq[0];
     for (int k = gtid(); k < nq; k += gstride())
@@ -444,12 +452,12 @@ void bottom_up(BvhBuffers& b, RoundCounters* rc, int n_bound, const int* leaf_fa
                const int* active, cudaStream_t s) {
     cudaMemsetAsync(b.upq, 0, sizeof(int), s);
     const int gT = tile_grid(n_bound);
-    k_bottom_up_tiles<kPack, kNodes><<<gT, kTileThreads, 0, s>>>(rc, b.child, b.iparent, b.lparent, b.range, b.llo,
+    pdl(k_bottom_up_tiles<kPack, kNodes>, gT, kTileThreads, 0, s)(rc, b.child, b.iparent, b.lparent, b.range, b.llo,
                                                                  b.lhi, b.nlo, b.nhi, b.visit, leaf_face, qscan,
                                                                  b.packed, meta_out, active, b.upq);
     note_launch();
     const int gU = std::max(1, std::min(gT, 4 * kNumSM));
-    k_bottom_up_upper<kPack, kNodes><<<gU, 256, 0, s>>>(rc, b.child, b.iparent, b.llo, b.lhi, b.nlo, b.nhi, b.visit,
+    pdl(k_bottom_up_upper<kPack, kNodes>, gU, 256, 0, s)(rc, b.child, b.iparent, b.llo, b.lhi, b.nlo, b.nhi, b.visit,
                                                         leaf_face, qscan, b.packed, b.upq, active);
     note_launch();
 }
@@ -485,6 +493,7 @@ __device__ __forceinline__ bool decide_pair(int f, int g, const int4* __restrict
 
 __global__ void __launch_bounds__(256) k_query_order(const RoundCounters* rc, const int* __restrict__ leaf_face,
                                                      const int* __restrict__ qscan, int* flags) {
+    pdl_wait();
     const int n = rc->n_live;
     for (int i = gtid(); i < n; i += gstride()) {
         const int f = leaf_face[i];
@@ -495,6 +504,7 @@ __global__ void __launch_bounds__(256) k_query_order(const RoundCounters* rc, co
 
 __global__ void __launch_bounds__(256) k_query_gather(const RoundCounters* rc, const int* __restrict__ leaf_face,
                                                       const int* __restrict__ scan, int* qsorted) {
+    pdl_wait();
     const int n = rc->n_live;
     for (int i = gtid(); i < n; i += gstride())
         if (scan[i + 1] != scan[i]) qsorted[scan[i]] = leaf_face[i];
@@ -529,6 +539,7 @@ __global__ void __launch_bounds__(kQueryThreads) k_traverse_list(const float4* _
                                                                   int pair_cap, RoundCounters* rc, int* redo,
                                                                   const int* __restrict__ fmesh,
                                                                   const int* __restrict__ mesh_root) {
+    pdl_wait();
     __shared__ int stack[kShortStack][kQueryThreads];
     int* n_list = &rc->pad[1];
     const int nq = rc->pad[2];
@@ -681,6 +692,7 @@ __global__ void __launch_bounds__(kQueryThreads) k_traverse_redo(const float4* _
                                                                   RoundCounters* rc, float eps, const int* redo,
                                                                   const int* __restrict__ fmesh,
                                                                   const int* __restrict__ mesh_root) {
+    pdl_wait();
     __shared__ int stack[kStackDepth][kQueryThreads];
     if (rc->pad[3] == 0) return;
     const int nq = rc->pad[2];
@@ -746,6 +758,7 @@ __global__ void __launch_bounds__(kQueryThreads) k_traverse_redo(const float4* _
 __global__ void __launch_bounds__(128, 8) k_pairs(const int4* __restrict__ tri, const float4* __restrict__ pos,
                                                const int2* __restrict__ pair_list, int pair_cap, unsigned char* hit,
                                                RoundCounters* rc, float eps, int4* xq, int xq_cap, int* xq_count) {
+    pdl_wait();
     const int n = min(rc->pad[1], pair_cap);
     unsigned exact = 0;
     for (int i = gtid(); i < n; i += gstride()) {
@@ -799,6 +812,7 @@ __global__ void __launch_bounds__(128, 8) k_pairs(const int4* __restrict__ tri, 
 __global__ void __launch_bounds__(64) k_pairs_exact(const int4* __restrict__ tri, const float4* __restrict__ pos,
                                                     const int4* __restrict__ xq, int xq_cap,
                                                     const int* __restrict__ xq_count, unsigned char* hit, float eps) {
+    pdl_wait();
     const int n = min(*xq_count, xq_cap);
     for (long long k = (long long)threadIdx.x * gridDim.x + blockIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
         const int4 e = xq[k];
@@ -821,6 +835,7 @@ __global__ void __launch_bounds__(64) k_pairs_exact(const int4* __restrict__ tri
 __global__ void k_mesh_roots(const RoundCounters* rc, const int* __restrict__ live_scan, const int2* __restrict__ range,
                              const int* __restrict__ mesh_f0, const int* __restrict__ mesh_nf, const int* d_count,
                              int* root) {
+    pdl_wait();
     const int n = *d_count;
     const int n_live = rc->n_live;
     for (int m = gtid(); m < n; m += gstride()) {
@@ -902,9 +917,9 @@ void bvh_build(BvhBuffers& b, const int4* tri, const float4* pos, RoundCounters*
     cudaMemsetAsync(b.scene, 0xFF, 3 * sizeof(unsigned), s);
     cudaMemsetAsync(b.scene + 3, 0x00, 3 * sizeof(unsigned), s);
     const int gF = grid_for(n_tris_bound, 256);
-    k_boxes<<<gF, 256, 0, s>>>(tri, pos, rc, b.box_lo, b.box_hi, b.live_scan, b.scene, all_faces ? 1 : 0); note_launch();
+    pdl(k_boxes, gF, 256, 0, s)(tri, pos, rc, b.box_lo, b.box_hi, b.live_scan, b.scene, all_faces ? 1 : 0); note_launch();
     exclusive_scan(b.live_scan, b.live_scan, &rc->n_tris, 1, &rc->n_live, b.scan_scratch, s, &rc->status, n_tris_bound);
-    k_morton<<<gF, 256, 0, s>>>(rc, b.live_scan, b.box_lo, b.box_hi, b.scene, b.keys[0], b.vals[0],
+    pdl(k_morton, gF, 256, 0, s)(rc, b.live_scan, b.box_lo, b.box_hi, b.scene, b.keys[0], b.vals[0],
                                 meshes ? meshes->fmesh : nullptr, meshes ? meshes->bits : 0); note_launch();
     // sort tiles from the launch's bound (about 2048 keys per tile; all kSortTiles from 2^19 on, where callers
     // cap their bounds); the histogram is
@@ -913,15 +928,15 @@ void bvh_build(BvhBuffers& b, const int4* tri, const float4* pos, RoundCounters*
     const int sort_tiles = (int)(st < 1 ? 1 : (st > kSortTiles ? kSortTiles : st));
     for (int pass = 0; pass < 4; ++pass) {
         const int in = pass & 1, out = in ^ 1;
-        k_rs_hist<<<sort_tiles, kSortThreads, 0, s>>>(b.keys[in], &rc->n_live, 8 * pass, b.hist); note_launch();
+        pdl(k_rs_hist, sort_tiles, kSortThreads, 0, s)(b.keys[in], &rc->n_live, 8 * pass, b.hist); note_launch();
         exclusive_scan(b.hist, b.hist, nullptr, 256 * sort_tiles, nullptr, b.scan_scratch, s, &rc->status, 0);
-        k_rs_scatter<<<sort_tiles, kSortThreads, 0, s>>>(b.keys[in], b.vals[in], b.keys[out], b.vals[out], &rc->n_live,
+        pdl(k_rs_scatter, sort_tiles, kSortThreads, 0, s)(b.keys[in], b.vals[in], b.keys[out], b.vals[out], &rc->n_live,
                                                          8 * pass, b.hist); note_launch();
     }
-    k_leaves<<<gF, 256, 0, s>>>(rc, b.vals[0], b.box_lo, b.box_hi, b.llo, b.lhi, b.visit, b.lparent); note_launch();
-    k_karras<<<gF, 256, 0, s>>>(rc, b.keys[0], b.child, b.iparent, b.lparent, b.range); note_launch();
+    pdl(k_leaves, gF, 256, 0, s)(rc, b.vals[0], b.box_lo, b.box_hi, b.llo, b.lhi, b.visit, b.lparent); note_launch();
+    pdl(k_karras, gF, 256, 0, s)(rc, b.keys[0], b.child, b.iparent, b.lparent, b.range); note_launch();
     if (meshes) {
-        k_mesh_roots<<<grid_for(meshes->count_bound, 256), 256, 0, s>>>(rc, b.live_scan, b.range, meshes->f0, meshes->nf,
+        pdl(k_mesh_roots, grid_for(meshes->count_bound, 256), 256, 0, s)(rc, b.live_scan, b.range, meshes->f0, meshes->nf,
                                                                           meshes->d_count, meshes->root);
         note_launch();
     }
@@ -932,6 +947,7 @@ void bvh_build(BvhBuffers& b, const int4* tri, const float4* pos, RoundCounters*
 __global__ void __launch_bounds__(256) k_refit_leaves(const RoundCounters* rc, const int4* __restrict__ tri,
                                                       const float4* __restrict__ pos, const int* __restrict__ vals,
                                                       float4* llo, float4* lhi, int* visit, const int* active) {
+    pdl_wait();
     if (active && *active == 0) return;
     const int n = rc->n_live;
     for (int i = gtid(); i < n; i += gstride()) {
@@ -946,7 +962,7 @@ __global__ void __launch_bounds__(256) k_refit_leaves(const RoundCounters* rc, c
 void bvh_refit(BvhBuffers& b, const int4* tri, const float4* pos, RoundCounters* rc, int n_tris_bound, cudaStream_t s,
                const int* active) {
     const int gF = grid_for(n_tris_bound, 256);
-    k_refit_leaves<<<gF, 256, 0, s>>>(rc, tri, pos, b.vals[0], b.llo, b.lhi, b.visit, active); note_launch();
+    pdl(k_refit_leaves, gF, 256, 0, s)(rc, tri, pos, b.vals[0], b.llo, b.lhi, b.visit, active); note_launch();
     bottom_up<false, true>(b, rc, n_tris_bound, nullptr, nullptr, nullptr, active, s);
 }
 
@@ -954,6 +970,7 @@ __global__ void __launch_bounds__(256) k_reuse_leaves(RoundCounters* rc, const i
                                                       const float4* __restrict__ box_lo, const float4* __restrict__ box_hi,
                                                       const int* __restrict__ new_ids, int* leaf_face, float4* llo,
                                                       float4* lhi, int* visit, const int* meta) {
+    pdl_wait();
     const int n = meta[0];
     if (gtid() == 0) rc->n_live = n;
     for (int i = gtid(); i < n; i += gstride()) {
@@ -978,6 +995,7 @@ __global__ void __launch_bounds__(256) k_reuse_leaves(RoundCounters* rc, const i
 // next[i] = the leaf's face in the next numbering; reads the current ids only, so it can be repeated
 __global__ void __launch_bounds__(256) k_remap_leaves(const int* meta, const int* __restrict__ fscan,
                                                       const int* __restrict__ leaf_face, int* next) {
+    pdl_wait();
     const int n = meta[0];
     for (int i = gtid(); i < n; i += gstride()) {
         const int f = leaf_face[i];
@@ -988,14 +1006,14 @@ __global__ void __launch_bounds__(256) k_remap_leaves(const int* meta, const int
 void bvh_refit_faces(BvhBuffers& b, const int4* tri, const float4* pos, RoundCounters* rc, int n_tris_bound,
                      cudaStream_t s, bool next_round, const int* qscan) {
     const int gF = grid_for(n_tris_bound, 256);
-    k_boxes<<<gF, 256, 0, s>>>(tri, pos, rc, b.box_lo, b.box_hi, b.live_scan, b.scene, 1); note_launch();
-    k_reuse_leaves<<<gF, 256, 0, s>>>(rc, tri, b.box_lo, b.box_hi, next_round ? (const int*)b.keys[1] : nullptr,
+    pdl(k_boxes, gF, 256, 0, s)(tri, pos, rc, b.box_lo, b.box_hi, b.live_scan, b.scene, 1); note_launch();
+    pdl(k_reuse_leaves, gF, 256, 0, s)(rc, tri, b.box_lo, b.box_hi, next_round ? (const int*)b.keys[1] : nullptr,
                                       b.vals[0], b.llo, b.lhi, b.visit, b.meta); note_launch();
     bottom_up<true, false>(b, rc, n_tris_bound, b.vals[0], qscan, b.meta, nullptr, s);
 }
 
 void bvh_remap(BvhBuffers& b, const int* fscan, int n_tris_bound, cudaStream_t s) {
-    k_remap_leaves<<<grid_for(n_tris_bound, 256), 256, 0, s>>>(b.meta, fscan, b.vals[0], (int*)b.keys[1]);
+    pdl(k_remap_leaves, grid_for(n_tris_bound, 256), 256, 0, s)(b.meta, fscan, b.vals[0], (int*)b.keys[1]);
     note_launch();
 }
 
@@ -1006,11 +1024,11 @@ void bvh_query(const BvhBuffers& b, const int4* tri, const float4* pos, const in
     cudaMemsetAsync(&rc->pad[1], 0, 3 * sizeof(int), s);  // list length, query count, redo count
     // query faces in leaf order (uses the sort's second buffers, free after the build)
     const int gF = grid_for(n_query_bound, 256);
-    k_query_order<<<gF, 256, 0, s>>>(rc, b.vals[0], qscan, b.live_scan);
+    pdl(k_query_order, gF, 256, 0, s)(rc, b.vals[0], qscan, b.live_scan);
     note_launch();
     exclusive_scan(b.live_scan, b.live_scan, &rc->n_live, 1, &rc->pad[2], b.scan_scratch, s, &rc->status,
                    n_query_bound);
-    k_query_gather<<<gF, 256, 0, s>>>(rc, b.vals[0], b.live_scan, b.vals[1]);
+    pdl(k_query_gather, gF, 256, 0, s)(rc, b.vals[0], b.live_scan, b.vals[1]);
     note_launch();
     // b.visit (free between a tree's bottom-up passes) holds the per-query redo marks
     // a function-local static initialiser runs once even when worker threads query concurrently
@@ -1020,16 +1038,16 @@ void bvh_query(const BvhBuffers& b, const int4* tri, const float4* pos, const in
             nb = 4;
         return nb;
     }();
-    k_traverse_list<<<grid_for(n_query_bound, kQueryThreads, blocks_per_sm), kQueryThreads, 0, s>>>(
+    pdl(k_traverse_list, grid_for(n_query_bound, kQueryThreads, blocks_per_sm), kQueryThreads, 0, s)(
         b.packed, b.box_lo, b.box_hi, b.vals[1], pair_list, pair_cap, rc, b.visit, fmesh, mesh_root);
     note_launch();
     cudaMemsetAsync(b.xq_count, 0, sizeof(int), s);
-    k_pairs<<<grid_for((long long)pair_cap, 128, 16), 128, 0, s>>>(tri, pos, pair_list, pair_cap, hit, rc, eps, b.xq,
+    pdl(k_pairs, grid_for((long long)pair_cap, 128, 16), 128, 0, s)(tri, pos, pair_list, pair_cap, hit, rc, eps, b.xq,
                                                                    b.xq_cap, b.xq_count);
     note_launch();
-    k_pairs_exact<<<4 * kNumSM, 64, 0, s>>>(tri, pos, b.xq, b.xq_cap, b.xq_count, hit, eps);
+    pdl(k_pairs_exact, 4 * kNumSM, 64, 0, s)(tri, pos, b.xq, b.xq_cap, b.xq_count, hit, eps);
     note_launch();
-    k_traverse_redo<<<grid_for(n_query_bound, kQueryThreads, 4), kQueryThreads, 0, s>>>(
+    pdl(k_traverse_redo, grid_for(n_query_bound, kQueryThreads, 4), kQueryThreads, 0, s)(
         b.packed, b.box_lo, b.box_hi, tri, pos, b.vals[1], hit, rc, eps, b.visit, fmesh, mesh_root);
     note_launch();
 }

@@ -57,11 +57,13 @@ __device__ D3 closest_point_triangle(D3 p, D3 a, D3 b, D3 c) {
 }
 
 __global__ void k_to_float4(const double* __restrict__ v, int n, float4* out) {
+    pdl_wait();
     for (int i = gtid(); i < n; i += gstride())
         out[i] = make_float4((float)v[3 * i], (float)v[3 * i + 1], (float)v[3 * i + 2], 0.f);
 }
 
 __global__ void k_to_int4(const int* __restrict__ f, int n, int nv, int4* out, int* status) {
+    pdl_wait();
     for (int i = gtid(); i < n; i += gstride()) {
         const int a = f[3 * i], b = f[3 * i + 1], c = f[3 * i + 2];
         if (a < 0 || b < 0 || c < 0 || a >= nv || b >= nv || c >= nv) {
@@ -142,6 +144,7 @@ __global__ void __launch_bounds__(kQT) k_point_mesh(const double* __restrict__ p
                                                     const float4* __restrict__ packed, const unsigned* __restrict__ scene,
                                                     const int* __restrict__ leaf_face, const RoundCounters* rc,
                                                     double* out_d2, int* out_face, int* status) {
+    pdl_wait();
     __shared__ int s_node[kStack][kQT];
     __shared__ float s_dist[kStack][kQT];
     __shared__ int s_list[kList][kQT];
@@ -263,6 +266,7 @@ __global__ void __launch_bounds__(kQT) k_point_mesh(const double* __restrict__ p
 // cosines on the squared edge lengths), in radians; NaN for a face with a repeated index.
 __global__ void k_face_min_angles(const double* __restrict__ V, const int* __restrict__ F, int nf, double* out_edge,
                                   double* out_igl) {
+    pdl_wait();
     for (int f = gtid(); f < nf; f += gstride()) {
         const int i0 = F[3 * f], i1 = F[3 * f + 1], i2 = F[3 * f + 2];
         if (i0 == i1 || i1 == i2 || i2 == i0) {
@@ -333,11 +337,11 @@ int pamo_point_mesh_sqdist(const double* points, int32_t n_points, const double*
         h.n_pts = n_vertices;
         h.n_tris = n_triangles;
         cudaMemcpyAsync(rc, &h, sizeof(h), cudaMemcpyHostToDevice, s);
-        k_to_float4<<<grid_for(n_vertices, kT), kT, 0, s>>>(vertices, n_vertices, pos);
-        k_to_int4<<<grid_for(n_triangles, kT), kT, 0, s>>>(triangles, n_triangles, n_vertices, tri, &rc->status);
+        pdl(k_to_float4, grid_for(n_vertices, kT), kT, 0, s)(vertices, n_vertices, pos);
+        pdl(k_to_int4, grid_for(n_triangles, kT), kT, 0, s)(triangles, n_triangles, n_vertices, tri, &rc->status);
         note_launches(2);
         bvh_build(b, tri, pos, rc, n_triangles, s, false, nullptr, false);
-        k_point_mesh<<<grid_for(n_points, kQT, 16), kQT, 0, s>>>(points, n_points, vertices, pos, tri, b.packed, b.scene,
+        pdl(k_point_mesh, grid_for(n_points, kQT, 16), kQT, 0, s)(points, n_points, vertices, pos, tri, b.packed, b.scene,
                                                                 b.vals[0], rc, out_sqdist, out_face, &rc->status);
         note_launch();
         r = cuda_status(cudaStreamSynchronize(s));
@@ -360,7 +364,7 @@ int pamo_face_min_angles(const double* vertices, const int32_t* triangles, int32
     if (!vertices || !triangles || n_triangles < 0 || (!out_edge_form && !out_igl_form)) return PAMO_ERR_INVALID_ARG;
     if (n_triangles == 0) return PAMO_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    k_face_min_angles<<<grid_for(n_triangles, kT), kT, 0, s>>>(vertices, triangles, n_triangles, out_edge_form,
+    pdl(k_face_min_angles, grid_for(n_triangles, kT), kT, 0, s)(vertices, triangles, n_triangles, out_edge_form,
                                                                out_igl_form);
     note_launch();
     return cuda_status(cudaStreamSynchronize(s));

@@ -147,6 +147,7 @@ int scratch_on_current_device(unsigned char** out) {
 
 // counters of this call: zero, then the mesh sizes (no host staging buffer involved)
 __global__ void k_noalloc_init(pamo::RoundCounters* rc, int n_points, int n_triangles) {
+    pamo::pdl_wait();
     int* w = (int*)rc;
     for (int i = threadIdx.x; i < (int)(sizeof(pamo::RoundCounters) / sizeof(int)); i += blockDim.x) w[i] = 0;
     __syncthreads();
@@ -173,7 +174,7 @@ extern "C" int pamo_self_intersect_noalloc(const float* points, const int32_t* t
     cudaStream_t s = (cudaStream_t)stream;
 
     // the counters and flags start from zero on every call (the array keeps the previous call's contents)
-    k_noalloc_init<<<1, 64, 0, s>>>(L.rc, n_points, n_triangles);
+    pamo::pdl(k_noalloc_init, 1, 64, 0, s)(L.rc, n_points, n_triangles);
     cudaMemsetAsync(L.hit, 0, n_triangles + 1, s);
 
     pamo::launch_load_points(points, n_points, L.pos, L.orig_pos, L.occ, s);

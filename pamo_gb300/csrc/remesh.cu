@@ -37,6 +37,7 @@ __device__ __forceinline__ float unord(unsigned u) { return __uint_as_float((u &
 // maxima (max((p - mean) - min) = max(p - mean) - min: rounding is monotone)
 __global__ void __launch_bounds__(kT) k_corner_bounds(const float* __restrict__ pts, const int* __restrict__ tris, int nf,
                                                       const float* mean, unsigned* ext, int np, int* status) {
+    pdl_wait();
     __shared__ float sm[6][kT / 32];
     float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
     const long long n = 3ll * nf;
@@ -84,6 +85,7 @@ __device__ __forceinline__ float extent_max(const unsigned* ext) {
 // when the counts are read)
 __global__ void k_normalise(const float* __restrict__ pts, int np, const int* __restrict__ tris, int nf,
                             const float* mean, const unsigned* ext, float band, float margin, float4* q, int4* tri) {
+    pdl_wait();
     const float t0 = unord(ext[0]), t1 = unord(ext[1]), t2 = unord(ext[2]), tmax = extent_max(ext);
     for (int v = gtid(); v < np; v += gstride()) {
         const float x = ((pts[3 * v] - mean[0]) - t0) / tmax, y = ((pts[3 * v + 1] - mean[1]) - t1) / tmax,
@@ -217,6 +219,7 @@ __device__ __forceinline__ void splat_range(const SplatBox& s, unsigned i0, unsi
 
 __global__ void __launch_bounds__(kT) k_splat(const float4* __restrict__ q, const int4* __restrict__ tri, int nf, int R,
                                               float band, unsigned* udf2, int2* queue, int* queued) {
+    pdl_wait();
     const float inv = 1.0f / (float)(R + 1), slack = kBoxSlack * band;
     const int lane = threadIdx.x & 31;
     for (long long f = gtid() >> 5; f < nf; f += gstride() >> 5) {
@@ -250,6 +253,7 @@ __global__ void __launch_bounds__(kT) k_splat(const float4* __restrict__ q, cons
 __global__ void __launch_bounds__(kT) k_splat_big(const float4* __restrict__ q, const int4* __restrict__ tri, int R,
                                                   float band, unsigned* udf2, const int2* __restrict__ queue,
                                                   const int* __restrict__ queued) {
+    pdl_wait();
     const int n = min(*queued, kSplatQueue);
     for (int k = gtid() >> 5; k < n; k += gstride() >> 5) {
         const int2 e = queue[k];
@@ -262,6 +266,7 @@ __global__ void __launch_bounds__(kT) k_splat_big(const float4* __restrict__ q, 
 }
 
 __global__ void k_fill_value(unsigned* p, long long n, unsigned v) {
+    pdl_wait();
     const long long n4 = n >> 2;
     for (long long i = gtid(); i < n4; i += gstride()) reinterpret_cast<uint4*>(p)[i] = make_uint4(v, v, v, v);
     if (gtid() < (n & 3)) p[4 * n4 + gtid()] = v;
@@ -276,6 +281,7 @@ __device__ __forceinline__ float distance_of(unsigned d2, float band) { return f
 // boundary. A warp takes 32 words, so that each lane stores one.
 __global__ void __launch_bounds__(kT) k_sign_bits(const unsigned* __restrict__ udf2, int R, int W, float band, float iso,
                                                   unsigned* far, unsigned* below, unsigned* out) {
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const long long words = (long long)R * R * W;
     for (long long w0 = 32ll * (gtid() >> 5); w0 < words; w0 += gstride()) {
@@ -329,6 +335,7 @@ __device__ __forceinline__ unsigned carries(unsigned p, unsigned s, unsigned cin
 
 __global__ void __launch_bounds__(kFillThreads) k_fill(const unsigned* __restrict__ far, unsigned* out, int R, int W,
                                                        long long plane_stride, long long row_stride, int* changed) {
+    pdl_wait();
     extern __shared__ unsigned fill_sm[];
     const int tiles = (R + kFillRows - 1) / kFillRows;
     const int plane = blockIdx.x / tiles, r0 = (blockIdx.x % tiles) * kFillRows;
@@ -439,6 +446,7 @@ __global__ void __launch_bounds__(kFillThreads) k_fill(const unsigned* __restric
 // The field at a sample is |udf - iso|, negative inside (not outside) unless it is zero: neg has those samples' bits.
 __global__ void k_negative(const unsigned* __restrict__ far, const unsigned* __restrict__ below,
                            const unsigned* __restrict__ out, long long words, unsigned* neg) {
+    pdl_wait();
     for (long long i = gtid(); i < words; i += gstride()) neg[i] = below[i] | (far[i] & ~out[i]);
 }
 
@@ -469,6 +477,7 @@ __device__ __forceinline__ void edge_bits(const unsigned* neg, long long i, int 
 // per word: the cells (named by their lowest sample) whose corners change sign, their number, and the number of quads
 __global__ void k_surface_counts(const unsigned* __restrict__ neg, int R, int W, unsigned* cells, int* ccount,
                                  int* qcount) {
+    pdl_wait();
     const long long words = (long long)R * R * W;
     for (long long i = gtid(); i < words; i += gstride()) {
         const long long row = i / W;
@@ -502,6 +511,7 @@ __global__ void __launch_bounds__(kT) k_cell_vertices(const unsigned* __restrict
                                                       const unsigned* __restrict__ cells, int R, int W, float iso,
                                                       const int* __restrict__ cscan, float band, float margin,
                                                       const unsigned* ext, float* verts) {
+    pdl_wait();
     const float t0 = unord(ext[0]), t1 = unord(ext[1]), t2 = unord(ext[2]), tmax = extent_max(ext);
     const int lane = threadIdx.x & 31;
     const long long words = (long long)R * R * W, RR = (long long)R * R;
@@ -547,6 +557,7 @@ __global__ void __launch_bounds__(kT) k_cell_vertices(const unsigned* __restrict
 __global__ void __launch_bounds__(kT) k_quads(const unsigned* __restrict__ neg, const unsigned* __restrict__ cells, int R,
                                               int W, const int* __restrict__ qscan, const int* __restrict__ cscan,
                                               int* tris) {
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const unsigned lower = (1u << lane) - 1u;
     const long long words = (long long)R * R * W;
@@ -693,17 +704,17 @@ int pamo_remesh(pamo_remesher* m, const float* points, const int32_t* triangles,
     cudaMemcpyAsync(d_mean, m->h_small + 4, 3 * sizeof(float), cudaMemcpyHostToDevice, s);
     cudaMemsetAsync(ext, 0xFF, 3 * sizeof(unsigned), s);
     cudaMemsetAsync(ext + 3, 0x00, 5 * sizeof(unsigned), s);  // the maxima, changed, queued
-    k_corner_bounds<<<grid_for(3ll * n_triangles, kT), kT, 0, s>>>(points, triangles, n_triangles, d_mean, ext, n_points,
+    pdl(k_corner_bounds, grid_for(3ll * n_triangles, kT), kT, 0, s)(points, triangles, n_triangles, d_mean, ext, n_points,
                                                                    &m->rc->status);
-    k_normalise<<<grid_for(std::max(n_points, n_triangles), kT), kT, 0, s>>>(points, n_points, triangles, n_triangles,
+    pdl(k_normalise, grid_for(std::max(n_points, n_triangles), kT), kT, 0, s)(points, n_points, triangles, n_triangles,
                                                                            d_mean, ext, band, margin, q, tri);
     const float band2 = band * band;
     unsigned band2_bits;
     std::memcpy(&band2_bits, &band2, sizeof(band2_bits));
-    k_fill_value<<<grid_for(NV / 4 + 1, kT), kT, 0, s>>>(udf2, NV, band2_bits);
-    k_splat<<<grid_for(32ll * n_triangles, kT), kT, 0, s>>>(q, tri, n_triangles, R, band, udf2, (int2*)m->queue.p, d_queued);
-    k_splat_big<<<8 * kNumSM, kT, 0, s>>>(q, tri, R, band, udf2, (const int2*)m->queue.p, d_queued);
-    k_sign_bits<<<grid_for(words, kT), kT, 0, s>>>(udf2, R, W, band, iso, far, below, out);
+    pdl(k_fill_value, grid_for(NV / 4 + 1, kT), kT, 0, s)(udf2, NV, band2_bits);
+    pdl(k_splat, grid_for(32ll * n_triangles, kT), kT, 0, s)(q, tri, n_triangles, R, band, udf2, (int2*)m->queue.p, d_queued);
+    pdl(k_splat_big, 8 * kNumSM, kT, 0, s)(q, tri, R, band, udf2, (const int2*)m->queue.p, d_queued);
+    pdl(k_sign_bits, grid_for(words, kT), kT, 0, s)(udf2, R, W, band, iso, far, below, out);
     note_launches(6);
     // flood fill: two passes over the planes of both orientations, the second of which notes whether it changed
     // anything, and the counts behind them; again until it did not (each repetition adds at least one sample)
@@ -716,11 +727,11 @@ int pamo_remesh(pamo_remesher* m, const float* points, const int32_t* triangles,
     for (long long batch = 0; batch < max_batches; ++batch) {
         for (int pass = 0; pass < 2; ++pass) {
             if (pass == 1) cudaMemsetAsync(d_changed, 0, sizeof(int), s);
-            k_fill<<<R * tiles, kFillThreads, fill_smem, s>>>(far, out, R, W, (long long)R * W, W, d_changed);
-            k_fill<<<R * tiles, kFillThreads, fill_smem, s>>>(far, out, R, W, W, (long long)R * W, d_changed);
+            pdl(k_fill, R * tiles, kFillThreads, fill_smem, s)(far, out, R, W, (long long)R * W, W, d_changed);
+            pdl(k_fill, R * tiles, kFillThreads, fill_smem, s)(far, out, R, W, W, (long long)R * W, d_changed);
         }
-        k_negative<<<grid_for(words, kT), kT, 0, s>>>(far, below, out, words, neg);
-        k_surface_counts<<<grid_for(words, kT), kT, 0, s>>>(neg, R, W, cells, ccount, qcount);
+        pdl(k_negative, grid_for(words, kT), kT, 0, s)(far, below, out, words, neg);
+        pdl(k_surface_counts, grid_for(words, kT), kT, 0, s)(neg, R, W, cells, ccount, qcount);
         note_launches(6);
         const ScanJob jobs[2] = {{ccount, ccount, nullptr, (int)words + 1, &m->rc->n_win, scratch},
                                  {qcount, qcount, nullptr, (int)words + 1, &m->rc->n_query, scratch + scan_scratch_ints()}};
@@ -738,9 +749,9 @@ int pamo_remesh(pamo_remesher* m, const float* points, const int32_t* triangles,
     m->nf = 2 * m->h_small[3];
     if ((r = m->verts.grow(((size_t)m->nv + 1) * 3 * sizeof(float))) || (r = m->tris.grow(((size_t)m->nf + 1) * 3 * sizeof(int))))
         return r;
-    k_cell_vertices<<<grid_for(words, kT), kT, 0, s>>>(udf2, neg, cells, R, W, iso, ccount, band, margin, ext,
+    pdl(k_cell_vertices, grid_for(words, kT), kT, 0, s)(udf2, neg, cells, R, W, iso, ccount, band, margin, ext,
                                                        (float*)m->verts.p);
-    k_quads<<<grid_for(words, kT), kT, 0, s>>>(neg, cells, R, W, qcount, ccount, (int*)m->tris.p);
+    pdl(k_quads, grid_for(words, kT), kT, 0, s)(neg, cells, R, W, qcount, ccount, (int*)m->tris.p);
     note_launches(2);
     if (cudaStreamSynchronize(s) != cudaSuccess) return PAMO_ERR_CUDA;
     if (out_n_points) *out_n_points = m->nv;

@@ -392,6 +392,7 @@ __device__ void grid_sum_finish(CSum acc, float2* partial, int* counter, float* 
 constexpr int kNormBlocks = 4 * 152;
 
 __global__ void __launch_bounds__(kT) k_norm_partial(const double* __restrict__ gt, int n, double* part) {
+    pdl_wait();
     __shared__ double sh[9][kT];
     const long long chunk = ((long long)n + gridDim.x - 1) / gridDim.x;
     const long long lo = chunk * blockIdx.x, hi = min((long long)n, lo + chunk);
@@ -422,6 +423,7 @@ __global__ void __launch_bounds__(kT) k_norm_partial(const double* __restrict__ 
 }
 
 __global__ void __launch_bounds__(kT) k_norm_final(const double* __restrict__ part, int nparts, int n, double* stats) {
+    pdl_wait();
     __shared__ double sh[9][kT];
     double s[3] = {0, 0, 0}, mn[3] = {1e300, 1e300, 1e300}, mx[3] = {-1e300, -1e300, -1e300};
     for (int b = threadIdx.x; b < nparts; b += blockDim.x)
@@ -461,6 +463,7 @@ __global__ void __launch_bounds__(kT) k_norm_final(const double* __restrict__ pa
 // V * scale + t in float64 (numpy), stored as float32 (the simulation arrays)
 template <typename T>
 __global__ void k_normalize(const T* __restrict__ in, int n, const double* __restrict__ st, float4* out, float4* copy) {
+    pdl_wait();
     const double s = st[3];
     for (int i = gtid(); i < n; i += gstride()) {
         const float4 p = make_float4((float)((double)in[3 * i] * s + st[4]), (float)((double)in[3 * i + 1] * s + st[5]),
@@ -471,6 +474,7 @@ __global__ void k_normalize(const T* __restrict__ in, int n, const double* __res
 }
 
 __global__ void k_denormalize(const float4* __restrict__ q, int n, const double* __restrict__ st, double* out) {
+    pdl_wait();
     const double s = st[3];
     for (int i = gtid(); i < n; i += gstride()) {
         const float4 p = q[i];
@@ -482,6 +486,7 @@ __global__ void k_denormalize(const float4* __restrict__ q, int n, const double*
 
 // int32 rows of 3 -> int4; an index outside [0, n_points) sets *bad and the face becomes (0, 0, 0)
 __global__ void k_tris4(const int* __restrict__ t, int n, int n_points, int4* out, int* bad) {
+    pdl_wait();
     for (int i = gtid(); i < n; i += gstride()) {
         int4 f = make_int4(t[3 * i], t[3 * i + 1], t[3 * i + 2], 0);
         if ((unsigned)f.x >= (unsigned)n_points || (unsigned)f.y >= (unsigned)n_points ||
@@ -515,6 +520,7 @@ __device__ __forceinline__ double dsq(D3 a, D3 b) {
 // simulation's weights array).
 __global__ void k_voronoi(const double* __restrict__ pts, const double* __restrict__ st, const int4* __restrict__ tri,
                           int nt, const int* __restrict__ inv_vs, double* wslot) {
+    pdl_wait();
     for (int f = gtid(); f < nt; f += gstride()) {
         const int4 t = tri[f];
         const D3 p[3] = {norm_pos(pts, t.x, st), norm_pos(pts, t.y, st), norm_pos(pts, t.z, st)};
@@ -548,6 +554,7 @@ __global__ void k_voronoi(const double* __restrict__ pts, const double* __restri
 }
 
 __global__ void k_weights_f32(const double* __restrict__ wslot, const int* __restrict__ vs_off, int n, float* w) {
+    pdl_wait();
     for (int i = gtid(); i < n; i += gstride()) {
         double acc = 0.0;
         for (int s = vs_off[i]; s < vs_off[i + 1]; ++s) acc += wslot[s];
@@ -557,6 +564,7 @@ __global__ void k_weights_f32(const double* __restrict__ wslot, const int* __res
 
 // elastic_preprocess_kernel (elastic_energy.py:7-37)
 __global__ void k_elastic_pre(const float4* __restrict__ xr, const int4* __restrict__ tri, int nt, float* area, float4* invDm) {
+    pdl_wait();
     for (int f = gtid(); f < nt; f += gstride()) {
         const int4 t = tri[f];
         const F3 x0 = f3(xr[t.x]), x1 = f3(xr[t.y]), x2 = f3(xr[t.z]);
@@ -583,6 +591,7 @@ __device__ __forceinline__ float hinge_angle(F3 x0, F3 x1, F3 x2, F3 x3) {
 }
 
 __global__ void k_hinge_pre(const float4* __restrict__ xr, const int4* __restrict__ hinge, int nh, float2* rest) {
+    pdl_wait();
     for (int h = gtid(); h < nh; h += gstride()) {
         const int4 i = hinge[h];
         const F3 x0 = f3(xr[i.x]), x1 = f3(xr[i.y]), x2 = f3(xr[i.z]), x3 = f3(xr[i.w]);
@@ -596,6 +605,7 @@ __global__ void k_hinge_pre(const float4* __restrict__ xr, const int4* __restric
 // one NaN angle anywhere disables the test. flag bit 0: some angle <= thres; bit 1: some angle is NaN.
 __global__ void k_min_angle(const double* __restrict__ pts, const double* __restrict__ st, const int4* __restrict__ tri,
                             int nt, double thres_deg, int* flag) {
+    pdl_wait();
     for (int f = gtid(); f < nt; f += gstride()) {
         const int4 t = tri[f];
         const D3 p[3] = {norm_pos(pts, t.x, st), norm_pos(pts, t.y, st), norm_pos(pts, t.z, st)};
@@ -648,6 +658,7 @@ __global__ void __launch_bounds__(kQT) k_closest_gt(const float4* __restrict__ q
                                                     const int* __restrict__ leaf_face, const int4* __restrict__ gtri,
                                                     const float4* __restrict__ gpos, const RoundCounters* grc,
                                                     float4* target, int* status) {
+    pdl_wait();
     __shared__ int stack[kStack][kQT];
     const int nl = grc->n_live;
     for (int i = gtid(); i < np; i += gstride()) {
@@ -727,6 +738,7 @@ __global__ void __launch_bounds__(kQT) k_closest_gt(const float4* __restrict__ q
 // rebuild when some vertex moved more than half the skin since the lists were built
 __global__ void k_disp_check(const float4* __restrict__ q, const float4* __restrict__ qref, int np, float half_skin,
                              SolverScalars* sc) {
+    pdl_wait();
     if (sc->abort) return;
     bool moved = false;
     for (int i = gtid(); i < np; i += gstride()) {
@@ -748,6 +760,7 @@ __global__ void __launch_bounds__(kQT) k_candidates(const float4* __restrict__ x
                                                     const RoundCounters* brc, float d_hat, float skin, int2* out,
                                                     int cap, int* qcount, const int* __restrict__ qoff,
                                                     SolverScalars* sc) {
+    pdl_wait();
     __shared__ int stack[kStack][kQT];
     if (sc->abort || !sc->rebuild) return;
     const float reach = 2.0f * sc->radius + d_hat + skin;
@@ -836,6 +849,7 @@ __global__ void __launch_bounds__(kQT) k_candidates(const float4* __restrict__ x
 // overflow of a candidate list: grow it and redo the iteration; otherwise the lists now hold positions q
 __global__ void k_cand_done(const float4* __restrict__ q, float4* qref, int np, int cap_pt, int cap_ee,
                             SolverScalars* sc) {
+    pdl_wait();
     if (sc->abort || !sc->rebuild) return;
     if (sc->n_cand_pt > cap_pt || sc->n_cand_ee > cap_ee) {
         if (gtid() == 0) sc->abort = 3;
@@ -852,6 +866,7 @@ __global__ void __launch_bounds__(kT) k_filter(const float4* __restrict__ x, con
                                                const int2* __restrict__ cee, const int4* __restrict__ tri,
                                                const int4* __restrict__ edge4, float d_hat, float ee_thres,
                                                int* cflag, int4* cid, int2* cty, SolverScalars* sc) {
+    pdl_wait();
     if (sc->abort) return;
     const float thr = 2.0f * sc->radius + d_hat;
     const int npt = sc->n_cand_pt, nee = sc->n_cand_ee;
@@ -891,6 +906,7 @@ __global__ void __launch_bounds__(kT) k_filter(const float4* __restrict__ x, con
 __global__ void __launch_bounds__(kT) k_contacts_scatter(const int* __restrict__ cflag, const int* __restrict__ cpos,
                                                          const int4* __restrict__ cid, const int2* __restrict__ cty,
                                                          int4* c_idx, int2* c_type, int* ccnt, SolverScalars* sc) {
+    pdl_wait();
     if (sc->abort) return;
     const int n = sc->n_cand_all;
     for (int g = gtid(); g < n; g += gstride()) {
@@ -912,6 +928,7 @@ __global__ void __launch_bounds__(kT) k_contacts_scatter(const int* __restrict__
 // of a contact are written at those positions, so each vertex's contact parts are contiguous and in code order.
 __global__ void __launch_bounds__(kT) k_cvert_fill(const int4* __restrict__ c_idx, const int* __restrict__ coff,
                                                    int* ccur, int* ctmp, const SolverScalars* sc) {
+    pdl_wait();
     if (sc->abort) return;
     const int n = 4 * sc->n_contacts;
     for (int s = gtid(); s < n; s += gstride()) {
@@ -924,6 +941,7 @@ __global__ void __launch_bounds__(kT) k_cvert_fill(const int4* __restrict__ c_id
 
 __global__ void __launch_bounds__(kT) k_cvert_rank(const int* __restrict__ coff, const int* __restrict__ ctmp,
                                                    int* cinv, int np, const SolverScalars* sc) {
+    pdl_wait();
     if (sc->abort) return;
     const int lane = threadIdx.x & 31;
     const long long warps = (long long)gridDim.x * (blockDim.x / 32);
@@ -1133,6 +1151,7 @@ __device__ __forceinline__ CSum energy_elements(const float4* __restrict__ x, co
 
 __global__ void __launch_bounds__(kT) k_energy(const float4* __restrict__ x, EnergyArgs A, SolverScalars* sc,
                                                float2* partial, int ls_n) {
+    pdl_wait();
     if (sc->abort) return;
     if (ls_n > 0 && sc->energy < sc->energy_prev) return;
     const CSum acc = energy_elements(x, A, sc->n_contacts, gtid(), gstride());
@@ -1146,6 +1165,7 @@ __global__ void __launch_bounds__(kT) k_energy(const float4* __restrict__ x, Ene
 __global__ void k_diff_elastic(const float4* __restrict__ x, const int4* __restrict__ tri, const float* __restrict__ area,
                                const float4* __restrict__ invDm, float mu, float la, float coeff, int nt, float4* gslot,
                                const int* __restrict__ inv_vs, const SolverScalars* sc) {
+    pdl_wait();
     if (sc->abort) return;
     for (int f = gtid(); f < nt; f += gstride()) {
         const int4 t = tri[f];
@@ -1201,6 +1221,7 @@ __device__ __forceinline__ M33 sym(M33 a) { return add(a, tr(a)); }
 __global__ void k_diff_hinge(const float4* __restrict__ x, const int4* __restrict__ hinge, const float2* __restrict__ rest,
                              float k, float coeff, int nh, float* blocks, float4* gslot, float4* hslot,
                              const int* __restrict__ inv_h, const SolverScalars* sc) {
+    pdl_wait();
     if (sc->abort) return;
     for (int h = gtid(); h < nh; h += gstride()) {
         const int4 id = hinge[h];
@@ -1287,6 +1308,7 @@ constexpr int kSpdWarps = 4;
 
 __global__ void __launch_bounds__(32 * kSpdWarps) k_spd_project(float* blocks, int nh, int sweeps,
                                                                 const SolverScalars* sc) {
+    pdl_wait();
     if (sc->abort) return;
     __shared__ float sA[kSpdWarps][3][81], sV[kSpdWarps][3][81];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1352,6 +1374,7 @@ __global__ void __launch_bounds__(32 * kSpdWarps) k_spd_project(float* blocks, i
 __global__ void k_diff_contact(const float4* __restrict__ x, const int4* __restrict__ cidx, const int2* __restrict__ ctype,
                                const float* __restrict__ cd, const SolverScalars* sc, float kappa, float dh, float coeff,
                                float4* cdd, float4* gslot, float4* hslot, const int* __restrict__ cinv) {
+    pdl_wait();
     if (sc->abort) return;
     const int n = sc->n_contacts;
     for (int b = gtid(); b < n; b += gstride()) {
@@ -1387,6 +1410,7 @@ __global__ void __launch_bounds__(kT) k_gather_grad(const float4* __restrict__ x
                                                     const float* __restrict__ w, float stiff, float coeff, int np,
                                                     const float4* __restrict__ gslot, const float4* __restrict__ hslot,
                                                     VertexSlots S, float4* grad, float4* hd, const SolverScalars* sc) {
+    pdl_wait();
     if (sc->abort) return;
     const int G = gather_width((long long)gridDim.x * blockDim.x, np);
     const long long ngroups = (long long)gridDim.x * blockDim.x / G;
@@ -1730,6 +1754,7 @@ template <int kThreads>
 __global__ void __launch_bounds__(kThreads) k_cg_start(const float4* __restrict__ grad, const float4* __restrict__ hd,
                                                        int np, float4* p, float4* r, float4* z, float4* v0,
                                                        SolverScalars* sc, float2* partial) {
+    pdl_wait();
     if (sc->abort) return;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
     grid_sum_finish(cg_init_vertices(grad, hd, np, p, r, z, v0, tid, nthreads), partial, &sc->red_count, &sc->z_r,
@@ -1740,6 +1765,7 @@ template <int kThreads>
 __global__ void __launch_bounds__(kThreads) k_cg_product(const float4* __restrict__ x, HvpArgs A,
                                                          const float4* __restrict__ z, const float4* __restrict__ vin,
                                                          float4* vout, int it, SolverScalars* sc, float2* partial) {
+    pdl_wait();
     if (sc->abort) return;
     const int nc = sc->n_contacts;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
@@ -1754,6 +1780,7 @@ template <int kThreads>
 __global__ void __launch_bounds__(kThreads) k_cg_update(HvpArgs A, const float4* __restrict__ v,
                                                         const float4* __restrict__ hd, float4* p, float4* r, float4* z,
                                                         SolverScalars* sc, float2* partial) {
+    pdl_wait();
     if (sc->abort) return;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
     const PrzLanes L = prz_lanes(tid, nthreads, A.np);
@@ -1911,6 +1938,7 @@ __global__ void __launch_bounds__(kClusterThreads) k_cg_cluster(const float4* __
 // cursors cleared.
 __global__ void k_iter_begin(const float4* __restrict__ q, float4* qpn, int* ccnt, int* ccur, int np,
                              SolverScalars* sc) {
+    pdl_wait();
     if (sc->abort) return;
     for (int i = gtid(); i <= np; i += gstride()) {
         if (i < np) {
@@ -1924,6 +1952,7 @@ __global__ void k_iter_begin(const float4* __restrict__ q, float4* qpn, int* ccn
 // After detection: the contact count, and the abort code when the list overflowed (energy.py:942-948 halves
 // the radius when the count exceeds max_blocks; a count above this build's capacity grows the list instead).
 __global__ void k_contacts_done(SolverScalars* sc, int cap, long long max_blocks) {
+    pdl_wait();
     if (sc->abort) return;
     const int raw = sc->n_contacts_raw;
     if ((long long)raw > max_blocks) {
@@ -1944,6 +1973,7 @@ __global__ void k_contacts_done(SolverScalars* sc, int cap, long long max_blocks
 // clamp_p_kernel (solver_kernels.py:68-85): keep |q_prev_newton + p - q_prev_detection| <= radius. Contacts are
 // detected at the start of every Newton iteration, so q_prev_detection equals q_prev_newton.
 __global__ void k_clamp_p(float4* p, const float4* __restrict__ qn, float radius, int np, const SolverScalars* sc) {
+    pdl_wait();
     if (sc->abort) return;
     for (int i = gtid(); i < np; i += gstride()) {
         const F3 pi = f3(p[i]), qni = f3(qn[i]);
@@ -1954,6 +1984,7 @@ __global__ void k_clamp_p(float4* p, const float4* __restrict__ qn, float radius
 
 // _ccd (system.py:368-391) sets ccd_step = 1; _line_search (:393-409) keeps the energy before the search.
 __global__ void k_before_ccd(SolverScalars* sc) {
+    pdl_wait();
     if (sc->abort) return;
     sc->ccd_step = 1.0f;
     sc->energy_prev = sc->energy;
@@ -1965,6 +1996,7 @@ __global__ void k_before_ccd(SolverScalars* sc) {
 __global__ void k_accd(const float4* __restrict__ x, const float4* __restrict__ vel, const int4* __restrict__ cidx,
                        const int2* __restrict__ ctype, SolverScalars* sc, float slackness, float thickness, int max_iters,
                        float ee_thres) {
+    pdl_wait();
     if (sc->abort) return;
     const int n = sc->n_contacts;
     for (long long bb = spread_first(); bb < n; bb += spread_stride()) {
@@ -2298,6 +2330,7 @@ template <class R>
 __global__ void k_accd_wide(const float4* __restrict__ x, const float4* __restrict__ vel, const int4* __restrict__ cidx,
                             const int2* __restrict__ ctype, SolverScalars* sc, float slackness_f, float thickness_f,
                             int max_iters, float ee_thres_f) {
+    pdl_wait();
     typedef Real<R> K;
     if (sc->abort) return;
     const R slackness = K::of(slackness_f), thickness = K::of(thickness_f), ee_thres = K::of(ee_thres_f);
@@ -2347,6 +2380,7 @@ __global__ void k_accd_wide(const float4* __restrict__ x, const float4* __restri
 // lowered the energy
 __global__ void k_line_search(const float4* __restrict__ q0, const float4* __restrict__ p, const SolverScalars* sc,
                               int n_halves, int np, float4* q) {
+    pdl_wait();
     if (sc->abort) return;
     if (n_halves > 0 && sc->energy < sc->energy_prev) return;
     const float a = sc->ccd_step * powf(0.5f, (float)n_halves);
@@ -2357,6 +2391,7 @@ __global__ void k_line_search(const float4* __restrict__ q0, const float4* __res
 }
 
 __global__ void k_iter_end(SolverScalars* sc) {
+    pdl_wait();
     if (sc->abort) return;
     sc->iters_done += 1;
 }
@@ -2687,7 +2722,7 @@ int Stage3::energy_grid() const {
 }
 
 void Stage3::launch_energy(const float4* x, int ls_n) {
-    k_energy<<<energy_grid(), kT, 0, stream>>>(x, energy_args(), sc, partial, ls_n);
+    pdl(k_energy, energy_grid(), kT, 0, stream)(x, energy_args(), sc, partial, ls_n);
     note_launch();
 }
 
@@ -2698,10 +2733,10 @@ void Stage3::newton_iteration() {
     const float la = P.elas_young_modulus * P.elas_poisson_ratio / ((1.f + P.elas_poisson_ratio) * (1.f - 2.f * P.elas_poisson_ratio));
     const int gC = grid_for((long long)cap_c, kT);
     // q_prev_newton = q; contacts at q (system.py:425-432, _detect_contact :308-318 with refitted LBVHs)
-    k_iter_begin<<<grid_for(NP + 1, kT), kT, 0, s>>>(q, q_prev_newton, c_cnt, c_cur, NP, sc);
+    pdl(k_iter_begin, grid_for(NP + 1, kT), kT, 0, s)(q, q_prev_newton, c_cnt, c_cur, NP, sc);
     note_launch();
     const float skin = 2.0f * P.contact_detection_radius + P.d_hat;
-    k_disp_check<<<grid_for(NP, kT), kT, 0, s>>>(q, q_ref, NP, 0.5f * skin, sc);
+    pdl(k_disp_check, grid_for(NP, kT), kT, 0, s)(q, q_ref, NP, 0.5f * skin, sc);
     note_launch();
     bvh_refit(tri_bvh, tri, q, tri_rc, NT, s, &sc->rebuild);
     bvh_refit(edge_bvh, edge4, q, edge_rc, NE, s, &sc->rebuild);
@@ -2712,11 +2747,11 @@ void Stage3::newton_iteration() {
     int* cnt_ee = cand_cnt + NP;
     int* off_pt = cand_off;
     int* off_ee = cand_off + NP;
-    k_candidates<false><<<grid_for(NP, kQT, 16), kQT, 0, s>>>(q, NP, tri, tri_bvh.child, tri_bvh.nlo, tri_bvh.nhi,
+    pdl(k_candidates<false>, grid_for(NP, kQT, 16), kQT, 0, s)(q, NP, tri, tri_bvh.child, tri_bvh.nlo, tri_bvh.nhi,
                                                              tri_bvh.llo, tri_bvh.lhi, tri_bvh.vals[0], tri_rc, P.d_hat,
                                                              skin, cand_pt, (int)cap_cpt, cnt_pt, nullptr, sc);
     note_launch();
-    k_candidates<true><<<grid_for(NE, kQT, 16), kQT, 0, s>>>(q, NE, edge4, edge_bvh.child, edge_bvh.nlo, edge_bvh.nhi,
+    pdl(k_candidates<true>, grid_for(NE, kQT, 16), kQT, 0, s)(q, NE, edge4, edge_bvh.child, edge_bvh.nlo, edge_bvh.nhi,
                                                             edge_bvh.llo, edge_bvh.lhi, edge_bvh.vals[0], edge_rc,
                                                             P.d_hat, skin, cand_ee, (int)cap_cee, cnt_ee, nullptr, sc);
     note_launch();
@@ -2727,56 +2762,56 @@ void Stage3::newton_iteration() {
         exclusive_scans(jobs, 2, s, &sc->status, std::max(NP, NE));
         note_launch();
     }
-    k_candidates<false><<<grid_for(NP, kQT, 16), kQT, 0, s>>>(q, NP, tri, tri_bvh.child, tri_bvh.nlo, tri_bvh.nhi,
+    pdl(k_candidates<false>, grid_for(NP, kQT, 16), kQT, 0, s)(q, NP, tri, tri_bvh.child, tri_bvh.nlo, tri_bvh.nhi,
                                                              tri_bvh.llo, tri_bvh.lhi, tri_bvh.vals[0], tri_rc, P.d_hat,
                                                              skin, cand_pt, (int)cap_cpt, cnt_pt, off_pt, sc);
     note_launch();
-    k_candidates<true><<<grid_for(NE, kQT, 16), kQT, 0, s>>>(q, NE, edge4, edge_bvh.child, edge_bvh.nlo, edge_bvh.nhi,
+    pdl(k_candidates<true>, grid_for(NE, kQT, 16), kQT, 0, s)(q, NE, edge4, edge_bvh.child, edge_bvh.nlo, edge_bvh.nhi,
                                                             edge_bvh.llo, edge_bvh.lhi, edge_bvh.vals[0], edge_rc,
                                                             P.d_hat, skin, cand_ee, (int)cap_cee, cnt_ee, off_ee, sc);
     note_launch();
-    k_cand_done<<<grid_for(NP, kT), kT, 0, s>>>(q, q_ref, NP, (int)cap_cpt, (int)cap_cee, sc);
+    pdl(k_cand_done, grid_for(NP, kT), kT, 0, s)(q, q_ref, NP, (int)cap_cpt, (int)cap_cee, sc);
     note_launch();
     // contacts in candidate order: flags, their prefix sums (the total is the contact count), the list, then each
     // vertex's contact corners (counted, offsets, filled, sorted)
     const int cap = (int)std::min<size_t>(cap_c, (size_t)P.max_blocks);
-    k_filter<<<grid_for((long long)(cap_cpt + cap_cee), kT), kT, 0, s>>>(q, cand_pt, cand_ee, tri, edge4, P.d_hat,
+    pdl(k_filter, grid_for((long long)(cap_cpt + cap_cee), kT), kT, 0, s)(q, cand_pt, cand_ee, tri, edge4, P.d_hat,
                                                                         P.ee_classify_thres, cflag, cid, cty, sc);
     note_launch();
     exclusive_scan(cflag, cpos, &sc->n_cand_all, 0, &sc->n_contacts_raw, scan_scratch, s, &sc->status,
                    (long long)(cap_cpt + cap_cee));
     note_launch();
-    k_contacts_done<<<1, 1, 0, s>>>(sc, cap, P.max_blocks);
+    pdl(k_contacts_done, 1, 1, 0, s)(sc, cap, P.max_blocks);
     note_launch();
-    k_contacts_scatter<<<grid_for((long long)(cap_cpt + cap_cee), kT), kT, 0, s>>>(cflag, cpos, cid, cty, c_idx, c_type,
+    pdl(k_contacts_scatter, grid_for((long long)(cap_cpt + cap_cee), kT), kT, 0, s)(cflag, cpos, cid, cty, c_idx, c_type,
                                                                                   c_cnt, sc);
     note_launch();
     exclusive_scan(c_cnt, c_off, nullptr, NP + 1, nullptr, scan_scratch, s, &sc->status, NP + 1);
     note_launch();
-    k_cvert_fill<<<grid_for(4ll * cap_c, kT), kT, 0, s>>>(c_idx, c_off, c_cur, c_tmp, sc);
+    pdl(k_cvert_fill, grid_for(4ll * cap_c, kT), kT, 0, s)(c_idx, c_off, c_cur, c_tmp, sc);
     note_launch();
-    k_cvert_rank<<<grid_for(32ll * NP, kT), kT, 0, s>>>(c_off, c_tmp, c_inv, NP, sc);
+    pdl(k_cvert_rank, grid_for(32ll * NP, kT), kT, 0, s)(c_off, c_tmp, c_inv, NP, sc);
     note_launch();
     // energy, gradient (coeff -1), Hessian diagonal and hinge blocks (system.py:433-434): per-corner parts into
     // the slot arrays, then summed per vertex
     launch_energy(q);
     const size_t nt3 = (size_t)3 * NT, cbase = nt3 + (size_t)4 * NH;
-    k_diff_elastic<<<grid_for(NT, kT), kT, 0, s>>>(q, tri, el_area, el_invDm, mu, la, -1.f, NT, gslot, inv_vs, sc);
+    pdl(k_diff_elastic, grid_for(NT, kT), kT, 0, s)(q, tri, el_area, el_invDm, mu, la, -1.f, NT, gslot, inv_vs, sc);
     note_launch();
     if (NH) {
-        k_diff_hinge<<<grid_for(NH, 128), 128, 0, s>>>(q, hinge, hinge_rest, P.hinge_stiffness, -1.f, NH, hinge_blocks,
+        pdl(k_diff_hinge, grid_for(NH, 128), 128, 0, s)(q, hinge, hinge_rest, P.hinge_stiffness, -1.f, NH, hinge_blocks,
                                                        gslot, hslot, inv_vs + nt3, sc);
         note_launch();
-        k_spd_project<<<grid_for((NH + 3 * kSpdWarps - 1) / (3 * kSpdWarps), 1, 16), 32 * kSpdWarps, 0, s>>>(
+        pdl(k_spd_project, grid_for((NH + 3 * kSpdWarps - 1) / (3 * kSpdWarps), 1, 16), 32 * kSpdWarps, 0, s)(
             hinge_blocks, NH, P.spd_max_iters, sc);
         note_launch();
     }
-    k_diff_contact<<<gC, kT, 0, s>>>(q, c_idx, c_type, c_d, sc, P.coll_stiffness, P.d_hat, -1.f, c_dd, gslot + cbase,
+    pdl(k_diff_contact, gC, kT, 0, s)(q, c_idx, c_type, c_d, sc, P.coll_stiffness, P.d_hat, -1.f, c_dd, gslot + cbase,
                                      hslot + cbase, c_inv);
     note_launch();
     VertexSlots S;
     S.vs_off = vs_off; S.coff = c_off; S.inv_vs = inv_vs; S.cinv = c_inv; S.cbase = (int)cbase;
-    k_gather_grad<<<grid_for((long long)kGather * NP, kT), kT, 0, s>>>(q, target, vweight, P.mesh2gt_dist_stiffness,
+    pdl(k_gather_grad, grid_for((long long)kGather * NP, kT), kT, 0, s)(q, target, vweight, P.mesh2gt_dist_stiffness,
                                                                       -1.f, NP, gslot, hslot, S, grad, hdiag, sc);
     note_launch();
     // Jacobi PCG (cg_solver.py:96-158)
@@ -2810,14 +2845,14 @@ void Stage3::newton_iteration() {
         const long long elems = (long long)NP + NT + NH;
         const int g = (int)std::max<long long>(1, std::min<long long>({(elems + 127) / 128, (long long)n_sm,
                                                                        (long long)kPartials / 2}));
-        k_cg_start<128><<<g, 128, 0, s>>>(grad, hdiag, NP, p, r, z, v[0], sc, partial);
+        pdl(k_cg_start<128>, g, 128, 0, s)(grad, hdiag, NP, p, r, z, v[0], sc, partial);
         note_launch();
         for (int it = 0; it < P.n_cg_iters; ++it) {
             float4* vin = (it & 1) ? v[1] : v[0];
             float4* vout = (it & 1) ? v[0] : v[1];
-            k_cg_product<128><<<g, 128, 0, s>>>(q, H, z, vin, vout, it, sc, partial);
+            pdl(k_cg_product<128>, g, 128, 0, s)(q, H, z, vin, vout, it, sc, partial);
             note_launch();
-            k_cg_update<128><<<g, 128, 0, s>>>(H, vout, hdiag, p, r, z, sc, partial);
+            pdl(k_cg_update<128>, g, 128, 0, s)(H, vout, hdiag, p, r, z, sc, partial);
             note_launch();
         }
     } else {
@@ -2854,18 +2889,18 @@ void Stage3::newton_iteration() {
         note_launch();
     }
     // step clamp, CCD, line search (system.py:441-459)
-    k_clamp_p<<<grid_for(NP, kT), kT, 0, s>>>(p, q_prev_newton, P.contact_detection_radius, NP, sc);
+    pdl(k_clamp_p, grid_for(NP, kT), kT, 0, s)(p, q_prev_newton, P.contact_detection_radius, NP, sc);
     note_launch();
-    k_before_ccd<<<1, 1, 0, s>>>(sc);
+    pdl(k_before_ccd, 1, 1, 0, s)(sc);
     note_launch();
     if (P.ccd_fp64 == 2)
-        k_accd_wide<WF><<<gC, kT, 0, s>>>(q, p, c_idx, c_type, sc, P.ccd_slackness, P.ccd_thickness, P.ccd_max_iters,
+        pdl(k_accd_wide<WF>, gC, kT, 0, s)(q, p, c_idx, c_type, sc, P.ccd_slackness, P.ccd_thickness, P.ccd_max_iters,
                                           P.ee_classify_thres);
     else if (P.ccd_fp64)
-        k_accd_wide<double><<<gC, kT, 0, s>>>(q, p, c_idx, c_type, sc, P.ccd_slackness, P.ccd_thickness,
+        pdl(k_accd_wide<double>, gC, kT, 0, s)(q, p, c_idx, c_type, sc, P.ccd_slackness, P.ccd_thickness,
                                               P.ccd_max_iters, P.ee_classify_thres);
     else
-        k_accd<<<gC, kT, 0, s>>>(q, p, c_idx, c_type, sc, P.ccd_slackness, P.ccd_thickness, P.ccd_max_iters,
+        pdl(k_accd, gC, kT, 0, s)(q, p, c_idx, c_type, sc, P.ccd_slackness, P.ccd_thickness, P.ccd_max_iters,
                                 P.ee_classify_thres);
     note_launch();
     const int g_ls = energy_grid();
@@ -2886,12 +2921,12 @@ void Stage3::newton_iteration() {
         note_launch();
     } else {
         for (int n = 0; n < P.n_line_search_iters; ++n) {
-            k_line_search<<<grid_for(NP, kT), kT, 0, s>>>(q_prev_newton, p, sc, n, NP, q);
+            pdl(k_line_search, grid_for(NP, kT), kT, 0, s)(q_prev_newton, p, sc, n, NP, q);
             note_launch();
             launch_energy(q, n);
         }
     }
-    k_iter_end<<<1, 1, 0, s>>>(sc);
+    pdl(k_iter_end, 1, 1, 0, s)(sc);
     note_launch();
 }
 
@@ -3017,22 +3052,22 @@ int Stage3::run_once(const double* gt_points, const int* gt_tris, int n_gt_point
         cudaMemcpyAsync(inv_vs, vs_host_list.data(), vs_host_list.size() * sizeof(int), cudaMemcpyHostToDevice, s);
 
     // normalisation (processing.py:15-21, 57-59)
-    k_norm_partial<<<kNormBlocks, kT, 0, s>>>(gt_points, NGP, d_norm + 16);
+    pdl(k_norm_partial, kNormBlocks, kT, 0, s)(gt_points, NGP, d_norm + 16);
     note_launch();
-    k_norm_final<<<1, kT, 0, s>>>(d_norm + 16, kNormBlocks, NGP, d_norm);
+    pdl(k_norm_final, 1, kT, 0, s)(d_norm + 16, kNormBlocks, NGP, d_norm);
     note_launch();
-    k_normalize<<<grid_for(NGP, kT), kT, 0, s>>>(gt_points, NGP, d_norm, gt_pos, nullptr);
+    pdl(k_normalize<double>, grid_for(NGP, kT), kT, 0, s)(gt_points, NGP, d_norm, gt_pos, nullptr);
     note_launch();
     std::memset(h_sc, 0, sizeof(SolverScalars));
     h_sc->radius = params.contact_detection_radius;
     h_sc->rebuild = 1;  // candidate lists are built in the first iteration
     h_sc->barrier_extra = test_barrier_extra;
     cudaMemcpyAsync(sc, h_sc, sizeof(SolverScalars), cudaMemcpyHostToDevice, s);
-    k_tris4<<<grid_for(NGT, kT), kT, 0, s>>>(gt_tris, NGT, NGP, gt_tri, &sc->status);
+    pdl(k_tris4, grid_for(NGT, kT), kT, 0, s)(gt_tris, NGT, NGP, gt_tri, &sc->status);
     note_launch();
-    k_normalize<<<grid_for(NP, kT), kT, 0, s>>>(points, NP, d_norm, q, q_rest);
+    pdl(k_normalize<double>, grid_for(NP, kT), kT, 0, s)(points, NP, d_norm, q, q_rest);
     note_launch();
-    k_tris4<<<grid_for(NT, kT), kT, 0, s>>>(tris, NT, NP, tri, &sc->status);
+    pdl(k_tris4, grid_for(NT, kT), kT, 0, s)(tris, NT, NP, tri, &sc->status);
     note_launch();
     cudaMemcpyAsync(h_sc, sc, sizeof(SolverScalars), cudaMemcpyDeviceToHost, s);
     if (cudaStreamSynchronize(s) != cudaSuccess) return fail(PAMO_ERR_CUDA, cudaGetErrorString(cudaGetLastError()));
@@ -3059,17 +3094,17 @@ int Stage3::run_once(const double* gt_points, const int* gt_tris, int n_gt_point
     cudaMemsetAsync(wslot, 0, ((size_t)3 * NT + (size_t)4 * NH) * sizeof(double), s);
     // the triangle positions of hslot hold no Hessian part: zero for the whole call
     cudaMemsetAsync(hslot, 0, ((size_t)3 * NT + (size_t)4 * NH) * sizeof(float4), s);
-    k_voronoi<<<grid_for(NT, kT), kT, 0, s>>>(points, d_norm, tri, NT, inv_vs, wslot);
+    pdl(k_voronoi, grid_for(NT, kT), kT, 0, s)(points, d_norm, tri, NT, inv_vs, wslot);
     note_launch();
-    k_weights_f32<<<grid_for(NP, kT), kT, 0, s>>>(wslot, vs_off, NP, vweight);
+    pdl(k_weights_f32, grid_for(NP, kT), kT, 0, s)(wslot, vs_off, NP, vweight);
     note_launch();
-    k_elastic_pre<<<grid_for(NT, kT), kT, 0, s>>>(q_rest, tri, NT, el_area, el_invDm);
+    pdl(k_elastic_pre, grid_for(NT, kT), kT, 0, s)(q_rest, tri, NT, el_area, el_invDm);
     note_launch();
     if (NH) {
-        k_hinge_pre<<<grid_for(NH, kT), kT, 0, s>>>(q_rest, hinge, NH, hinge_rest);
+        pdl(k_hinge_pre, grid_for(NH, kT), kT, 0, s)(q_rest, hinge, NH, hinge_rest);
         note_launch();
     }
-    k_min_angle<<<grid_for(NT, kT), kT, 0, s>>>(points, d_norm, tri, NT, (double)params.min_angle_thres, &sc->accepted);
+    pdl(k_min_angle, grid_for(NT, kT), kT, 0, s)(points, d_norm, tri, NT, (double)params.min_angle_thres, &sc->accepted);
     note_launch();
     cudaMemcpyAsync(h_sc, sc, sizeof(SolverScalars), cudaMemcpyDeviceToHost, s);
     if (cudaStreamSynchronize(s) != cudaSuccess) return fail(PAMO_ERR_CUDA, cudaGetErrorString(cudaGetLastError()));
@@ -3099,7 +3134,7 @@ int Stage3::run_once(const double* gt_points, const int* gt_tris, int n_gt_point
         for (int step = 0; step < n_iters; ++step) {
             ++stats.steps;
             // _update_vertex_target: closest points on the GT surface
-            k_closest_gt<<<grid_for(NP, kQT, 16), kQT, 0, s>>>(q, NP, gt_bvh.child, gt_bvh.nlo, gt_bvh.nhi, gt_bvh.llo,
+            pdl(k_closest_gt, grid_for(NP, kQT, 16), kQT, 0, s)(q, NP, gt_bvh.child, gt_bvh.nlo, gt_bvh.nhi, gt_bvh.llo,
                                                               gt_bvh.lhi, gt_bvh.vals[0], gt_tri, gt_pos, gt_rc, target,
                                                               &sc->status);
             note_launch();
@@ -3142,7 +3177,7 @@ int Stage3::run_once(const double* gt_points, const int* gt_tris, int n_gt_point
         }
         stats.newton_iters = done;
     }
-    k_denormalize<<<grid_for(NP, kT), kT, 0, s>>>(q, NP, d_norm, out_points);
+    pdl(k_denormalize, grid_for(NP, kT), kT, 0, s)(q, NP, d_norm, out_points);
     note_launch();
     cudaMemcpyAsync(h_sc, sc, sizeof(SolverScalars), cudaMemcpyDeviceToHost, s);
     cudaEventRecord(ev_out, s);

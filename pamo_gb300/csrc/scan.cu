@@ -62,6 +62,7 @@ struct ScanJobs {
 };
 
 __global__ void __launch_bounds__(kThreads) k_scan(ScanJobs jobs, int* err) {
+    pdl_wait();
     const ScanJob& J = jobs.j[blockIdx.y];
     const int* in = J.in;
     int* out = J.out;
@@ -188,7 +189,7 @@ void exclusive_scans(const ScanJob* jobs, int count, cudaStream_t s, int* err, l
         const long long want = (n_bound + n_add + kPass - 1) / kPass;
         tiles = (int)(want < 1 ? 1 : (want > kScanTiles ? kScanTiles : want));
     }
-    k_scan<<<dim3(tiles, count), kThreads, 0, s>>>(all, err); note_launch();
+    pdl(k_scan, dim3(tiles, count), kThreads, 0, s)(all, err); note_launch();
 }
 
 void exclusive_scan(const int* in, int* out, const int* d_n, int n_add, int* d_total, int* scratch, cudaStream_t s,

@@ -27,6 +27,7 @@ constexpr float kU32MaxF = 4294967296.0f;      // (float)UINT32_MAX
 // ------------------------------------------------------------------ set-up
 __global__ void k_undo_stuck(const int* __restrict__ verts_undo, int n, int* tmp_undo, int* undo_list,
                              const int* __restrict__ pts_map, int map_len) {
+    pdl_wait();
     for (int a = gtid(); a < n; a += gstride()) {
         const int x = verts_undo[a];
         tmp_undo[a] = x;
@@ -35,6 +36,7 @@ __global__ void k_undo_stuck(const int* __restrict__ verts_undo, int n, int* tmp
 }
 
 __global__ void k_invalid_mark(const int* __restrict__ verts_undo, int n, unsigned char* invalid, int len) {
+    pdl_wait();
     for (int a = gtid(); a < n; a += gstride()) {
         const int x = verts_undo[a];
         if (x >= 0 && x < len) invalid[x] = 1;  // compute_invalid_vertices_table, :880-889
@@ -42,6 +44,7 @@ __global__ void k_invalid_mark(const int* __restrict__ verts_undo, int n, unsign
 }
 
 __global__ void k_load_points(const float* __restrict__ pts, int n, float4* pos, float4* orig, int* occ) {
+    pdl_wait();
     for (int v = gtid(); v < n; v += gstride()) {
         const float4 p = make_float4(pts[3 * v], pts[3 * v + 1], pts[3 * v + 2], 0.f);
         pos[v] = p;
@@ -52,6 +55,7 @@ __global__ void k_load_points(const float* __restrict__ pts, int n, float4* pos,
 }
 
 __global__ void k_load_points4(const float4* __restrict__ pts, int n, float4* pos, float4* orig, int* occ) {
+    pdl_wait();
     for (int v = gtid(); v < n; v += gstride()) {
         const float4 p = pts[v];
         pos[v] = p;
@@ -62,6 +66,7 @@ __global__ void k_load_points4(const float4* __restrict__ pts, int n, float4* po
 }
 
 __global__ void k_load_tris(const int* __restrict__ tris, int n, int n_pts, int4* tri, RoundCounters* rc) {
+    pdl_wait();
     for (int f = gtid(); f < n; f += gstride()) {
         const int a = tris[3 * f], b = tris[3 * f + 1], c = tris[3 * f + 2];
         const bool dead = (a == -1 && b == -1 && c == -1);
@@ -72,16 +77,19 @@ __global__ void k_load_tris(const int* __restrict__ tris, int n, int n_pts, int4
 }
 
 __global__ void k_copy4(const int4* __restrict__ src, int4* dst, int n) {
+    pdl_wait();
     for (int f = gtid(); f < n; f += gstride()) dst[f] = src[f];
 }
 
 __global__ void k_shuffle_flags(Feistel fb, int* flags) {
+    pdl_wait();
     const long long n = (long long)fb.n;
     for (long long i = gtid(); i < n; i += gstride()) flags[i] = feistel(fb, fb.size, (unsigned long long)i) < fb.m ? 1 : 0;
     if (gtid() == 0) flags[n] = 0;
 }
 
 __global__ void k_shuffle_gather(Feistel fb, const int* __restrict__ scan, const int4* __restrict__ src, int4* dst) {
+    pdl_wait();
     const long long n = (long long)fb.n;
     for (long long i = gtid(); i < n; i += gstride()) {
         const unsigned long long g = feistel(fb, fb.size, (unsigned long long)i);
@@ -194,6 +202,7 @@ __device__ __forceinline__ float acc_value(const CSum& a) { return a.value(); }
 __global__ void __launch_bounds__(kT) k_face_counts(const int4* __restrict__ tri, const RoundCounters* rc, int* valence,
                                                     int* ecount, int* vedges, const float4* __restrict__ pos,
                                                     float4* fgeo, int plane_df) {
+    pdl_wait();
     const int n = rc->n_tris;
     for (int f = gtid(); f < n; f += gstride()) {
         const int4 t = tri[f];
@@ -237,6 +246,7 @@ __global__ void __launch_bounds__(kT) k_fill_adjacency(const int4* __restrict__ 
                                                        const int* __restrict__ nt_off, int* cursor, int* nt,
                                                        const int* __restrict__ edge_off, int2* edges,
                                                        const int* __restrict__ voff, int* vcursor, int* eorder) {
+    pdl_wait();
     const int n = rc->n_tris;
     for (int f = gtid(); f < n; f += gstride()) {
         const int4 t = tri[f];
@@ -261,6 +271,7 @@ __global__ void __launch_bounds__(kT) k_fill_adjacency(const int4* __restrict__ 
 }
 
 __global__ void __launch_bounds__(kT) k_sort_adjacency(const RoundCounters* rc, const int* __restrict__ nt_off, int* nt) {
+    pdl_wait();
     const int n = rc->n_pts;
     for (int v = gtid(); v < n; v += gstride()) {
         const int a = nt_off[v], b = nt_off[v + 1];
@@ -296,6 +307,7 @@ __global__ void __launch_bounds__(kT) k_quadrics(const RoundCounters* rc, const 
                                                  const int* __restrict__ nt, const int4* __restrict__ tri,
                                                  const float4* __restrict__ fgeo, Quadric* q, int* nxt,
                                                  int2* spc, Quadric* qlo) {
+    pdl_wait();
     const int n = rc->n_pts;
     const size_t planes = 4 * (size_t)rc->n_tris;
     for (int v = gtid(); v < n; v += gstride()) {
@@ -634,8 +646,9 @@ __global__ void __launch_bounds__(kT) k_edge_cost(const RoundCounters* rc, const
                                                   uint32_t* cost, unsigned long long* vmin, const float* d_scale,
                                                   float tres, int is_stuck_host, const int* is_stuck_dev,
                                                   const int* __restrict__ vmesh, const int* __restrict__ mesh_stuck,
-                                                  float* raw_out = nullptr, float4* place_out = nullptr,
-                                                  const Quadric* __restrict__ qlo = nullptr) {
+                                                  float* raw_out, float4* place_out,
+                                                  const Quadric* __restrict__ qlo) {
+    pdl_wait();
     int is_stuck = 0;
     float scale = 0.0f;
     if constexpr (!kBatch) {
@@ -678,6 +691,7 @@ __global__ void __launch_bounds__(kT) k_edge_cost(const RoundCounters* rc, const
 }
 
 __global__ void k_edge_cost_capacity(RoundCounters* rc, int* d_cap) {
+    pdl_wait();
     const int n = rc->n_edges;
     int grow = 0;
     if (n > *d_cap) {
@@ -688,12 +702,14 @@ __global__ void k_edge_cost_capacity(RoundCounters* rc, int* d_cap) {
 }
 
 __global__ void k_edge_cost_zero(const RoundCounters* rc, uint32_t* cost, int len) {
+    pdl_wait();
     if (!rc->pad[0]) return;
     for (int i = gtid(); i < len; i += gstride()) cost[i] = 0u;
 }
 
 __global__ void __launch_bounds__(kT) k_face_keys(const RoundCounters* rc, const int4* __restrict__ tri,
                                                   const unsigned long long* __restrict__ vmin, unsigned long long* fkey) {
+    pdl_wait();
     const int n = rc->n_tris;
     for (int f = gtid(); f < n; f += gstride()) {
         const int4 t = tri[f];
@@ -737,7 +753,8 @@ __global__ void __launch_bounds__(kT) k_collapse(RoundCounters* rc, const int* _
                                                  const unsigned long long* __restrict__ fkey, const int* __restrict__ nt_off,
                                                  const int* __restrict__ nt, int4* tri, const int4* __restrict__ orig_tri,
                                                  float4* pos, const float4* __restrict__ orig_pos, int* occ, int* win,
-                                                 const float4* __restrict__ place = nullptr) {
+                                                 const float4* __restrict__ place) {
+    pdl_wait();
     const int n = rc->n_edges;
     if (gtid() == 0) win[n] = 0;
     for (int i = gtid(); i < n; i += gstride()) {
@@ -776,12 +793,13 @@ __global__ void __launch_bounds__(kT) k_collapse(RoundCounters* rc, const int* _
 }
 
 __global__ void k_compact_winners(const RoundCounters* rc, const int* __restrict__ scan, int* collapsed) {
+    pdl_wait();
     const int n = rc->n_edges;
     for (int e = gtid(); e < n; e += gstride())
         if (scan[e + 1] != scan[e]) collapsed[scan[e]] = e;
 }
 
-__global__ void __launch_bounds__(kT) k_remove_invalid(const RoundCounters* rc, int4* tri) {  // :218-232
+__global__ void __launch_bounds__(kT) k_remove_invalid(const RoundCounters* rc, int4* tri) { pdl_wait();  // :218-232
     const int n = rc->n_tris;
     for (int f = gtid(); f < n; f += gstride()) {
         const int4 t = tri[f];
@@ -791,6 +809,7 @@ __global__ void __launch_bounds__(kT) k_remove_invalid(const RoundCounters* rc, 
 }
 
 __global__ void __launch_bounds__(kT) k_line_detect(RoundCounters* rc, const int2* __restrict__ edges, const float4* pos) {
+    pdl_wait();
     const int n = rc->n_edges;
     int found = 0;
     for (int e = gtid(); e < n; e += gstride()) {
@@ -805,6 +824,7 @@ __global__ void __launch_bounds__(kT) k_line_detect(RoundCounters* rc, const int
 // then the collapsed-list bookkeeping of forward() (:1004-1016).
 __global__ void k_line_apply(RoundCounters* rc, const int2* __restrict__ edges, const int* __restrict__ nt_off,
                              const int* __restrict__ nt, int4* tri, float4* pos, int* occ, int* collapsed, int cap) {
+    pdl_wait();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     const int h = rc->n_win;
     int k = h;
@@ -832,6 +852,7 @@ __global__ void k_line_apply(RoundCounters* rc, const int2* __restrict__ edges, 
 // ------------------------------------------------------------------ rollback
 __global__ void k_mark_query(const RoundCounters* rc, const int* __restrict__ collapsed, const int2* __restrict__ edges,
                              const int* __restrict__ nt_off, const int* __restrict__ nt, int* qflag) {
+    pdl_wait();
     const int n = rc->n_considered;
     for (int c = gtid(); c < n; c += gstride()) {
         const int2 ed = edges[collapsed[c]];
@@ -841,6 +862,7 @@ __global__ void k_mark_query(const RoundCounters* rc, const int* __restrict__ co
 }
 
 __global__ void k_compact_flags(const int* __restrict__ scan, const int* d_n, int* out) {
+    pdl_wait();
     const int n = *d_n;
     for (int i = gtid(); i < n; i += gstride())
         if (scan[i + 1] != scan[i]) out[scan[i]] = i;
@@ -849,6 +871,7 @@ __global__ void k_compact_flags(const int* __restrict__ scan, const int* d_n, in
 __global__ void k_undo_check(RoundCounters* rc, const int* __restrict__ collapsed, const int2* __restrict__ edges,
                              const int* __restrict__ nt_off, const int* __restrict__ nt, const unsigned char* __restrict__ hit,
                              int* uflag) {
+    pdl_wait();
     const int n = rc->n_considered;
     if (gtid() == 0) uflag[n] = 0;
     for (int c = gtid(); c < n; c += gstride()) {
@@ -861,6 +884,7 @@ __global__ void k_undo_check(RoundCounters* rc, const int* __restrict__ collapse
 }
 
 __global__ void k_after_check(RoundCounters* rc) {
+    pdl_wait();
     const int nu = rc->n_undo;
     if (rc->passes < 8) rc->undo_per_pass[rc->passes] = nu;
     rc->passes += 1;
@@ -874,6 +898,7 @@ __global__ void k_undo_apply(RoundCounters* rc, const int* __restrict__ collapse
                              int4* tri, const int4* __restrict__ orig_tri, float4* pos, const float4* __restrict__ orig_pos,
                              int* occ, int* tmp_undo, int* undo_list, const int* __restrict__ pts_map, int map_len,
                              int list_cap) {
+    pdl_wait();
     const int n = rc->n_considered;
     const int first = rc->first_undo;
     for (int c = gtid(); c < n; c += gstride()) {
@@ -897,10 +922,11 @@ __global__ void k_undo_apply(RoundCounters* rc, const int* __restrict__ collapse
     }
 }
 
-__global__ void k_after_apply(RoundCounters* rc) { rc->first_undo += 2 * rc->n_undo; }
+__global__ void k_after_apply(RoundCounters* rc) { pdl_wait(); rc->first_undo += 2 * rc->n_undo; }
 
 // ------------------------------------------------------------------ outputs
 __global__ void k_live_flags(const RoundCounters* rc, const int4* __restrict__ tri, int* flags) {
+    pdl_wait();
     const int n = rc->n_tris;
     for (int f = gtid(); f < n; f += gstride()) flags[f] = (tri[f].x >= 0) ? 1 : 0;
     if (gtid() == 0) flags[n] = 0;
@@ -909,6 +935,7 @@ __global__ void k_live_flags(const RoundCounters* rc, const int4* __restrict__ t
 __global__ void k_compact_mesh(RoundCounters* rc, const float4* __restrict__ pos, const int* __restrict__ occ,
                                const int* __restrict__ pts_map, const int4* __restrict__ tri, const int* __restrict__ fscan,
                                float4* out_pos, int4* out_tri) {
+    pdl_wait();
     const int np = rc->n_pts, nf = rc->n_tris;
     for (int v = gtid(); v < np; v += gstride())
         if (occ[v]) out_pos[pts_map[v]] = pos[v];
@@ -926,6 +953,7 @@ __global__ void k_compact_mesh(RoundCounters* rc, const float4* __restrict__ pos
 __global__ void k_export_round(int np, int nf, const float4* __restrict__ pos, const int4* __restrict__ tri,
                                const int* __restrict__ occ, const int* __restrict__ pts_map, const int* __restrict__ undo,
                                float* verts, int* tris, int* vocc, int* vmap, int* vundo, int nu) {
+    pdl_wait();
     for (int v = gtid(); v < np; v += gstride()) {
         const float4 p = pos[v];
         verts[3 * v] = p.x;
@@ -946,6 +974,7 @@ __global__ void k_export_round(int np, int nf, const float4* __restrict__ pos, c
 
 __global__ void k_export_mesh(int np, int nf, const float4* __restrict__ pos, const int4* __restrict__ tri,
                               const float* __restrict__ add, float* verts, int* tris) {
+    pdl_wait();
     const float ax = add ? add[0] : 0.f, ay = add ? add[1] : 0.f, az = add ? add[2] : 0.f;
     for (int v = gtid(); v < np; v += gstride()) {
         const float4 p = pos[v];
@@ -968,6 +997,7 @@ __global__ void k_export_mesh(int np, int nf, const float4* __restrict__ pos, co
 // *ls = *next; the round's counters as forward() sets them (a stuck round starts its undo list with the
 // carried-over entries)
 __global__ void k_round_begin(RoundCounters* rc, LoopState* ls, const LoopState* next) {
+    pdl_wait();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     const LoopState L = *next;
     *ls = L;
@@ -983,6 +1013,7 @@ __global__ void k_round_begin(RoundCounters* rc, LoopState* ls, const LoopState*
 
 // not stuck and undo vertices carried in: the invalid table is cleared (cusimp_free.cu:905-908)
 __global__ void k_invalid_clear_dev(const LoopState* ls, unsigned char* invalid, int len) {
+    pdl_wait();
     if (ls->is_stuck || ls->nu == 0) return;
     for (int i = gtid(); i < len; i += gstride()) invalid[i] = 0;
 }
@@ -991,6 +1022,7 @@ __global__ void k_invalid_clear_dev(const LoopState* ls, unsigned char* invalid,
 // then the carried vertices are marked invalid (:880-889)
 __global__ void k_undo_book_dev(const int* __restrict__ verts_undo, const LoopState* ls, int* tmp_undo, int* undo_list,
                                 const int* __restrict__ pts_map, int map_len, unsigned char* invalid, int len) {
+    pdl_wait();
     const int n = ls->nu;
     const bool stuck = ls->is_stuck != 0;
     for (int a = gtid(); a < n; a += gstride()) {
@@ -1008,6 +1040,7 @@ __global__ void k_round_prologue_dev(const LoopState* ls, const RoundCounters* r
                                      int* pts_map_prev, const float4* __restrict__ pts_in, float4* pos, float4* orig_pos,
                                      int* occ, const int4* __restrict__ tri_in, int4* tri, int4* orig_tri, int* valence,
                                      int* cursor, int* vedges, int* vcursor, int* qflag) {
+    pdl_wait();
     const int nm = ls->np, np = rc->n_pts, nf = rc->n_tris;
     const int n = max(max(nm, np + 1), nf + 1);
     for (int i = gtid(); i < n; i += gstride()) {
@@ -1031,11 +1064,13 @@ __global__ void k_round_prologue_dev(const LoopState* ls, const RoundCounters* r
 }
 
 __global__ void k_fill_u64_dev(const RoundCounters* rc, unsigned long long* p, unsigned long long v) {
+    pdl_wait();
     const int n = rc->n_pts + 1;
     for (int i = gtid(); i < n; i += gstride()) p[i] = v;
 }
 
 __global__ void k_zero_face_bytes_dev(const RoundCounters* rc, unsigned char* p) {
+    pdl_wait();
     const int n = rc->n_tris + 1;
     for (int i = gtid(); i < n; i += gstride()) p[i] = 0;
 }
@@ -1043,6 +1078,7 @@ __global__ void k_zero_face_bytes_dev(const RoundCounters* rc, unsigned char* p)
 // After compaction: the next round's state (pamo/__init__.py:131-159: sizes, undo vertices, the no-progress
 // count and is_stuck) computed from this round's start state; recomputing it after an undo pass is harmless.
 __global__ void k_round_end(const RoundCounters* rc, const LoopState* ls, LoopState* next) {
+    pdl_wait();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     LoopState L = *ls;
     const int nf = rc->n_tris_out;
@@ -1063,6 +1099,7 @@ __global__ void k_round_end(const RoundCounters* rc, const LoopState* ls, LoopSt
 // overwrites pts_map before an undo pass may follow); undo entries index it with this round's vertex ids (< np)
 // undo vertices carried to the next round (the host loop's copy of the previous undo list)
 __global__ void k_copy_undo_dev(const RoundCounters* rc, const int* __restrict__ src, int* dst, int cap) {
+    pdl_wait();
     const int n = min(rc->n_vertices_undo, cap);
     for (int i = gtid(); i < n; i += gstride()) dst[i] = src[i];
 }
@@ -1087,64 +1124,64 @@ void launch_undo_bookkeeping(const int* verts_undo, int n_verts_undo, int is_stu
                              const int* pts_map, int pts_map_len, unsigned char* invalid, int invalid_len, cudaStream_t s) {
     if (is_stuck) {
         if (n_verts_undo > 0)
-            k_undo_stuck<<<grid_for(n_verts_undo, kT), kT, 0, s>>>(verts_undo, n_verts_undo, tmp_undo, undo_list, pts_map,
+            pdl(k_undo_stuck, grid_for(n_verts_undo, kT), kT, 0, s)(verts_undo, n_verts_undo, tmp_undo, undo_list, pts_map,
                                                                    pts_map_len); note_launch();
     } else if (n_verts_undo != 0) {
         cudaMemsetAsync(invalid, 0, invalid_len, s);
     }
     if (n_verts_undo > 0)
-        k_invalid_mark<<<grid_for(n_verts_undo, kT), kT, 0, s>>>(verts_undo, n_verts_undo, invalid, invalid_len); note_launch();
+        pdl(k_invalid_mark, grid_for(n_verts_undo, kT), kT, 0, s)(verts_undo, n_verts_undo, invalid, invalid_len); note_launch();
 }
 
 void launch_load_points(const float* pts, int n, float4* pos, float4* orig_pos, int* occ, cudaStream_t s) {
-    k_load_points<<<grid_for(n, kT), kT, 0, s>>>(pts, n, pos, orig_pos, occ); note_launch();
+    pdl(k_load_points, grid_for(n, kT), kT, 0, s)(pts, n, pos, orig_pos, occ); note_launch();
 }
 void launch_load_points4(const float4* pts, int n, float4* pos, float4* orig_pos, int* occ, cudaStream_t s) {
-    k_load_points4<<<grid_for(n, kT), kT, 0, s>>>(pts, n, pos, orig_pos, occ); note_launch();
+    pdl(k_load_points4, grid_for(n, kT), kT, 0, s)(pts, n, pos, orig_pos, occ); note_launch();
 }
 void launch_load_tris(const int* tris, int n, int n_pts, int4* tri, RoundCounters* rc, cudaStream_t s) {
-    k_load_tris<<<grid_for(n, kT), kT, 0, s>>>(tris, n, n_pts, tri, rc); note_launch();
+    pdl(k_load_tris, grid_for(n, kT), kT, 0, s)(tris, n, n_pts, tri, rc); note_launch();
 }
 void launch_load_tris4(const int4* tris, int n, int4* tri, cudaStream_t s) {
-    k_copy4<<<grid_for(n, kT), kT, 0, s>>>(tris, tri, n); note_launch();
+    pdl(k_copy4, grid_for(n, kT), kT, 0, s)(tris, tri, n); note_launch();
 }
 void launch_copy_tris(const int4* src, int4* dst, int n, cudaStream_t s) {
-    k_copy4<<<grid_for(n, kT), kT, 0, s>>>(src, dst, n); note_launch();
+    pdl(k_copy4, grid_for(n, kT), kT, 0, s)(src, dst, n); note_launch();
 }
 void launch_shuffle_tris(const Feistel& fb, int* flags, int* scan_scratch, int4* src, int4* dst, int n, cudaStream_t s,
                          int* err) {
     (void)n;
     const int g = grid_for((long long)fb.n, kT);
-    k_shuffle_flags<<<g, kT, 0, s>>>(fb, flags); note_launch();
+    pdl(k_shuffle_flags, g, kT, 0, s)(fb, flags); note_launch();
     exclusive_scan(flags, flags, nullptr, (int)fb.n + 1, nullptr, scan_scratch, s, err, 0);
-    k_shuffle_gather<<<g, kT, 0, s>>>(fb, flags, src, dst); note_launch();
+    pdl(k_shuffle_gather, g, kT, 0, s)(fb, flags, src, dst); note_launch();
 }
 
 void launch_face_counts(const int4* tri, const RoundCounters* rc, int n_tris_bound, int* valence, int* ecount,
                         int* vedges, cudaStream_t s, const float4* pos, float4* fgeo, bool plane_df) {
-    k_face_counts<<<grid_for(n_tris_bound, kT), kT, 0, s>>>(tri, rc, valence, ecount, vedges, pos, fgeo,
+    pdl(k_face_counts, grid_for(n_tris_bound, kT), kT, 0, s)(tri, rc, valence, ecount, vedges, pos, fgeo,
                                                             plane_df ? 1 : 0);
     note_launch();
 }
 void launch_fill_adjacency(const int4* tri, const RoundCounters* rc, int n_tris_bound, const int* nt_off, int* cursor,
                            int* nt, const int* edge_off, int2* edges, const int* voff, int* vcursor, int* eorder,
                            cudaStream_t s) {
-    k_fill_adjacency<<<grid_for(n_tris_bound, kT), kT, 0, s>>>(tri, rc, nt_off, cursor, nt, edge_off, edges, voff, vcursor,
+    pdl(k_fill_adjacency, grid_for(n_tris_bound, kT), kT, 0, s)(tri, rc, nt_off, cursor, nt, edge_off, edges, voff, vcursor,
                                                                eorder);
     note_launch();
 }
 void launch_sort_adjacency(const RoundCounters* rc, int n_pts_bound, const int* nt_off, int* nt, cudaStream_t s) {
-    k_sort_adjacency<<<grid_for(n_pts_bound, kT), kT, 0, s>>>(rc, nt_off, nt); note_launch();
+    pdl(k_sort_adjacency, grid_for(n_pts_bound, kT), kT, 0, s)(rc, nt_off, nt); note_launch();
 }
 void launch_quadrics(const RoundCounters* rc, int n_pts_bound, const int* nt_off, const int* nt, const int4* tri,
                      const float4* fgeo, Quadric* q, int* nxt, int2* spc, cudaStream_t s, Quadric* qlo) {
-    if (qlo) k_quadrics<true><<<grid_for(n_pts_bound, kT), kT, 0, s>>>(rc, nt_off, nt, tri, fgeo, q, nxt, spc, qlo);
-    else k_quadrics<false><<<grid_for(n_pts_bound, kT), kT, 0, s>>>(rc, nt_off, nt, tri, fgeo, q, nxt, spc, nullptr);
+    if (qlo) pdl(k_quadrics<true>, grid_for(n_pts_bound, kT), kT, 0, s)(rc, nt_off, nt, tri, fgeo, q, nxt, spc, qlo);
+    else pdl(k_quadrics<false>, grid_for(n_pts_bound, kT), kT, 0, s)(rc, nt_off, nt, tri, fgeo, q, nxt, spc, nullptr);
     note_launch();
 }
 void launch_edge_cost_capacity(RoundCounters* rc, int* d_cap, uint32_t* edge_cost, int phys_len, cudaStream_t s) {
-    k_edge_cost_capacity<<<1, 1, 0, s>>>(rc, d_cap); note_launch();
-    k_edge_cost_zero<<<grid_for(phys_len, kT), kT, 0, s>>>(rc, edge_cost, phys_len); note_launch();
+    pdl(k_edge_cost_capacity, 1, 1, 0, s)(rc, d_cap); note_launch();
+    pdl(k_edge_cost_zero, grid_for(phys_len, kT), kT, 0, s)(rc, edge_cost, phys_len); note_launch();
 }
 void launch_edge_cost(const RoundCounters* rc, int n_edges_bound, const int* eorder, const int2* edges, const int* nt_off,
                       const int* nt, const int4* tri, const float4* pos, const Quadric* q, const float4* fgeo,
@@ -1154,7 +1191,7 @@ void launch_edge_cost(const RoundCounters* rc, int n_edges_bound, const int* eor
                       bool device_pow, int mode, float* raw, float4* place, const Quadric* qlo) {
     const int g = grid_for(n_edges_bound, kT);
 #define PAMO_COST_MODE(M, P, O)                                                                                      \
-    k_edge_cost<false, P, false, M, O><<<g, kT, 0, s>>>(rc, eorder, edges, nt_off, nt, tri, pos, q, fgeo, nxt,       \
+    pdl(k_edge_cost<false, P, false, M, O>, g, kT, 0, s)(rc, eorder, edges, nt_off, nt, tri, pos, q, fgeo, nxt,       \
                                                         spc, invalid, cost, vmin, d_scale, tres, is_stuck, is_stuck_dev,  \
                                                         nullptr, nullptr, raw, place, qlo)
     if (!legacy && mode == 1) {
@@ -1183,19 +1220,19 @@ void launch_edge_cost(const RoundCounters* rc, int n_edges_bound, const int* eor
 #undef PAMO_COST_MODE
     if (legacy) {
         if (device_pow)
-            k_edge_cost<true, true, false><<<g, kT, 0, s>>>(rc, eorder, edges, nt_off, nt, tri, pos, q, fgeo, nxt, spc, invalid,
-                                                            cost, vmin, d_scale, tres, 0, nullptr, nullptr, nullptr);
+            pdl(k_edge_cost<true, true, false>, g, kT, 0, s)(rc, eorder, edges, nt_off, nt, tri, pos, q, fgeo, nxt, spc, invalid,
+                                                            cost, vmin, d_scale, tres, 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
         else
-            k_edge_cost<true, false, false><<<g, kT, 0, s>>>(rc, eorder, edges, nt_off, nt, tri, pos, q, fgeo, nxt, spc, invalid,
-                                                             cost, vmin, d_scale, tres, 0, nullptr, nullptr, nullptr);
+            pdl(k_edge_cost<true, false, false>, g, kT, 0, s)(rc, eorder, edges, nt_off, nt, tri, pos, q, fgeo, nxt, spc, invalid,
+                                                             cost, vmin, d_scale, tres, 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
     } else if (device_pow) {
-        k_edge_cost<false, true, false><<<g, kT, 0, s>>>(rc, eorder, edges, nt_off, nt, tri, pos, q, fgeo, nxt, spc, invalid,
+        pdl(k_edge_cost<false, true, false>, g, kT, 0, s)(rc, eorder, edges, nt_off, nt, tri, pos, q, fgeo, nxt, spc, invalid,
                                                          cost, vmin, d_scale, tres, is_stuck, is_stuck_dev, nullptr,
-                                                         nullptr);
+                                                         nullptr, nullptr, nullptr, nullptr);
     } else {
-        k_edge_cost<false, false, false><<<g, kT, 0, s>>>(rc, eorder, edges, nt_off, nt, tri, pos, q, fgeo, nxt, spc, invalid,
+        pdl(k_edge_cost<false, false, false>, g, kT, 0, s)(rc, eorder, edges, nt_off, nt, tri, pos, q, fgeo, nxt, spc, invalid,
                                                           cost, vmin, d_scale, tres, is_stuck, is_stuck_dev, nullptr,
-                                                          nullptr);
+                                                          nullptr, nullptr, nullptr, nullptr);
     }
     note_launch();
 }
@@ -1207,104 +1244,106 @@ void launch_edge_cost_batch(const RoundCounters* rc, int n_edges_bound, const in
                             float tres, cudaStream_t s, bool device_pow) {
     const int g = grid_for(n_edges_bound, kT);
     if (device_pow)
-        k_edge_cost<false, true, true><<<g, kT, 0, s>>>(rc, eorder, edges, nt_off, nt, tri, pos, q, fgeo, nxt, spc, invalid,
-                                                        cost, vmin, mesh_scale, tres, 0, nullptr, vmesh, mesh_stuck);
+        pdl(k_edge_cost<false, true, true>, g, kT, 0, s)(rc, eorder, edges, nt_off, nt, tri, pos, q, fgeo, nxt, spc, invalid,
+                                                        cost, vmin, mesh_scale, tres, 0, nullptr, vmesh, mesh_stuck, nullptr, nullptr,
+                                                        nullptr);
     else
-        k_edge_cost<false, false, true><<<g, kT, 0, s>>>(rc, eorder, edges, nt_off, nt, tri, pos, q, fgeo, nxt, spc, invalid,
-                                                         cost, vmin, mesh_scale, tres, 0, nullptr, vmesh, mesh_stuck);
+        pdl(k_edge_cost<false, false, true>, g, kT, 0, s)(rc, eorder, edges, nt_off, nt, tri, pos, q, fgeo, nxt, spc, invalid,
+                                                         cost, vmin, mesh_scale, tres, 0, nullptr, vmesh, mesh_stuck, nullptr, nullptr,
+                                                        nullptr);
     note_launch();
 }
 void launch_face_keys(const RoundCounters* rc, int n_tris_bound, const int4* tri, const unsigned long long* vmin,
                       unsigned long long* fkey, cudaStream_t s) {
-    k_face_keys<<<grid_for(n_tris_bound, kT), kT, 0, s>>>(rc, tri, vmin, fkey); note_launch();
+    pdl(k_face_keys, grid_for(n_tris_bound, kT), kT, 0, s)(rc, tri, vmin, fkey); note_launch();
 }
 void launch_collapse(RoundCounters* rc, int n_edges_bound, const int* eorder, const int2* edges, const uint32_t* cost,
                      uint32_t collapse_t, const unsigned long long* fkey, const int* nt_off, const int* nt, int4* tri,
                      const int4* orig_tri, float4* pos, const float4* orig_pos, int* occ, int* win, cudaStream_t s,
                      bool restore, const float4* place) {
     if (restore && place)
-        k_collapse<true, true><<<grid_for(n_edges_bound, kT), kT, 0, s>>>(rc, eorder, edges, cost, collapse_t, fkey,
+        pdl(k_collapse<true, true>, grid_for(n_edges_bound, kT), kT, 0, s)(rc, eorder, edges, cost, collapse_t, fkey,
                                                                           nt_off, nt, tri, orig_tri, pos, orig_pos, occ,
                                                                           win, place);
     else if (restore)
-        k_collapse<true><<<grid_for(n_edges_bound, kT), kT, 0, s>>>(rc, eorder, edges, cost, collapse_t, fkey, nt_off, nt,
-                                                                    tri, orig_tri, pos, orig_pos, occ, win);
+        pdl(k_collapse<true>, grid_for(n_edges_bound, kT), kT, 0, s)(rc, eorder, edges, cost, collapse_t, fkey, nt_off, nt,
+                                                                    tri, orig_tri, pos, orig_pos, occ, win, nullptr);
     else
-        k_collapse<false><<<grid_for(n_edges_bound, kT), kT, 0, s>>>(rc, eorder, edges, cost, collapse_t, fkey, nt_off, nt,
-                                                                     tri, orig_tri, pos, orig_pos, occ, win);
+        pdl(k_collapse<false>, grid_for(n_edges_bound, kT), kT, 0, s)(rc, eorder, edges, cost, collapse_t, fkey, nt_off, nt,
+                                                                     tri, orig_tri, pos, orig_pos, occ, win, nullptr);
     note_launch();
 }
 void launch_compact_winners(const RoundCounters* rc, int n_edges_bound, const int* win_scan, int* collapsed,
                             cudaStream_t s) {
-    k_compact_winners<<<grid_for(n_edges_bound, kT), kT, 0, s>>>(rc, win_scan, collapsed); note_launch();
+    pdl(k_compact_winners, grid_for(n_edges_bound, kT), kT, 0, s)(rc, win_scan, collapsed); note_launch();
 }
 void launch_remove_invalid(const RoundCounters* rc, int n_tris_bound, int4* tri, cudaStream_t s) {
-    k_remove_invalid<<<grid_for(n_tris_bound, kT), kT, 0, s>>>(rc, tri); note_launch();
+    pdl(k_remove_invalid, grid_for(n_tris_bound, kT), kT, 0, s)(rc, tri); note_launch();
 }
 void launch_line_edges(RoundCounters* rc, int n_edges_bound, const int2* edges, const int* nt_off, const int* nt,
                        int4* tri, float4* pos, int* occ, int* line_buf, int line_cap, int* collapsed, cudaStream_t s) {
     (void)line_buf;
-    k_line_detect<<<grid_for(n_edges_bound, kT), kT, 0, s>>>(rc, edges, pos); note_launch();
-    k_line_apply<<<1, 32, 0, s>>>(rc, edges, nt_off, nt, tri, pos, occ, collapsed, line_cap); note_launch();
+    pdl(k_line_detect, grid_for(n_edges_bound, kT), kT, 0, s)(rc, edges, pos); note_launch();
+    pdl(k_line_apply, 1, 32, 0, s)(rc, edges, nt_off, nt, tri, pos, occ, collapsed, line_cap); note_launch();
 }
 void launch_line_detect(RoundCounters* rc, int n_edges_bound, const int2* edges, const float4* pos, cudaStream_t s) {
-    k_line_detect<<<grid_for(n_edges_bound, kT), kT, 0, s>>>(rc, edges, pos); note_launch();
+    pdl(k_line_detect, grid_for(n_edges_bound, kT), kT, 0, s)(rc, edges, pos); note_launch();
 }
 void launch_mark_query(const RoundCounters* rc, int n_edges_bound, const int* collapsed, const int2* edges,
                        const int* nt_off, const int* nt, int* qflag, cudaStream_t s) {
-    k_mark_query<<<grid_for(n_edges_bound, kT), kT, 0, s>>>(rc, collapsed, edges, nt_off, nt, qflag); note_launch();
+    pdl(k_mark_query, grid_for(n_edges_bound, kT), kT, 0, s)(rc, collapsed, edges, nt_off, nt, qflag); note_launch();
 }
 void launch_compact_flags(const int* scan, int n_bound, const int* d_n, int* out_list, cudaStream_t s) {
-    k_compact_flags<<<grid_for(n_bound, kT), kT, 0, s>>>(scan, d_n, out_list); note_launch();
+    pdl(k_compact_flags, grid_for(n_bound, kT), kT, 0, s)(scan, d_n, out_list); note_launch();
 }
 void launch_undo_check(RoundCounters* rc, int n_edges_bound, const int* collapsed, const int2* edges, const int* nt_off,
                        const int* nt, const unsigned char* hit, int* uflag, cudaStream_t s) {
-    k_undo_check<<<grid_for(n_edges_bound, kT), kT, 0, s>>>(rc, collapsed, edges, nt_off, nt, hit, uflag); note_launch();
+    pdl(k_undo_check, grid_for(n_edges_bound, kT), kT, 0, s)(rc, collapsed, edges, nt_off, nt, hit, uflag); note_launch();
 }
 void launch_undo_apply(RoundCounters* rc, int n_edges_bound, const int* collapsed, const int* uscan, const int2* edges,
                        const int* nt_off, const int* nt, int4* tri, const int4* orig_tri, float4* pos,
                        const float4* orig_pos, int* occ, int* tmp_undo, int* undo_list, const int* pts_map,
                        int list_cap, cudaStream_t s) {
-    k_undo_apply<<<grid_for(n_edges_bound, kT), kT, 0, s>>>(rc, collapsed, uscan, edges, nt_off, nt, tri, orig_tri, pos,
+    pdl(k_undo_apply, grid_for(n_edges_bound, kT), kT, 0, s)(rc, collapsed, uscan, edges, nt_off, nt, tri, orig_tri, pos,
                                                             orig_pos, occ, tmp_undo, undo_list, pts_map, list_cap, list_cap); note_launch();
-    k_after_apply<<<1, 1, 0, s>>>(rc); note_launch();
+    pdl(k_after_apply, 1, 1, 0, s)(rc); note_launch();
 }
 void launch_after_check(RoundCounters* rc, cudaStream_t s) {
-    k_after_check<<<1, 1, 0, s>>>(rc); note_launch();
+    pdl(k_after_check, 1, 1, 0, s)(rc); note_launch();
 }
 
 void launch_live_flags(const RoundCounters* rc, int n_tris_bound, const int4* tri, int* flags, cudaStream_t s) {
-    k_live_flags<<<grid_for(n_tris_bound, kT), kT, 0, s>>>(rc, tri, flags); note_launch();
+    pdl(k_live_flags, grid_for(n_tris_bound, kT), kT, 0, s)(rc, tri, flags); note_launch();
 }
 void launch_compact_mesh(RoundCounters* rc, int n_pts_bound, int n_tris_bound, const float4* pos, const int* occ,
                          const int* pts_map, const int4* tri, const int* face_scan, float4* out_pos, int4* out_tri,
                          cudaStream_t s) {
     const int n = n_pts_bound > n_tris_bound ? n_pts_bound : n_tris_bound;
-    k_compact_mesh<<<grid_for(n, kT), kT, 0, s>>>(rc, pos, occ, pts_map, tri, face_scan, out_pos, out_tri); note_launch();
+    pdl(k_compact_mesh, grid_for(n, kT), kT, 0, s)(rc, pos, occ, pts_map, tri, face_scan, out_pos, out_tri); note_launch();
 }
 void launch_export_round(const RoundCounters* rc, int n_pts, int n_tris, const float4* pos, const int4* tri,
                          const int* occ, const int* pts_map, const int* undo_list, float* verts, int* tris,
                          int* verts_occ, int* verts_map, int* verts_undo, int n_undo, cudaStream_t s) {
     (void)rc;
     const int n = n_pts > n_tris ? n_pts : n_tris;
-    k_export_round<<<grid_for(n, kT), kT, 0, s>>>(n_pts, n_tris, pos, tri, occ, pts_map, undo_list, verts, tris, verts_occ,
+    pdl(k_export_round, grid_for(n, kT), kT, 0, s)(n_pts, n_tris, pos, tri, occ, pts_map, undo_list, verts, tris, verts_occ,
                                                   verts_map, verts_undo, n_undo); note_launch();
 }
 void launch_export_mesh(int n_pts, int n_tris, const float4* pos, const int4* tri, const float* add, float* verts,
                         int* tris, cudaStream_t s) {
     const int n = n_pts > n_tris ? n_pts : n_tris;
-    k_export_mesh<<<grid_for(n, kT), kT, 0, s>>>(n_pts, n_tris, pos, tri, add, verts, tris); note_launch();
+    pdl(k_export_mesh, grid_for(n, kT), kT, 0, s)(n_pts, n_tris, pos, tri, add, verts, tris); note_launch();
 }
 
 // ---- device-driven rounds ----
 void launch_round_begin(RoundCounters* rc, LoopState* ls, const LoopState* next, cudaStream_t s) {
-    k_round_begin<<<1, 32, 0, s>>>(rc, ls, next); note_launch();
+    pdl(k_round_begin, 1, 32, 0, s)(rc, ls, next); note_launch();
 }
 void launch_undo_bookkeeping_dev(const int* verts_undo, const LoopState* ls, int n_undo_bound, int* tmp_undo,
                                  int* undo_list, const int* pts_map, int pts_map_len, unsigned char* invalid,
                                  int invalid_len, cudaStream_t s) {
-    k_invalid_clear_dev<<<grid_for(invalid_len, kT), kT, 0, s>>>(ls, invalid, invalid_len); note_launch();
-    k_undo_book_dev<<<grid_for(n_undo_bound, kT), kT, 0, s>>>(verts_undo, ls, tmp_undo, undo_list, pts_map, pts_map_len,
+    pdl(k_invalid_clear_dev, grid_for(invalid_len, kT), kT, 0, s)(ls, invalid, invalid_len); note_launch();
+    pdl(k_undo_book_dev, grid_for(n_undo_bound, kT), kT, 0, s)(verts_undo, ls, tmp_undo, undo_list, pts_map, pts_map_len,
                                                              invalid, invalid_len); note_launch();
 }
 void launch_round_prologue_dev(const LoopState* ls, const RoundCounters* rc, int n_pts_bound, int n_tris_bound,
@@ -1312,21 +1351,21 @@ void launch_round_prologue_dev(const LoopState* ls, const RoundCounters* rc, int
                                float4* orig_pos, int* occ, const int4* tri_in, int4* tri, int4* orig_tri, int* valence,
                                int* cursor, int* vedges, int* vcursor, int* qflag, cudaStream_t s) {
     const int n = (n_pts_bound > n_tris_bound ? n_pts_bound : n_tris_bound) + 1;
-    k_round_prologue_dev<<<grid_for(n, kT), kT, 0, s>>>(ls, rc, pts_map, pts_map_prev, pts_in, pos, orig_pos, occ, tri_in,
+    pdl(k_round_prologue_dev, grid_for(n, kT), kT, 0, s)(ls, rc, pts_map, pts_map_prev, pts_in, pos, orig_pos, occ, tri_in,
                                                         tri, orig_tri, valence, cursor, vedges, vcursor, qflag);
     note_launch();
 }
 void launch_fill_u64_dev(const RoundCounters* rc, int n_pts_bound, unsigned long long* p, unsigned long long v,
                          cudaStream_t s) {
-    k_fill_u64_dev<<<grid_for(n_pts_bound + 1, kT), kT, 0, s>>>(rc, p, v); note_launch();
+    pdl(k_fill_u64_dev, grid_for(n_pts_bound + 1, kT), kT, 0, s)(rc, p, v); note_launch();
 }
 void launch_zero_face_bytes_dev(const RoundCounters* rc, int n_tris_bound, unsigned char* p, cudaStream_t s) {
-    k_zero_face_bytes_dev<<<grid_for(n_tris_bound + 1, kT), kT, 0, s>>>(rc, p); note_launch();
+    pdl(k_zero_face_bytes_dev, grid_for(n_tris_bound + 1, kT), kT, 0, s)(rc, p); note_launch();
 }
 void launch_round_end(const RoundCounters* rc, const LoopState* ls, LoopState* next, const int* undo_list, int* undo_in,
                       int undo_cap, int n_undo_bound, cudaStream_t s) {
-    k_round_end<<<1, 32, 0, s>>>(rc, ls, next); note_launch();
-    k_copy_undo_dev<<<grid_for(n_undo_bound, kT), kT, 0, s>>>(rc, undo_list, undo_in, undo_cap); note_launch();
+    pdl(k_round_end, 1, 32, 0, s)(rc, ls, next); note_launch();
+    pdl(k_copy_undo_dev, grid_for(n_undo_bound, kT), kT, 0, s)(rc, undo_list, undo_in, undo_cap); note_launch();
 }
 
 }  // namespace pamo
