@@ -577,7 +577,7 @@ struct pamo_csr {
     Buf<unsigned long long> vmin;
     Buf<unsigned char> invalid;
     Buf<int4> tri, orig_tri, tri_in, tri_next, res_tri, tri_load;
-    Buf<int> ecount, qflag, qlist, fflags, nt, nxt, fmesh, shuffle_flags;
+    Buf<int> ecount, qflag, fflags, nt, nxt, fmesh, shuffle_flags;
     Buf<int2> spc;
     Buf<float4> fgeo;
     Buf<float> face_mean;
@@ -603,7 +603,6 @@ struct pamo_csr {
     RoundCounters* rc = nullptr;
     BatchCtl* ctl = nullptr;
     BatchCtl* h_ctl = nullptr;
-    LoopState* zero_ls = nullptr;
     int* scan_scratch = nullptr;
     std::vector<int> rounds;
     std::vector<BatchMesh> h_mesh;
@@ -652,8 +651,6 @@ struct pamo_csr {
         if ((r = check(cudaMalloc((void**)&rc, sizeof(RoundCounters)), "cudaMalloc"))) return r;
         if ((r = check(cudaMalloc((void**)&ctl, sizeof(BatchCtl)), "cudaMalloc"))) return r;
         if ((r = check(cudaMallocHost((void**)&h_ctl, sizeof(BatchCtl)), "cudaMallocHost"))) return r;
-        if ((r = check(cudaMalloc((void**)&zero_ls, sizeof(LoopState)), "cudaMalloc"))) return r;
-        cudaMemset(zero_ls, 0, sizeof(LoopState));
         if ((r = check(cudaMalloc((void**)&scan_scratch, kMaxScanJobs * scan_scratch_ints() * sizeof(int)), "cudaMalloc")))
             return r;
         for (int k = 0; k < kMaxScanJobs; ++k)
@@ -668,7 +665,7 @@ struct pamo_csr {
         release(occ); release(valence); release(cursor); release(vedges); release(vcursor); release(vmesh);
         release(vscan); release(quad); release(vmin); release(invalid); release(tri); release(orig_tri);
         release(tri_in); release(tri_next); release(res_tri); release(tri_load); release(ecount); release(qflag);
-        release(qlist); release(fflags); release(nt); release(nxt); release(spc); release(fmesh); release(shuffle_flags);
+        release(fflags); release(nt); release(nxt); release(spc); release(fmesh); release(shuffle_flags);
         release(fgeo); release(face_mean); release(fkey); release(hit); release(edges); release(exact_list);
         release(eorder); release(win); release(winners); release(lines); release(considered); release(uflag);
         release(cost); release(map_reg); release(undo_list_reg); release(tmp_undo_reg); release(undo_in_reg);
@@ -681,7 +678,6 @@ struct pamo_csr {
         if (rc) cudaFree(rc);
         if (ctl) cudaFree(ctl);
         if (h_ctl) cudaFreeHost(h_ctl);
-        if (zero_ls) cudaFree(zero_ls);
         if (scan_scratch) cudaFree(scan_scratch);
         rc = nullptr;
     }
@@ -697,7 +693,7 @@ struct pamo_csr {
             return r;
         if ((r = grow(tri, fc)) || (r = grow(orig_tri, fc)) || (r = grow(tri_in, fc)) || (r = grow(tri_next, fc)) ||
             (r = grow(res_tri, fc)) || (r = grow(tri_load, fc)) || (r = grow(ecount, fc + 1)) ||
-            (r = grow(qflag, fc + 1)) || (r = grow(qlist, fc)) || (r = grow(fflags, fc + 1)) || (r = grow(nt, 3 * fc)) ||
+            (r = grow(qflag, fc + 1)) || (r = grow(fflags, fc + 1)) || (r = grow(nt, 3 * fc)) ||
             (r = grow(nxt, 3 * fc)) || (r = grow(spc, 3 * fc)) || (r = grow(fmesh, fc)) ||
             (r = grow(fgeo, 6 * fc)) || (r = grow(face_mean, 3 * fc)) || (r = grow(fkey, fc)) || (r = grow(hit, fc + 1)))
             return r;
@@ -748,9 +744,9 @@ struct pamo_csr {
     // one intersection check over the meshes being checked, then their undo counts (kb_after_check)
     void check_pass(int Vb, int Fb, int Eb, int M, const BvhMeshes& bm) {
         cudaStream_t s = stream;
-        launch_zero_face_bytes_dev(rc, Fb, hit.p, s);
-        bvh_build(bvh, tri.p, pos.p, rc, Fb, s, false, qflag.p, false, &bm);
-        bvh_query(bvh, tri.p, pos.p, qlist.p, qflag.p, hit.p, exact_list.p, (int)exact_list.n, rc, Fb, kTriEpsB, s,
+        const BvhQuery query{qflag.p, hit.p};
+        bvh_build(bvh, tri.p, pos.p, rc, Fb, s, false, query, false, &bm);
+        bvh_query(bvh, tri.p, pos.p, query, exact_list.p, (int)exact_list.n, rc, Fb, kTriEpsB, s,
                   fmesh.p, mesh_root.p);
         launch_undo_check(rc, Eb, considered.p, edges.p, valence.p, nt.p, hit.p, uflag.p, s);
         exclusive_scan(uflag.p, uflag.p, &rc->n_considered, 1, &rc->n_undo, scan_scratch, s, &rc->status, Eb);
@@ -770,8 +766,13 @@ struct pamo_csr {
         pdl(kb_fill_slots, gM, kT, 0, s)(ctl, slot_v0.p, slot_np.p, slot_f0.p, slot_nf.p, vmesh.p, fmesh.p); note_launch();
         pdl(kb_undo_book, gM, kT, 0, s)(ctl, slot_mesh.p, mesh.p, undo_in_reg.p, tmp_undo_reg.p, undo_list_reg.p,
                                        map_reg.p, invalid_reg.p); note_launch();
-        launch_round_prologue_dev(zero_ls, rc, Vb, Fb, nullptr, nullptr, pos_in.p, pos.p, orig_pos.p, occ.p, tri_in.p,
-                                  tri.p, orig_tri.p, valence.p, cursor.p, vedges.p, vcursor.p, qflag.p, s);
+        RoundStart rs;
+        rs.rc = rc;
+        rs.pts_in = pos_in.p; rs.pos = pos.p; rs.orig_pos = orig_pos.p; rs.occ = occ.p;
+        rs.tri_in = tri_in.p; rs.tri = tri.p; rs.orig_tri = orig_tri.p;
+        rs.valence = valence.p; rs.cursor = cursor.p; rs.vedges = vedges.p; rs.vcursor = vcursor.p;
+        rs.qflag = qflag.p; rs.vmin = vmin.p;
+        launch_round_prologue_dev(rs, Vb, Fb, s);
         // adjacency, quadrics (per element: rings never leave a mesh)
         launch_face_counts(tri.p, rc, Fb, valence.p, ecount.p, vedges.p, s, pos.p, fgeo.p);
         {
@@ -783,14 +784,12 @@ struct pamo_csr {
         }
         launch_fill_adjacency(tri.p, rc, Fb, valence.p, cursor.p, nt.p, ecount.p, edges.p, vedges.p, vcursor.p,
                               eorder.p, s);
-        launch_sort_adjacency(rc, Vb, valence.p, nt.p, s);
         const int* nt_off = valence.p;
-        launch_quadrics(rc, Vb, nt_off, nt.p, tri.p, fgeo.p, quad.p, nxt.p, spc.p, s);
+        launch_ring_quadrics(rc, Vb, nt_off, nt.p, tri.p, fgeo.p, quad.p, nxt.p, spc.p, s);
         // cost with each mesh's stale costs and invalid table, then the costs back to the meshes' regions
         pdl(kb_slot_edges, gM, kT, 0, s)(ctl, slot_mesh.p, mesh.p, ecount.p, rc); note_launch();
         pdl(kb_gather, grid_for(std::max(Eb, Vb), kT), kT, 0, s)(rc, slot_mesh.p, mesh.p, vmesh.p, edges.p, ecost_reg.p,
                                                                invalid_reg.p, cost.p, invalid.p); note_launch();
-        launch_fill_u64_dev(rc, Vb, vmin.p, ~0ull, s);
         launch_edge_cost_batch(rc, Eb, eorder.p, edges.p, nt_off, nt.p, tri.p, pos.p, quad.p, fgeo.p, nxt.p, spc.p, invalid.p,
                                cost.p, vmin.p, slot_scale.p, slot_stuck.p, vmesh.p, threshold, s, skinny_pow);
         pdl(kb_scatter_costs, grid_for(Eb, kT), kT, 0, s)(rc, slot_mesh.p, mesh.p, vmesh.p, edges.p, cost.p, ecost_reg.p);
@@ -800,17 +799,13 @@ struct pamo_csr {
         launch_collapse(rc, Eb, eorder.p, edges.p, cost.p, collapse_t, fkey.p, nt_off, nt.p, tri.p, orig_tri.p, pos.p,
                         orig_pos.p, occ.p, win.p, s);
         exclusive_scan(win.p, win.p, &rc->n_edges, 1, &rc->n_win, scan_scratch, s, &rc->status, Eb);
-        launch_compact_winners(rc, Eb, win.p, winners.p, s);
-        launch_remove_invalid(rc, Fb, tri.p, s);
-        launch_line_detect(rc, Eb, edges.p, pos.p, s);
+        launch_after_collapse(rc, Eb, Fb, win.p, winners.p, edges.p, nt_off, nt.p, tri.p, pos.p, occ.p, 0, false, s);
         pdl(kb_line_apply, 1, 32, 0, s)(rc, ctl, slot_mesh.p, mesh.p, vmesh.p, edges.p, nt_off, nt.p, tri.p, pos.p, occ.p,
                                        lines.p, (int)lines.n); note_launch();
         pdl(kb_considered, 1, kCtlThreads, 0, s)(ctl, slot_mesh.p, mesh.p, win.p, rc); note_launch();
         pdl(kb_considered_fill, gM, kT, 0, s)(ctl, slot_mesh.p, mesh.p, winners.p, lines.p, considered.p); note_launch();
         // faces whose intersections decide the undo: rings of the considered collapsed edges
         launch_mark_query(rc, Eb, considered.p, edges.p, nt_off, nt.p, qflag.p, s);
-        exclusive_scan(qflag.p, qflag.p, &rc->n_tris, 1, &rc->n_query, scan_scratch, s, &rc->status, Fb);
-        launch_compact_flags(qflag.p, Fb, &rc->n_tris, qlist.p, s);
         // intersection checks and undo passes (cusimp_free.cu:1014-1040), per mesh
         BvhMeshes bm;
         bm.fmesh = fmesh.p;

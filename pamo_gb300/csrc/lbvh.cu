@@ -21,6 +21,7 @@ constexpr int kSortThreads = 256;
 constexpr int kQueryThreads = 128;
 constexpr int kStackDepth = 64;  // enough for any tree (depth <= 62 + 1)
 constexpr int kShortStack = 24;  // first walk: deeper queries are handed to the second walk
+constexpr int kExactThreads = 64;
 constexpr int kPairChunk = 32;   // list slots a lane takes at a time
 constexpr int kQueryBit = 1 << 30;  // set on a packed leaf's face id when the face is a query face
 
@@ -41,16 +42,32 @@ __device__ __forceinline__ unsigned expand10(unsigned v) {
 }
 
 // ---------------------------------------------------------------- boxes + scene bounds
+// One pass over the faces before a build or a refit, which also prepares the pass that follows: the counters of
+// bvh_query, the hit flags (q.hit), the number of query faces on a round's first check (rc->n_query) and, for a refit, the
+// arrival counts of the carried tree's nodes (leaves: their number). They were five memsets and kernels of their own.
 __global__ void __launch_bounds__(256) k_boxes(const int4* __restrict__ tri, const float4* __restrict__ pos,
-                                                const RoundCounters* rc, float4* box_lo, float4* box_hi, int* live,
-                                                unsigned* scene, int all_faces) {
+                                                RoundCounters* rc, float4* box_lo, float4* box_hi, int* live,
+                                                unsigned* scene, int all_faces, BvhQuery q, int* xq_count, int* visit,
+                                                const int* leaves) {
     pdl_wait();
+    if (gtid() == 0) {
+        rc->pad[1] = rc->pad[2] = rc->pad[3] = 0;  // pair list length, query count, redo count
+        *xq_count = 0;
+    }
+    if (leaves) {
+        const int m = *leaves - 1;
+        for (int i = gtid(); i < m; i += gstride()) visit[i] = 0;
+    }
+    const bool count = q.flags && rc->passes == 0;
+    int marked = 0;
     const int n = rc->n_tris;
     float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
     for (int f = gtid(); f < n; f += gstride()) {
         int4 t = tri[f];
         int is_live = (t.x != -1);
-        live[f] = all_faces ? 1 : is_live;
+        if (!leaves) live[f] = all_faces ? 1 : is_live;
+        if (q.hit) q.hit[f] = 0;
+        if (count) marked += q.flags[f];
         if (!is_live) {
             if (all_faces) {  // an empty box: overlaps nothing
                 box_lo[f] = make_float4(INFINITY, INFINITY, INFINITY, 0.f);
@@ -66,6 +83,11 @@ __global__ void __launch_bounds__(256) k_boxes(const int4* __restrict__ tri, con
         mn[0] = fminf(mn[0], lo.x); mn[1] = fminf(mn[1], lo.y); mn[2] = fminf(mn[2], lo.z);
         mx[0] = fmaxf(mx[0], hi.x); mx[1] = fmaxf(mx[1], hi.y); mx[2] = fmaxf(mx[2], hi.z);
     }
+    if (count) {
+        for (int o = 16; o > 0; o >>= 1) marked += __shfl_xor_sync(0xffffffffu, marked, o);
+        if ((threadIdx.x & 31) == 0 && marked) atomicAdd(&rc->n_query, marked);
+    }
+    if (leaves) return;  // a refit has no codes to make
     if (gtid() == 0) live[n] = 0;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -90,7 +112,7 @@ __global__ void __launch_bounds__(256) k_boxes(const int4* __restrict__ tri, con
 // Morton code, so that the sort groups each mesh's faces and every Karras node under a mesh boundary covers one mesh
 __global__ void __launch_bounds__(256) k_morton(const RoundCounters* rc, const int* live_scan, const float4* box_lo,
                                                  const float4* box_hi, const unsigned* scene, unsigned* keys, int* vals,
-                                                 const int* __restrict__ fmesh, int mesh_bits) {
+                                                 const int* __restrict__ fmesh, int mesh_bits, int* visit) {
     pdl_wait();
     const int n = rc->n_tris;
     float lo[3], ext[3];
@@ -119,6 +141,7 @@ __global__ void __launch_bounds__(256) k_morton(const RoundCounters* rc, const i
         }
         keys[i] = key;
         vals[i] = f;
+        visit[i] = 0;  // the nodes' arrival counts (one node fewer than leaves)
     }
 }
 
@@ -200,23 +223,11 @@ __device__ __forceinline__ int delta(const unsigned* k, int n, int i, int j) {
     return 32 + __clz((unsigned)(i ^ j));
 }
 
-__global__ void __launch_bounds__(256) k_leaves(const RoundCounters* rc, const int* vals, const float4* box_lo,
-                                                 const float4* box_hi, float4* llo, float4* lhi, int* visit, int* lparent) {
-    pdl_wait();
-    const int n = rc->n_live;
-    for (int i = gtid(); i < n; i += gstride()) {
-        int f = vals[i];
-        llo[i] = box_lo[f];
-        lhi[i] = box_hi[f];
-        if (i < n - 1) visit[i] = 0;
-        if (n == 1) lparent[0] = -1;
-    }
-}
-
 __global__ void __launch_bounds__(256) k_karras(const RoundCounters* rc, const unsigned* keys, int2* child, int* iparent,
                                                  int* lparent, int2* range) {
     pdl_wait();
     const int n = rc->n_live;
+    if (n == 1 && gtid() == 0) lparent[0] = -1;
     for (int i = gtid(); i < n - 1; i += gstride()) {
         const int d = (delta(keys, n, i, i + 1) - delta(keys, n, i, i - 1)) >= 0 ? 1 : -1;
         const int dmin = delta(keys, n, i, i - d);
@@ -281,18 +292,13 @@ __device__ __forceinline__ int arrive_acq_rel(int* p) {
     return old;
 }
 
-// The packed 64-byte record of node p (both children's boxes, child references, leaf face ids with the query bit).
-__device__ __forceinline__ void write_packed(int p, int2 c, float4 alo, float4 ahi, float4 clo, float4 chi,
-                                             const int* leaf_face, const int* qscan, float4* packed) {
-    int fa = -1, fc = -1;
-    if (c.x < 0) {
-        fa = leaf_face[~c.x];
-        if (qscan && fa >= 0 && qscan[fa + 1] != qscan[fa]) fa |= kQueryBit;
-    }
-    if (c.y < 0) {
-        fc = leaf_face[~c.y];
-        if (qscan && fc >= 0 && qscan[fc + 1] != qscan[fc]) fc |= kQueryBit;
-    }
+// The face id of a packed leaf with its query bit
+__device__ __forceinline__ int packed_face(int f, const int* qflag) {
+    return qflag && f >= 0 && qflag[f] ? f | kQueryBit : f;
+}
+// The packed 64-byte record of node p (both children's boxes, child references, leaf face ids fa and fc).
+__device__ __forceinline__ void write_packed(int p, int2 c, float4 alo, float4 ahi, float4 clo, float4 chi, int fa,
+                                             int fc, float4* packed) {
     float4* rec = packed + 4 * (size_t)p;
     alo.w = __int_as_float(c.x);
     ahi.w = __int_as_float(fa);
@@ -309,7 +315,7 @@ __device__ __forceinline__ void write_packed(int p, int2 c, float4 alo, float4 a
 template <bool kPack>
 __device__ void climb_from(RoundCounters* rc, int p, const int2* child, const int* iparent, const float4* llo,
                            const float4* lhi, float4* nlo, float4* nhi, int* visit, const int* leaf_face,
-                           const int* qscan, float4* packed) {
+                           const int* qflag, float4* packed) {
     {
         int guard = 0;
         int2 c = child[p];
@@ -328,7 +334,9 @@ __device__ void climb_from(RoundCounters* rc, int p, const int2* child, const in
             const float4 bhi = make_float4(fmaxf(ahi.x, chi.x), fmaxf(ahi.y, chi.y), fmaxf(ahi.z, chi.z), 0.f);
             __stcg(&nlo[p], blo);  // the parent's second arrival reads it
             __stcg(&nhi[p], bhi);
-            if (kPack) write_packed(p, c, alo, ahi, clo, chi, leaf_face, qscan, packed);
+            if (kPack)
+                write_packed(p, c, alo, ahi, clo, chi, c.x < 0 ? packed_face(__ldcg(&leaf_face[~c.x]), qflag) : -1,
+                             c.y < 0 ? packed_face(__ldcg(&leaf_face[~c.y]), qflag) : -1, packed);
             if (pp < 0) break;
             // the parent's topology is fixed: loaded before its arrival count, not after
             const int2 cn = child[pp];
@@ -341,23 +349,36 @@ __device__ void climb_from(RoundCounters* rc, int p, const int2* child, const in
     }
 }
 
-template <bool kPack, bool kNodes>
+// kLeaf: where the leaves' boxes come from. kLeafGiven: llo/lhi; kLeafBuild: the boxes of the leaves' faces (leaf_face);
+// kLeafReuse: the same for a carried tree, *meta leaves, with the face ids of new_ids where it is given (they become
+// leaf_face); a leaf whose face is gone has an empty box. llo/lhi receive the boxes for the nodes above the tile.
+// The tile's topology is loaded into shared memory with its leaves: loaded from global memory node by node, it put a
+// dependent load of an L2 latency into every level of the climb.
+enum { kLeafGiven = 0, kLeafBuild = 1, kLeafReuse = 2 };
+
+template <bool kPack, bool kNodes, int kLeaf>
 __global__ void __launch_bounds__(kTileThreads, 3) k_bottom_up_tiles(RoundCounters* rc, const int2* child,
                                                                   const int* iparent, const int* lparent,
-                                                                  const int2* range, const float4* llo,
-                                                                  const float4* lhi, float4* nlo, float4* nhi, int* visit,
-                                                                  const int* leaf_face, const int* qscan, float4* packed,
-                                                                  int* meta_out, const int* active, int* upq) {
+                                                                  const int2* range, float4* llo, float4* lhi, float4* nlo,
+                                                                  float4* nhi, int* visit, int* leaf_face,
+                                                                  const int* __restrict__ new_ids,
+                                                                  const float4* __restrict__ box_lo,
+                                                                  const float4* __restrict__ box_hi,
+                                                                  const int* __restrict__ qflag, float4* packed, int* meta,
+                                                                  const int* active, int* upq, int climb) {
     pdl_wait();
-    __shared__ int svisit[kTileLeaves];
+    __shared__ int svisit[kTileLeaves], sface[kTileLeaves], sparent[kTileLeaves];
+    __shared__ int2 srange[kTileLeaves], schild[kTileLeaves];
     __shared__ float4 slo[kTileLeaves], shi[kTileLeaves];    // internal nodes a .. b-2
     __shared__ float4 sllo[kTileLeaves], slhi[kTileLeaves];  // leaves a .. b-1
     if (active && *active == 0) return;
-    const int n = rc->n_live;
-    if (kPack && blockIdx.x == 0 && threadIdx.x == 0) meta_out[0] = n;
-    // one tile per block (a single wave): a chain leaving its tile climbs on here, nothing waits for it; several
-    // tiles per block: the nodes above the tiles are queued for k_bottom_up_upper
-    const bool climb = (long long)gridDim.x * kTileLeaves >= n;
+    const int n = kLeaf == kLeafReuse ? *meta : rc->n_live;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (kLeaf == kLeafReuse) rc->n_live = n;
+        else if (kPack) *meta = n;
+    }
+    // climb: one tile per block, and a chain leaving its tile climbs on here, nothing waits for it; else several
+    // tiles per block, and the nodes above the tiles are queued for k_bottom_up_upper
     // tiles in a block-stride loop: the leaf count is read on the device and may exceed the launch's bound
     for (int a = blockIdx.x * kTileLeaves; a < n; a += gridDim.x * kTileLeaves) {
         const int b = min(a + kTileLeaves, n);  // leaves [a, b)
@@ -367,11 +388,37 @@ __global__ void __launch_bounds__(kTileThreads, 3) k_bottom_up_tiles(RoundCounte
         float4 blo = make_float4(0.f, 0.f, 0.f, 0.f), bhi = blo;
         int p = -1;
         if (leaf < b) {
-            blo = __ldcg(&llo[leaf]);
-            bhi = __ldcg(&lhi[leaf]);
+            p = lparent[leaf];
+            if (leaf < n - 1) {
+                srange[threadIdx.x] = range[leaf];
+                schild[threadIdx.x] = child[leaf];
+                sparent[threadIdx.x] = iparent[leaf];
+            }
+            if constexpr (kLeaf == kLeafGiven) {
+                blo = __ldcg(&llo[leaf]);
+                bhi = __ldcg(&lhi[leaf]);
+                if (kPack) sface[threadIdx.x] = packed_face(leaf_face[leaf], qflag);
+            } else {
+                int f;
+                if (kLeaf == kLeafReuse && new_ids) {
+                    f = new_ids[leaf];
+                    __stcg(&leaf_face[leaf], f);
+                } else {
+                    f = leaf_face[leaf];
+                }
+                if (f >= 0) {
+                    blo = box_lo[f];
+                    bhi = box_hi[f];
+                } else {
+                    blo = make_float4(INFINITY, INFINITY, INFINITY, 0.f);
+                    bhi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
+                }
+                __stcg(&llo[leaf], blo);
+                __stcg(&lhi[leaf], bhi);
+                if (kPack) sface[threadIdx.x] = packed_face(f, qflag);
+            }
             sllo[threadIdx.x] = blo;
             slhi[threadIdx.x] = bhi;
-            p = lparent[leaf];
         }
         __syncthreads();
         int ref = ~leaf;
@@ -381,10 +428,9 @@ __global__ void __launch_bounds__(kTileThreads, 3) k_bottom_up_tiles(RoundCounte
                 atomicOr(&rc->status, kErrIterLimit);
                 break;
             }
-            const int2 rg = range[p];
-            const int2 c = child[p];
-            const int pp = iparent[p];
-            if (!(rg.x >= a && rg.y < b)) {
+            // a node's index is one end of its range: a node with its index outside the tile leaves the tile
+            const int k = p - a;
+            if (!(p >= a && p < b && srange[k].x >= a && srange[k].y < b)) {
                 // leaving the tile: this child's box goes to global memory for the other child's chain; with
                 // several tiles per block the second arrival queues p for k_bottom_up_upper instead of climbing
                 // on, so that no chain through the upper tree holds this block at the next tile's barrier
@@ -395,14 +441,15 @@ __global__ void __launch_bounds__(kTileThreads, 3) k_bottom_up_tiles(RoundCounte
                 if (!climb) {
                     if (arrive_release(&visit[p]) != 0) upq[1 + atomicAdd(upq, 1)] = p;
                 } else if (arrive_acq_rel(&visit[p]) != 0) {
-                    climb_from<kPack>(rc, p, child, iparent, llo, lhi, nlo, nhi, visit, leaf_face, qscan, packed);
+                    climb_from<kPack>(rc, p, child, iparent, llo, lhi, nlo, nhi, visit, leaf_face, qflag, packed);
                 }
                 break;
             }
             __threadfence_block();
-            if (atomicAdd(&svisit[p - a], 1) == 0) break;
+            if (atomicAdd(&svisit[k], 1) == 0) break;
             __threadfence_block();
             // both children are in this tile
+            const int2 c = schild[k];
             float4 alo, ahi, clo, chi;
             if (c.x < 0) { alo = sllo[~c.x - a]; ahi = slhi[~c.x - a]; }
             else { alo = slo[c.x - a]; ahi = shi[c.x - a]; }
@@ -410,15 +457,17 @@ __global__ void __launch_bounds__(kTileThreads, 3) k_bottom_up_tiles(RoundCounte
             else { clo = slo[c.y - a]; chi = shi[c.y - a]; }
             blo = make_float4(fminf(alo.x, clo.x), fminf(alo.y, clo.y), fminf(alo.z, clo.z), 0.f);
             bhi = make_float4(fmaxf(ahi.x, chi.x), fmaxf(ahi.y, chi.y), fmaxf(ahi.z, chi.z), 0.f);
-            slo[p - a] = blo;
-            shi[p - a] = bhi;
+            slo[k] = blo;
+            shi[k] = bhi;
             if (kNodes) {
                 __stcg(&nlo[p], blo);
                 __stcg(&nhi[p], bhi);
             }
-            if (kPack) write_packed(p, c, alo, ahi, clo, chi, leaf_face, qscan, packed);
+            if (kPack)
+                write_packed(p, c, alo, ahi, clo, chi, c.x < 0 ? sface[~c.x - a] : -1, c.y < 0 ? sface[~c.y - a] : -1,
+                             packed);
             ref = p;
-            p = pp;
+            p = sparent[k];
         }
     }
 }
@@ -429,36 +478,38 @@ template <bool kPack, bool kNodes>
 __global__ void __launch_bounds__(256) k_bottom_up_upper(RoundCounters* rc, const int2* child, const int* iparent,
                                                          const float4* llo, const float4* lhi, float4* nlo,
                                                          float4* nhi, int* visit, const int* leaf_face,
-                                                         const int* qscan, float4* packed, const int* upq,
+                                                         const int* qflag, float4* packed, const int* upq,
                                                          const int* active) {
     pdl_wait();
     if (active && *active == 0) return;
     const int nq = upq[0];
     for (int k = gtid(); k < nq; k += gstride())
-        climb_from<kPack>(rc, upq[1 + k], child, iparent, llo, lhi, nlo, nhi, visit, leaf_face, qscan, packed);
+        climb_from<kPack>(rc, upq[1 + k], child, iparent, llo, lhi, nlo, nhi, visit, leaf_face, qflag, packed);
 }
 
-// blocks for k_bottom_up_tiles: a tile per block up to the resident count (the bound may be capped below the
-// leaf count, which the block-stride loop covers)
+// blocks for k_bottom_up_tiles: a tile per block (a carried tree has up to 4/3 of the faces), except for a capped bound,
+// whose block-stride loop covers any number
 inline int tile_grid(int n_bound) {
-    int g = (n_bound + kTileLeaves - 1) / kTileLeaves;
-    if (n_bound >= (1 << 19) && g < 3 * kNumSM) g = 3 * kNumSM;
-    return g < 1 ? 1 : g;
+    if (n_bound >= (1 << 19)) return std::max((n_bound + kTileLeaves - 1) / kTileLeaves, 3 * kNumSM);
+    return (n_bound + n_bound / 3 + kTileLeaves) / kTileLeaves;
 }
 
-// The whole bottom-up pass: the tiles, then the nodes above them.
-template <bool kPack, bool kNodes>
-void bottom_up(BvhBuffers& b, RoundCounters* rc, int n_bound, const int* leaf_face, const int* qscan, int* meta_out,
-               const int* active, cudaStream_t s) {
-    cudaMemsetAsync(b.upq, 0, sizeof(int), s);
+// The whole bottom-up pass: the tiles, then the nodes above them (climbed within the tiles' kernel where each block has
+// one tile).
+template <bool kPack, bool kNodes, int kLeaf>
+void bottom_up(BvhBuffers& b, RoundCounters* rc, int n_bound, const int* new_ids, const int* qflag, const int* active,
+               cudaStream_t s) {
+    const bool climb = n_bound != (1 << 19);  // where callers cap their bounds
+    if (!climb) cudaMemsetAsync(b.upq, 0, sizeof(int), s);
     const int gT = tile_grid(n_bound);
-    pdl(k_bottom_up_tiles<kPack, kNodes>, gT, kTileThreads, 0, s)(rc, b.child, b.iparent, b.lparent, b.range, b.llo,
-                                                                 b.lhi, b.nlo, b.nhi, b.visit, leaf_face, qscan,
-                                                                 b.packed, meta_out, active, b.upq);
+    pdl(k_bottom_up_tiles<kPack, kNodes, kLeaf>, gT, kTileThreads, 0, s)(
+        rc, b.child, b.iparent, b.lparent, b.range, b.llo, b.lhi, b.nlo, b.nhi, b.visit, b.vals[0], new_ids, b.box_lo,
+        b.box_hi, qflag, b.packed, b.meta, active, b.upq, climb ? 1 : 0);
     note_launch();
+    if (climb) return;
     const int gU = std::max(1, std::min(gT, 4 * kNumSM));
     pdl(k_bottom_up_upper<kPack, kNodes>, gU, 256, 0, s)(rc, b.child, b.iparent, b.llo, b.lhi, b.nlo, b.nhi, b.visit,
-                                                        leaf_face, qscan, b.packed, b.upq, active);
+                                                        b.vals[0], qflag, b.packed, b.upq, active);
     note_launch();
 }
 
@@ -491,23 +542,34 @@ __device__ __forceinline__ bool decide_pair(int f, int g, const int4* __restrict
            (need_b && pair_decide_exact(q0, q1, q2, qt, g0, g1, g2, gt, eps));
 }
 
-__global__ void __launch_bounds__(256) k_query_order(const RoundCounters* rc, const int* __restrict__ leaf_face,
-                                                     const int* __restrict__ qscan, int* flags) {
+// The query faces in leaf order: a block takes chunks of 1024 leaves and a place for each chunk's queries in one atomic
+// (the chunks come in any order, which only sets which walks run side by side). In place of a flag kernel, a scan and a
+// gather.
+__global__ void __launch_bounds__(256) k_query_gather(RoundCounters* rc, const int* __restrict__ leaf_face,
+                                                      const int* __restrict__ qflag, int* qsorted) {
     pdl_wait();
+    __shared__ int sm[33];
+    __shared__ int s_base;
     const int n = rc->n_live;
-    for (int i = gtid(); i < n; i += gstride()) {
-        const int f = leaf_face[i];
-        flags[i] = (f >= 0 && qscan[f + 1] != qscan[f]) ? 1 : 0;  // f < 0: a leaf whose face is gone
+    for (int lo = blockIdx.x * 1024; lo < n; lo += gridDim.x * 1024) {
+        int f[4], cnt = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int i = lo + 4 * threadIdx.x + k;
+            f[k] = i < n ? leaf_face[i] : -1;  // -1: a leaf whose face is gone
+            if (f[k] >= 0 && !qflag[f[k]]) f[k] = -1;
+            cnt += f[k] >= 0;
+        }
+        int tot;
+        int at = block_exclusive_scan(cnt, &tot, sm);
+        if (threadIdx.x == 0) s_base = tot ? atomicAdd(&rc->pad[2], tot) : 0;
+        __syncthreads();
+        at += s_base;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (f[k] >= 0) qsorted[at++] = f[k];
+        __syncthreads();
     }
-    if (gtid() == 0) flags[n] = 0;
-}
-
-__global__ void __launch_bounds__(256) k_query_gather(const RoundCounters* rc, const int* __restrict__ leaf_face,
-                                                      const int* __restrict__ scan, int* qsorted) {
-    pdl_wait();
-    const int n = rc->n_live;
-    for (int i = gtid(); i < n; i += gstride())
-        if (scan[i + 1] != scan[i]) qsorted[scan[i]] = leaf_face[i];
 }
 
 __device__ __forceinline__ bool box_overlap4(float4 qlo, float4 qhi, float4 lo, float4 hi) {
@@ -680,77 +742,6 @@ __global__ void __launch_bounds__(kQueryThreads) k_traverse_list(const float4* _
     if (lane == 0 && npairs) atomicAdd(&rc->n_pairs, npairs);
 }
 
-// Second walk, only when the first marked queries: each marked query walks the whole tree again with a stack
-// deep enough for any tree (the Karras split prefix grows by at least one of the 62 key bits per level) and
-// decides every pair in place (pairs already listed are decided twice, which sets the same flags).
-__global__ void __launch_bounds__(kQueryThreads) k_traverse_redo(const float4* __restrict__ packed,
-                                                                  const float4* __restrict__ box_lo,
-                                                                  const float4* __restrict__ box_hi,
-                                                                  const int4* __restrict__ tri,
-                                                                  const float4* __restrict__ pos,
-                                                                  const int* __restrict__ qsorted, unsigned char* hit,
-                                                                  RoundCounters* rc, float eps, const int* redo,
-                                                                  const int* __restrict__ fmesh,
-                                                                  const int* __restrict__ mesh_root) {
-    pdl_wait();
-    __shared__ int stack[kStackDepth][kQueryThreads];
-    if (rc->pad[3] == 0) return;
-    const int nq = rc->pad[2];
-    unsigned exact = 0;
-    for (int qi = gtid(); qi < nq; qi += gstride()) {
-        if (redo[qi] == 0) continue;
-        const int f = qsorted[qi];
-        int node = query_root(f, fmesh, mesh_root);
-        if (node < 0) continue;
-        const float4 qlo = box_lo[f], qhi = box_hi[f];
-        int sp = 0;
-        int guard = 0;
-        while (true) {
-            if (++guard > (1 << 22)) {
-                atomicOr(&rc->status, kErrIterLimit);
-                break;
-            }
-            const float4* rec = packed + 4 * (size_t)node;
-            const float4 alo = __ldg(rec), ahi = __ldg(rec + 1), blo = __ldg(rec + 2), bhi = __ldg(rec + 3);
-            int next[2];
-            int nn = 0;
-#pragma unroll
-            for (int side = 0; side < 2; ++side) {
-                const float4 lo = side ? blo : alo, hi = side ? bhi : ahi;
-                if (!box_overlap4(qlo, qhi, lo, hi)) continue;
-                const int x = __float_as_int(lo.w);
-                if (x < 0) {
-                    const int graw = __float_as_int(hi.w);
-                    const int g = graw & ~kQueryBit;
-                    if (g == f) continue;
-                    if (g < f && (graw & kQueryBit)) continue;
-                    if (decide_pair(f, g, tri, pos, eps, exact)) {
-                        hit[f] = 1;
-                        hit[g] = 1;
-                    }
-                } else {
-                    next[nn++] = x;
-                }
-            }
-            if (nn == 2) {
-                if (sp >= kStackDepth) {
-                    atomicOr(&rc->status, kErrStackOverflow);
-                    break;
-                }
-                stack[sp++][threadIdx.x] = next[1];
-                node = next[0];
-            } else if (nn == 1) {
-                node = next[0];
-            } else {
-                if (sp == 0) break;
-                node = stack[--sp][threadIdx.x];
-            }
-        }
-    }
-    for (int o = 16; o > 0; o >>= 1) exact += __shfl_xor_sync(0xffffffffu, exact, o);
-    if ((threadIdx.x & 31) == 0 && exact) atomicAdd(&rc->n_exact, (unsigned long long)exact);
-}
-
 // k_pairs decides every listed pair by the float certificates; each order of a pair they cannot decide (the float64
 // path, a few pairs in a thousand) is queued in xq, and k_pairs_exact runs those one per thread spread over every SM
 // (decided where they were listed, they clustered in a few warps and the float64 pipes of a few SMs set the time).
@@ -807,11 +798,80 @@ __global__ void __launch_bounds__(128, 8) k_pairs(const int4* __restrict__ tri, 
     if ((threadIdx.x & 31) == 0 && exact) atomicAdd(&rc->n_exact, (unsigned long long)exact);
 }
 
+// Second walk, only when the first marked queries: each marked query walks the whole tree again with a stack
+// deep enough for any tree (the Karras split prefix grows by at least one of the 62 key bits per level) and
+// decides every pair in place (pairs already listed are decided twice, which sets the same flags).
+__device__ void redo_walks(const float4* __restrict__ packed, const float4* __restrict__ box_lo,
+                           const float4* __restrict__ box_hi, const int4* __restrict__ tri,
+                           const float4* __restrict__ pos, const int* __restrict__ qsorted, unsigned char* hit,
+                           RoundCounters* rc, float eps, const int* redo, const int* __restrict__ fmesh,
+                           const int* __restrict__ mesh_root) {
+    __shared__ int stack[kStackDepth][kExactThreads];
+    const int nq = rc->pad[2];
+    unsigned exact = 0;
+    for (int qi = gtid(); qi < nq; qi += gstride()) {
+        if (redo[qi] == 0) continue;
+        const int f = qsorted[qi];
+        int node = query_root(f, fmesh, mesh_root);
+        if (node < 0) continue;
+        const float4 qlo = box_lo[f], qhi = box_hi[f];
+        int sp = 0;
+        int guard = 0;
+        while (true) {
+            if (++guard > (1 << 22)) {
+                atomicOr(&rc->status, kErrIterLimit);
+                break;
+            }
+            const float4* rec = packed + 4 * (size_t)node;
+            const float4 alo = __ldg(rec), ahi = __ldg(rec + 1), blo = __ldg(rec + 2), bhi = __ldg(rec + 3);
+            int next[2];
+            int nn = 0;
+#pragma unroll
+            for (int side = 0; side < 2; ++side) {
+                const float4 lo = side ? blo : alo, hi = side ? bhi : ahi;
+                if (!box_overlap4(qlo, qhi, lo, hi)) continue;
+                const int x = __float_as_int(lo.w);
+                if (x < 0) {
+                    const int graw = __float_as_int(hi.w);
+                    const int g = graw & ~kQueryBit;
+                    if (g == f) continue;
+                    if (g < f && (graw & kQueryBit)) continue;
+                    if (decide_pair(f, g, tri, pos, eps, exact)) {
+                        hit[f] = 1;
+                        hit[g] = 1;
+                    }
+                } else {
+                    next[nn++] = x;
+                }
+            }
+            if (nn == 2) {
+                if (sp >= kStackDepth) {
+                    atomicOr(&rc->status, kErrStackOverflow);
+                    break;
+                }
+                stack[sp++][threadIdx.x] = next[1];
+                node = next[0];
+            } else if (nn == 1) {
+                node = next[0];
+            } else {
+                if (sp == 0) break;
+                node = stack[--sp][threadIdx.x];
+            }
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) exact += __shfl_xor_sync(0xffffffffu, exact, o);
+    if ((threadIdx.x & 31) == 0 && exact) atomicAdd(&rc->n_exact, (unsigned long long)exact);
+}
+
 // The queued pairs, one per thread, consecutive pairs on different SMs (block-cyclic: item k goes to block
 // k mod blocks).
-__global__ void __launch_bounds__(64) k_pairs_exact(const int4* __restrict__ tri, const float4* __restrict__ pos,
+__global__ void __launch_bounds__(kExactThreads) k_pairs_exact(const int4* __restrict__ tri, const float4* __restrict__ pos,
                                                     const int4* __restrict__ xq, int xq_cap,
-                                                    const int* __restrict__ xq_count, unsigned char* hit, float eps) {
+                                                    const int* __restrict__ xq_count, unsigned char* hit, float eps,
+                                                    const float4* __restrict__ packed, const float4* __restrict__ box_lo,
+                                                    const float4* __restrict__ box_hi, const int* __restrict__ qsorted,
+                                                    RoundCounters* rc, const int* redo, const int* __restrict__ fmesh,
+                                                    const int* __restrict__ mesh_root) {
     pdl_wait();
     const int n = min(*xq_count, xq_cap);
     for (long long k = (long long)threadIdx.x * gridDim.x + blockIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
@@ -827,6 +887,7 @@ __global__ void __launch_bounds__(64) k_pairs_exact(const int4* __restrict__ tri
             hit[g] = 1;
         }
     }
+    if (rc->pad[3] != 0) redo_walks(packed, box_lo, box_hi, tri, pos, qsorted, hit, rc, eps, redo, fmesh, mesh_root);
 }
 
 // The subtree root of each mesh: its live faces are the leaves [live_scan[f0], live_scan[f0 + nf]) of a tree built
@@ -913,14 +974,15 @@ void bvh_carve(BvhBuffers& b, int cap, char* base, bool clear_scan_scratch) {
 }
 
 void bvh_build(BvhBuffers& b, const int4* tri, const float4* pos, RoundCounters* rc, int n_tris_bound, cudaStream_t s,
-               bool all_faces, const int* qscan, bool nodes, const BvhMeshes* meshes) {
+               bool all_faces, const BvhQuery& query, bool nodes, const BvhMeshes* meshes) {
     cudaMemsetAsync(b.scene, 0xFF, 3 * sizeof(unsigned), s);
     cudaMemsetAsync(b.scene + 3, 0x00, 3 * sizeof(unsigned), s);
     const int gF = grid_for(n_tris_bound, 256);
-    pdl(k_boxes, gF, 256, 0, s)(tri, pos, rc, b.box_lo, b.box_hi, b.live_scan, b.scene, all_faces ? 1 : 0); note_launch();
+    pdl(k_boxes, gF, 256, 0, s)(tri, pos, rc, b.box_lo, b.box_hi, b.live_scan, b.scene, all_faces ? 1 : 0, query,
+                                   b.xq_count, b.visit, nullptr); note_launch();
     exclusive_scan(b.live_scan, b.live_scan, &rc->n_tris, 1, &rc->n_live, b.scan_scratch, s, &rc->status, n_tris_bound);
     pdl(k_morton, gF, 256, 0, s)(rc, b.live_scan, b.box_lo, b.box_hi, b.scene, b.keys[0], b.vals[0],
-                                meshes ? meshes->fmesh : nullptr, meshes ? meshes->bits : 0); note_launch();
+                                meshes ? meshes->fmesh : nullptr, meshes ? meshes->bits : 0, b.visit); note_launch();
     // sort tiles from the launch's bound (about 2048 keys per tile; all kSortTiles from 2^19 on, where callers
     // cap their bounds); the histogram is
     // digit-major over the tiles, so its scan gives each tile's output offset per digit
@@ -933,15 +995,14 @@ void bvh_build(BvhBuffers& b, const int4* tri, const float4* pos, RoundCounters*
         pdl(k_rs_scatter, sort_tiles, kSortThreads, 0, s)(b.keys[in], b.vals[in], b.keys[out], b.vals[out], &rc->n_live,
                                                          8 * pass, b.hist); note_launch();
     }
-    pdl(k_leaves, gF, 256, 0, s)(rc, b.vals[0], b.box_lo, b.box_hi, b.llo, b.lhi, b.visit, b.lparent); note_launch();
     pdl(k_karras, gF, 256, 0, s)(rc, b.keys[0], b.child, b.iparent, b.lparent, b.range); note_launch();
     if (meshes) {
         pdl(k_mesh_roots, grid_for(meshes->count_bound, 256), 256, 0, s)(rc, b.live_scan, b.range, meshes->f0, meshes->nf,
                                                                           meshes->d_count, meshes->root);
         note_launch();
     }
-    if (nodes) bottom_up<true, true>(b, rc, n_tris_bound, b.vals[0], qscan, b.meta, nullptr, s);
-    else bottom_up<true, false>(b, rc, n_tris_bound, b.vals[0], qscan, b.meta, nullptr, s);
+    if (nodes) bottom_up<true, true, kLeafBuild>(b, rc, n_tris_bound, nullptr, query.flags, nullptr, s);
+    else bottom_up<true, false, kLeafBuild>(b, rc, n_tris_bound, nullptr, query.flags, nullptr, s);
 }
 
 __global__ void __launch_bounds__(256) k_refit_leaves(const RoundCounters* rc, const int4* __restrict__ tri,
@@ -963,72 +1024,24 @@ void bvh_refit(BvhBuffers& b, const int4* tri, const float4* pos, RoundCounters*
                const int* active) {
     const int gF = grid_for(n_tris_bound, 256);
     pdl(k_refit_leaves, gF, 256, 0, s)(rc, tri, pos, b.vals[0], b.llo, b.lhi, b.visit, active); note_launch();
-    bottom_up<false, true>(b, rc, n_tris_bound, nullptr, nullptr, nullptr, active, s);
-}
-
-__global__ void __launch_bounds__(256) k_reuse_leaves(RoundCounters* rc, const int4* __restrict__ tri,
-                                                      const float4* __restrict__ box_lo, const float4* __restrict__ box_hi,
-                                                      const int* __restrict__ new_ids, int* leaf_face, float4* llo,
-                                                      float4* lhi, int* visit, const int* meta) {
-    pdl_wait();
-    const int n = meta[0];
-    if (gtid() == 0) rc->n_live = n;
-    for (int i = gtid(); i < n; i += gstride()) {
-        int f;
-        if (new_ids) {
-            f = new_ids[i];
-            leaf_face[i] = f;
-        } else {
-            f = leaf_face[i];
-        }
-        if (f >= 0 && tri[f].x != -1) {
-            llo[i] = box_lo[f];
-            lhi[i] = box_hi[f];
-        } else {
-            llo[i] = make_float4(INFINITY, INFINITY, INFINITY, 0.f);
-            lhi[i] = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
-        }
-        if (i < n - 1) visit[i] = 0;
-    }
-}
-
-// next[i] = the leaf's face in the next numbering; reads the current ids only, so it can be repeated
-__global__ void __launch_bounds__(256) k_remap_leaves(const int* meta, const int* __restrict__ fscan,
-                                                      const int* __restrict__ leaf_face, int* next) {
-    pdl_wait();
-    const int n = meta[0];
-    for (int i = gtid(); i < n; i += gstride()) {
-        const int f = leaf_face[i];
-        next[i] = (f >= 0 && fscan[f + 1] != fscan[f]) ? fscan[f] : -1;
-    }
+    bottom_up<false, true, kLeafGiven>(b, rc, n_tris_bound, nullptr, nullptr, active, s);
 }
 
 void bvh_refit_faces(BvhBuffers& b, const int4* tri, const float4* pos, RoundCounters* rc, int n_tris_bound,
-                     cudaStream_t s, bool next_round, const int* qscan) {
-    const int gF = grid_for(n_tris_bound, 256);
-    pdl(k_boxes, gF, 256, 0, s)(tri, pos, rc, b.box_lo, b.box_hi, b.live_scan, b.scene, 1); note_launch();
-    pdl(k_reuse_leaves, gF, 256, 0, s)(rc, tri, b.box_lo, b.box_hi, next_round ? (const int*)b.keys[1] : nullptr,
-                                      b.vals[0], b.llo, b.lhi, b.visit, b.meta); note_launch();
-    bottom_up<true, false>(b, rc, n_tris_bound, b.vals[0], qscan, b.meta, nullptr, s);
+                     cudaStream_t s, bool next_round, const BvhQuery& query) {
+    pdl(k_boxes, grid_for(n_tris_bound, 256), 256, 0, s)(tri, pos, rc, b.box_lo, b.box_hi, b.live_scan, b.scene, 1, query,
+                                                       b.xq_count, b.visit, b.meta); note_launch();
+    bottom_up<true, false, kLeafReuse>(b, rc, n_tris_bound, next_round ? (const int*)b.keys[1] : nullptr, query.flags,
+                                       nullptr, s);
 }
 
-void bvh_remap(BvhBuffers& b, const int* fscan, int n_tris_bound, cudaStream_t s) {
-    pdl(k_remap_leaves, grid_for(n_tris_bound, 256), 256, 0, s)(b.meta, fscan, b.vals[0], (int*)b.keys[1]);
-    note_launch();
-}
+BvhRemap bvh_remap(const BvhBuffers& b) { return {b.meta, b.vals[0], (int*)b.keys[1]}; }
 
-void bvh_query(const BvhBuffers& b, const int4* tri, const float4* pos, const int* qlist, const int* qscan,
-               unsigned char* hit, int2* pair_list, int pair_cap, RoundCounters* rc, int n_query_bound, float eps,
-               cudaStream_t s, const int* fmesh, const int* mesh_root) {
-    (void)qlist;
-    cudaMemsetAsync(&rc->pad[1], 0, 3 * sizeof(int), s);  // list length, query count, redo count
-    // query faces in leaf order (uses the sort's second buffers, free after the build)
-    const int gF = grid_for(n_query_bound, 256);
-    pdl(k_query_order, gF, 256, 0, s)(rc, b.vals[0], qscan, b.live_scan);
-    note_launch();
-    exclusive_scan(b.live_scan, b.live_scan, &rc->n_live, 1, &rc->pad[2], b.scan_scratch, s, &rc->status,
-                   n_query_bound);
-    pdl(k_query_gather, gF, 256, 0, s)(rc, b.vals[0], b.live_scan, b.vals[1]);
+void bvh_query(const BvhBuffers& b, const int4* tri, const float4* pos, const BvhQuery& query, int2* pair_list,
+               int pair_cap, RoundCounters* rc, int n_query_bound, float eps, cudaStream_t s, const int* fmesh,
+               const int* mesh_root) {
+    // the query faces go to one of the sort's second buffers, free after the build
+    pdl(k_query_gather, grid_for((n_query_bound + 3) / 4, 256), 256, 0, s)(rc, b.vals[0], query.flags, b.vals[1]);
     note_launch();
     // b.visit (free between a tree's bottom-up passes) holds the per-query redo marks
     // a function-local static initialiser runs once even when worker threads query concurrently
@@ -1041,14 +1054,11 @@ void bvh_query(const BvhBuffers& b, const int4* tri, const float4* pos, const in
     pdl(k_traverse_list, grid_for(n_query_bound, kQueryThreads, blocks_per_sm), kQueryThreads, 0, s)(
         b.packed, b.box_lo, b.box_hi, b.vals[1], pair_list, pair_cap, rc, b.visit, fmesh, mesh_root);
     note_launch();
-    cudaMemsetAsync(b.xq_count, 0, sizeof(int), s);
-    pdl(k_pairs, grid_for((long long)pair_cap, 128, 16), 128, 0, s)(tri, pos, pair_list, pair_cap, hit, rc, eps, b.xq,
-                                                                   b.xq_cap, b.xq_count);
+    pdl(k_pairs, grid_for((long long)pair_cap, 128, 16), 128, 0, s)(tri, pos, pair_list, pair_cap, query.hit, rc, eps, b.xq,
+                                                                  b.xq_cap, b.xq_count);
     note_launch();
-    pdl(k_pairs_exact, 4 * kNumSM, 64, 0, s)(tri, pos, b.xq, b.xq_cap, b.xq_count, hit, eps);
-    note_launch();
-    pdl(k_traverse_redo, grid_for(n_query_bound, kQueryThreads, 4), kQueryThreads, 0, s)(
-        b.packed, b.box_lo, b.box_hi, tri, pos, b.vals[1], hit, rc, eps, b.visit, fmesh, mesh_root);
+    pdl(k_pairs_exact, 4 * kNumSM, kExactThreads, 0, s)(tri, pos, b.xq, b.xq_cap, b.xq_count, query.hit, eps, b.packed,
+                                                       b.box_lo, b.box_hi, b.vals[1], rc, b.visit, fmesh, mesh_root);
     note_launch();
 }
 

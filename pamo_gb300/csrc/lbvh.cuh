@@ -48,6 +48,13 @@ struct BvhMeshes {
     int* root = nullptr;
 };
 
+// The query of a check: flags[f] != 0 marks the query faces (face ids below 2^30), hit[f] receives the result. Both null:
+// the tree is built for other uses.
+struct BvhQuery {
+    const int* flags = nullptr;
+    unsigned char* hit = nullptr;
+};
+
 size_t bvh_bytes(int cap);
 // Lays the buffers out from base; clear_scan_scratch zeroes the tree's scan scratch (synchronous), which
 // memory that is not zero-initialised needs before its first build.
@@ -56,22 +63,28 @@ void bvh_carve(BvhBuffers& b, int cap, char* base, bool clear_scan_scratch = tru
 // Builds the LBVH over faces with tri[f].x != -1 (count from rc->n_tris); writes rc->n_live. With all_faces,
 // every face slot below rc->n_tris is a leaf and a removed face has an empty box, so that the tree can be
 // refitted after faces are removed or restored (bvh_refit_faces) and carried to the next round (bvh_remap).
-// qscan (exclusive scan of the query flags, or null) marks the query faces in the packed leaves for bvh_query.
+// The query's flags mark its faces in the packed leaves for bvh_query and its hit flags are cleared.
 // nodes: also keep the internal node boxes nlo/nhi for every node (the traversals of the projection stage read
 // them); the packed records that bvh_query reads are always written.
 void bvh_build(BvhBuffers& b, const int4* tri, const float4* pos, RoundCounters* rc, int n_tris_bound, cudaStream_t s,
-               bool all_faces = false, const int* qscan = nullptr, bool nodes = true,
+               bool all_faces = false, const BvhQuery& query = BvhQuery(), bool nodes = true,
                const BvhMeshes* meshes = nullptr);
 
 // New boxes for the leaves of a tree built with all_faces (a removed face, or a leaf whose face is gone, gets an
 // empty box that overlaps nothing); sets rc->n_live to the tree's leaf count. next_round: first take the leaf
-// face ids bvh_remap computed for this round's numbering.
+// face ids that the compaction left for this round's numbering (bvh_remap).
 void bvh_refit_faces(BvhBuffers& b, const int4* tri, const float4* pos, RoundCounters* rc, int n_tris_bound,
-                     cudaStream_t s, bool next_round, const int* qscan = nullptr);
+                     cudaStream_t s, bool next_round, const BvhQuery& query);
 
-// After a compaction with exclusive scan fscan of the kept faces: the leaves' face ids in the new numbering
-// (-1 for faces not kept), kept aside until bvh_refit_faces(next_round = true); repeating it is harmless.
-void bvh_remap(BvhBuffers& b, const int* fscan, int n_tris_bound, cudaStream_t s);
+// For the compaction kernel (exclusive scan fscan of the kept faces): next[i] for i < *leaves, the face of leaf i in the
+// new numbering (-1 for a face not kept), from leaf_face; kept aside until bvh_refit_faces(next_round = true), and
+// repeating it is harmless.
+struct BvhRemap {
+    const int* leaves = nullptr;  // null: no tree is carried
+    const int* leaf_face = nullptr;
+    int* next = nullptr;
+};
+BvhRemap bvh_remap(const BvhBuffers& b);
 
 // Recomputes the leaf and node boxes of a tree built by bvh_build over the same faces after the positions
 // moved (same topology and leaf order; the tree may bound more loosely than a rebuilt one). With `active`,
@@ -79,16 +92,14 @@ void bvh_remap(BvhBuffers& b, const int* fscan, int n_tris_bound, cudaStream_t s
 void bvh_refit(BvhBuffers& b, const int4* tri, const float4* pos, RoundCounters* rc, int n_tris_bound, cudaStream_t s,
                const int* active = nullptr);
 
-// For every face in the query list that is still live: hit[f] = 1 iff some live face g != f with an
-// overlapping closed AABB makes the reference's pair test true in either order. Query faces are taken
-// as the faces f with qscan[f + 1] != qscan[f] (qscan: exclusive scan of the query flags), visited in leaf
-// order. The tree must have been built or refitted with the same qscan (face ids below 2^30). Candidate pairs
-// go through pair_list (capacity pair_cap; queries beyond it decide their pairs in place).
-// qlist is unused (kept for callers that hold one).
+// For every query face that is still live: hit[f] = 1 iff some live face g != f with an overlapping closed AABB makes
+// the reference's pair test true in either order. The query faces are visited in leaf order. The tree must have been
+// built or refitted with the same query just before. Candidate pairs go through pair_list (capacity pair_cap; queries
+// beyond it decide their pairs in place).
 // With fmesh and mesh_root (from a bvh_build with BvhMeshes), each query walks only its own mesh's subtree, so
 // pairs never join two meshes.
-void bvh_query(const BvhBuffers& b, const int4* tri, const float4* pos, const int* qlist, const int* qscan,
-               unsigned char* hit, int2* pair_list, int pair_cap, RoundCounters* rc, int n_query_bound, float eps,
-               cudaStream_t s, const int* fmesh = nullptr, const int* mesh_root = nullptr);
+void bvh_query(const BvhBuffers& b, const int4* tri, const float4* pos, const BvhQuery& query, int2* pair_list,
+               int pair_cap, RoundCounters* rc, int n_query_bound, float eps, cudaStream_t s, const int* fmesh = nullptr,
+               const int* mesh_root = nullptr);
 
 }  // namespace pamo

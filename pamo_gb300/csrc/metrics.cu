@@ -340,7 +340,7 @@ int pamo_point_mesh_sqdist(const double* points, int32_t n_points, const double*
         pdl(k_to_float4, grid_for(n_vertices, kT), kT, 0, s)(vertices, n_vertices, pos);
         pdl(k_to_int4, grid_for(n_triangles, kT), kT, 0, s)(triangles, n_triangles, n_vertices, tri, &rc->status);
         note_launches(2);
-        bvh_build(b, tri, pos, rc, n_triangles, s, false, nullptr, false);
+        bvh_build(b, tri, pos, rc, n_triangles, s, false, BvhQuery(), false);
         pdl(k_point_mesh, grid_for(n_points, kQT, 16), kQT, 0, s)(points, n_points, vertices, pos, tri, b.packed, b.scene,
                                                                 b.vals[0], rc, out_sqdist, out_face, &rc->status);
         note_launch();

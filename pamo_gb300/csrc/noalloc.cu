@@ -64,7 +64,6 @@ struct Layout {
     int* occ;
     int4* tri;
     int* qflag;
-    int* qlist;
     unsigned char* hit;
     int2* exact;
     char* bvh;
@@ -86,7 +85,6 @@ Layout carve(unsigned char* base) {
     L.occ = (int*)take((kNoAllocMaxPoints + 2) * sizeof(int));
     L.tri = (int4*)take((kNoAllocMaxTriangles + 2) * sizeof(int4));
     L.qflag = (int*)take((kNoAllocMaxTriangles + 2) * sizeof(int));
-    L.qlist = (int*)take((kNoAllocMaxTriangles + 2) * sizeof(int));
     L.hit = (unsigned char*)take(kNoAllocMaxTriangles + 2);
     L.exact = (int2*)take((size_t)kExactCap * sizeof(int2));
     L.bvh = (char*)take(pamo::bvh_bytes(kNoAllocMaxTriangles));
@@ -175,16 +173,13 @@ extern "C" int pamo_self_intersect_noalloc(const float* points, const int32_t* t
 
     // the counters and flags start from zero on every call (the array keeps the previous call's contents)
     pamo::pdl(k_noalloc_init, 1, 64, 0, s)(L.rc, n_points, n_triangles);
-    cudaMemsetAsync(L.hit, 0, n_triangles + 1, s);
 
     pamo::launch_load_points(points, n_points, L.pos, L.orig_pos, L.occ, s);
     pamo::launch_load_tris(triangles, n_triangles, n_points, L.tri, L.rc, s);
     pamo::launch_live_flags(L.rc, n_triangles, L.tri, L.qflag, s);
-    pamo::exclusive_scan(L.qflag, L.qflag, &L.rc->n_tris, 1, &L.rc->n_query, L.scan_scratch, s, &L.rc->status,
-                         n_triangles);
-    pamo::launch_compact_flags(L.qflag, n_triangles, &L.rc->n_tris, L.qlist, s);
-    pamo::bvh_build(bvh, L.tri, L.pos, L.rc, n_triangles, s, false, L.qflag, false);
-    pamo::bvh_query(bvh, L.tri, L.pos, L.qlist, L.qflag, L.hit, L.exact, kExactCap, L.rc, n_triangles, kTriEps, s);
+    const pamo::BvhQuery query{L.qflag, L.hit};
+    pamo::bvh_build(bvh, L.tri, L.pos, L.rc, n_triangles, s, false, query, false);
+    pamo::bvh_query(bvh, L.tri, L.pos, query, L.exact, kExactCap, L.rc, n_triangles, kTriEps, s);
     cudaMemcpyAsync(face_hit, L.hit, n_triangles, cudaMemcpyDeviceToDevice, s);
     int status = 0;
     cudaMemcpyAsync(&status, &L.rc->status, sizeof(int), cudaMemcpyDeviceToHost, s);

@@ -114,7 +114,7 @@ struct pamo_ctx {
 
     // ---- per-face ----
     DevBuf<int4> tri, orig_tri, tri_in, tri_out;
-    DevBuf<int> ecount, qflag, qlist, fflags, nt, shuffle_flags;
+    DevBuf<int> ecount, qflag, fflags, nt, shuffle_flags;
     DevBuf<int> nxt;        // per CSR slot: the vertex after the ring's vertex in the slot's face
     DevBuf<int2> spc;       // per CSR slot: the vertex before it and its corner
     DevBuf<float4> fgeo;    // per face: a 64-byte ring record, then the planes (room for six float4 per face)
@@ -287,7 +287,7 @@ struct pamo_ctx {
         };
         fr(edge_cost); fr(invalid); fr(pts_map); fr(pts_map_prev); fr(undo_list); fr(tmp_undo);
         fr(pos); fr(orig_pos); fr(pos_in); fr(pos_out); fr(occ); fr(valence); fr(cursor); fr(quad); fr(quad_lo); fr(vmin); fr(undo_in);
-        fr(nxt); fr(spc); fr(fgeo); fr(tri); fr(orig_tri); fr(tri_in); fr(tri_out); fr(ecount); fr(qflag); fr(qlist); fr(fflags); fr(nt);
+        fr(nxt); fr(spc); fr(fgeo); fr(tri); fr(orig_tri); fr(tri_in); fr(tri_out); fr(ecount); fr(qflag); fr(fflags); fr(nt);
         fr(shuffle_flags); fr(fkey); fr(eorder); fr(vedges); fr(vcursor); fr(hit); fr(edges); fr(win); fr(collapsed); fr(uflag); fr(face_mean); fr(exact_list); fr(place); fr(probe_raw);
         if (bvh_mem) cudaFree(bvh_mem);
         bvh_mem = nullptr;
@@ -361,7 +361,7 @@ struct pamo_ctx {
              undo_in.bytes();
         b += nxt.bytes() + spc.bytes() + fgeo.bytes();
         b += tri.bytes() + orig_tri.bytes() + tri_in.bytes() + tri_out.bytes() + ecount.bytes() + qflag.bytes() +
-             qlist.bytes() + fflags.bytes() + nt.bytes() + shuffle_flags.bytes() + fkey.bytes() + hit.bytes() +
+             fflags.bytes() + nt.bytes() + shuffle_flags.bytes() + fkey.bytes() + hit.bytes() +
              edges.bytes() + win.bytes() + collapsed.bytes() + uflag.bytes() + eorder.bytes() + exact_list.bytes() +
              face_mean.bytes();
         b += edge_cost.bytes() + invalid.bytes() + pts_map.bytes() + pts_map_prev.bytes() + undo_list.bytes() +
@@ -390,7 +390,7 @@ struct pamo_ctx {
         const size_t nc = c + c / 5;
         int r;
         if ((r = grow(tri, nc)) || (r = grow(orig_tri, nc)) || (r = grow(tri_in, nc)) || (r = grow(tri_out, nc)) ||
-            (r = grow(ecount, nc + 1)) || (r = grow(qflag, nc + 1)) || (r = grow(qlist, nc)) || (r = grow(fflags, nc + 1)) ||
+            (r = grow(ecount, nc + 1)) || (r = grow(qflag, nc + 1)) || (r = grow(fflags, nc + 1)) ||
             (r = grow(nt, 3 * nc)) || (r = grow(nxt, 3 * nc)) || (r = grow(spc, 3 * nc)) || (r = grow(fgeo, 6 * nc)) || (r = grow(shuffle_flags, 2 * nc + 40)) || (r = grow(fkey, nc)) || (r = grow(hit, nc)) ||
             (r = grow(eorder, 2 * nc)) ||
             (r = grow(edges, 2 * nc)) || (r = grow(win, 2 * nc + 1)) || (r = grow(collapsed, 2 * nc)) ||
@@ -441,12 +441,12 @@ struct pamo_ctx {
         cudaMemsetAsync(vcursor.p, 0, (nP + 1) * sizeof(int), s);
         launch_face_counts(tri.p, rc, nT, valence.p, ecount.p, vedges.p, s, pos.p, fgeo.p);
         scan_adjacency_counts(s, std::max(nP, nT));
-        launch_fill_adjacency(tri.p, rc, nT, valence.p, cursor.p, nt.p, ecount.p, edges.p, vedges.p, vcursor.p, eorder.p, s);
-        launch_sort_adjacency(rc, nP, valence.p, nt.p, s);
+        launch_fill_adjacency(tri.p, rc, nT, valence.p, cursor.p, nt.p, ecount.p, edges.p, vedges.p, vcursor.p, eorder.p, s,
+                              d_ecap);
         const int* nt_off = valence.p;
         const int eb = 2 * nT;
-        launch_quadrics(rc, nP, nt_off, nt.p, tri.p, fgeo.p, quad.p, nxt.p, spc.p, s);
-        launch_edge_cost_capacity(rc, d_ecap, edge_cost.p, (int)edge_cost.n, s);
+        launch_ring_quadrics(rc, nP, nt_off, nt.p, tri.p, fgeo.p, quad.p, nxt.p, spc.p, s, nullptr, edge_cost.p,
+                             (int)edge_cost.n);
         cudaMemsetAsync(vmin.p, 0xFF, (nP + 1) * sizeof(unsigned long long), s);
         launch_edge_cost(rc, eb, eorder.p, edges.p, nt_off, nt.p, tri.p, pos.p, quad.p, fgeo.p, nxt.p, spc.p, invalid.p, edge_cost.p, vmin.p,
                          d_scale, threshold, 0, s, nullptr, true, skinny_pow);
@@ -487,9 +487,8 @@ struct pamo_ctx {
         launch_face_counts(tri.p, rc, nT, valence.p, ecount.p, vedges.p, s, pos.p, fgeo.p, mode > 0);
         scan_adjacency_counts(s, std::max(nP, nT));
         launch_fill_adjacency(tri.p, rc, nT, valence.p, cursor.p, nt.p, ecount.p, edges.p, vedges.p, vcursor.p, eorder.p, s);
-        launch_sort_adjacency(rc, nP, valence.p, nt.p, s);
         Quadric* qlo = mode > 0 ? quad_lo.p : nullptr;
-        launch_quadrics(rc, nP, valence.p, nt.p, tri.p, fgeo.p, quad.p, nxt.p, spc.p, s, qlo);
+        launch_ring_quadrics(rc, nP, valence.p, nt.p, tri.p, fgeo.p, quad.p, nxt.p, spc.p, s, qlo);
         cudaMemsetAsync(vmin.p, 0xFF, (nP + 1) * sizeof(unsigned long long), s);
         cudaMemsetAsync(probe_raw.p, 0xFF, probe_raw.n * sizeof(float), s);  // NaN where no cost is computed
         launch_edge_cost(rc, 2 * nT, eorder.p, edges.p, valence.p, nt.p, tri.p, pos.p, quad.p, fgeo.p, nxt.p, spc.p, invalid.p,
@@ -524,19 +523,25 @@ struct pamo_ctx {
         const int list_cap = (int)undo_list.n;
         const uint32_t collapse_t = collapse_threshold(threshold);
         if (kind != 1) {
-            launch_round_begin(rc, d_ls, d_ls + 1, s);
-            launch_undo_bookkeeping_dev(undo_in.p, d_ls, list_cap, tmp_undo.p, undo_list.p, pts_map.p, (int)pts_map.n,
-                                        invalid.p, (int)invalid.n, s);
-            launch_round_prologue_dev(d_ls, rc, nPb, nTb, pts_map.p, pts_map_prev.p, pos_in.p, pos.p, orig_pos.p, occ.p,
-                                      tri_in.p, tri.p, orig_tri.p, valence.p, cursor.p, vedges.p, vcursor.p, qflag.p, s);
-            launch_face_counts(tri.p, rc, nTb, valence.p, ecount.p, vedges.p, s, pos.p, fgeo.p, precision > 0);
+            RoundStart rs;
+            rs.next = d_ls + 1; rs.ls = d_ls; rs.rc = rc;
+            rs.invalid = invalid.p; rs.invalid_len = (int)invalid.n;
+            rs.pts_map = pts_map.p; rs.pts_map_prev = pts_map_prev.p;
+            rs.pts_in = pos_in.p; rs.pos = pos.p; rs.orig_pos = orig_pos.p; rs.occ = occ.p;
+            rs.tri_in = tri_in.p; rs.tri = tri.p; rs.orig_tri = orig_tri.p;
+            rs.valence = valence.p; rs.cursor = cursor.p; rs.vedges = vedges.p; rs.vcursor = vcursor.p;
+            rs.qflag = qflag.p; rs.vmin = vmin.p;
+            launch_round_prologue_dev(rs, nPb, nTb, s);
+            UndoBook book;
+            book.ls = d_ls; book.verts_undo = undo_in.p; book.tmp_undo = tmp_undo.p; book.undo_list = undo_list.p;
+            book.pts_map = pts_map.p; book.map_len = (int)pts_map.n;
+            book.invalid = invalid.p; book.invalid_len = (int)invalid.n;
+            launch_face_counts(tri.p, rc, nTb, valence.p, ecount.p, vedges.p, s, pos.p, fgeo.p, precision > 0, book);
             scan_adjacency_counts(s, std::max(nPb, nTb));
             launch_fill_adjacency(tri.p, rc, nTb, valence.p, cursor.p, nt.p, ecount.p, edges.p, vedges.p, vcursor.p,
-                                  eorder.p, s);
-            launch_sort_adjacency(rc, nPb, valence.p, nt.p, s);
-            launch_quadrics(rc, nPb, nt_off, nt.p, tri.p, fgeo.p, quad.p, nxt.p, spc.p, s, qlo_ptr());
-            launch_edge_cost_capacity(rc, d_ecap, edge_cost.p, (int)edge_cost.n, s);
-            launch_fill_u64_dev(rc, nPb, vmin.p, ~0ull, s);
+                                  eorder.p, s, d_ecap);
+            launch_ring_quadrics(rc, nPb, nt_off, nt.p, tri.p, fgeo.p, quad.p, nxt.p, spc.p, s, qlo_ptr(), edge_cost.p,
+                                 (int)edge_cost.n);
             cost_begin(s);
             launch_edge_cost(rc, eb, eorder.p, edges.p, nt_off, nt.p, tri.p, pos.p, quad.p, fgeo.p, nxt.p, spc.p, invalid.p, edge_cost.p,
                              vmin.p, d_scale, threshold, 0, s, &d_ls->is_stuck, false, skinny_pow, precision, nullptr,
@@ -546,30 +551,24 @@ struct pamo_ctx {
             launch_collapse(rc, eb, eorder.p, edges.p, edge_cost.p, collapse_t, fkey.p, nt_off, nt.p, tri.p, orig_tri.p,
                             pos.p, orig_pos.p, occ.p, win.p, s, true, place_ptr());
             exclusive_scan(win.p, win.p, &rc->n_edges, 1, &rc->n_win, scan_scratch, s, &rc->status, eb);
-            launch_compact_winners(rc, eb, win.p, collapsed.p, s);
-            launch_remove_invalid(rc, nTb, tri.p, s);
-            launch_line_edges(rc, eb, edges.p, nt_off, nt.p, tri.p, pos.p, occ.p, nullptr, (int)collapsed.n,
-                              collapsed.p, s);
+            launch_after_collapse(rc, eb, nTb, win.p, collapsed.p, edges.p, nt_off, nt.p, tri.p, pos.p, occ.p,
+                                  (int)collapsed.n, true, s);
             launch_mark_query(rc, eb, collapsed.p, edges.p, nt_off, nt.p, qflag.p, s);
-            exclusive_scan(qflag.p, qflag.p, &rc->n_tris, 1, &rc->n_query, scan_scratch, s, &rc->status, nTb);
-            launch_compact_flags(qflag.p, nTb, &rc->n_tris, qlist.p, s);
         } else {
             launch_undo_apply(rc, eb, collapsed.p, uflag.p, edges.p, nt_off, nt.p, tri.p, orig_tri.p, pos.p, orig_pos.p,
                               occ.p, tmp_undo.p, undo_list.p, pts_map_prev.p, list_cap, s);
         }
         // intersection check; the LBVH spans every face slot of the round and is refitted when reused
-        launch_zero_face_bytes_dev(rc, nTb, hit.p, s);
-        if (kind == 0) bvh_build(bvh, tri.p, pos.p, rc, nTb, s, true, qflag.p, false);
-        else bvh_refit_faces(bvh, tri.p, pos.p, rc, nTb, s, kind == 2, qflag.p);
-        bvh_query(bvh, tri.p, pos.p, qlist.p, qflag.p, hit.p, exact_list.p, pair_cap(), rc, nTb, kTriEps, s);
-        launch_undo_check(rc, eb, collapsed.p, edges.p, nt_off, nt.p, hit.p, uflag.p, s);
-        exclusive_scan(uflag.p, uflag.p, &rc->n_considered, 1, &rc->n_undo, scan_scratch, s, &rc->status, eb);
-        launch_after_check(rc, s);
-        // compaction map (cusimp_free.cu:1042-1045), compaction (pamo/__init__.py:136-140), next round's state
-        launch_live_flags(rc, nTb, tri.p, fflags.p, s);
-        scan_compaction_maps(s, std::max(nPb, nTb));
-        launch_compact_mesh(rc, nPb, nTb, pos.p, occ.p, pts_map.p, tri.p, fflags.p, pos_out.p, tri_out.p, s);
-        bvh_remap(bvh, fflags.p, nTb, s);  // the tree's leaves in the next round's face numbering
+        const BvhQuery query{qflag.p, hit.p};
+        if (kind == 0) bvh_build(bvh, tri.p, pos.p, rc, nTb, s, true, query, false);
+        else bvh_refit_faces(bvh, tri.p, pos.p, rc, nTb, s, kind == 2, query);
+        bvh_query(bvh, tri.p, pos.p, query, exact_list.p, pair_cap(), rc, nTb, kTriEps, s);
+        launch_undo_check(rc, eb, collapsed.p, edges.p, nt_off, nt.p, hit.p, uflag.p, s, tri.p, fflags.p);
+        // the undo edges, and the compaction (cusimp_free.cu:1042-1045, pamo/__init__.py:136-140) with the tree's leaves
+        // in the next round's face numbering; then the next round's state
+        scan_undo_and_maps(s, std::max(eb, std::max(nPb, nTb)));
+        launch_compact_mesh(rc, nPb, nTb, pos.p, occ.p, pts_map.p, tri.p, fflags.p, pos_out.p, tri_out.p, s, true,
+                            bvh_remap(bvh));
         launch_round_end(rc, d_ls, d_ls + 1, undo_list.p, undo_in.p, (int)std::min(undo_in.n, undo_list.n), list_cap, s);
     }
 
@@ -583,12 +582,14 @@ struct pamo_ctx {
         exclusive_scans(jobs, 3, s, &rc->status, bound);
     }
 
-    // The vertex compaction map (occ -> pts_map) and the live-face offsets, scanned by one launch.
-    void scan_compaction_maps(cudaStream_t s, long long bound) {
+    // The undo edges' offsets (their total the undo count), the vertex compaction map (occ -> pts_map) and the live-face
+    // offsets, scanned by one launch.
+    void scan_undo_and_maps(cudaStream_t s, long long bound) {
         const size_t sz = scan_scratch_ints();
-        const ScanJob jobs[2] = {{occ.p, pts_map.p, &rc->n_pts, 1, nullptr, scan_scratch},
-                                 {fflags.p, fflags.p, &rc->n_tris, 1, nullptr, scan_scratch + sz}};
-        exclusive_scans(jobs, 2, s, &rc->status, bound);
+        const ScanJob jobs[3] = {{uflag.p, uflag.p, &rc->n_considered, 1, &rc->n_undo, scan_scratch},
+                                 {occ.p, pts_map.p, &rc->n_pts, 1, nullptr, scan_scratch + sz},
+                                 {fflags.p, fflags.p, &rc->n_tris, 1, nullptr, scan_scratch + 2 * sz}};
+        exclusive_scans(jobs, 3, s, &rc->status, bound);
     }
 
     // Enqueue round_dev through a cached graph of its size class (or directly when graphs are off or the
@@ -701,17 +702,17 @@ struct pamo_ctx {
         cudaMemsetAsync(vcursor.p, 0, (nP + 1) * sizeof(int), s);
         launch_face_counts(tri.p, rc, nT, valence.p, ecount.p, vedges.p, s, pos.p, fgeo.p, precision > 0);
         scan_adjacency_counts(s, std::max(nP, nT));
-        launch_fill_adjacency(tri.p, rc, nT, valence.p, cursor.p, nt.p, ecount.p, edges.p, vedges.p, vcursor.p, eorder.p, s);
-        launch_sort_adjacency(rc, nP, valence.p, nt.p, s);
+        launch_fill_adjacency(tri.p, rc, nT, valence.p, cursor.p, nt.p, ecount.p, edges.p, vedges.p, vcursor.p, eorder.p, s,
+                              d_ecap);
         const int* nt_off = valence.p;
         const int eb = 2 * nT;
         prof.end(kPhAdj, s);
 
         // cost and selection
         prof.begin(kPhQuad, s);
-        launch_quadrics(rc, nP, nt_off, nt.p, tri.p, fgeo.p, quad.p, nxt.p, spc.p, s, qlo_ptr());
+        launch_ring_quadrics(rc, nP, nt_off, nt.p, tri.p, fgeo.p, quad.p, nxt.p, spc.p, s, qlo_ptr(), edge_cost.p,
+                             (int)edge_cost.n);
         prof.end(kPhQuad, s);
-        launch_edge_cost_capacity(rc, d_ecap, edge_cost.p, (int)edge_cost.n, s);
         cudaMemsetAsync(vmin.p, 0xFF, (nP + 1) * sizeof(unsigned long long), s);
         prof.begin(kPhCost, s);
         cost_begin(s);
@@ -725,28 +726,25 @@ struct pamo_ctx {
         launch_collapse(rc, eb, eorder.p, edges.p, edge_cost.p, collapse_t, fkey.p, nt_off, nt.p, tri.p, orig_tri.p, pos.p,
                         orig_pos.p, occ.p, win.p, s, true, place_ptr());
         exclusive_scan(win.p, win.p, &rc->n_edges, 1, &rc->n_win, scan_scratch, s, &rc->status, eb);
-        launch_compact_winners(rc, eb, win.p, collapsed.p, s);
+        launch_after_collapse(rc, eb, nT, win.p, collapsed.p, edges.p, nt_off, nt.p, tri.p, pos.p, occ.p, (int)collapsed.n,
+                              true, s);
         prof.end(kPhCollapse, s);
         prof.begin(kPhMarks, s);
-        launch_remove_invalid(rc, nT, tri.p, s);
-        launch_line_edges(rc, eb, edges.p, nt_off, nt.p, tri.p, pos.p, occ.p, nullptr, (int)collapsed.n, collapsed.p, s);
 
         // faces whose intersections decide the undo: rings of the considered collapsed edges
         cudaMemsetAsync(qflag.p, 0, (nT + 1) * sizeof(int), s);
         launch_mark_query(rc, eb, collapsed.p, edges.p, nt_off, nt.p, qflag.p, s);
-        exclusive_scan(qflag.p, qflag.p, &rc->n_tris, 1, &rc->n_query, scan_scratch, s, &rc->status, nT);
-        launch_compact_flags(qflag.p, nT, &rc->n_tris, qlist.p, s);
         prof.end(kPhMarks, s);
 
         // self-intersection check and undo passes (cusimp_free.cu:1014-1040)
         const int list_cap = (int)undo_list.n;
         auto check_pass = [&]() {
-            cudaMemsetAsync(hit.p, 0, nT + 1, s);
+            const BvhQuery query{qflag.p, hit.p};
             prof.begin(kPhBvh, s);
-            bvh_build(bvh, tri.p, pos.p, rc, nT, s, false, qflag.p, false);
+            bvh_build(bvh, tri.p, pos.p, rc, nT, s, false, query, false);
             prof.end(kPhBvh, s);
             prof.begin(kPhQuery, s);
-            bvh_query(bvh, tri.p, pos.p, qlist.p, qflag.p, hit.p, exact_list.p, pair_cap(), rc, nT, kTriEps, s);
+            bvh_query(bvh, tri.p, pos.p, query, exact_list.p, pair_cap(), rc, nT, kTriEps, s);
             prof.end(kPhQuery, s);
             launch_undo_check(rc, eb, collapsed.p, edges.p, nt_off, nt.p, hit.p, uflag.p, s);
             exclusive_scan(uflag.p, uflag.p, &rc->n_considered, 1, &rc->n_undo, scan_scratch, s, &rc->status, eb);
@@ -1260,12 +1258,9 @@ int pamo_self_intersect(pamo_ctx* ctx, const float* points, const int32_t* trian
     launch_load_tris(triangles, n_triangles, n_points, ctx->tri.p, ctx->rc, s);
     // every live face queries
     launch_live_flags(ctx->rc, n_triangles, ctx->tri.p, ctx->qflag.p, s);
-    exclusive_scan(ctx->qflag.p, ctx->qflag.p, &ctx->rc->n_tris, 1, &ctx->rc->n_query, ctx->scan_scratch, s,
-                   &ctx->rc->status, n_triangles);
-    launch_compact_flags(ctx->qflag.p, n_triangles, &ctx->rc->n_tris, ctx->qlist.p, s);
-    cudaMemsetAsync(ctx->hit.p, 0, n_triangles + 1, s);
-    bvh_build(ctx->bvh, ctx->tri.p, ctx->pos.p, ctx->rc, n_triangles, s, false, ctx->qflag.p, false);
-    bvh_query(ctx->bvh, ctx->tri.p, ctx->pos.p, ctx->qlist.p, ctx->qflag.p, ctx->hit.p, ctx->exact_list.p,
+    const BvhQuery query{ctx->qflag.p, ctx->hit.p};
+    bvh_build(ctx->bvh, ctx->tri.p, ctx->pos.p, ctx->rc, n_triangles, s, false, query, false);
+    bvh_query(ctx->bvh, ctx->tri.p, ctx->pos.p, query, ctx->exact_list.p,
               ctx->pair_cap(), ctx->rc, n_triangles, kTriEps, s);
     cudaMemcpyAsync(face_hit, ctx->hit.p, n_triangles, cudaMemcpyDeviceToDevice, s);
     if ((r = ctx->read_counters())) return r;

@@ -12,6 +12,8 @@
 //     of scanning the whole intersection list per collapsed edge (:776-827).
 #include <cstdint>
 #include <type_traits>
+#include <algorithm>
+
 #include "scan.cuh"
 #include "simp_round.cuh"
 #include "round_ops.cuh"
@@ -201,9 +203,23 @@ __device__ __forceinline__ float acc_value(const CSum& a) { return a.value(); }
 // plane_df (precision mode): the planes as double-float pairs, fgeo[4n + 2f] (hi) and fgeo[4n + 2f + 1] (lo)
 __global__ void __launch_bounds__(kT) k_face_counts(const int4* __restrict__ tri, const RoundCounters* rc, int* valence,
                                                     int* ecount, int* vedges, const float4* __restrict__ pos,
-                                                    float4* fgeo, int plane_df) {
+                                                    float4* fgeo, int plane_df, UndoBook book) {
     pdl_wait();
     const int n = rc->n_tris;
+    if (book.ls) {
+        // stuck: the undo list restarts from the carried vertices mapped through the previous map (:869-878);
+        // then the carried vertices are marked invalid (:880-889)
+        const int m = book.ls->nu;
+        const bool stuck = book.ls->is_stuck != 0;
+        for (int a = gtid(); a < m; a += gstride()) {
+            const int x = book.verts_undo[a];
+            if (stuck) {
+                book.tmp_undo[a] = x;
+                book.undo_list[a] = (x >= 0 && x < book.map_len) ? book.pts_map[x] : 0;
+            }
+            if (x >= 0 && x < book.invalid_len) book.invalid[x] = 1;
+        }
+    }
     for (int f = gtid(); f < n; f += gstride()) {
         const int4 t = tri[f];
         if (face_killed(t)) {
@@ -242,12 +258,21 @@ __global__ void __launch_bounds__(kT) k_face_counts(const int4* __restrict__ tri
     if (gtid() == 0) ecount[n] = 0;
 }
 
-__global__ void __launch_bounds__(kT) k_fill_adjacency(const int4* __restrict__ tri, const RoundCounters* rc,
+// d_cap (or null): the length of the edge costs as the reference sizes them; rc->pad[0] says whether it grew, and then the
+// costs start from zero (k_ring_quadrics)
+__global__ void __launch_bounds__(kT) k_fill_adjacency(const int4* __restrict__ tri, RoundCounters* rc,
                                                        const int* __restrict__ nt_off, int* cursor, int* nt,
                                                        const int* __restrict__ edge_off, int2* edges,
-                                                       const int* __restrict__ voff, int* vcursor, int* eorder) {
+                                                       const int* __restrict__ voff, int* vcursor, int* eorder,
+                                                       int* d_cap) {
     pdl_wait();
     const int n = rc->n_tris;
+    if (d_cap && gtid() == 0) {
+        const int ne = rc->n_edges;
+        const int grow = ne > *d_cap;
+        if (grow) *d_cap = ne + ne / 5;
+        rc->pad[0] = grow;
+    }
     for (int f = gtid(); f < n; f += gstride()) {
         const int4 t = tri[f];
         if (face_killed(t)) continue;
@@ -270,11 +295,55 @@ __global__ void __launch_bounds__(kT) k_fill_adjacency(const int4* __restrict__ 
     }
 }
 
-__global__ void __launch_bounds__(kT) k_sort_adjacency(const RoundCounters* rc, const int* __restrict__ nt_off, int* nt) {
-    pdl_wait();
-    const int n = rc->n_pts;
-    for (int v = gtid(); v < n; v += gstride()) {
-        const int a = nt_off[v], b = nt_off[v + 1];
+// ------------------------------------------------------------------ quadrics (compute_vert_Q_kernel, :337-366)
+__device__ __forceinline__ void face_plane(const float4* __restrict__ pos, int4 t, float p[4]) {
+    const V3 v0 = v3(pos[t.x]), v1 = v3(pos[t.y]), v2 = v3(pos[t.z]);
+    V3 n = vcross(vsub(v1, v0), vsub(v2, v0));
+    n = vdiv(n, vnorm(n));
+    p[0] = n.x;
+    p[1] = n.y;
+    p[2] = n.z;
+    p[3] = -vdot(n, v0);
+}
+
+// Sorts r[0 .. N) ascending (N a power of two) by Batcher's odd-even merge exchange, all in registers.
+template <int N>
+__device__ __forceinline__ void sort_registers(int (&r)[N]) {
+#pragma unroll
+    for (int p = 1; p < N; p *= 2)
+#pragma unroll
+        for (int k = p; k >= 1; k /= 2)
+#pragma unroll
+            for (int j = k % p; j + k < N; j += 2 * k)
+#pragma unroll
+                for (int i = 0; i < k; ++i)
+                    if (i + j + k < N && (i + j) / (2 * p) == (i + j + k) / (2 * p)) {
+                        const int lo = min(r[i + j], r[i + j + k]), hi = max(r[i + j], r[i + j + k]);
+                        r[i + j] = lo;
+                        r[i + j + k] = hi;
+                    }
+}
+
+// The faces nt[a, b) of a ring into ascending order. The rings are filled by atomics, so their order is arbitrary. A ring
+// of up to 16 faces (nearly all) is sorted in registers; sorted in place, its loads and stores were a chain of L2
+// latencies (22 us of a mean round of 1.29 ms from 5.24M faces, 9.4 us of one of 0.25 ms from 1,280).
+template <int N>
+__device__ __forceinline__ void sort_ring_small(int* nt, int a, int m) {
+    int r[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) r[k] = k < m ? nt[a + k] : 0x7fffffff;
+    sort_registers<N>(r);
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+        if (k < m) nt[a + k] = r[k];
+}
+__device__ __forceinline__ void sort_ring(int* nt, int a, int b) {
+    const int m = b - a;
+    if (m <= 8) {
+        sort_ring_small<8>(nt, a, m);
+    } else if (m <= 16) {
+        sort_ring_small<16>(nt, a, m);
+    } else {
         for (int i = a + 1; i < b; ++i) {
             const int x = nt[i];
             int j = i - 1;
@@ -287,56 +356,64 @@ __global__ void __launch_bounds__(kT) k_sort_adjacency(const RoundCounters* rc, 
     }
 }
 
-// ------------------------------------------------------------------ quadrics (compute_vert_Q_kernel, :337-366)
-__device__ __forceinline__ void face_plane(const float4* __restrict__ pos, int4 t, float p[4]) {
-    const V3 v0 = v3(pos[t.x]), v1 = v3(pos[t.y]), v2 = v3(pos[t.z]);
-    V3 n = vcross(vsub(v1, v0), vsub(v2, v0));
-    n = vdiv(n, vnorm(n));
-    p[0] = n.x;
-    p[1] = n.y;
-    p[2] = n.z;
-    p[3] = -vdot(n, v0);
-}
-
-// Quadrics from the face planes of fgeo; also, per ring slot s of v (face t = tri[nt[s]]), nxt[s] = the vertex
-// after v in t (the link condition's per-slot value) and spc[s] = (the vertex before v, the corner c of v: the
-// first of t.x, t.y, t.z equal to v), from which the ring passes rebuild t without reading it.
+// The rings in face order, then the quadrics from the face planes of fgeo; also, per ring slot s of v (face t =
+// tri[nt[s]]), nxt[s] = the vertex after v in t (the link condition's per-slot value) and spc[s] = (the vertex before v,
+// the corner c of v: the first of t.x, t.y, t.z equal to v), from which the ring passes rebuild t without reading it.
+// Four slots at a time, so that their gathers are in flight together; the sums run in slot order.
 // kComp (precision mode): every entry summed with compensation (products by TwoProd, sums by TwoSum), rounded once
+// cost (or null): zeroed where the edge costs grew (rc->pad[0], k_fill_adjacency)
 template <bool kComp>
-__global__ void __launch_bounds__(kT) k_quadrics(const RoundCounters* rc, const int* __restrict__ nt_off,
-                                                 const int* __restrict__ nt, const int4* __restrict__ tri,
-                                                 const float4* __restrict__ fgeo, Quadric* q, int* nxt,
-                                                 int2* spc, Quadric* qlo) {
+__global__ void __launch_bounds__(kT) k_ring_quadrics(const RoundCounters* rc, const int* __restrict__ nt_off, int* nt,
+                                                      const int4* __restrict__ tri, const float4* __restrict__ fgeo,
+                                                      Quadric* q, int* nxt, int2* spc, Quadric* qlo, uint32_t* cost,
+                                                      int cost_len) {
     pdl_wait();
+    if (cost && rc->pad[0])
+        for (int i = gtid(); i < cost_len; i += gstride()) cost[i] = 0u;
     const int n = rc->n_pts;
     const size_t planes = 4 * (size_t)rc->n_tris;
     for (int v = gtid(); v < n; v += gstride()) {
         float m00 = 0.f, m01 = 0.f, m02 = 0.f, m03 = 0.f, m11 = 0.f, m12 = 0.f, m13 = 0.f, m22 = 0.f, m23 = 0.f, m33 = 0.f;
         CSum c[10];
-        const int b = nt_off[v + 1];
-        for (int s = nt_off[v]; s < b; ++s) {
-            const int f = nt[s];
-            const int4 t = tri[f];
-            const int corner = t.x == v ? 0 : (t.y == v ? 1 : 2);
-            nxt[s] = corner == 0 ? t.y : (corner == 1 ? t.z : t.x);
-            spc[s] = make_int2(corner == 0 ? t.z : (corner == 1 ? t.x : t.y), corner);
-            if constexpr (kComp) {  // double-float planes (face_plane_df), double-float products and sums
-                const float4 ph = fgeo[planes + 2 * (size_t)f], pl = fgeo[planes + 2 * (size_t)f + 1];
-                const DF d[4] = {{ph.x, pl.x}, {ph.y, pl.y}, {ph.z, pl.z}, {ph.w, pl.w}};
-                const int ij[10][2] = {{0, 0}, {0, 1}, {0, 2}, {0, 3}, {1, 1}, {1, 2}, {1, 3}, {2, 2}, {2, 3}, {3, 3}};
+        const int a = nt_off[v], b = nt_off[v + 1];
+        sort_ring(nt, a, b);
+        for (int s0 = a; s0 < b; s0 += 4) {
+            int f4[4];
+            int4 t4[4];
+            float4 p4[4];
 #pragma unroll
-                for (int k = 0; k < 10; ++k) {
-                    const DF pr = df_mul(d[ij[k][0]], d[ij[k][1]]);
-                    c[k].add(pr.hi);
-                    c[k].c += pr.lo;
+            for (int k = 0; k < 4; ++k) f4[k] = s0 + k < b ? nt[s0 + k] : -1;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (f4[k] < 0) continue;
+                t4[k] = tri[f4[k]];
+                p4[k] = kComp ? fgeo[planes + 2 * (size_t)f4[k]] : fgeo[planes + f4[k]];
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (f4[k] < 0) continue;
+                const int s = s0 + k;
+                const int4 t = t4[k];
+                const int corner = t.x == v ? 0 : (t.y == v ? 1 : 2);
+                nxt[s] = corner == 0 ? t.y : (corner == 1 ? t.z : t.x);
+                spc[s] = make_int2(corner == 0 ? t.z : (corner == 1 ? t.x : t.y), corner);
+                if constexpr (kComp) {  // double-float planes (face_plane_df), double-float products and sums
+                    const float4 ph = p4[k], pl = fgeo[planes + 2 * (size_t)f4[k] + 1];
+                    const DF d[4] = {{ph.x, pl.x}, {ph.y, pl.y}, {ph.z, pl.z}, {ph.w, pl.w}};
+                    const int ij[10][2] = {{0, 0}, {0, 1}, {0, 2}, {0, 3}, {1, 1}, {1, 2}, {1, 3}, {2, 2}, {2, 3}, {3, 3}};
+#pragma unroll
+                    for (int e = 0; e < 10; ++e) {
+                        const DF pr = df_mul(d[ij[e][0]], d[ij[e][1]]);
+                        c[e].add(pr.hi);
+                        c[e].c += pr.lo;
+                    }
+                } else {
+                    const float p[4] = {p4[k].x, p4[k].y, p4[k].z, p4[k].w};
+                    m00 += p[0] * p[0]; m01 += p[0] * p[1]; m02 += p[0] * p[2]; m03 += p[0] * p[3];
+                    m11 += p[1] * p[1]; m12 += p[1] * p[2]; m13 += p[1] * p[3];
+                    m22 += p[2] * p[2]; m23 += p[2] * p[3];
+                    m33 += p[3] * p[3];
                 }
-            } else {
-                const float4 pl = fgeo[planes + f];
-                const float p[4] = {pl.x, pl.y, pl.z, pl.w};
-                m00 += p[0] * p[0]; m01 += p[0] * p[1]; m02 += p[0] * p[2]; m03 += p[0] * p[3];
-                m11 += p[1] * p[1]; m12 += p[1] * p[2]; m13 += p[1] * p[3];
-                m22 += p[2] * p[2]; m23 += p[2] * p[3];
-                m33 += p[3] * p[3];
             }
         }
         if constexpr (kComp) {  // each entry as hi (q) + lo (qlo)
@@ -690,23 +767,6 @@ __global__ void __launch_bounds__(kT) k_edge_cost(const RoundCounters* rc, const
     }
 }
 
-__global__ void k_edge_cost_capacity(RoundCounters* rc, int* d_cap) {
-    pdl_wait();
-    const int n = rc->n_edges;
-    int grow = 0;
-    if (n > *d_cap) {
-        *d_cap = n + n / 5;
-        grow = 1;
-    }
-    rc->pad[0] = grow;
-}
-
-__global__ void k_edge_cost_zero(const RoundCounters* rc, uint32_t* cost, int len) {
-    pdl_wait();
-    if (!rc->pad[0]) return;
-    for (int i = gtid(); i < len; i += gstride()) cost[i] = 0u;
-}
-
 __global__ void __launch_bounds__(kT) k_face_keys(const RoundCounters* rc, const int4* __restrict__ tri,
                                                   const unsigned long long* __restrict__ vmin, unsigned long long* fkey) {
     pdl_wait();
@@ -792,43 +852,13 @@ __global__ void __launch_bounds__(kT) k_collapse(RoundCounters* rc, const int* _
     }
 }
 
-__global__ void k_compact_winners(const RoundCounters* rc, const int* __restrict__ scan, int* collapsed) {
-    pdl_wait();
-    const int n = rc->n_edges;
-    for (int e = gtid(); e < n; e += gstride())
-        if (scan[e + 1] != scan[e]) collapsed[scan[e]] = e;
-}
-
-__global__ void __launch_bounds__(kT) k_remove_invalid(const RoundCounters* rc, int4* tri) { pdl_wait();  // :218-232
-    const int n = rc->n_tris;
-    for (int f = gtid(); f < n; f += gstride()) {
-        const int4 t = tri[f];
-        if (face_killed(t)) continue;
-        if (t.x == t.y || t.y == t.z || t.z == t.x) tri[f] = make_int4(-1, -1, -1, 0);
-    }
-}
-
-__global__ void __launch_bounds__(kT) k_line_detect(RoundCounters* rc, const int2* __restrict__ edges, const float4* pos) {
-    pdl_wait();
-    const int n = rc->n_edges;
-    int found = 0;
-    for (int e = gtid(); e < n; e += gstride()) {
-        const int2 ed = edges[e];
-        const float4 p = pos[ed.x], q = pos[ed.y];
-        if (p.x == q.x && p.y == q.y && p.z == q.z) found = 1;
-    }
-    if (__any_sync(0xffffffffu, found) && (threadIdx.x & 31) == 0) atomicAdd(&rc->n_line, 1);
-}
-
 // remove_line_edge_collapse (:234-274), applied in edge order by one thread when any coincident edge exists;
 // then the collapsed-list bookkeeping of forward() (:1004-1016).
-__global__ void k_line_apply(RoundCounters* rc, const int2* __restrict__ edges, const int* __restrict__ nt_off,
-                             const int* __restrict__ nt, int4* tri, float4* pos, int* occ, int* collapsed, int cap) {
-    pdl_wait();
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+__device__ void line_apply(RoundCounters* rc, const int2* __restrict__ edges, const int* __restrict__ nt_off,
+                           const int* __restrict__ nt, int4* tri, float4* pos, int* occ, int* collapsed, int cap) {
     const int h = rc->n_win;
     int k = h;
-    if (rc->n_line > 0) {
+    if (*(volatile int*)&rc->n_line > 0) {
         const int n = rc->n_edges;
         for (int e = 0; e < n; ++e) {
             const int2 ed = edges[e];
@@ -849,6 +879,41 @@ __global__ void k_line_apply(RoundCounters* rc, const int2* __restrict__ edges, 
     rc->n_considered = (h == 0) ? 0 : (k < roundup ? k : roundup);
 }
 
+// After the collapses, in one launch: the winners' list in edge order, the faces that became degenerate removed
+// (:218-232), the edges with coincident endpoints counted in rc->n_line, and, with kLines, line_apply by the block that
+// finishes last (rc->pad[4] counts them; zero at a round's start). The three passes touch different arrays.
+template <bool kLines>
+__global__ void __launch_bounds__(kT) k_after_collapse(RoundCounters* rc, const int* __restrict__ scan, int* collapsed,
+                                                       const int2* __restrict__ edges, const int* __restrict__ nt_off,
+                                                       const int* __restrict__ nt, int4* tri, float4* pos, int* occ,
+                                                       int line_cap) {
+    pdl_wait();
+    const int ne = rc->n_edges, nf = rc->n_tris;
+    int found = 0;
+    for (int e = gtid(); e < ne; e += gstride()) {
+        if (scan[e + 1] != scan[e]) collapsed[scan[e]] = e;
+        const int2 ed = edges[e];
+        const float4 p = pos[ed.x], q = pos[ed.y];
+        if (p.x == q.x && p.y == q.y && p.z == q.z) found = 1;
+    }
+    for (int f = gtid(); f < nf; f += gstride()) {
+        const int4 t = tri[f];
+        if (face_killed(t)) continue;
+        if (t.x == t.y || t.y == t.z || t.z == t.x) tri[f] = make_int4(-1, -1, -1, 0);
+    }
+    if (__any_sync(0xffffffffu, found) && (threadIdx.x & 31) == 0) atomicAdd(&rc->n_line, 1);
+    if constexpr (kLines) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            if (atomicAdd(&rc->pad[4], 1) == (int)gridDim.x - 1) {
+                __threadfence();
+                line_apply(rc, edges, nt_off, nt, tri, pos, occ, collapsed, line_cap);
+            }
+        }
+    }
+}
+
 // ------------------------------------------------------------------ rollback
 __global__ void k_mark_query(const RoundCounters* rc, const int* __restrict__ collapsed, const int2* __restrict__ edges,
                              const int* __restrict__ nt_off, const int* __restrict__ nt, int* qflag) {
@@ -861,17 +926,16 @@ __global__ void k_mark_query(const RoundCounters* rc, const int* __restrict__ co
     }
 }
 
-__global__ void k_compact_flags(const int* __restrict__ scan, const int* d_n, int* out) {
-    pdl_wait();
-    const int n = *d_n;
-    for (int i = gtid(); i < n; i += gstride())
-        if (scan[i + 1] != scan[i]) out[scan[i]] = i;
-}
-
+// with fflags: also the faces that the compaction keeps (k_live_flags)
 __global__ void k_undo_check(RoundCounters* rc, const int* __restrict__ collapsed, const int2* __restrict__ edges,
                              const int* __restrict__ nt_off, const int* __restrict__ nt, const unsigned char* __restrict__ hit,
-                             int* uflag) {
+                             int* uflag, const int4* __restrict__ tri, int* fflags) {
     pdl_wait();
+    if (fflags) {
+        const int nf = rc->n_tris;
+        for (int f = gtid(); f < nf; f += gstride()) fflags[f] = (tri[f].x >= 0) ? 1 : 0;
+        if (gtid() == 0) fflags[nf] = 0;
+    }
     const int n = rc->n_considered;
     if (gtid() == 0) uflag[n] = 0;
     for (int c = gtid(); c < n; c += gstride()) {
@@ -883,12 +947,16 @@ __global__ void k_undo_check(RoundCounters* rc, const int* __restrict__ collapse
     }
 }
 
-__global__ void k_after_check(RoundCounters* rc) {
-    pdl_wait();
+__device__ __forceinline__ void after_check(RoundCounters* rc) {
     const int nu = rc->n_undo;
     if (rc->passes < 8) rc->undo_per_pass[rc->passes] = nu;
     rc->passes += 1;
     rc->n_vertices_undo += 2 * nu;
+}
+
+__global__ void k_after_check(RoundCounters* rc) {
+    pdl_wait();
+    after_check(rc);
 }
 
 // undo_collapse_kernel (:829-867) + rearrange_index_of_undo_vertices (:869-878). The map is the compaction
@@ -932,10 +1000,19 @@ __global__ void k_live_flags(const RoundCounters* rc, const int4* __restrict__ t
     if (gtid() == 0) flags[n] = 0;
 }
 
+// check: also the counters after an intersection check (k_after_check). remap: also the carried tree's leaves in the
+// next round's face numbering.
 __global__ void k_compact_mesh(RoundCounters* rc, const float4* __restrict__ pos, const int* __restrict__ occ,
                                const int* __restrict__ pts_map, const int4* __restrict__ tri, const int* __restrict__ fscan,
-                               float4* out_pos, int4* out_tri) {
+                               float4* out_pos, int4* out_tri, int check, BvhRemap remap) {
     pdl_wait();
+    if (remap.leaves) {
+        const int n = *remap.leaves;
+        for (int i = gtid(); i < n; i += gstride()) {
+            const int f = remap.leaf_face[i];
+            remap.next[i] = (f >= 0 && fscan[f + 1] != fscan[f]) ? fscan[f] : -1;
+        }
+    }
     const int np = rc->n_pts, nf = rc->n_tris;
     for (int v = gtid(); v < np; v += gstride())
         if (occ[v]) out_pos[pts_map[v]] = pos[v];
@@ -947,6 +1024,7 @@ __global__ void k_compact_mesh(RoundCounters* rc, const float4* __restrict__ pos
     if (gtid() == 0) {
         rc->n_pts_out = pts_map[np];
         rc->n_tris_out = fscan[nf];
+        if (check) after_check(rc);
     }
 }
 
@@ -994,92 +1072,68 @@ __global__ void k_export_mesh(int np, int nf, const float4* __restrict__ pos, co
 // The same steps as the host-sized launchers, with every size read from the device (LoopState, RoundCounters),
 // so that one captured graph serves every round of a size class.
 
-// *ls = *next; the round's counters as forward() sets them (a stuck round starts its undo list with the
-// carried-over entries)
-__global__ void k_round_begin(RoundCounters* rc, LoopState* ls, const LoopState* next) {
+// The start of a round in one launch. With r.next (device-driven rounds): *ls = *next, the round's counters as forward()
+// sets them (a stuck round starts its undo list with the carried-over entries), the invalid table cleared when undo
+// vertices are carried into a round that is not stuck (cusimp_free.cu:905-908), and the previous compaction map kept;
+// the sizes come from *next, since the counters are written here. Without: the sizes are rc's. Then the round's
+// arrays.
+__global__ void k_round_prologue_dev(RoundStart r) {
     pdl_wait();
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const LoopState L = *next;
-    *ls = L;
-    RoundCounters z = {};
-    z.n_pts = L.np;
-    z.n_tris = L.nf;
-    if (L.is_stuck) {
-        z.first_undo = L.nu;
-        z.n_vertices_undo = L.nu;
-    }
-    *rc = z;
-}
-
-// not stuck and undo vertices carried in: the invalid table is cleared (cusimp_free.cu:905-908)
-__global__ void k_invalid_clear_dev(const LoopState* ls, unsigned char* invalid, int len) {
-    pdl_wait();
-    if (ls->is_stuck || ls->nu == 0) return;
-    for (int i = gtid(); i < len; i += gstride()) invalid[i] = 0;
-}
-
-// stuck: the undo list restarts from the carried vertices mapped through the previous map (:869-878);
-// then the carried vertices are marked invalid (:880-889)
-__global__ void k_undo_book_dev(const int* __restrict__ verts_undo, const LoopState* ls, int* tmp_undo, int* undo_list,
-                                const int* __restrict__ pts_map, int map_len, unsigned char* invalid, int len) {
-    pdl_wait();
-    const int n = ls->nu;
-    const bool stuck = ls->is_stuck != 0;
-    for (int a = gtid(); a < n; a += gstride()) {
-        const int x = verts_undo[a];
-        if (stuck) {
-            tmp_undo[a] = x;
-            undo_list[a] = (x >= 0 && x < map_len) ? pts_map[x] : 0;
+    int nm = 0, np, nf;
+    if (r.next) {
+        const LoopState L = *r.next;
+        nm = np = L.np;
+        nf = L.nf;
+        if (gtid() == 0) {
+            *r.ls = L;
+            RoundCounters z = {};
+            z.n_pts = L.np;
+            z.n_tris = L.nf;
+            if (L.is_stuck) {
+                z.first_undo = L.nu;
+                z.n_vertices_undo = L.nu;
+            }
+            *r.rc = z;
         }
-        if (x >= 0 && x < len) invalid[x] = 1;
+        if (!L.is_stuck && L.nu != 0)
+            for (int i = gtid(); i < r.invalid_len; i += gstride()) r.invalid[i] = 0;
+    } else {
+        np = r.rc->n_pts;
+        nf = r.rc->n_tris;
     }
-}
-
-// the start of a device round (launch_round_prologue_dev)
-__global__ void k_round_prologue_dev(const LoopState* ls, const RoundCounters* rc, const int* __restrict__ pts_map,
-                                     int* pts_map_prev, const float4* __restrict__ pts_in, float4* pos, float4* orig_pos,
-                                     int* occ, const int4* __restrict__ tri_in, int4* tri, int4* orig_tri, int* valence,
-                                     int* cursor, int* vedges, int* vcursor, int* qflag) {
-    pdl_wait();
-    const int nm = ls->np, np = rc->n_pts, nf = rc->n_tris;
-    const int n = max(max(nm, np + 1), nf + 1);
+    const int n = max(np + 1, nf + 1);
     for (int i = gtid(); i < n; i += gstride()) {
-        if (i < nm) pts_map_prev[i] = pts_map[i];
+        if (i < nm) r.pts_map_prev[i] = r.pts_map[i];
         if (i < np) {
-            const float4 p = pts_in[i];
-            pos[i] = p;
-            orig_pos[i] = p;
-            occ[i] = 1;
+            const float4 p = r.pts_in[i];
+            r.pos[i] = p;
+            r.orig_pos[i] = p;
+            r.occ[i] = 1;
         } else if (i == np) {
-            occ[np] = 0;
+            r.occ[np] = 0;
         }
-        if (i <= np) valence[i] = cursor[i] = vedges[i] = vcursor[i] = 0;
+        if (i <= np) {
+            r.valence[i] = r.cursor[i] = r.vedges[i] = r.vcursor[i] = 0;
+            r.vmin[i] = ~0ull;
+        }
         if (i < nf) {
-            const int4 t = tri_in[i];
-            tri[i] = t;
-            orig_tri[i] = t;
+            const int4 t = r.tri_in[i];
+            r.tri[i] = t;
+            r.orig_tri[i] = t;
         }
-        if (i <= nf) qflag[i] = 0;
+        if (i <= nf) r.qflag[i] = 0;
     }
-}
-
-__global__ void k_fill_u64_dev(const RoundCounters* rc, unsigned long long* p, unsigned long long v) {
-    pdl_wait();
-    const int n = rc->n_pts + 1;
-    for (int i = gtid(); i < n; i += gstride()) p[i] = v;
-}
-
-__global__ void k_zero_face_bytes_dev(const RoundCounters* rc, unsigned char* p) {
-    pdl_wait();
-    const int n = rc->n_tris + 1;
-    for (int i = gtid(); i < n; i += gstride()) p[i] = 0;
 }
 
 // After compaction: the next round's state (pamo/__init__.py:131-159: sizes, undo vertices, the no-progress
 // count and is_stuck) computed from this round's start state; recomputing it after an undo pass is harmless.
-__global__ void k_round_end(const RoundCounters* rc, const LoopState* ls, LoopState* next) {
+// Also the undo vertices carried to the next round (the host loop's copy of the previous undo list).
+__global__ void k_round_end(const RoundCounters* rc, const LoopState* ls, LoopState* next, const int* __restrict__ undo_list,
+                            int* undo_in, int undo_cap) {
     pdl_wait();
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    const int n = min(rc->n_vertices_undo, undo_cap);
+    for (int i = gtid(); i < n; i += gstride()) undo_in[i] = undo_list[i];
+    if (gtid() != 0) return;
     LoopState L = *ls;
     const int nf = rc->n_tris_out;
     if (nf == L.nf) {
@@ -1093,15 +1147,6 @@ __global__ void k_round_end(const RoundCounters* rc, const LoopState* ls, LoopSt
     L.nf = nf;
     L.nu = rc->n_vertices_undo;
     *next = L;
-}
-
-// the previous round's compaction map, kept for the undo passes of this round (the round's own compaction
-// overwrites pts_map before an undo pass may follow); undo entries index it with this round's vertex ids (< np)
-// undo vertices carried to the next round (the host loop's copy of the previous undo list)
-__global__ void k_copy_undo_dev(const RoundCounters* rc, const int* __restrict__ src, int* dst, int cap) {
-    pdl_wait();
-    const int n = min(rc->n_vertices_undo, cap);
-    for (int i = gtid(); i < n; i += gstride()) dst[i] = src[i];
 }
 
 }  // namespace
@@ -1158,30 +1203,26 @@ void launch_shuffle_tris(const Feistel& fb, int* flags, int* scan_scratch, int4*
 }
 
 void launch_face_counts(const int4* tri, const RoundCounters* rc, int n_tris_bound, int* valence, int* ecount,
-                        int* vedges, cudaStream_t s, const float4* pos, float4* fgeo, bool plane_df) {
+                        int* vedges, cudaStream_t s, const float4* pos, float4* fgeo, bool plane_df,
+                        const UndoBook& book) {
     pdl(k_face_counts, grid_for(n_tris_bound, kT), kT, 0, s)(tri, rc, valence, ecount, vedges, pos, fgeo,
-                                                            plane_df ? 1 : 0);
+                                                            plane_df ? 1 : 0, book);
     note_launch();
 }
-void launch_fill_adjacency(const int4* tri, const RoundCounters* rc, int n_tris_bound, const int* nt_off, int* cursor,
+void launch_fill_adjacency(const int4* tri, RoundCounters* rc, int n_tris_bound, const int* nt_off, int* cursor,
                            int* nt, const int* edge_off, int2* edges, const int* voff, int* vcursor, int* eorder,
-                           cudaStream_t s) {
+                           cudaStream_t s, int* d_cap) {
     pdl(k_fill_adjacency, grid_for(n_tris_bound, kT), kT, 0, s)(tri, rc, nt_off, cursor, nt, edge_off, edges, voff, vcursor,
-                                                               eorder);
+                                                               eorder, d_cap);
     note_launch();
 }
-void launch_sort_adjacency(const RoundCounters* rc, int n_pts_bound, const int* nt_off, int* nt, cudaStream_t s) {
-    pdl(k_sort_adjacency, grid_for(n_pts_bound, kT), kT, 0, s)(rc, nt_off, nt); note_launch();
-}
-void launch_quadrics(const RoundCounters* rc, int n_pts_bound, const int* nt_off, const int* nt, const int4* tri,
-                     const float4* fgeo, Quadric* q, int* nxt, int2* spc, cudaStream_t s, Quadric* qlo) {
-    if (qlo) pdl(k_quadrics<true>, grid_for(n_pts_bound, kT), kT, 0, s)(rc, nt_off, nt, tri, fgeo, q, nxt, spc, qlo);
-    else pdl(k_quadrics<false>, grid_for(n_pts_bound, kT), kT, 0, s)(rc, nt_off, nt, tri, fgeo, q, nxt, spc, nullptr);
+void launch_ring_quadrics(const RoundCounters* rc, int n_pts_bound, const int* nt_off, int* nt, const int4* tri,
+                          const float4* fgeo, Quadric* q, int* nxt, int2* spc, cudaStream_t s, Quadric* qlo,
+                          uint32_t* cost, int cost_len) {
+    const int g = grid_for(n_pts_bound, kT);
+    if (qlo) pdl(k_ring_quadrics<true>, g, kT, 0, s)(rc, nt_off, nt, tri, fgeo, q, nxt, spc, qlo, cost, cost_len);
+    else pdl(k_ring_quadrics<false>, g, kT, 0, s)(rc, nt_off, nt, tri, fgeo, q, nxt, spc, nullptr, cost, cost_len);
     note_launch();
-}
-void launch_edge_cost_capacity(RoundCounters* rc, int* d_cap, uint32_t* edge_cost, int phys_len, cudaStream_t s) {
-    pdl(k_edge_cost_capacity, 1, 1, 0, s)(rc, d_cap); note_launch();
-    pdl(k_edge_cost_zero, grid_for(phys_len, kT), kT, 0, s)(rc, edge_cost, phys_len); note_launch();
 }
 void launch_edge_cost(const RoundCounters* rc, int n_edges_bound, const int* eorder, const int2* edges, const int* nt_off,
                       const int* nt, const int4* tri, const float4* pos, const Quadric* q, const float4* fgeo,
@@ -1273,32 +1314,24 @@ void launch_collapse(RoundCounters* rc, int n_edges_bound, const int* eorder, co
                                                                      tri, orig_tri, pos, orig_pos, occ, win, nullptr);
     note_launch();
 }
-void launch_compact_winners(const RoundCounters* rc, int n_edges_bound, const int* win_scan, int* collapsed,
-                            cudaStream_t s) {
-    pdl(k_compact_winners, grid_for(n_edges_bound, kT), kT, 0, s)(rc, win_scan, collapsed); note_launch();
-}
-void launch_remove_invalid(const RoundCounters* rc, int n_tris_bound, int4* tri, cudaStream_t s) {
-    pdl(k_remove_invalid, grid_for(n_tris_bound, kT), kT, 0, s)(rc, tri); note_launch();
-}
-void launch_line_edges(RoundCounters* rc, int n_edges_bound, const int2* edges, const int* nt_off, const int* nt,
-                       int4* tri, float4* pos, int* occ, int* line_buf, int line_cap, int* collapsed, cudaStream_t s) {
-    (void)line_buf;
-    pdl(k_line_detect, grid_for(n_edges_bound, kT), kT, 0, s)(rc, edges, pos); note_launch();
-    pdl(k_line_apply, 1, 32, 0, s)(rc, edges, nt_off, nt, tri, pos, occ, collapsed, line_cap); note_launch();
-}
-void launch_line_detect(RoundCounters* rc, int n_edges_bound, const int2* edges, const float4* pos, cudaStream_t s) {
-    pdl(k_line_detect, grid_for(n_edges_bound, kT), kT, 0, s)(rc, edges, pos); note_launch();
+void launch_after_collapse(RoundCounters* rc, int n_edges_bound, int n_tris_bound, const int* win_scan, int* collapsed,
+                           const int2* edges, const int* nt_off, const int* nt, int4* tri, float4* pos, int* occ,
+                           int line_cap, bool lines, cudaStream_t s) {
+    const int g = grid_for(std::max(n_edges_bound, n_tris_bound), kT);
+    if (lines)
+        pdl(k_after_collapse<true>, g, kT, 0, s)(rc, win_scan, collapsed, edges, nt_off, nt, tri, pos, occ, line_cap);
+    else
+        pdl(k_after_collapse<false>, g, kT, 0, s)(rc, win_scan, collapsed, edges, nt_off, nt, tri, pos, occ, line_cap);
+    note_launch();
 }
 void launch_mark_query(const RoundCounters* rc, int n_edges_bound, const int* collapsed, const int2* edges,
                        const int* nt_off, const int* nt, int* qflag, cudaStream_t s) {
     pdl(k_mark_query, grid_for(n_edges_bound, kT), kT, 0, s)(rc, collapsed, edges, nt_off, nt, qflag); note_launch();
 }
-void launch_compact_flags(const int* scan, int n_bound, const int* d_n, int* out_list, cudaStream_t s) {
-    pdl(k_compact_flags, grid_for(n_bound, kT), kT, 0, s)(scan, d_n, out_list); note_launch();
-}
 void launch_undo_check(RoundCounters* rc, int n_edges_bound, const int* collapsed, const int2* edges, const int* nt_off,
-                       const int* nt, const unsigned char* hit, int* uflag, cudaStream_t s) {
-    pdl(k_undo_check, grid_for(n_edges_bound, kT), kT, 0, s)(rc, collapsed, edges, nt_off, nt, hit, uflag); note_launch();
+                       const int* nt, const unsigned char* hit, int* uflag, cudaStream_t s, const int4* tri,
+                       int* fflags) {
+    pdl(k_undo_check, grid_for(n_edges_bound, kT), kT, 0, s)(rc, collapsed, edges, nt_off, nt, hit, uflag, tri, fflags); note_launch();
 }
 void launch_undo_apply(RoundCounters* rc, int n_edges_bound, const int* collapsed, const int* uscan, const int2* edges,
                        const int* nt_off, const int* nt, int4* tri, const int4* orig_tri, float4* pos,
@@ -1317,9 +1350,10 @@ void launch_live_flags(const RoundCounters* rc, int n_tris_bound, const int4* tr
 }
 void launch_compact_mesh(RoundCounters* rc, int n_pts_bound, int n_tris_bound, const float4* pos, const int* occ,
                          const int* pts_map, const int4* tri, const int* face_scan, float4* out_pos, int4* out_tri,
-                         cudaStream_t s) {
+                         cudaStream_t s, bool check, const BvhRemap& remap) {
     const int n = n_pts_bound > n_tris_bound ? n_pts_bound : n_tris_bound;
-    pdl(k_compact_mesh, grid_for(n, kT), kT, 0, s)(rc, pos, occ, pts_map, tri, face_scan, out_pos, out_tri); note_launch();
+    pdl(k_compact_mesh, grid_for(n, kT), kT, 0, s)(rc, pos, occ, pts_map, tri, face_scan, out_pos, out_tri, check ? 1 : 0,
+                                           remap); note_launch();
 }
 void launch_export_round(const RoundCounters* rc, int n_pts, int n_tris, const float4* pos, const int4* tri,
                          const int* occ, const int* pts_map, const int* undo_list, float* verts, int* tris,
@@ -1336,36 +1370,14 @@ void launch_export_mesh(int n_pts, int n_tris, const float4* pos, const int4* tr
 }
 
 // ---- device-driven rounds ----
-void launch_round_begin(RoundCounters* rc, LoopState* ls, const LoopState* next, cudaStream_t s) {
-    pdl(k_round_begin, 1, 32, 0, s)(rc, ls, next); note_launch();
-}
-void launch_undo_bookkeeping_dev(const int* verts_undo, const LoopState* ls, int n_undo_bound, int* tmp_undo,
-                                 int* undo_list, const int* pts_map, int pts_map_len, unsigned char* invalid,
-                                 int invalid_len, cudaStream_t s) {
-    pdl(k_invalid_clear_dev, grid_for(invalid_len, kT), kT, 0, s)(ls, invalid, invalid_len); note_launch();
-    pdl(k_undo_book_dev, grid_for(n_undo_bound, kT), kT, 0, s)(verts_undo, ls, tmp_undo, undo_list, pts_map, pts_map_len,
-                                                             invalid, invalid_len); note_launch();
-}
-void launch_round_prologue_dev(const LoopState* ls, const RoundCounters* rc, int n_pts_bound, int n_tris_bound,
-                               const int* pts_map, int* pts_map_prev, const float4* pts_in, float4* pos,
-                               float4* orig_pos, int* occ, const int4* tri_in, int4* tri, int4* orig_tri, int* valence,
-                               int* cursor, int* vedges, int* vcursor, int* qflag, cudaStream_t s) {
+void launch_round_prologue_dev(const RoundStart& r, int n_pts_bound, int n_tris_bound, cudaStream_t s) {
     const int n = (n_pts_bound > n_tris_bound ? n_pts_bound : n_tris_bound) + 1;
-    pdl(k_round_prologue_dev, grid_for(n, kT), kT, 0, s)(ls, rc, pts_map, pts_map_prev, pts_in, pos, orig_pos, occ, tri_in,
-                                                        tri, orig_tri, valence, cursor, vedges, vcursor, qflag);
+    pdl(k_round_prologue_dev, grid_for(n, kT), kT, 0, s)(r);
     note_launch();
-}
-void launch_fill_u64_dev(const RoundCounters* rc, int n_pts_bound, unsigned long long* p, unsigned long long v,
-                         cudaStream_t s) {
-    pdl(k_fill_u64_dev, grid_for(n_pts_bound + 1, kT), kT, 0, s)(rc, p, v); note_launch();
-}
-void launch_zero_face_bytes_dev(const RoundCounters* rc, int n_tris_bound, unsigned char* p, cudaStream_t s) {
-    pdl(k_zero_face_bytes_dev, grid_for(n_tris_bound + 1, kT), kT, 0, s)(rc, p); note_launch();
 }
 void launch_round_end(const RoundCounters* rc, const LoopState* ls, LoopState* next, const int* undo_list, int* undo_in,
                       int undo_cap, int n_undo_bound, cudaStream_t s) {
-    pdl(k_round_end, 1, 32, 0, s)(rc, ls, next); note_launch();
-    pdl(k_copy_undo_dev, grid_for(n_undo_bound, kT), kT, 0, s)(rc, undo_list, undo_in, undo_cap); note_launch();
+    pdl(k_round_end, grid_for(n_undo_bound, kT, 1), kT, 0, s)(rc, ls, next, undo_list, undo_in, undo_cap); note_launch();
 }
 
 }  // namespace pamo

@@ -3,6 +3,7 @@
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
+#include "lbvh.cuh"
 #include "pamo_common.cuh"
 
 namespace pamo {
@@ -57,23 +58,37 @@ void launch_shuffle_tris(const Feistel& fb, int* flags, int* scan_scratch, int4*
 void launch_copy_tris(const int4* src, int4* dst, int n, cudaStream_t s);
 
 // ---- adjacency ----
+// The bookkeeping of the undo vertices carried into a device round (cusimp_free.cu:869-889), done beside the face counts:
+// invalid marked, and in a stuck round the undo list restarted through the previous map. ls null: none.
+struct UndoBook {
+    const LoopState* ls = nullptr;
+    const int* verts_undo = nullptr;
+    int* tmp_undo = nullptr;
+    int* undo_list = nullptr;
+    const int* pts_map = nullptr;
+    int map_len = 0;
+    unsigned char* invalid = nullptr;
+    int invalid_len = 0;
+};
 // with fgeo: also the per-face geometry the rings read (from pos; room for six float4 per face): a 64-byte record per
 // face (fgeo[4f .. 4f + 3]: edge lengths, normal, corner positions), then the planes after all n faces' records, one
 // float4 per face (fgeo[4n + f]) or, with plane_df (precision mode), a double-float pair (fgeo[4n + 2f], +1)
 void launch_face_counts(const int4* tri, const RoundCounters* rc, int n_tris_bound, int* valence, int* ecount,
                         int* vedges, cudaStream_t s, const float4* pos = nullptr, float4* fgeo = nullptr,
-                        bool plane_df = false);
-void launch_fill_adjacency(const int4* tri, const RoundCounters* rc, int n_tris_bound, const int* nt_off, int* cursor,
+                        bool plane_df = false, const UndoBook& book = UndoBook());
+// d_cap (or null): the length of the edge costs as the reference sizes them, grown to the round's edges
+void launch_fill_adjacency(const int4* tri, RoundCounters* rc, int n_tris_bound, const int* nt_off, int* cursor,
                            int* nt, const int* edge_off, int2* edges, const int* voff, int* vcursor, int* eorder,
-                           cudaStream_t s);
-void launch_sort_adjacency(const RoundCounters* rc, int n_pts_bound, const int* nt_off, int* nt, cudaStream_t s);
+                           cudaStream_t s, int* d_cap = nullptr);
 
 // ---- cost, selection, collapse ----
+// The rings sorted by face, and the quadrics.
 // qlo (precision mode; needs the plane_df planes): each quadric as a double-float sum, hi parts to q, lo to qlo
 // nxt, spc: per ring slot, the vertex after the ring's vertex in the slot's face and (the vertex before it, its corner)
-void launch_quadrics(const RoundCounters* rc, int n_pts_bound, const int* nt_off, const int* nt, const int4* tri,
-                     const float4* fgeo, Quadric* q, int* nxt, int2* spc, cudaStream_t s, Quadric* qlo = nullptr);
-void launch_edge_cost_capacity(RoundCounters* rc, int* d_cap, uint32_t* edge_cost, int phys_len, cudaStream_t s);
+// cost (or null), cost_len: the edge costs, zeroed when their length grew (launch_fill_adjacency)
+void launch_ring_quadrics(const RoundCounters* rc, int n_pts_bound, const int* nt_off, int* nt, const int4* tri,
+                          const float4* fgeo, Quadric* q, int* nxt, int2* spc, cudaStream_t s, Quadric* qlo = nullptr,
+                          uint32_t* cost = nullptr, int cost_len = 0);
 // mode: 0 the reference's arithmetic; precision mode 1 (double-float quadrics q + qlo, compensated sums) or 2 (as 1,
 // placement at the quadric's minimiser, written to place[e]). raw (optional): each edge's cost before clamp and quantisation (NaN where
 // none is computed); place (optional, required by mode 2): each edge's placement.
@@ -98,20 +113,20 @@ void launch_collapse(RoundCounters* rc, int n_edges_bound, const int* eorder, co
                      uint32_t collapse_t, const unsigned long long* fkey, const int* nt_off, const int* nt, int4* tri,
                      const int4* orig_tri, float4* pos, const float4* orig_pos, int* occ, int* win, cudaStream_t s,
                      bool restore = true, const float4* place = nullptr);
-void launch_compact_winners(const RoundCounters* rc, int n_edges_bound, const int* win_scan, int* collapsed,
-                            cudaStream_t s);
-void launch_remove_invalid(const RoundCounters* rc, int n_tris_bound, int4* tri, cudaStream_t s);
-void launch_line_edges(RoundCounters* rc, int n_edges_bound, const int2* edges, const int* nt_off, const int* nt,
-                       int4* tri, float4* pos, int* occ, int* line_buf, int line_cap, int* collapsed, cudaStream_t s);
+// After the collapses: the winners' list, the degenerate faces removed and the edges with coincident endpoints counted in
+// rc->n_line; with lines, also collapsed in edge order and appended to the list (up to line_cap), with rc->n_collapsed
+// and rc->n_considered. Needs rc->pad[4] = 0, which a round starts with.
+void launch_after_collapse(RoundCounters* rc, int n_edges_bound, int n_tris_bound, const int* win_scan, int* collapsed,
+                           const int2* edges, const int* nt_off, const int* nt, int4* tri, float4* pos, int* occ,
+                           int line_cap, bool lines, cudaStream_t s);
 
 // ---- self-intersection rollback ----
-// counts coincident-endpoint edges into rc->n_line (the first half of launch_line_edges)
-void launch_line_detect(RoundCounters* rc, int n_edges_bound, const int2* edges, const float4* pos, cudaStream_t s);
 void launch_mark_query(const RoundCounters* rc, int n_edges_bound, const int* collapsed, const int2* edges,
                        const int* nt_off, const int* nt, int* qflag, cudaStream_t s);
-void launch_compact_flags(const int* scan, int n_bound, const int* d_n, int* out_list, cudaStream_t s);
+// fflags (or null): also the live faces of tri, as launch_live_flags
 void launch_undo_check(RoundCounters* rc, int n_edges_bound, const int* collapsed, const int2* edges, const int* nt_off,
-                       const int* nt, const unsigned char* hit, int* uflag, cudaStream_t s);
+                       const int* nt, const unsigned char* hit, int* uflag, cudaStream_t s,
+                       const int4* tri = nullptr, int* fflags = nullptr);
 void launch_undo_apply(RoundCounters* rc, int n_edges_bound, const int* collapsed, const int* uscan, const int2* edges,
                        const int* nt_off, const int* nt, int4* tri, const int4* orig_tri, float4* pos,
                        const float4* orig_pos, int* occ, int* tmp_undo, int* undo_list, const int* pts_map,
@@ -119,9 +134,10 @@ void launch_undo_apply(RoundCounters* rc, int n_edges_bound, const int* collapse
 
 // ---- outputs ----
 void launch_live_flags(const RoundCounters* rc, int n_tris_bound, const int4* tri, int* flags, cudaStream_t s);
+// check: also launch_after_check's counters; remap: also the carried tree's leaves in the new numbering
 void launch_compact_mesh(RoundCounters* rc, int n_pts_bound, int n_tris_bound, const float4* pos, const int* occ,
                          const int* pts_map, const int4* tri, const int* face_scan, float4* out_pos, int4* out_tri,
-                         cudaStream_t s);
+                         cudaStream_t s, bool check = false, const BvhRemap& remap = BvhRemap());
 void launch_export_round(const RoundCounters* rc, int n_pts, int n_tris, const float4* pos, const int4* tri,
                          const int* occ, const int* pts_map, const int* undo_list, float* verts, int* tris,
                          int* verts_occ, int* verts_map, int* verts_undo, int n_undo, cudaStream_t s);
@@ -156,21 +172,28 @@ void launch_center(const float* pts, const int* tris, int n_pts, int n_tris, flo
 void launch_after_check(RoundCounters* rc, cudaStream_t s);
 
 // ---- device-driven rounds: sizes from LoopState / RoundCounters, host values only bound the grids ----
-void launch_round_begin(RoundCounters* rc, LoopState* ls, const LoopState* next, cudaStream_t s);
-void launch_undo_bookkeeping_dev(const int* verts_undo, const LoopState* ls, int n_undo_bound, int* tmp_undo,
-                                 int* undo_list, const int* pts_map, int pts_map_len, unsigned char* invalid,
-                                 int invalid_len, cudaStream_t s);
-// Start of a device round, after the undo bookkeeping, in one launch: pts_map_prev[0, ls->np) = pts_map (the
-// previous round's map, read by this round's undo passes); pos = orig_pos = the round's points, occ = 1 and
-// occ[n_pts] = 0; tri = orig_tri = the round's faces; valence, cursor, vedges, vcursor = 0 over n_pts + 1 entries;
-// qflag = 0 over n_tris + 1 entries.
-void launch_round_prologue_dev(const LoopState* ls, const RoundCounters* rc, int n_pts_bound, int n_tris_bound,
-                               const int* pts_map, int* pts_map_prev, const float4* pts_in, float4* pos,
-                               float4* orig_pos, int* occ, const int4* tri_in, int4* tri, int4* orig_tri, int* valence,
-                               int* cursor, int* vedges, int* vcursor, int* qflag, cudaStream_t s);
-void launch_fill_u64_dev(const RoundCounters* rc, int n_pts_bound, unsigned long long* p, unsigned long long v,
-                         cudaStream_t s);
-void launch_zero_face_bytes_dev(const RoundCounters* rc, int n_tris_bound, unsigned char* p, cudaStream_t s);
+// The start of a round in one launch: pos = orig_pos = the round's points, occ = 1 and occ[n_pts] = 0; tri = orig_tri = the
+// round's faces; valence, cursor, vedges, vcursor = 0 and vmin = ~0 over n_pts + 1 entries; qflag = 0 over n_tris + 1
+// entries. With next (device-driven rounds; null: the sizes are rc's and the rest is not touched) also *ls = *next, rc as
+// forward() sets it, the invalid table cleared where undo vertices are carried into a round that is not stuck, and
+// pts_map_prev[0, n_pts) = pts_map (the previous round's map, read by this round's undo passes).
+struct RoundStart {
+    const LoopState* next = nullptr;
+    LoopState* ls = nullptr;
+    RoundCounters* rc = nullptr;
+    unsigned char* invalid = nullptr;
+    int invalid_len = 0;
+    const int* pts_map = nullptr;
+    int* pts_map_prev = nullptr;
+    const float4* pts_in = nullptr;
+    float4 *pos = nullptr, *orig_pos = nullptr;
+    int* occ = nullptr;
+    const int4* tri_in = nullptr;
+    int4 *tri = nullptr, *orig_tri = nullptr;
+    int *valence = nullptr, *cursor = nullptr, *vedges = nullptr, *vcursor = nullptr, *qflag = nullptr;
+    unsigned long long* vmin = nullptr;
+};
+void launch_round_prologue_dev(const RoundStart& r, int n_pts_bound, int n_tris_bound, cudaStream_t s);
 void launch_round_end(const RoundCounters* rc, const LoopState* ls, LoopState* next, const int* undo_list, int* undo_in,
                       int undo_cap, int n_undo_bound, cudaStream_t s);
 
