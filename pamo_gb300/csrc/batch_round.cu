@@ -581,7 +581,6 @@ struct pamo_csr {
     Buf<int2> spc;
     Buf<float4> fgeo;
     Buf<float> face_mean;
-    Buf<unsigned long long> fkey;
     Buf<unsigned char> hit;
     Buf<int2> edges, exact_list;
     Buf<int> eorder, win, winners, lines, considered, uflag;
@@ -666,7 +665,7 @@ struct pamo_csr {
         release(vscan); release(quad); release(vmin); release(invalid); release(tri); release(orig_tri);
         release(tri_in); release(tri_next); release(res_tri); release(tri_load); release(ecount); release(qflag);
         release(fflags); release(nt); release(nxt); release(spc); release(fmesh); release(shuffle_flags);
-        release(fgeo); release(face_mean); release(fkey); release(hit); release(edges); release(exact_list);
+        release(fgeo); release(face_mean); release(hit); release(edges); release(exact_list);
         release(eorder); release(win); release(winners); release(lines); release(considered); release(uflag);
         release(cost); release(map_reg); release(undo_list_reg); release(tmp_undo_reg); release(undo_in_reg);
         release(invalid_reg); release(ecost_reg); release(mesh); release(slot_mesh); release(slot_v0);
@@ -695,7 +694,7 @@ struct pamo_csr {
             (r = grow(res_tri, fc)) || (r = grow(tri_load, fc)) || (r = grow(ecount, fc + 1)) ||
             (r = grow(qflag, fc + 1)) || (r = grow(fflags, fc + 1)) || (r = grow(nt, 3 * fc)) ||
             (r = grow(nxt, 3 * fc)) || (r = grow(spc, 3 * fc)) || (r = grow(fmesh, fc)) ||
-            (r = grow(fgeo, 6 * fc)) || (r = grow(face_mean, 3 * fc)) || (r = grow(fkey, fc)) || (r = grow(hit, fc + 1)))
+            (r = grow(fgeo, 6 * fc)) || (r = grow(face_mean, 3 * fc)) || (r = grow(hit, fc + 1)))
             return r;
         if ((r = grow(edges, ec)) || (r = grow(eorder, ec)) || (r = grow(win, ec + 1)) || (r = grow(winners, ec)) ||
             (r = grow(lines, ec)) || (r = grow(considered, ec)) || (r = grow(uflag, ec + 1)) || (r = grow(cost, ec)) ||
@@ -795,8 +794,7 @@ struct pamo_csr {
         pdl(kb_scatter_costs, grid_for(Eb, kT), kT, 0, s)(rc, slot_mesh.p, mesh.p, vmesh.p, edges.p, cost.p, ecost_reg.p);
         note_launch();
         // selection and collapse
-        launch_face_keys(rc, Fb, tri.p, vmin.p, fkey.p, s);
-        launch_collapse(rc, Eb, eorder.p, edges.p, cost.p, collapse_t, fkey.p, nt_off, nt.p, tri.p, orig_tri.p, pos.p,
+        launch_collapse(rc, Eb, eorder.p, edges.p, cost.p, collapse_t, vmin.p, nxt.p, spc.p, nt_off, nt.p, tri.p, orig_tri.p, pos.p,
                         orig_pos.p, occ.p, win.p, s);
         exclusive_scan(win.p, win.p, &rc->n_edges, 1, &rc->n_win, scan_scratch, s, &rc->status, Eb);
         launch_after_collapse(rc, Eb, Fb, win.p, winners.p, edges.p, nt_off, nt.p, tri.p, pos.p, occ.p, 0, false, s);

@@ -118,7 +118,6 @@ struct pamo_ctx {
     DevBuf<int> nxt;        // per CSR slot: the vertex after the ring's vertex in the slot's face
     DevBuf<int2> spc;       // per CSR slot: the vertex before it and its corner
     DevBuf<float4> fgeo;    // per face: a 64-byte ring record, then the planes (room for six float4 per face)
-    DevBuf<unsigned long long> fkey;
     DevBuf<unsigned char> hit;
     BvhBuffers bvh;
     char* bvh_mem = nullptr;
@@ -288,7 +287,7 @@ struct pamo_ctx {
         fr(edge_cost); fr(invalid); fr(pts_map); fr(pts_map_prev); fr(undo_list); fr(tmp_undo);
         fr(pos); fr(orig_pos); fr(pos_in); fr(pos_out); fr(occ); fr(valence); fr(cursor); fr(quad); fr(quad_lo); fr(vmin); fr(undo_in);
         fr(nxt); fr(spc); fr(fgeo); fr(tri); fr(orig_tri); fr(tri_in); fr(tri_out); fr(ecount); fr(qflag); fr(fflags); fr(nt);
-        fr(shuffle_flags); fr(fkey); fr(eorder); fr(vedges); fr(vcursor); fr(hit); fr(edges); fr(win); fr(collapsed); fr(uflag); fr(face_mean); fr(exact_list); fr(place); fr(probe_raw);
+        fr(shuffle_flags); fr(eorder); fr(vedges); fr(vcursor); fr(hit); fr(edges); fr(win); fr(collapsed); fr(uflag); fr(face_mean); fr(exact_list); fr(place); fr(probe_raw);
         if (bvh_mem) cudaFree(bvh_mem);
         bvh_mem = nullptr;
         prof.destroy();
@@ -361,7 +360,7 @@ struct pamo_ctx {
              undo_in.bytes();
         b += nxt.bytes() + spc.bytes() + fgeo.bytes();
         b += tri.bytes() + orig_tri.bytes() + tri_in.bytes() + tri_out.bytes() + ecount.bytes() + qflag.bytes() +
-             fflags.bytes() + nt.bytes() + shuffle_flags.bytes() + fkey.bytes() + hit.bytes() +
+             fflags.bytes() + nt.bytes() + shuffle_flags.bytes() + hit.bytes() +
              edges.bytes() + win.bytes() + collapsed.bytes() + uflag.bytes() + eorder.bytes() + exact_list.bytes() +
              face_mean.bytes();
         b += edge_cost.bytes() + invalid.bytes() + pts_map.bytes() + pts_map_prev.bytes() + undo_list.bytes() +
@@ -391,7 +390,7 @@ struct pamo_ctx {
         int r;
         if ((r = grow(tri, nc)) || (r = grow(orig_tri, nc)) || (r = grow(tri_in, nc)) || (r = grow(tri_out, nc)) ||
             (r = grow(ecount, nc + 1)) || (r = grow(qflag, nc + 1)) || (r = grow(fflags, nc + 1)) ||
-            (r = grow(nt, 3 * nc)) || (r = grow(nxt, 3 * nc)) || (r = grow(spc, 3 * nc)) || (r = grow(fgeo, 6 * nc)) || (r = grow(shuffle_flags, 2 * nc + 40)) || (r = grow(fkey, nc)) || (r = grow(hit, nc)) ||
+            (r = grow(nt, 3 * nc)) || (r = grow(nxt, 3 * nc)) || (r = grow(spc, 3 * nc)) || (r = grow(fgeo, 6 * nc)) || (r = grow(shuffle_flags, 2 * nc + 40)) || (r = grow(hit, nc)) ||
             (r = grow(eorder, 2 * nc)) ||
             (r = grow(edges, 2 * nc)) || (r = grow(win, 2 * nc + 1)) || (r = grow(collapsed, 2 * nc)) ||
             (r = grow(uflag, 2 * nc + 1)) || (r = grow(face_mean, 3 * nc)) ||
@@ -450,8 +449,7 @@ struct pamo_ctx {
         cudaMemsetAsync(vmin.p, 0xFF, (nP + 1) * sizeof(unsigned long long), s);
         launch_edge_cost(rc, eb, eorder.p, edges.p, nt_off, nt.p, tri.p, pos.p, quad.p, fgeo.p, nxt.p, spc.p, invalid.p, edge_cost.p, vmin.p,
                          d_scale, threshold, 0, s, nullptr, true, skinny_pow);
-        launch_face_keys(rc, nT, tri.p, vmin.p, fkey.p, s);
-        launch_collapse(rc, eb, eorder.p, edges.p, edge_cost.p, collapse_t, fkey.p, nt_off, nt.p, tri.p, orig_tri.p, pos.p,
+        launch_collapse(rc, eb, eorder.p, edges.p, edge_cost.p, collapse_t, vmin.p, nxt.p, spc.p, nt_off, nt.p, tri.p, orig_tri.p, pos.p,
                         orig_pos.p, occ.p, win.p, s, false);
         exclusive_scan(occ.p, pts_map.p, &rc->n_pts, 1, nullptr, scan_scratch, s, &rc->status, nP);
         if ((r = read_counters())) return r;
@@ -547,8 +545,7 @@ struct pamo_ctx {
                              vmin.p, d_scale, threshold, 0, s, &d_ls->is_stuck, false, skinny_pow, precision, nullptr,
                              place_ptr(), qlo_ptr());
             cost_end(s);
-            launch_face_keys(rc, nTb, tri.p, vmin.p, fkey.p, s);
-            launch_collapse(rc, eb, eorder.p, edges.p, edge_cost.p, collapse_t, fkey.p, nt_off, nt.p, tri.p, orig_tri.p,
+            launch_collapse(rc, eb, eorder.p, edges.p, edge_cost.p, collapse_t, vmin.p, nxt.p, spc.p, nt_off, nt.p, tri.p, orig_tri.p,
                             pos.p, orig_pos.p, occ.p, win.p, s, true, place_ptr());
             exclusive_scan(win.p, win.p, &rc->n_edges, 1, &rc->n_win, scan_scratch, s, &rc->status, eb);
             launch_after_collapse(rc, eb, nTb, win.p, collapsed.p, edges.p, nt_off, nt.p, tri.p, pos.p, occ.p,
@@ -722,8 +719,7 @@ struct pamo_ctx {
         cost_end(s);
         prof.end(kPhCost, s);
         prof.begin(kPhCollapse, s);
-        launch_face_keys(rc, nT, tri.p, vmin.p, fkey.p, s);
-        launch_collapse(rc, eb, eorder.p, edges.p, edge_cost.p, collapse_t, fkey.p, nt_off, nt.p, tri.p, orig_tri.p, pos.p,
+        launch_collapse(rc, eb, eorder.p, edges.p, edge_cost.p, collapse_t, vmin.p, nxt.p, spc.p, nt_off, nt.p, tri.p, orig_tri.p, pos.p,
                         orig_pos.p, occ.p, win.p, s, true, place_ptr());
         exclusive_scan(win.p, win.p, &rc->n_edges, 1, &rc->n_win, scan_scratch, s, &rc->status, eb);
         launch_after_collapse(rc, eb, nT, win.p, collapsed.p, edges.p, nt_off, nt.p, tri.p, pos.p, occ.p, (int)collapsed.n,

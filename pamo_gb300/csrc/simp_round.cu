@@ -4,9 +4,8 @@
 // result:
 //   * vertex->face lists are filled with atomics and then sorted per vertex, so every float sum over a ring
 //     runs in ascending face order and the round is deterministic;
-//   * the per-face minimum key of propagate_edge_cost_kernel (:587-610) is computed as the minimum over the
-//     face's three vertices of a per-vertex minimum (two 64-bit atomicMin per edge instead of one per ring
-//     face); both are the minimum over all edges touching the face;
+//   * the per-face minimum key of propagate_edge_cost_kernel (:587-610) is replaced by a per-vertex minimum (two
+//     64-bit atomicMin per edge instead of one per ring face), whose minimum over a face's vertices it is;
 //   * winners are listed in ascending edge order through a scan instead of an atomic counter;
 //   * the undo check marks intersecting faces in a flag array and tests ring membership in O(ring) instead
 //     of scanning the whole intersection list per collapsed edge (:776-827).
@@ -767,20 +766,6 @@ __global__ void __launch_bounds__(kT) k_edge_cost(const RoundCounters* rc, const
     }
 }
 
-__global__ void __launch_bounds__(kT) k_face_keys(const RoundCounters* rc, const int4* __restrict__ tri,
-                                                  const unsigned long long* __restrict__ vmin, unsigned long long* fkey) {
-    pdl_wait();
-    const int n = rc->n_tris;
-    for (int f = gtid(); f < n; f += gstride()) {
-        const int4 t = tri[f];
-        if (face_killed(t)) continue;
-        unsigned long long k = vmin[t.x];
-        k = min(k, vmin[t.y]);
-        k = min(k, vmin[t.z]);
-        fkey[f] = k;
-    }
-}
-
 // ------------------------------------------------------------------ collapse (collapse_edge_kernel, :639-774)
 __device__ __forceinline__ bool is_skinny(V3 p, V3 q, V3 r) {  // :617-637
     const V3 pq = vsub(q, p), pr = vsub(r, p), qr = vsub(r, q);
@@ -804,13 +789,34 @@ __device__ __forceinline__ bool ring_has_skinny(int w, const int* __restrict__ n
 }
 
 
+// An edge wins when its key is the least over every face that touches it, that is when no vertex of the rings of u and v
+// has a smaller one in vmin (the least key of its edges; a face's key is the least of its three vertices', and u and v
+// lie in all faces of their rings). vmin[u] and vmin[v] alone reject nearly every edge before a ring is read; the
+// reference's per-face keys (:587-610) are not made. Slots four at a time, their gathers in flight together.
+__device__ __forceinline__ bool ring_keys_at_least(int a, int b, unsigned long long key, const int* __restrict__ nxt,
+                                                   const int2* __restrict__ spc,
+                                                   const unsigned long long* __restrict__ vmin) {
+    for (int s0 = a; s0 < b; s0 += 4) {
+        bool low = false;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int s = min(s0 + k, b - 1);
+            low |= vmin[nxt[s]] < key;
+            low |= vmin[spc[s].x] < key;
+        }
+        if (low) return false;
+    }
+    return true;
+}
+
 // kRestore = false: CUSimp's collapse (cusimp.cu:512-585), without the skinny-ring restore
 // kOpt (precision mode 2): the collapse places at the edge's precomputed placement instead of the midpoint
 template <bool kRestore, bool kOpt = false>
 __global__ void __launch_bounds__(kT) k_collapse(RoundCounters* rc, const int* __restrict__ eorder,
                                                  const int2* __restrict__ edges,
                                                  const uint32_t* __restrict__ cost, uint32_t collapse_t,
-                                                 const unsigned long long* __restrict__ fkey, const int* __restrict__ nt_off,
+                                                 const unsigned long long* __restrict__ vmin, const int* __restrict__ nxt,
+                                                 const int2* __restrict__ spc, const int* __restrict__ nt_off,
                                                  const int* __restrict__ nt, int4* tri, const int4* __restrict__ orig_tri,
                                                  float4* pos, const float4* __restrict__ orig_pos, int* occ, int* win,
                                                  const float4* __restrict__ place) {
@@ -825,10 +831,9 @@ __global__ void __launch_bounds__(kT) k_collapse(RoundCounters* rc, const int* _
             const int2 ed = edges[e];
             const int u = ed.x, v = ed.y;
             const unsigned long long key = ((unsigned long long)c << 32) | (unsigned)e;
-            bool ok = true;
-            for (int s = nt_off[u]; s < nt_off[u + 1] && ok; ++s) ok = (fkey[nt[s]] == key);
-            for (int s = nt_off[v]; s < nt_off[v + 1] && ok; ++s) ok = (fkey[nt[s]] == key);
-            if (ok) {
+            if (vmin[u] == key && vmin[v] == key &&
+                ring_keys_at_least(nt_off[u], nt_off[u + 1], key, nxt, spc, vmin) &&
+                ring_keys_at_least(nt_off[v], nt_off[v + 1], key, nxt, spc, vmin)) {
                 w = 1;
                 const V3 v0 = v3(pos[u]), v1 = v3(pos[v]);
                 V3 vm = vdiv(vadd(v0, v1), 2.0f);
@@ -921,8 +926,16 @@ __global__ void k_mark_query(const RoundCounters* rc, const int* __restrict__ co
     const int n = rc->n_considered;
     for (int c = gtid(); c < n; c += gstride()) {
         const int2 ed = edges[collapsed[c]];
-        for (int s = nt_off[ed.x]; s < nt_off[ed.x + 1]; ++s) qflag[nt[s]] = 1;
-        for (int s = nt_off[ed.y]; s < nt_off[ed.y + 1]; ++s) qflag[nt[s]] = 1;
+        for (int side = 0; side < 2; ++side) {
+            const int w = side ? ed.y : ed.x, b = nt_off[w + 1];
+            for (int s0 = nt_off[w]; s0 < b; s0 += 4) {  // four slots at a time: their loads are in flight together
+                int f[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) f[k] = nt[min(s0 + k, b - 1)];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) qflag[f[k]] = 1;
+            }
+        }
     }
 }
 
@@ -941,8 +954,12 @@ __global__ void k_undo_check(RoundCounters* rc, const int* __restrict__ collapse
     for (int c = gtid(); c < n; c += gstride()) {
         const int2 ed = edges[collapsed[c]];
         int f = 0;
-        for (int s = nt_off[ed.x]; s < nt_off[ed.x + 1] && !f; ++s) f = hit[nt[s]];
-        for (int s = nt_off[ed.y]; s < nt_off[ed.y + 1] && !f; ++s) f = hit[nt[s]];
+        for (int side = 0; side < 2 && !f; ++side) {
+            const int w = side ? ed.y : ed.x, b = nt_off[w + 1];
+            for (int s0 = nt_off[w]; s0 < b && !f; s0 += 4)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) f |= hit[nt[min(s0 + k, b - 1)]];
+        }
         uflag[c] = f ? 1 : 0;
     }
 }
@@ -1294,23 +1311,20 @@ void launch_edge_cost_batch(const RoundCounters* rc, int n_edges_bound, const in
                                                         nullptr);
     note_launch();
 }
-void launch_face_keys(const RoundCounters* rc, int n_tris_bound, const int4* tri, const unsigned long long* vmin,
-                      unsigned long long* fkey, cudaStream_t s) {
-    pdl(k_face_keys, grid_for(n_tris_bound, kT), kT, 0, s)(rc, tri, vmin, fkey); note_launch();
-}
 void launch_collapse(RoundCounters* rc, int n_edges_bound, const int* eorder, const int2* edges, const uint32_t* cost,
-                     uint32_t collapse_t, const unsigned long long* fkey, const int* nt_off, const int* nt, int4* tri,
+                     uint32_t collapse_t, const unsigned long long* vmin, const int* nxt, const int2* spc,
+                     const int* nt_off, const int* nt, int4* tri,
                      const int4* orig_tri, float4* pos, const float4* orig_pos, int* occ, int* win, cudaStream_t s,
                      bool restore, const float4* place) {
     if (restore && place)
-        pdl(k_collapse<true, true>, grid_for(n_edges_bound, kT), kT, 0, s)(rc, eorder, edges, cost, collapse_t, fkey,
+        pdl(k_collapse<true, true>, grid_for(n_edges_bound, kT), kT, 0, s)(rc, eorder, edges, cost, collapse_t, vmin, nxt, spc,
                                                                           nt_off, nt, tri, orig_tri, pos, orig_pos, occ,
                                                                           win, place);
     else if (restore)
-        pdl(k_collapse<true>, grid_for(n_edges_bound, kT), kT, 0, s)(rc, eorder, edges, cost, collapse_t, fkey, nt_off, nt,
+        pdl(k_collapse<true>, grid_for(n_edges_bound, kT), kT, 0, s)(rc, eorder, edges, cost, collapse_t, vmin, nxt, spc, nt_off, nt,
                                                                     tri, orig_tri, pos, orig_pos, occ, win, nullptr);
     else
-        pdl(k_collapse<false>, grid_for(n_edges_bound, kT), kT, 0, s)(rc, eorder, edges, cost, collapse_t, fkey, nt_off, nt,
+        pdl(k_collapse<false>, grid_for(n_edges_bound, kT), kT, 0, s)(rc, eorder, edges, cost, collapse_t, vmin, nxt, spc, nt_off, nt,
                                                                      tri, orig_tri, pos, orig_pos, occ, win, nullptr);
     note_launch();
 }

@@ -107,10 +107,10 @@ void launch_edge_cost_batch(const RoundCounters* rc, int n_edges_bound, const in
                             uint32_t* cost,
                             unsigned long long* vmin, const float* mesh_scale, const int* mesh_stuck, const int* vmesh,
                             float tres, cudaStream_t s, bool device_pow = false);
-void launch_face_keys(const RoundCounters* rc, int n_tris_bound, const int4* tri, const unsigned long long* vmin,
-                      unsigned long long* fkey, cudaStream_t s);
+// vmin: the least key (cost << 32 | edge) over the edges of each vertex
 void launch_collapse(RoundCounters* rc, int n_edges_bound, const int* eorder, const int2* edges, const uint32_t* cost,
-                     uint32_t collapse_t, const unsigned long long* fkey, const int* nt_off, const int* nt, int4* tri,
+                     uint32_t collapse_t, const unsigned long long* vmin, const int* nxt, const int2* spc,
+                     const int* nt_off, const int* nt, int4* tri,
                      const int4* orig_tri, float4* pos, const float4* orig_pos, int* occ, int* win, cudaStream_t s,
                      bool restore = true, const float4* place = nullptr);
 // After the collapses: the winners' list, the degenerate faces removed and the edges with coincident endpoints counted in
