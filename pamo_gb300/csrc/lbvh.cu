@@ -22,7 +22,7 @@ constexpr int kQueryThreads = 128;
 constexpr int kStackDepth = 64;  // enough for any tree (depth <= 62 + 1)
 constexpr int kShortStack = 24;  // first walk: deeper queries are handed to the second walk
 constexpr int kExactThreads = 64;
-constexpr int kPairChunk = 32;   // list slots a lane takes at a time
+constexpr int kPairChunk = 128;  // list slots a warp takes at a time
 constexpr int kQueryBit = 1 << 30;  // set on a packed leaf's face id when the face is a query face
 
 __device__ __forceinline__ unsigned f2ord(float f) {
@@ -421,8 +421,10 @@ __global__ void __launch_bounds__(kTileThreads, 3) k_bottom_up_tiles(RoundCounte
             slhi[threadIdx.x] = bhi;
         }
         __syncthreads();
+        // up to the tile's edge, in shared memory alone
         int ref = ~leaf;
         int guard = 0;
+        bool leaves_tile = false;
         while (p >= 0) {
             if (++guard > 4096) {
                 atomicOr(&rc->status, kErrIterLimit);
@@ -431,18 +433,7 @@ __global__ void __launch_bounds__(kTileThreads, 3) k_bottom_up_tiles(RoundCounte
             // a node's index is one end of its range: a node with its index outside the tile leaves the tile
             const int k = p - a;
             if (!(p >= a && p < b && srange[k].x >= a && srange[k].y < b)) {
-                // leaving the tile: this child's box goes to global memory for the other child's chain; with
-                // several tiles per block the second arrival queues p for k_bottom_up_upper instead of climbing
-                // on, so that no chain through the upper tree holds this block at the next tile's barrier
-                if (ref >= 0 && !kNodes) {
-                    __stcg(&nlo[ref], blo);
-                    __stcg(&nhi[ref], bhi);
-                }
-                if (!climb) {
-                    if (arrive_release(&visit[p]) != 0) upq[1 + atomicAdd(upq, 1)] = p;
-                } else if (arrive_acq_rel(&visit[p]) != 0) {
-                    climb_from<kPack>(rc, p, child, iparent, llo, lhi, nlo, nhi, visit, leaf_face, qflag, packed);
-                }
+                leaves_tile = true;
                 break;
             }
             __threadfence_block();
@@ -450,24 +441,43 @@ __global__ void __launch_bounds__(kTileThreads, 3) k_bottom_up_tiles(RoundCounte
             __threadfence_block();
             // both children are in this tile
             const int2 c = schild[k];
-            float4 alo, ahi, clo, chi;
-            if (c.x < 0) { alo = sllo[~c.x - a]; ahi = slhi[~c.x - a]; }
-            else { alo = slo[c.x - a]; ahi = shi[c.x - a]; }
-            if (c.y < 0) { clo = sllo[~c.y - a]; chi = slhi[~c.y - a]; }
-            else { clo = slo[c.y - a]; chi = shi[c.y - a]; }
+            const float4 alo = c.x < 0 ? sllo[~c.x - a] : slo[c.x - a], ahi = c.x < 0 ? slhi[~c.x - a] : shi[c.x - a];
+            const float4 clo = c.y < 0 ? sllo[~c.y - a] : slo[c.y - a], chi = c.y < 0 ? slhi[~c.y - a] : shi[c.y - a];
             blo = make_float4(fminf(alo.x, clo.x), fminf(alo.y, clo.y), fminf(alo.z, clo.z), 0.f);
             bhi = make_float4(fmaxf(ahi.x, chi.x), fmaxf(ahi.y, chi.y), fmaxf(ahi.z, chi.z), 0.f);
             slo[k] = blo;
             shi[k] = bhi;
-            if (kNodes) {
-                __stcg(&nlo[p], blo);
-                __stcg(&nhi[p], bhi);
-            }
-            if (kPack)
-                write_packed(p, c, alo, ahi, clo, chi, c.x < 0 ? sface[~c.x - a] : -1, c.y < 0 ? sface[~c.y - a] : -1,
-                             packed);
             ref = p;
             p = sparent[k];
+        }
+        // the chains that leave the tile go on before the tile's records are written, whose stores they need not wait
+        // for: this child's box goes to global memory for the other child's chain; with several tiles per block the
+        // second arrival queues p for k_bottom_up_upper instead of climbing on, so that no chain through the upper
+        // tree holds this block at the next tile's barrier
+        if (leaves_tile) {
+            if (ref >= 0) {
+                __stcg(&nlo[ref], blo);
+                __stcg(&nhi[ref], bhi);
+            }
+            if (!climb) {
+                if (arrive_release(&visit[p]) != 0) upq[1 + atomicAdd(upq, 1)] = p;
+            } else if (arrive_acq_rel(&visit[p]) != 0) {
+                climb_from<kPack>(rc, p, child, iparent, llo, lhi, nlo, nhi, visit, leaf_face, qflag, packed);
+            }
+        }
+        __syncthreads();
+        // the tile's own nodes, one per thread: consecutive records
+        const int k = threadIdx.x;
+        if (leaf < b && leaf < n - 1 && srange[k].x >= a && srange[k].y < b) {
+            const int2 c = schild[k];
+            if (kNodes) {
+                __stcg(&nlo[leaf], slo[k]);
+                __stcg(&nhi[leaf], shi[k]);
+            }
+            if (kPack)
+                write_packed(leaf, c, c.x < 0 ? sllo[~c.x - a] : slo[c.x - a], c.x < 0 ? slhi[~c.x - a] : shi[c.x - a],
+                             c.y < 0 ? sllo[~c.y - a] : slo[c.y - a], c.y < 0 ? slhi[~c.y - a] : shi[c.y - a],
+                             c.x < 0 ? sface[~c.x - a] : -1, c.y < 0 ? sface[~c.y - a] : -1, packed);
         }
     }
 }
@@ -577,21 +587,19 @@ __device__ __forceinline__ bool box_overlap4(float4 qlo, float4 qhi, float4 lo, 
 }
 
 // First walk: candidate pairs go to the pair list. The loop is flat: a thread whose query is done takes its
-// next query in the same iteration in which the other lanes of its warp take their next node, so the lanes
-// stay busy until the warp runs out of queries. From then on, a lane without work takes the bottom entry of the
-// pending stack of a lane that has some (the subtree nearest the root, the largest), together with that lane's query
-// face and box, so that a few long walks are shared by the warp instead of setting the launch's time. A walk whose
-// pair does not fit the list, or whose deferred siblings do not fit the short stack, stops and marks its query in
-// redo[] (counted in rc->pad[3]) for the second walk.
+// next query in the same iteration in which the other lanes of its warp take their next node. A lane without work or
+// queries of its own takes the bottom entry of the pending stack of a lane that has some (the subtree nearest the root,
+// the largest), together with that lane's query face and box: the r-th such lane gives to the r-th idle one through
+// shared memory. Where there are fewer queries than lanes, each warp takes few of them (the first `own` lanes) and its other
+// lanes live on shares, so that a walk of a hundred dependent loads is the work of several lanes from the start. With a
+// lane per query and shares found by searching the votes bit by bit, a launch took 43 us of a round from 1,280 faces and
+// 79 us of one from a height field of 286k.
+// The pairs of a step go to the warp's chunk of the list, one atomic on its length serving many steps; unused slots of
+// its last chunk are set to -1. A walk whose pair does not fit the list, or whose deferred siblings do not fit the short
+// stack, stops and marks its query in redo[] (counted in rc->pad[3]) for the second walk.
 // With fmesh, a query walks only the subtree of its own mesh (mesh_root; < 0: the mesh has one leaf, no pair).
 __device__ __forceinline__ int query_root(int f, const int* __restrict__ fmesh, const int* __restrict__ mesh_root) {
     return fmesh ? mesh_root[fmesh[f]] : 0;
-}
-
-// the lane of the r-th set bit of m (r < popc(m))
-__device__ __forceinline__ int nth_lane(unsigned m, int r) {
-    for (int k = 0; k < r; ++k) m &= m - 1u;
-    return __ffs(m) - 1;
 }
 
 __global__ void __launch_bounds__(kQueryThreads) k_traverse_list(const float4* __restrict__ packed,
@@ -603,23 +611,25 @@ __global__ void __launch_bounds__(kQueryThreads) k_traverse_list(const float4* _
                                                                   const int* __restrict__ mesh_root) {
     pdl_wait();
     __shared__ int stack[kShortStack][kQueryThreads];
+    __shared__ int2 share_q[kQueryThreads];  // (query face, query), with the node in share_lo.w and the box
+    __shared__ float4 share_lo[kQueryThreads], share_hi[kQueryThreads];
     int* n_list = &rc->pad[1];
     const int nq = rc->pad[2];
     const bool empty = rc->n_live < 2;
     unsigned long long npairs = 0;
-    // each lane fills its own chunk of kPairChunk list slots, so that one atomic on the list length serves
-    // many pairs (a single counter is an L2 hot spot); unused slots of a lane's last chunk are set to -1
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, me = threadIdx.x, w0 = me & ~31;
     const unsigned lower = (1u << lane) - 1u;
-    int cbase = -1, cused = kPairChunk;
-    int qi = gtid() - gstride();  // this lane's query iterator
+    const int warps = gstride() >> 5;
+    const int own = max(1, min(32, (nq + warps - 1) / warps));
+    int cbase = -1, cused = kPairChunk;  // the warp's chunk
+    int qi = (gtid() >> 5) * own + lane - warps * own;  // this lane's query iterator
     int wq = -1;                  // the query of the current walk (the lane's own or a shared one)
-    bool supply = true;           // this lane may still get queries of its own
+    bool supply = lane < own;     // this lane may still get queries of its own
     int f = 0, node = -1, sp = 0, bot = 0, guard = 0;  // pending entries: stack[bot .. sp)
     float4 qlo = make_float4(0.f, 0.f, 0.f, 0.f), qhi = qlo;
     while (true) {
         if (node < 0 && supply) {
-            qi += gstride();
+            qi += warps * own;
             if (qi >= nq) {
                 supply = false;
             } else {
@@ -637,106 +647,114 @@ __global__ void __launch_bounds__(kQueryThreads) k_traverse_list(const float4* _
                 }
             }
         }
-        // sharing, once lanes are out of queries (every lane takes part: the shuffles need the whole warp)
+        // sharing, once lanes are out of queries (every lane takes part in the votes)
         const bool idle = node < 0 && !supply;
         const unsigned I = __ballot_sync(0xffffffffu, idle);
         if (I == 0xffffffffu) break;
-        const unsigned D = __ballot_sync(0xffffffffu, node >= 0 && sp > bot);
+        const bool gives = node >= 0 && sp > bot;
+        const unsigned D = __ballot_sync(0xffffffffu, gives);
         if (I != 0u && D != 0u) {
-            int partner = -1;
-            if (idle) {
-                const int r = __popc(I & lower);
-                if (r < __popc(D)) partner = nth_lane(D, r);
-            } else if ((D >> lane) & 1u) {
-                const int r = __popc(D & lower);
-                if (r < __popc(I)) partner = nth_lane(I, r);
+            const int r = __popc((idle ? I : D) & lower), shares = min(__popc(I), __popc(D));
+            if (gives && r < shares) {
+                share_q[w0 + r] = make_int2(f, wq);
+                share_lo[w0 + r] = make_float4(qlo.x, qlo.y, qlo.z, __int_as_float(stack[bot++][me]));
+                share_hi[w0 + r] = qhi;
             }
-            int give = -1;
-            if (!idle && partner >= 0) give = stack[bot++][threadIdx.x];
-            const int src = (idle && partner >= 0) ? partner : lane;
-            const int g_node = __shfl_sync(0xffffffffu, give, src);
-            const int g_f = __shfl_sync(0xffffffffu, f, src);
-            const int g_wq = __shfl_sync(0xffffffffu, wq, src);
-            const float4 g_lo = make_float4(__shfl_sync(0xffffffffu, qlo.x, src), __shfl_sync(0xffffffffu, qlo.y, src),
-                                            __shfl_sync(0xffffffffu, qlo.z, src), 0.f);
-            const float4 g_hi = make_float4(__shfl_sync(0xffffffffu, qhi.x, src), __shfl_sync(0xffffffffu, qhi.y, src),
-                                            __shfl_sync(0xffffffffu, qhi.z, src), 0.f);
-            if (idle && partner >= 0) {
-                node = g_node;
-                f = g_f;
-                wq = g_wq;
-                qlo = g_lo;
-                qhi = g_hi;
+            __syncwarp();
+            if (idle && r < shares) {
+                const int2 q = share_q[w0 + r];
+                qlo = share_lo[w0 + r];
+                qhi = share_hi[w0 + r];
+                node = __float_as_int(qlo.w);
+                f = q.x;
+                wq = q.y;
                 sp = bot = 0;
                 guard = 0;
             }
+            __syncwarp();
         }
-        if (node < 0) continue;
-        if (++guard > (1 << 22)) {
-            atomicOr(&rc->status, kErrIterLimit);
-            node = -1;
-            continue;
-        }
-        const float4* rec = packed + 4 * (size_t)node;
-        const float4 alo = __ldg(rec), ahi = __ldg(rec + 1), blo = __ldg(rec + 2), bhi = __ldg(rec + 3);
-        int next[2];
-        int nn = 0;
+        int hit0 = -1, hit1 = -1;
         bool abandon = false;
+        if (node >= 0) {
+            if (++guard > (1 << 22)) {
+                atomicOr(&rc->status, kErrIterLimit);
+                node = -1;
+            } else {
+                const float4* rec = packed + 4 * (size_t)node;
+                const float4 alo = __ldg(rec), ahi = __ldg(rec + 1), blo = __ldg(rec + 2), bhi = __ldg(rec + 3);
+                int next[2];
+                int nn = 0;
 #pragma unroll
-        for (int side = 0; side < 2; ++side) {
-            const float4 lo = side ? blo : alo, hi = side ? bhi : ahi;
-            if (!box_overlap4(qlo, qhi, lo, hi)) continue;
-            const int x = __float_as_int(lo.w);
-            if (x < 0) {
-                const int graw = __float_as_int(hi.w);
-                const int g = graw & ~kQueryBit;
-                if (g == f) continue;
-                if (g < f && (graw & kQueryBit)) continue;  // the lower query face owns the pair
-                if (cused == kPairChunk) {
-                    const unsigned am = __activemask();
-                    const int leader = __ffs(am) - 1;
-                    int b = 0;
-                    if (lane == leader) b = atomicAdd(n_list, kPairChunk * __popc(am));
-                    b = __shfl_sync(am, b, leader);
-                    cbase = b + kPairChunk * __popc(am & lower);
-                    cused = 0;
+                for (int side = 0; side < 2; ++side) {
+                    const float4 lo = side ? blo : alo, hi = side ? bhi : ahi;
+                    if (!box_overlap4(qlo, qhi, lo, hi)) continue;
+                    const int x = __float_as_int(lo.w);
+                    if (x < 0) {
+                        const int graw = __float_as_int(hi.w);
+                        const int g = graw & ~kQueryBit;
+                        if (g == f) continue;
+                        if (g < f && (graw & kQueryBit)) continue;  // the lower query face owns the pair
+                        if (side) hit1 = g;
+                        else hit0 = g;
+                    } else {
+                        next[nn++] = x;
+                    }
                 }
-                const int at = cbase + cused++;
+                if (nn == 2) {
+                    if (sp >= kShortStack && bot > 0) {  // entries given away at the bottom: move the rest down
+                        for (int k = bot; k < sp; ++k) stack[k - bot][me] = stack[k][me];
+                        sp -= bot;
+                        bot = 0;
+                    }
+                    if (sp >= kShortStack) {
+                        abandon = true;
+                    } else {
+                        stack[sp++][me] = next[1];
+                        node = next[0];
+                    }
+                } else if (nn == 1) {
+                    node = next[0];
+                } else {
+                    node = sp > bot ? stack[--sp][me] : -1;
+                }
+            }
+        }
+        const unsigned m0 = __ballot_sync(0xffffffffu, hit0 >= 0), m1 = __ballot_sync(0xffffffffu, hit1 >= 0);
+        if ((m0 | m1) != 0u) {
+            const int n0 = __popc(m0), n = n0 + __popc(m1);
+            int fresh = -1;
+            if (cused + n > kPairChunk) {
+                if (lane == 0) fresh = atomicAdd(n_list, kPairChunk);
+                fresh = __shfl_sync(0xffffffffu, fresh, 0);
+            }
+#pragma unroll
+            for (int side = 0; side < 2; ++side) {
+                const int g = side ? hit1 : hit0;
+                if (g < 0) continue;
+                const int k = cused + (side ? n0 + __popc(m1 & lower) : __popc(m0 & lower));
+                const int at = k < kPairChunk ? cbase + k : fresh + (k - kPairChunk);
                 if (at < pair_cap) {
                     pairs_out[at] = make_int2(f, g);
                     ++npairs;
                 } else {
                     abandon = true;
                 }
-            } else {
-                next[nn++] = x;
             }
-        }
-        if (nn == 2) {
-            if (sp >= kShortStack && bot > 0) {  // entries given away at the bottom: move the rest down
-                for (int k = bot; k < sp; ++k) stack[k - bot][threadIdx.x] = stack[k][threadIdx.x];
-                sp -= bot;
-                bot = 0;
+            cused += n;
+            if (fresh >= 0) {
+                cbase = fresh;
+                cused -= kPairChunk;
             }
-            if (sp >= kShortStack) {
-                abandon = true;
-            } else {
-                stack[sp++][threadIdx.x] = next[1];
-                node = next[0];
-            }
-        } else if (nn == 1) {
-            node = next[0];
-        } else {
-            node = sp > bot ? stack[--sp][threadIdx.x] : -1;
         }
         if (abandon) {
             redo[wq] = 1;
             atomicAdd(&rc->pad[3], 1);
             node = -1;
+            sp = bot = 0;
         }
     }
     if (cbase >= 0)
-        for (int k = cused; k < kPairChunk && cbase + k < pair_cap; ++k) pairs_out[cbase + k] = make_int2(-1, -1);
+        for (int k = cused + lane; k < kPairChunk && cbase + k < pair_cap; k += 32) pairs_out[cbase + k] = make_int2(-1, -1);
     __syncwarp();
     for (int o = 16; o > 0; o >>= 1) npairs += __shfl_xor_sync(0xffffffffu, npairs, o);
     if (lane == 0 && npairs) atomicAdd(&rc->n_pairs, npairs);
@@ -746,6 +764,8 @@ __global__ void __launch_bounds__(kQueryThreads) k_traverse_list(const float4* _
 // path, a few pairs in a thousand) is queued in xq, and k_pairs_exact runs those one per thread spread over every SM
 // (decided where they were listed, they clustered in a few warps and the float64 pipes of a few SMs set the time).
 // An order that finds the queue full is decided in place. Either way it sets the same flags.
+// The certificate that settles nearly every pair is the same for both orders and is tried first and once; with the walk
+// above, one intersection check of 327,680 faces went from 705 to 566 us.
 __global__ void __launch_bounds__(128, 8) k_pairs(const int4* __restrict__ tri, const float4* __restrict__ pos,
                                                const int2* __restrict__ pair_list, int pair_cap, unsigned char* hit,
                                                RoundCounters* rc, float eps, int4* xq, int xq_cap, int* xq_count) {
@@ -764,11 +784,24 @@ __global__ void __launch_bounds__(128, 8) k_pairs(const int4* __restrict__ tri, 
         if (shared >= 2) continue;
         const float4 q0 = pos[qt.x], q1 = pos[qt.y], q2 = pos[qt.z];
         const float4 g0 = pos[gt.x], g1 = pos[gt.y], g2 = pos[gt.z];
-        PairGeom ga, gb;
+        PairGeom ga;
         pair_geom(g0, g1, g2, gt, q0, q1, q2, qt, ga);  // reference order: the hit is "current"
-        pair_geom(q0, q1, q2, qt, g0, g1, g2, gt, gb);  // the order seen from g's own query
-        const bool need_a = !pair_certainly_disjoint(ga);
-        const bool need_b = !pair_certainly_disjoint(gb);
+        // the order seen from g's own query: the same translated faces with A and B exchanged, unless the translation
+        // rounds the other way; then the tests of one side against the other's plane are the same ones
+        int mx, my, mz;
+        pair_translation(q0, q1, q2, g0, g1, g2, mx, my, mz);
+        const bool same = mx == ga.mx && my == ga.my && mz == ga.mz;
+        if (same && pair_separated(ga)) continue;
+        bool need_a, need_b;
+        if (same) {
+            need_a = !pair_negligible(ga.A, ga.B, ga.cmax);
+            need_b = !pair_negligible(ga.B, ga.A, ga.cmax);
+        } else {
+            need_a = !pair_certainly_disjoint(ga);
+            PairGeom gb;
+            pair_geom(q0, q1, q2, qt, g0, g1, g2, gt, gb);
+            need_b = !pair_certainly_disjoint(gb);
+        }
         if (!need_a && !need_b) continue;
         exact += (unsigned)need_a + (unsigned)need_b;
         // one queue slot per order, taken for the whole warp by one atomic
@@ -1051,7 +1084,8 @@ void bvh_query(const BvhBuffers& b, const int4* tri, const float4* pos, const Bv
             nb = 4;
         return nb;
     }();
-    pdl(k_traverse_list, grid_for(n_query_bound, kQueryThreads, blocks_per_sm), kQueryThreads, 0, s)(
+    // four lanes a query while the GPU has room (k_traverse_list spreads them)
+    pdl(k_traverse_list, grid_for(4ll * n_query_bound, kQueryThreads, blocks_per_sm), kQueryThreads, 0, s)(
         b.packed, b.box_lo, b.box_hi, b.vals[1], pair_list, pair_cap, rc, b.visit, fmesh, mesh_root);
     note_launch();
     pdl(k_pairs, grid_for((long long)pair_cap, 128, 16), 128, 0, s)(tri, pos, pair_list, pair_cap, query.hit, rc, eps, b.xq,

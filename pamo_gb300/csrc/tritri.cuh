@@ -227,15 +227,26 @@ struct PairGeom {
     Tri9 A, B;  // A = BVH hit ("current"), B = querying face, both translated
     int shared, sa, sb;
     float cmax;
+    int mx, my, mz;  // the translation taken off
 };
+
+// the translation of a pair: the floored means of the six coordinates, summed in the order of the pair
+__device__ __forceinline__ void pair_translation(const float4 c0, const float4 c1, const float4 c2, const float4 q0,
+                                                 const float4 q1, const float4 q2, int& mx, int& my, int& mz) {
+    mx = floor_mean6(c0.x, c1.x, c2.x, q0.x, q1.x, q2.x);
+    my = floor_mean6(c0.y, c1.y, c2.y, q0.y, q1.y, q2.y);
+    mz = floor_mean6(c0.z, c1.z, c2.z, q0.z, q1.z, q2.z);
+}
 
 __device__ __forceinline__ void pair_geom(const float4 c0, const float4 c1, const float4 c2, const int4 ct, const float4 q0,
                                           const float4 q1, const float4 q2, const int4 qt, PairGeom& g) {
     g.A = {{{c0.x, c0.y, c0.z}, {c1.x, c1.y, c1.z}, {c2.x, c2.y, c2.z}}};
     g.B = {{{q0.x, q0.y, q0.z}, {q1.x, q1.y, q1.z}, {q2.x, q2.y, q2.z}}};
-    const int mx = floor_mean6(g.A.v[0][0], g.A.v[1][0], g.A.v[2][0], g.B.v[0][0], g.B.v[1][0], g.B.v[2][0]);
-    const int my = floor_mean6(g.A.v[0][1], g.A.v[1][1], g.A.v[2][1], g.B.v[0][1], g.B.v[1][1], g.B.v[2][1]);
-    const int mz = floor_mean6(g.A.v[0][2], g.A.v[1][2], g.A.v[2][2], g.B.v[0][2], g.B.v[1][2], g.B.v[2][2]);
+    int mx, my, mz;
+    pair_translation(c0, c1, c2, q0, q1, q2, mx, my, mz);
+    g.mx = mx;
+    g.my = my;
+    g.mz = mz;
 #pragma unroll
     for (int v = 0; v < 3; ++v) {
         g.A.v[v][0] -= mx; g.A.v[v][1] -= my; g.A.v[v][2] -= mz;
@@ -261,20 +272,24 @@ __device__ __forceinline__ void pair_geom(const float4 c0, const float4 c1, cons
         for (int d = 0; d < 3; ++d) g.cmax = fmaxf(g.cmax, fmaxf(fabsf(g.A.v[v][d]), fabsf(g.B.v[v][d])));
 }
 
-// true when the reference's decision is certainly "no intersection" without the fp64 path
-__device__ __forceinline__ bool pair_certainly_disjoint(const PairGeom& g) {
-    if (g.shared >= 2) return true;
-    {
-        const float e6 = 1e-6f;
-        int s = 0;
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-            s += (same_eps(g.A.v[i], g.B.v[0], e6) || same_eps(g.A.v[i], g.B.v[1], e6) || same_eps(g.A.v[i], g.B.v[2], e6)) ? 1 : 0;
-        if (s >= 2) return true;
-    }
-    if (coplanar_f(g.A, g.B, g.cmax) == 1) return true;
+// The two grounds on which the reference's decision is certainly "no intersection" without the fp64 path.
+// The faces lie on one side of each other's plane (of either plane, for faces without a common vertex): the same for both
+// orders of a pair.
+__device__ __forceinline__ bool pair_separated(const PairGeom& g) {
     if (g.shared == 0) return strictly_one_side(g.A, g.B, -1, g.cmax) || strictly_one_side(g.B, g.A, -1, g.cmax);
     return strictly_one_side(g.A, g.B, g.sb, g.cmax) && strictly_one_side(g.B, g.A, g.sa, g.cmax);
+}
+// Two vertices of A coincide with vertices of B, or B lies in A's plane: this order's.
+__device__ __forceinline__ bool pair_negligible(const Tri9& A, const Tri9& B, float cmax) {
+    const float e6 = 1e-6f;
+    int s = 0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        s += (same_eps(A.v[i], B.v[0], e6) || same_eps(A.v[i], B.v[1], e6) || same_eps(A.v[i], B.v[2], e6)) ? 1 : 0;
+    return s >= 2 || coplanar_f(A, B, cmax) == 1;
+}
+__device__ __forceinline__ bool pair_certainly_disjoint(const PairGeom& g) {
+    return g.shared >= 2 || pair_separated(g) || pair_negligible(g.A, g.B, g.cmax);
 }
 
 // the reference's fp64 decision on a translated pair

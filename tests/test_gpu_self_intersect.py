@@ -21,6 +21,18 @@ def test_flags_match_oracle(seed, amp):
     assert np.array_equal(got, ref)
 
 
+@pytest.mark.parametrize("faces", [1, 2, 3, 31, 33, 511, 512, 513, 1025, 1537, 2880])
+def test_flags_at_the_edges_of_tiles_and_warps(faces):
+    """Trees of one leaf to several bottom-up tiles of 512, and walks of one to many queries a warp."""
+    import pamo_gb300
+
+    v, f = meshes.tangled(12, seed=21, amp=0.3)
+    f = np.ascontiguousarray(f[np.random.default_rng(2).permutation(len(f))[:faces]])
+    ref, _ = orc.Oracle().self_intersect(v, f)
+    got = pamo_gb300.self_intersect(torch.from_numpy(v).cuda(), torch.from_numpy(f).cuda()).cpu().numpy()
+    assert np.array_equal(got, ref)
+
+
 def test_star_shaped_input_is_clean():
     import pamo_gb300
     from pamo_gb300 import synth
