@@ -926,8 +926,13 @@ __global__ void __launch_bounds__(kT) k_contacts_scatter(const int* __restrict__
 // vertex offsets coff into ctmp (in the order the atomics come), then ranked within each vertex's range by one
 // warp (ascending codes), which gives each corner its position cinv[4b + k] = coff[v] + rank. The per-corner parts
 // of a contact are written at those positions, so each vertex's contact parts are contiguous and in code order.
+// Contacts are detected to 20 times the distance at which the barrier begins, so nearly all of them have no term. A vertex
+// whose contacts all have none (cact, marked by the energy pass) has only zero parts: its corners get no positions, no
+// parts are written for them, and its sums leave them out; the other vertices' sums keep every part in its place. With
+// 157,922 contacts on 12,828 faces the zero parts were most of the PCG's traffic.
 __global__ void __launch_bounds__(kT) k_cvert_fill(const int4* __restrict__ c_idx, const int* __restrict__ coff,
-                                                   int* ccur, int* ctmp, const SolverScalars* sc) {
+                                                   const int* __restrict__ cact, int* ccur, int* ctmp,
+                                                   const SolverScalars* sc) {
     pdl_wait();
     if (sc->abort) return;
     const int n = 4 * sc->n_contacts;
@@ -935,17 +940,19 @@ __global__ void __launch_bounds__(kT) k_cvert_fill(const int4* __restrict__ c_id
         const int4 id = c_idx[s >> 2];
         const int k = s & 3;
         const int v = k == 0 ? id.x : k == 1 ? id.y : k == 2 ? id.z : id.w;
-        ctmp[coff[v] + atomicAdd(&ccur[v], 1)] = s;
+        if (cact[v]) ctmp[coff[v] + atomicAdd(&ccur[v], 1)] = s;
     }
 }
 
 __global__ void __launch_bounds__(kT) k_cvert_rank(const int* __restrict__ coff, const int* __restrict__ ctmp,
-                                                   int* cinv, int np, const SolverScalars* sc) {
+                                                   const int* __restrict__ cact, int* cinv, int np,
+                                                   const SolverScalars* sc) {
     pdl_wait();
     if (sc->abort) return;
     const int lane = threadIdx.x & 31;
     const long long warps = (long long)gridDim.x * (blockDim.x / 32);
     for (long long v = gtid() / 32; v < np; v += warps) {
+        if (!cact[v]) continue;
         const int a = coff[v], m = coff[v + 1] - a;
         for (int b0 = 0; b0 < m; b0 += 32) {
             const int x = b0 + lane < m ? ctmp[a + b0 + lane] : INT_MAX;
@@ -969,6 +976,7 @@ constexpr int kGather = 8;
 struct VertexSlots {
     const int* vs_off;   // NP + 1 offsets of the static parts
     const int* coff;     // NP + 1 offsets of the contact parts
+    const int* cact;     // NP marks: the vertex has contact parts that are not zero
     const int* inv_vs;   // position of static code 3f + c (triangle corner) or 3 NT + 4h + a (hinge slot)
     const int* cinv;     // position (after cbase) of contact code 4b + k
     int cbase;           // 3 NT + 4 NH
@@ -984,7 +992,7 @@ __device__ __forceinline__ VRange vertex_range(const VertexSlots& S, int i, bool
         R.m1 = S.vs_off[i + 1] - R.a;
         const int c0 = S.coff[i];
         R.ca = S.cbase + c0;
-        R.m = R.m1 + S.coff[i + 1] - c0;
+        R.m = S.cact[i] ? R.m1 + S.coff[i + 1] - c0 : R.m1;
     }
     return R;
 }
@@ -1091,6 +1099,7 @@ struct EnergyArgs {
     int2* ctype;
     float* cd;
     float kappa, d_hat, ee_thres;
+    int* cact;  // or null: marks the vertices of contacts with a barrier term
 };
 
 namespace {
@@ -1142,6 +1151,7 @@ __device__ __forceinline__ CSum energy_elements(const float4* __restrict__ x, co
             }
             A.ctype[b] = t;
             A.cd[b] = d;
+            if (A.cact && !(d >= A.d_hat)) A.cact[i.x] = A.cact[i.y] = A.cact[i.z] = A.cact[i.w] = 1;
             e = d < A.d_hat ? barrier(d, A.d_hat) * A.kappa : 0.f;
         }
         acc.add(e);
@@ -1370,25 +1380,32 @@ __global__ void __launch_bounds__(32 * kSpdWarps) k_spd_project(float* blocks, i
     }
 }
 
-// collision_diff_kernel (collision_energy.py:192-254)
+// collision_diff_kernel (collision_energy.py:192-254). cneed[b]: contact b has parts to write (here and in the PCG).
 __global__ void k_diff_contact(const float4* __restrict__ x, const int4* __restrict__ cidx, const int2* __restrict__ ctype,
                                const float* __restrict__ cd, const SolverScalars* sc, float kappa, float dh, float coeff,
-                               float4* cdd, float4* gslot, float4* hslot, const int* __restrict__ cinv) {
+                               float4* cdd, float4* gslot, float4* hslot, const int* __restrict__ cinv,
+                               const int* __restrict__ cact, int* cneed) {
     pdl_wait();
     if (sc->abort) return;
     const int n = sc->n_contacts;
     for (int b = gtid(); b < n; b += gstride()) {
         const float d = cd[b];
         const int* at = cinv + 4 * (size_t)b;
-        if (d >= dh) {  // no barrier term: zero parts
+        const int4 i = cidx[b];
+        if (d >= dh) {  // no barrier term: zero parts, at the vertices that have others
             const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+            const int ids[4] = {i.x, i.y, i.z, i.w};
+            int need = 0;
             for (int k = 0; k < 4; ++k) {
+                if (!cact[ids[k]]) continue;
                 gslot[at[k]] = zero;
                 hslot[at[k]] = zero;
+                need = 1;
             }
+            cneed[b] = need;
             continue;
         }
-        const int4 i = cidx[b];
+        cneed[b] = 1;
         const F3 x0 = f3(x[i.x]), x1 = f3(x[i.y]), x2 = f3(x[i.z]), x3 = f3(x[i.w]);
         const int2 t = ctype[b];
         F3 g[4];
@@ -1457,6 +1474,7 @@ struct HvpArgs {
     const int4* cidx;
     const float* cd;
     const float4* cdd;
+    const int* cneed;
     float kappa, d_hat;
     float4* aslot;  // per-corner parts of H v (triangles, hinges, then contacts at S.cbase)
     VertexSlots S;
@@ -1467,7 +1485,7 @@ __device__ __forceinline__ F3 cg_dir(const float4* __restrict__ z, const float4*
 }
 
 // The vertex ids of element g of hvp_elements (a triangle, hinge or contact; zeros for a vertex term or past
-// the end). They do not change during a solve, so a thread loads those of its first element once.
+// the end).
 __device__ __forceinline__ int4 element_ids(const HvpArgs& A, int nc, long long g) {
     const long long e1 = A.np, e2 = e1 + A.nt, e3 = e2 + A.nh, total = e3 + nc;
     if (g < e1 || g >= total) return make_int4(0, 0, 0, 0);
@@ -1476,8 +1494,7 @@ __device__ __forceinline__ int4 element_ids(const HvpArgs& A, int nc, long long 
     return A.cidx[g - e3];
 }
 
-// Where the corners' parts of element g go in A.aslot (unused entries zero; the vertex terms have none). Like the
-// ids they are fixed during a solve, so a thread loads those of its first element once.
+// Where the corners' parts of element g go in A.aslot (unused entries zero; the vertex terms have none).
 __device__ __forceinline__ int4 element_slots(const HvpArgs& A, int nc, long long g) {
     const long long e1 = A.np, e2 = e1 + A.nt, e3 = e2 + A.nh, total = e3 + nc;
     if (g < e1 || g >= total) return make_int4(0, 0, 0, 0);
@@ -1493,111 +1510,162 @@ __device__ __forceinline__ int4 element_slots(const HvpArgs& A, int nc, long lon
     return make_int4(A.S.cbase + at[0], A.S.cbase + at[1], A.S.cbase + at[2], A.S.cbase + at[3]);
 }
 
-// The corners' parts of H v over the elements gtid, gtid + stride, ... into A.aslot; returns this thread's part of
-// v.Av. The direction is v = z + s v_prev, written to vout by the vertex terms. ids0 = element_ids(first),
-// at0 = element_slots(first).
-__device__ __forceinline__ CSum hvp_elements(const float4* __restrict__ x, const HvpArgs& A, const float4* __restrict__ z,
-                                             const float4* __restrict__ vprev, float4* vout, float s, int nc,
-                                             long long first, long long stride, int4 ids0, int4 at0) {
+// What a product with an element's Hessian needs besides the direction: a triangle's or contact's factors, or a hinge's
+// block (kHingeStride floats), fixed during a solve, so that a thread keeps those of its first element in registers for
+// all its iterations (a barrier's acquire empties L1: read again they came from L2, 192 bytes a hinge).
+enum { kElNone = 0, kElVertex = 1, kElTri = 2, kElHinge = 3, kElContact = 4, kElContactOff = 5 };
+struct HvpElement {
+    int kind;
+    int index;   // of the vertex
+    int4 ids, at;
+    float e[kHingeStride];
+};
+
+__device__ __forceinline__ HvpElement load_element(const float4* __restrict__ x, const HvpArgs& A, int nc, long long g) {
     const long long e1 = A.np, e2 = e1 + A.nt, e3 = e2 + A.nh, total = e3 + nc;
-    CSum acc;
-    for (long long g = first; g < total; g += stride) {
-        const bool cached = g == first;
-        if (g < e1) {
-            const int i = (int)g;
-            const F3 vi = cg_dir(z, vprev, s, i);
-            vout[i] = f4(vi);
-            const float wi = A.w[i] * A.m2gt_k;
-            acc.add(dot(vi, vi * wi));
-        } else if (g < e2) {
-            const int f = (int)(g - e1);
-            const int4 t = cached ? ids0 : A.tri[f];
-            const ElasticLocal L = elastic_local(x, t, A.area[f], A.invDm[f]);
-            const F3 v0 = cg_dir(z, vprev, s, t.x), v1 = cg_dir(z, vprev, s, t.y), v2 = cg_dir(z, vprev, s, t.z);
-            const F3 dx01 = v1 - v0, dx02 = v2 - v0;
-            const Mat2 dDs = {dot(L.b1, dx01), dot(L.b1, dx02), dot(L.b2, dx01), dot(L.b2, dx02)};
-            const Mat2 dF = mmul(dDs, L.invDm);
-            const Mat2 I = {1.f, 0.f, 0.f, 1.f};
-            const Mat2 E = mscale(0.5f, madd(mmul(mtr(L.F), L.F), mscale(-1.f, I)));
-            const float trE = mtrace(E);
-            const Mat2 dE = mscale(0.5f, madd(mmul(mtr(dF), L.F), mmul(mtr(L.F), dF)));
-            const float trdE = mtrace(dE);
-            const Mat2 dP = madd(mmul(dF, madd(mscale(2.f * A.mu, E), mscale(A.la * trE, I))),
-                                 mmul(L.F, madd(mscale(2.f * A.mu, dE), mscale(A.la * trdE, I))));
-            const Mat2 dH = mmul(mscale(L.W, dP), mtr(L.invDm));
-            const F3 df1 = dH.a * L.b1 + dH.c * L.b2;
-            const F3 df2 = dH.b * L.b1 + dH.d * L.b2;
-            const F3 df0 = -df1 - df2;
-            const int4 at = cached ? at0 : element_slots(A, nc, g);
-            A.aslot[at.x] = f4(df0);
-            A.aslot[at.y] = f4(df1);
-            A.aslot[at.z] = f4(df2);
-            acc.add(dot(v0, df0) + dot(v1, df1) + dot(v2, df2));
-        } else if (g < e3) {
-            const int h = (int)(g - e2);
-            const int4 id = cached ? ids0 : A.hinge[h];
-            const int ids[4] = {id.x, id.y, id.z, id.w};
-            // H v with the fourth block row/column minus the sums of the first three: for w_a = v_a - v_3,
-            // (H v)_a = sum_b A_ab w_b (a < 3), (H v)_3 = -sum_a (H v)_a, and v.H v = w.A w
-            const float4* B4 = reinterpret_cast<const float4*>(A.blocks + (size_t)h * kHingeStride);
-            float Bm[kHingeStride];
+    HvpElement E;
+    E.kind = kElNone;
+    E.index = 0;
+    E.ids = E.at = make_int4(0, 0, 0, 0);
+    if (g >= total) return E;
+    if (g < e1) {
+        E.kind = kElVertex;
+        E.index = (int)g;
+        E.e[0] = A.w[g] * A.m2gt_k;
+        return E;
+    }
+    if (g >= e3 && !A.cneed[g - e3]) return E;  // no parts
+    E.ids = element_ids(A, nc, g);
+    E.at = element_slots(A, nc, g);
+    if (g < e2) {
+        const int f = (int)(g - e1);
+        E.kind = kElTri;
+        const ElasticLocal L = elastic_local(x, E.ids, A.area[f], A.invDm[f]);
+        const Mat2 I = {1.f, 0.f, 0.f, 1.f};
+        const Mat2 S = mscale(0.5f, madd(mmul(mtr(L.F), L.F), mscale(-1.f, I)));
+        const Mat2 M = madd(mscale(2.f * A.mu, S), mscale(A.la * mtrace(S), I));
+        E.e[0] = L.b1.x; E.e[1] = L.b1.y; E.e[2] = L.b1.z;
+        E.e[3] = L.b2.x; E.e[4] = L.b2.y; E.e[5] = L.b2.z;
+        E.e[6] = L.F.a; E.e[7] = L.F.b; E.e[8] = L.F.c; E.e[9] = L.F.d;
+        E.e[10] = L.invDm.a; E.e[11] = L.invDm.b; E.e[12] = L.invDm.c; E.e[13] = L.invDm.d;
+        E.e[14] = M.a; E.e[15] = M.b; E.e[16] = M.c; E.e[17] = M.d;
+        E.e[18] = L.W;
+    } else if (g < e3) {
+        E.kind = kElHinge;
+        const float4* B4 = reinterpret_cast<const float4*>(A.blocks + (size_t)(g - e2) * kHingeStride);
 #pragma unroll
-            for (int k = 0; k < kHingeStride / 4; ++k) {
-                const float4 b = B4[k];
-                Bm[4 * k] = b.x; Bm[4 * k + 1] = b.y; Bm[4 * k + 2] = b.z; Bm[4 * k + 3] = b.w;
-            }
-            const F3 d3 = cg_dir(z, vprev, s, ids[3]);
-            float w[9];
+        for (int k = 0; k < kHingeStride / 4; ++k) {
+            const float4 b = B4[k];
+            E.e[4 * k] = b.x; E.e[4 * k + 1] = b.y; E.e[4 * k + 2] = b.z; E.e[4 * k + 3] = b.w;
+        }
+    } else {
+        const int b = (int)(g - e3);
+        const float dist = A.cd[b];
+        if (dist >= A.d_hat) {  // no barrier term: zero parts, at the vertices that have others
+            E.kind = kElContactOff;
+            if (!A.S.cact[E.ids.x]) E.at.x = -1;
+            if (!A.S.cact[E.ids.y]) E.at.y = -1;
+            if (!A.S.cact[E.ids.z]) E.at.z = -1;
+            if (!A.S.cact[E.ids.w]) E.at.w = -1;
+            return E;
+        }
+        E.kind = kElContact;
+        E.e[12] = barrier_d2(dist, A.d_hat) * A.kappa;
 #pragma unroll
-            for (int b = 0; b < 3; ++b) {
-                const F3 wb = cg_dir(z, vprev, s, ids[b]) - d3;
-                w[3 * b] = wb.x; w[3 * b + 1] = wb.y; w[3 * b + 2] = wb.z;
-            }
-            float u[9];
-#pragma unroll
-            for (int i = 0; i < 9; ++i) {
-                float t = 0.f;
-#pragma unroll
-                for (int j = 0; j < 9; ++j) t += Bm[sym9(i, j)] * w[j];
-                u[i] = t;
-            }
-            float vhv = 0.f;
-            F3 sum = {0.f, 0.f, 0.f};
-            const int4 at4 = cached ? at0 : element_slots(A, nc, g);
-            const int at[4] = {at4.x, at4.y, at4.z, at4.w};
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                const F3 ua = {u[3 * a], u[3 * a + 1], u[3 * a + 2]};
-                A.aslot[at[a]] = f4(ua);
-                sum = sum + ua;
-                vhv += w[3 * a] * ua.x + w[3 * a + 1] * ua.y + w[3 * a + 2] * ua.z;
-            }
-            A.aslot[at[3]] = f4(-sum);
-            acc.add(vhv);
-        } else {
-            const int b = (int)(g - e3);
-            const float dist = A.cd[b];
-            float4* as = A.aslot;
-            const int4 at4 = cached ? at0 : element_slots(A, nc, g);
-            const int at[4] = {at4.x, at4.y, at4.z, at4.w};
-            if (dist >= A.d_hat) {  // no barrier term: zero parts
-                const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-                for (int k = 0; k < 4; ++k) as[at[k]] = zero;
-                continue;
-            }
-            const float c = barrier_d2(dist, A.d_hat) * A.kappa;
-            const int4 i = cached ? ids0 : A.cidx[b];
-            const int ids[4] = {i.x, i.y, i.z, i.w};
-            F3 gg[4];
-            float sd = 0.f;
-            for (int k = 0; k < 4; ++k) {
-                gg[k] = f3(A.cdd[4 * (size_t)b + k]);
-                sd += dot(gg[k], cg_dir(z, vprev, s, ids[k]));
-            }
-            for (int k = 0; k < 4; ++k) as[at[k]] = f4(gg[k] * (sd * c));
-            acc.add(sd * sd * c);
+        for (int k = 0; k < 4; ++k) {
+            const float4 d = A.cdd[4 * (size_t)b + k];
+            E.e[3 * k] = d.x; E.e[3 * k + 1] = d.y; E.e[3 * k + 2] = d.z;
         }
     }
+    return E;
+}
+
+// The corners' parts of H v of one element into A.aslot; returns its part of v.Av. The direction is v = z + s v_prev,
+// written to vout by the vertex terms.
+__device__ __forceinline__ float apply_element(const HvpElement& E, const HvpArgs& A, const float4* __restrict__ z,
+                                               const float4* __restrict__ vprev, float4* vout, float s) {
+    if (E.kind == kElNone) return 0.f;
+    if (E.kind == kElVertex) {
+        const F3 vi = cg_dir(z, vprev, s, E.index);
+        vout[E.index] = f4(vi);
+        return dot(vi, vi * E.e[0]);
+    }
+    if (E.kind == kElTri) {
+        const F3 v0 = cg_dir(z, vprev, s, E.ids.x), v1 = cg_dir(z, vprev, s, E.ids.y), v2 = cg_dir(z, vprev, s, E.ids.z);
+        const F3 b1 = {E.e[0], E.e[1], E.e[2]}, b2 = {E.e[3], E.e[4], E.e[5]};
+        const Mat2 F = {E.e[6], E.e[7], E.e[8], E.e[9]}, invDm = {E.e[10], E.e[11], E.e[12], E.e[13]},
+                   M = {E.e[14], E.e[15], E.e[16], E.e[17]};
+        const Mat2 I = {1.f, 0.f, 0.f, 1.f};
+        const F3 dx01 = v1 - v0, dx02 = v2 - v0;
+        const Mat2 dDs = {dot(b1, dx01), dot(b1, dx02), dot(b2, dx01), dot(b2, dx02)};
+        const Mat2 dF = mmul(dDs, invDm);
+        const Mat2 dE = mscale(0.5f, madd(mmul(mtr(dF), F), mmul(mtr(F), dF)));
+        const float trdE = mtrace(dE);
+        const Mat2 dP = madd(mmul(dF, M), mmul(F, madd(mscale(2.f * A.mu, dE), mscale(A.la * trdE, I))));
+        const Mat2 dH = mmul(mscale(E.e[18], dP), mtr(invDm));
+        const F3 df1 = dH.a * b1 + dH.c * b2;
+        const F3 df2 = dH.b * b1 + dH.d * b2;
+        const F3 df0 = -df1 - df2;
+        A.aslot[E.at.x] = f4(df0);
+        A.aslot[E.at.y] = f4(df1);
+        A.aslot[E.at.z] = f4(df2);
+        return dot(v0, df0) + dot(v1, df1) + dot(v2, df2);
+    }
+    const int ids[4] = {E.ids.x, E.ids.y, E.ids.z, E.ids.w}, at[4] = {E.at.x, E.at.y, E.at.z, E.at.w};
+    if (E.kind == kElHinge) {
+        // H v with the fourth block row/column minus the sums of the first three: for w_a = v_a - v_3,
+        // (H v)_a = sum_b A_ab w_b (a < 3), (H v)_3 = -sum_a (H v)_a, and v.H v = w.A w
+        const F3 d3 = cg_dir(z, vprev, s, ids[3]);
+        float w[9];
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+            const F3 wb = cg_dir(z, vprev, s, ids[b]) - d3;
+            w[3 * b] = wb.x; w[3 * b + 1] = wb.y; w[3 * b + 2] = wb.z;
+        }
+        float u[9];
+#pragma unroll
+        for (int i = 0; i < 9; ++i) {
+            float t = 0.f;
+#pragma unroll
+            for (int j = 0; j < 9; ++j) t += E.e[sym9(i, j)] * w[j];
+            u[i] = t;
+        }
+        float vhv = 0.f;
+        F3 sum = {0.f, 0.f, 0.f};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const F3 ua = {u[3 * a], u[3 * a + 1], u[3 * a + 2]};
+            A.aslot[at[a]] = f4(ua);
+            sum = sum + ua;
+            vhv += w[3 * a] * ua.x + w[3 * a + 1] * ua.y + w[3 * a + 2] * ua.z;
+        }
+        A.aslot[at[3]] = f4(-sum);
+        return vhv;
+    }
+    if (E.kind == kElContactOff) {
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k = 0; k < 4; ++k)
+            if (at[k] >= 0) A.aslot[at[k]] = zero;
+        return 0.f;
+    }
+    float sd = 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) sd += dot(F3{E.e[3 * k], E.e[3 * k + 1], E.e[3 * k + 2]}, cg_dir(z, vprev, s, ids[k]));
+    const float c = E.e[12];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) A.aslot[at[k]] = f4(F3{E.e[3 * k], E.e[3 * k + 1], E.e[3 * k + 2]} * (sd * c));
+    return sd * sd * c;
+}
+
+// The corners' parts of H v over the elements first, first + stride, ... into A.aslot; returns this thread's part of
+// v.Av.
+__device__ __forceinline__ CSum hvp_elements(const float4* __restrict__ x, const HvpArgs& A, const float4* __restrict__ z,
+                                             const float4* __restrict__ vprev, float4* vout, float s, int nc,
+                                             long long first, long long stride) {
+    const long long total = (long long)A.np + A.nt + A.nh + nc;
+    CSum acc;
+    for (long long g = first; g < total; g += stride)
+        acc.add(apply_element(load_element(x, A, nc, g), A, z, vprev, vout, s));
     return acc;
 }
 
@@ -1657,8 +1725,25 @@ __device__ __forceinline__ PrzVertex prz_load(const HvpArgs& A, const float4* __
     return pv;
 }
 
-// p += alpha v, r -= alpha Av when v.Av > 1e-16, z = r / diag; returns z.r part. `pre` holds the values of the
-// group's first vertex, loaded before the block partials of v.Av were summed.
+// p += alpha v, r -= alpha Av when v.Av > 1e-16, z = r / diag; returns z.r
+__device__ __forceinline__ float prz_update(const PrzVertex& pv, float4* p, float4* r, float4* z, int i, float vAv,
+                                            float alpha) {
+    float4 ri = pv.r;
+    if (vAv > 1e-16f) {
+        float4 pi = pv.p;
+        pi.x += alpha * pv.v.x; pi.y += alpha * pv.v.y; pi.z += alpha * pv.v.z;
+        ri.x -= alpha * pv.av.x; ri.y -= alpha * pv.av.y; ri.z -= alpha * pv.av.z;
+        p[i] = pi;
+        r[i] = ri;
+    }
+    const float4 d = pv.d;
+    const float4 zz = make_float4(ri.x / d.x, ri.y / d.y, ri.z / d.z, 0.f);
+    z[i] = zz;
+    return zz.x * ri.x + zz.y * ri.y + zz.z * ri.z;
+}
+
+// The same over a thread's vertices; returns z.r part. `pre` holds the values of the group's first vertex, loaded before
+// the block partials of v.Av were summed.
 __device__ __forceinline__ CSum cg_prz_vertices(const HvpArgs& A, const float4* __restrict__ v,
                                                 const float4* __restrict__ hd, float4* p, float4* r, float4* z,
                                                 float zr, float vAv, const PrzLanes& L, const PrzVertex& pre) {
@@ -1669,19 +1754,7 @@ __device__ __forceinline__ CSum cg_prz_vertices(const HvpArgs& A, const float4* 
         const bool valid = i < A.np;
         const PrzVertex pv = k == 0 ? pre : prz_load(A, v, hd, p, r, valid ? i : 0, valid, L,
                                                      vertex_range(A.S, valid ? i : 0, valid));
-        if (!valid || L.lane != 0) continue;
-        float4 ri = pv.r;
-        if (vAv > 1e-16f) {
-            float4 pi = pv.p;
-            pi.x += alpha * pv.v.x; pi.y += alpha * pv.v.y; pi.z += alpha * pv.v.z;
-            ri.x -= alpha * pv.av.x; ri.y -= alpha * pv.av.y; ri.z -= alpha * pv.av.z;
-            p[i] = pi;
-            r[i] = ri;
-        }
-        const float4 d = pv.d;
-        const float4 zz = make_float4(ri.x / d.x, ri.y / d.y, ri.z / d.z, 0.f);
-        z[i] = zz;
-        acc.add(zz.x * ri.x + zz.y * ri.y + zz.z * ri.z);
+        if (valid && L.lane == 0) acc.add(prz_update(pv, p, r, z, i, vAv, alpha));
     }
     return acc;
 }
@@ -1745,6 +1818,60 @@ struct CgState {
     unsigned count;  // grid_barrier's counter, zeroed before each stage-3 run
 };
 
+constexpr int kCgK = 2;  // threads that stand for one of the sums' threads in the default launch shape on large meshes
+
+// The total over the block of the sums of its first kThreads threads (all threads call it and all get it), added as
+// block_reduce adds them; buf alternates between two buffers, so that one block barrier a call is enough.
+template <int kThreads>
+__device__ __forceinline__ CSum block_total(CSum v, float2 (*ws)[kThreads / 32], int& buf) {
+    constexpr int W = kThreads / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp < W) {
+        for (int o = 16; o > 0; o >>= 1) {
+            CSum w;
+            w.s = __shfl_down_sync(0xffffffffu, v.s, o);
+            w.c = __shfl_down_sync(0xffffffffu, v.c, o);
+            if (lane + o < 32) v.merge(w);
+        }
+        if (lane == 0) ws[buf][warp] = make_float2(v.s, v.c);
+    }
+    __syncthreads();
+    CSum w[W];
+#pragma unroll
+    for (int i = 0; i < W; ++i) {
+        const float2 t = ws[buf][i];
+        w[i].s = t.x;
+        w[i].c = t.y;
+    }
+#pragma unroll
+    for (int o = W / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < o; ++i) w[i].merge(w[i + o]);
+    buf ^= 1;
+    return w[0];
+}
+
+// Stores the block's partial, waits for the grid and returns this thread's share of the partials (block b goes to thread
+// b mod kThreads, in block order). partial alternates between two buffers: one is rewritten only after the next barrier,
+// which every block reaches after it has read it. (Without the counter, each block polling every block's partial with the
+// number of the sum beside it, the wait was slower: 24.1 -> 31.0 ms on the smaller project case, 152 blocks polling
+// 152 slots.)
+template <int kThreads>
+__device__ __forceinline__ CSum grid_exchange(CSum part, float2* partial, CgState* bar, int* status, unsigned extra) {
+    if (threadIdx.x == 0) partial[blockIdx.x] = make_float2(part.s, part.c);
+    grid_barrier(&bar->count, status, extra);
+    CSum a;
+    if (threadIdx.x < kThreads)
+        for (int b = threadIdx.x; b < (int)gridDim.x; b += kThreads) {
+            const float2 w = __ldcg(&partial[b]);
+            CSum t;
+            t.s = w.x;
+            t.c = w.y;
+            a.merge(t);
+        }
+    return a;
+}
+
 // The same solve as two ordinary launches per iteration (cg_mode 7), for when a cooperative launch, which needs its
 // whole grid resident at once, would wait for other streams' work to drain (many solves at a time on one GPU): each
 // kernel is one phase of k_cg_solve with the same grid, threads and elements, and its block partials are summed by the
@@ -1770,9 +1897,7 @@ __global__ void __launch_bounds__(kThreads) k_cg_product(const float4* __restric
     const int nc = sc->n_contacts;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
     const float s_dir = it == 0 ? 0.f : sc->z_r / sc->z_r_last;
-    const int4 ids0 = element_ids(A, nc, tid);
-    const int4 at0 = element_slots(A, nc, tid);
-    grid_sum_finish(hvp_elements(x, A, z, vin, vout, s_dir, nc, tid, nthreads, ids0, at0), partial, &sc->red_count,
+    grid_sum_finish(hvp_elements(x, A, z, vin, vout, s_dir, nc, tid, nthreads), partial, &sc->red_count,
                     &sc->v_A_v, nullptr);
 }
 
@@ -1793,43 +1918,149 @@ __global__ void __launch_bounds__(kThreads) k_cg_update(HvpArgs A, const float4*
 }
 
 // The whole Jacobi PCG solve (cg_solver.py:96-158, n_cg_iters iterations) as one cooperative kernel: each
-// iteration is the Hessian product phase and the p/r/z phase, with a grid barrier after each. Every block
+// iteration is the Hessian product phase and the p/r/z phase, with a grid-wide sum after each. Every block
 // forms the same totals (v.Av, z.r) from the block partials in block order.
-template <int kThreads>
-__global__ void __launch_bounds__(kThreads) k_cg_solve(const float4* __restrict__ x, HvpArgs A, const float4* __restrict__ grad,
-                                                 const float4* __restrict__ hd, float4* p, float4* r, float4* z,
-                                                 float4* v0, float4* v1, int n_iters, SolverScalars* sc,
-                                                 float2* partial, CgState* bar) {
+// The sums are those of a grid of kThreads threads a block, thread t taking elements t, t + threads, ... (and vertices
+// likewise). With K > 1, K threads stand for each of them: its k-th element belongs to thread k mod K, and the values are
+// added in the element order, so the bits do not depend on K while K elements' chains of loads run side by side. A
+// thread's first element and vertex stay in registers for the whole solve. Before this and the marks of contacts without a
+// barrier term, an iteration took 6.7 us on 1,534 faces without contacts and 20 us on 12,828 faces with 157,922. K = 1 is
+// the faster where each thread has one element (a whole projection 21.4 against 22.6 ms), K = 2 where it has more (79.2
+// against 69.0 ms before the marks; K = 4 spills: 97.3 ms).
+template <int kThreads, int K>
+__global__ void __launch_bounds__(kThreads* K) k_cg_solve(const float4* __restrict__ x, HvpArgs A,
+                                                          const float4* __restrict__ grad, const float4* __restrict__ hd,
+                                                          float4* p, float4* r, float4* z, float4* v0, float4* v1,
+                                                          int n_iters, SolverScalars* sc, float2* partial,
+                                                          CgState* bar) {
+    __shared__ float2 ws[2][kThreads / 32];
+    __shared__ float val[2][K > 1 ? K : 1][kThreads];
+    __shared__ unsigned need_sm[2];
     if (sc->abort) return;
     const int nc = sc->n_contacts;
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
-    float2* part_a = partial;
-    float2* part_b = partial + gridDim.x;
-    const int4 ids0 = element_ids(A, nc, tid);
-    const int4 at0 = element_slots(A, nc, tid);  // fixed for the whole solve
-    const PrzLanes L = prz_lanes(tid, nthreads, A.np);
-    const VRange R0 = vertex_range(A.S, L.group < A.np ? L.group : 0, L.group < A.np);  // the group's first vertex
+    const int t = threadIdx.x % kThreads, k = threadIdx.x / kThreads;
+    const int tid = blockIdx.x * kThreads + t, nthreads = gridDim.x * kThreads;
+    const long long total = (long long)A.np + A.nt + A.nh + nc;
     const unsigned extra = (unsigned)sc->barrier_extra;
-    store_partial(cg_init_vertices(grad, hd, A.np, p, r, z, v0, tid, nthreads), part_a);
-    grid_barrier(&bar->count, &sc->status, extra);
-    float zr = grid_partials_sum(part_a), zr_last = zr;
+    float2 *part_a = partial, *part_b = partial + gridDim.x;
+    int wbuf = 0, vbuf = 0;
+    // adds the K threads' values in their order to the first one's sum
+    auto add = [&](CSum& acc, float x_) {
+        if constexpr (K == 1) {
+            acc.add(x_);
+        } else {
+            val[vbuf][k][t] = x_;
+            __syncthreads();
+            if (k == 0)
+#pragma unroll
+                for (int i = 0; i < K; ++i) acc.add(val[vbuf][i][t]);
+            vbuf ^= 1;
+        }
+    };
+    const long long first = tid + (long long)k * nthreads, stride = (long long)K * nthreads;
+    // the same number of rounds in every thread (the adds meet in barriers)
+    const int el_rounds = (int)((total + stride - 1) / stride), v_rounds = (int)((A.np + stride - 1) / stride);
+    // the rounds after the first in which the thread (the block, where the adds meet in barriers) has parts to write: a
+    // contact without any adds nothing; rounds past 64 are all taken
+    unsigned long long need = 0;
+    for (int q = 1; q < min(el_rounds, 64); ++q) {
+        const long long g = first + q * stride, c = g - ((long long)A.np + A.nt + A.nh);
+        if (g < total && (c < 0 || A.cneed[c])) need |= 1ull << q;
+    }
+    if constexpr (K > 1) {
+        if (threadIdx.x < 2) need_sm[threadIdx.x] = 0;
+        __syncthreads();
+        const unsigned lo = __reduce_or_sync(0xffffffffu, (unsigned)need),
+                       hi = __reduce_or_sync(0xffffffffu, (unsigned)(need >> 32));
+        if ((threadIdx.x & 31) == 0) {
+            atomicOr(&need_sm[0], lo);
+            atomicOr(&need_sm[1], hi);
+        }
+        __syncthreads();
+        need = (unsigned long long)need_sm[1] << 32 | need_sm[0];
+    }
+    const HvpElement E = load_element(x, A, nc, first);
+    const PrzLanes L = prz_lanes(tid, nthreads, A.np);
+    const int prz_rounds = (L.rounds + K - 1) / K;
+    const int own = L.group + k * L.groups;  // the group's first vertex, kept by its lane 0
+    const bool own_ok = k < L.rounds && own < A.np;
+    const VRange R0 = vertex_range(A.S, own_ok ? own : 0, own_ok);
+    CSum acc;
+    for (int q = 0; q < v_rounds; ++q) {
+        const long long i = first + q * stride;
+        float zr_i = 0.f;
+        if (i < A.np) {
+            const float4 g = grad[i], d = hd[i], zero = make_float4(0.f, 0.f, 0.f, 0.f);
+            p[i] = zero;
+            r[i] = g;
+            const float4 zz = make_float4(g.x / (d.x + 1e-6f), g.y / (d.y + 1e-6f), g.z / (d.z + 1e-6f), 0.f);
+            z[i] = zz;
+            v0[i] = zero;
+            zr_i = zz.x * g.x + zz.y * g.y + zz.z * g.z;
+        }
+        add(acc, zr_i);
+    }
+    CSum share = grid_exchange<kThreads>(block_total<kThreads>(acc, ws, wbuf), part_a, bar, &sc->status, extra);
+    F3 pi{}, ri{}, zi{}, vi{}, di{};
+    float wi = 0.f;
+    if (own_ok && L.lane == 0) {
+        ri = f3(r[own]);
+        zi = f3(z[own]);
+        di = f3(hd[own]);
+        wi = A.w[own] * A.m2gt_k;
+    }
+    CSum sum = block_total<kThreads>(share, ws, wbuf);
+    float zr = sum.s + sum.c, zr_last = zr;
     for (int it = 0; it < n_iters; ++it) {
         const float4* vin = (it & 1) ? v1 : v0;
         float4* vout = (it & 1) ? v0 : v1;
         const float s_dir = it == 0 ? 0.f : zr / zr_last;
-        // partials alternate between two buffers phase by phase: a buffer is rewritten only after the next
-        // barrier, which every block reaches after it has read that buffer
-        store_partial(hvp_elements(x, A, z, vin, vout, s_dir, nc, tid, nthreads, ids0, at0), part_b);
-        grid_barrier(&bar->count, &sc->status, extra);
-        // the first vertex's loads and slot gather go out before the partials are summed (they do not depend on
-        // v.Av)
-        const PrzVertex pre = prz_load(A, vout, hd, p, r, L.group < A.np ? L.group : 0, L.group < A.np, L, R0);
-        const float vAv = grid_partials_sum(part_b);
-        store_partial(cg_prz_vertices(A, vout, hd, p, r, z, zr, vAv, L, pre), part_a);
-        grid_barrier(&bar->count, &sc->status, extra);
+        acc = CSum();
+        add(acc, apply_element(E, A, z, vin, vout, s_dir));
+        auto later = [&](int q) {
+            add(acc, apply_element(load_element(x, A, nc, first + q * stride), A, z, vin, vout, s_dir));
+        };
+        for (unsigned long long m = need; m; m &= m - 1ull) later(__ffsll(m) - 1);
+        for (int q = 64; q < el_rounds; ++q) later(q);
+        share = grid_exchange<kThreads>(block_total<kThreads>(acc, ws, wbuf), part_b, bar, &sc->status, extra);
+        // the first vertex's slot gather goes out before the partials are summed (it does not depend on v.Av)
+        F3 unused;
+        const F3 own_g = gather_range(A.aslot, nullptr, unused, R0, L.lane, L.G);
+        sum = block_total<kThreads>(share, ws, wbuf);
+        const float vAv = sum.s + sum.c, alpha = zr / vAv;
+        acc = CSum();
+        for (int q = 0; q < prz_rounds; ++q) {
+            const int i = own + q * K * L.groups;
+            const bool valid = k + q * K < L.rounds && i < A.np;
+            float zr_i = 0.f;
+            if (q == 0) {
+                if (valid && L.lane == 0) {
+                    vi = zi + s_dir * vi;
+                    const F3 av = vi * wi + own_g;
+                    if (vAv > 1e-16f) {
+                        pi.x += alpha * vi.x; pi.y += alpha * vi.y; pi.z += alpha * vi.z;
+                        ri.x -= alpha * av.x; ri.y -= alpha * av.y; ri.z -= alpha * av.z;
+                    }
+                    zi = F3{ri.x / di.x, ri.y / di.y, ri.z / di.z};
+                    z[i] = f4(zi);
+                    zr_i = zi.x * ri.x + zi.y * ri.y + zi.z * ri.z;
+                }
+            } else {
+                const PrzVertex pv = prz_load(A, vout, hd, p, r, valid ? i : 0, valid, L,
+                                              vertex_range(A.S, valid ? i : 0, valid));
+                if (valid && L.lane == 0) zr_i = prz_update(pv, p, r, z, i, vAv, alpha);
+            }
+            add(acc, zr_i);
+        }
+        share = grid_exchange<kThreads>(block_total<kThreads>(acc, ws, wbuf), part_a, bar, &sc->status, extra);
+        sum = block_total<kThreads>(share, ws, wbuf);
         zr_last = zr;
-        zr = grid_partials_sum(part_a);
+        zr = sum.s + sum.c;
         if (blockIdx.x == 0 && threadIdx.x == 0) sc->v_A_v = vAv;
+    }
+    if (own_ok && L.lane == 0) {
+        p[own] = f4(pi);
+        r[own] = f4(ri);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         sc->z_r = zr;
@@ -1909,8 +2140,6 @@ __global__ void __launch_bounds__(kClusterThreads) k_cg_cluster(const float4* __
         __syncthreads();
         return v;
     };
-    const int4 ids0 = element_ids(A, nc, tid);
-    const int4 at0 = element_slots(A, nc, tid);
     const PrzLanes L = prz_lanes(tid, nthreads, A.np);
     const VRange R0 = vertex_range(A.S, L.group < A.np ? L.group : 0, L.group < A.np);  // the group's first vertex
     float zr = cluster_total(cg_init_vertices(grad, hd, A.np, p, r, z, v0, tid, nthreads)), zr_last = zr;
@@ -1919,7 +2148,7 @@ __global__ void __launch_bounds__(kClusterThreads) k_cg_cluster(const float4* __
         const float4* vin = (it & 1) ? v1 : v0;
         float4* vout = (it & 1) ? v0 : v1;
         const float s_dir = it == 0 ? 0.f : zr / zr_last;
-        vAv = cluster_total(hvp_elements(x, A, z, vin, vout, s_dir, nc, tid, nthreads, ids0, at0));
+        vAv = cluster_total(hvp_elements(x, A, z, vin, vout, s_dir, nc, tid, nthreads));
         const PrzVertex pre = prz_load(A, vout, hd, p, r, L.group < A.np ? L.group : 0, L.group < A.np, L, R0);
         const float zr_new = cluster_total(cg_prz_vertices(A, vout, hd, p, r, z, zr, vAv, L, pre));
         zr_last = zr;
@@ -1934,9 +2163,9 @@ __global__ void __launch_bounds__(kClusterThreads) k_cg_cluster(const float4* __
 }
 
 // ------------------------------------------------------------------ iteration bookkeeping
-// Start of a Newton iteration (system.py:425-432): q_prev_newton = q; the per-vertex contact counts and fill
-// cursors cleared.
-__global__ void k_iter_begin(const float4* __restrict__ q, float4* qpn, int* ccnt, int* ccur, int np,
+// Start of a Newton iteration (system.py:425-432): q_prev_newton = q; the per-vertex contact counts, fill cursors
+// and marks cleared.
+__global__ void k_iter_begin(const float4* __restrict__ q, float4* qpn, int* ccnt, int* ccur, int* cact, int np,
                              SolverScalars* sc) {
     pdl_wait();
     if (sc->abort) return;
@@ -1944,6 +2173,7 @@ __global__ void k_iter_begin(const float4* __restrict__ q, float4* qpn, int* ccn
         if (i < np) {
             qpn[i] = q[i];
             ccur[i] = 0;
+            cact[i] = 0;
         }
         ccnt[i] = 0;
     }
@@ -2447,7 +2677,7 @@ void Stage3::release() {
     };
     fp(gt_pos); fp(gt_tri); fp(gt_bvh_mem); fp(q); fp(q_rest); fp(q_prev_newton); fp(p); fp(target);
     fp(grad); fp(hdiag); fp(r); fp(z); fp(v[0]); fp(v[1]); fp(vweight);
-    fp(cand_cnt); fp(cand_off); fp(cflag); fp(cpos); fp(cid); fp(cty); fp(vs_off); fp(inv_vs); fp(c_cnt); fp(c_off);
+    fp(cand_cnt); fp(cand_off); fp(cflag); fp(cpos); fp(cid); fp(cty); fp(vs_off); fp(inv_vs); fp(c_cnt); fp(c_off); fp(c_act);
     fp(c_cur); fp(c_tmp); fp(c_inv); fp(gslot); fp(hslot); fp(aslot); fp(scan_scratch);
     cap_cf = cap_vs = cap_vso = cap_slot = cap_cq = 0;
     fp(q_ref); fp(cand_pt); fp(cand_ee); fp(tri); fp(edge4); fp(el_area); fp(el_invDm);
@@ -2497,7 +2727,7 @@ int Stage3::ensure(int np, int nt, int ne, int nh, int ngp, int ngt) {
             int dev = 0, nsm = 0, occ = 0;
             cudaGetDevice(&dev);
             cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_cg_solve<128>, 128, 0);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_cg_solve<128, 1>, 128, 0);
             coop_max_blocks = std::max(1, nsm * std::max(occ, 0));
             int occ_ls = 0;
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_ls, k_line_search_coop, kT, 0);
@@ -2640,7 +2870,7 @@ int Stage3::ensure_slots() {
     }
     const size_t nv = (size_t)NP + 2;
     if (cap_vso < nv || !vs_off) {
-        for (int** b : {&vs_off, &c_cnt, &c_off, &c_cur}) {
+        for (int** b : {&vs_off, &c_cnt, &c_off, &c_cur, &c_act}) {
             dfree(*b);
             *b = nullptr;
             c = 0;
@@ -2713,6 +2943,7 @@ EnergyArgs Stage3::energy_args() const {
     A.nt = NT; A.hinge = hinge; A.rest = hinge_rest; A.hinge_k = P.hinge_stiffness; A.nh = NH;
     A.cidx = c_idx; A.ctype = c_type; A.cd = c_d; A.kappa = P.coll_stiffness; A.d_hat = P.d_hat;
     A.ee_thres = P.ee_classify_thres;
+    A.cact = nullptr;
     return A;
 }
 
@@ -2722,7 +2953,9 @@ int Stage3::energy_grid() const {
 }
 
 void Stage3::launch_energy(const float4* x, int ls_n) {
-    pdl(k_energy, energy_grid(), kT, 0, stream)(x, energy_args(), sc, partial, ls_n);
+    EnergyArgs A = energy_args();
+    if (ls_n < 0) A.cact = c_act;
+    pdl(k_energy, energy_grid(), kT, 0, stream)(x, A, sc, partial, ls_n);
     note_launch();
 }
 
@@ -2733,7 +2966,7 @@ void Stage3::newton_iteration() {
     const float la = P.elas_young_modulus * P.elas_poisson_ratio / ((1.f + P.elas_poisson_ratio) * (1.f - 2.f * P.elas_poisson_ratio));
     const int gC = grid_for((long long)cap_c, kT);
     // q_prev_newton = q; contacts at q (system.py:425-432, _detect_contact :308-318 with refitted LBVHs)
-    pdl(k_iter_begin, grid_for(NP + 1, kT), kT, 0, s)(q, q_prev_newton, c_cnt, c_cur, NP, sc);
+    pdl(k_iter_begin, grid_for(NP + 1, kT), kT, 0, s)(q, q_prev_newton, c_cnt, c_cur, c_act, NP, sc);
     note_launch();
     const float skin = 2.0f * P.contact_detection_radius + P.d_hat;
     pdl(k_disp_check, grid_for(NP, kT), kT, 0, s)(q, q_ref, NP, 0.5f * skin, sc);
@@ -2786,15 +3019,15 @@ void Stage3::newton_iteration() {
     pdl(k_contacts_scatter, grid_for((long long)(cap_cpt + cap_cee), kT), kT, 0, s)(cflag, cpos, cid, cty, c_idx, c_type,
                                                                                   c_cnt, sc);
     note_launch();
-    exclusive_scan(c_cnt, c_off, nullptr, NP + 1, nullptr, scan_scratch, s, &sc->status, NP + 1);
-    note_launch();
-    pdl(k_cvert_fill, grid_for(4ll * cap_c, kT), kT, 0, s)(c_idx, c_off, c_cur, c_tmp, sc);
-    note_launch();
-    pdl(k_cvert_rank, grid_for(32ll * NP, kT), kT, 0, s)(c_off, c_tmp, c_inv, NP, sc);
-    note_launch();
     // energy, gradient (coeff -1), Hessian diagonal and hinge blocks (system.py:433-434): per-corner parts into
     // the slot arrays, then summed per vertex
     launch_energy(q);
+    exclusive_scan(c_cnt, c_off, nullptr, NP + 1, nullptr, scan_scratch, s, &sc->status, NP + 1);
+    note_launch();
+    pdl(k_cvert_fill, grid_for(4ll * cap_c, kT), kT, 0, s)(c_idx, c_off, c_act, c_cur, c_tmp, sc);
+    note_launch();
+    pdl(k_cvert_rank, grid_for(32ll * NP, kT), kT, 0, s)(c_off, c_tmp, c_act, c_inv, NP, sc);
+    note_launch();
     const size_t nt3 = (size_t)3 * NT, cbase = nt3 + (size_t)4 * NH;
     pdl(k_diff_elastic, grid_for(NT, kT), kT, 0, s)(q, tri, el_area, el_invDm, mu, la, -1.f, NT, gslot, inv_vs, sc);
     note_launch();
@@ -2807,10 +3040,10 @@ void Stage3::newton_iteration() {
         note_launch();
     }
     pdl(k_diff_contact, gC, kT, 0, s)(q, c_idx, c_type, c_d, sc, P.coll_stiffness, P.d_hat, -1.f, c_dd, gslot + cbase,
-                                     hslot + cbase, c_inv);
+                                     hslot + cbase, c_inv, c_act, cflag);
     note_launch();
     VertexSlots S;
-    S.vs_off = vs_off; S.coff = c_off; S.inv_vs = inv_vs; S.cinv = c_inv; S.cbase = (int)cbase;
+    S.vs_off = vs_off; S.coff = c_off; S.cact = c_act; S.inv_vs = inv_vs; S.cinv = c_inv; S.cbase = (int)cbase;
     pdl(k_gather_grad, grid_for((long long)kGather * NP, kT), kT, 0, s)(q, target, vweight, P.mesh2gt_dist_stiffness,
                                                                       -1.f, NP, gslot, hslot, S, grad, hdiag, sc);
     note_launch();
@@ -2819,7 +3052,7 @@ void Stage3::newton_iteration() {
     H.w = vweight; H.m2gt_k = P.mesh2gt_dist_stiffness; H.np = NP;
     H.tri = tri; H.area = el_area; H.invDm = el_invDm; H.mu = mu; H.la = la; H.nt = NT;
     H.hinge = hinge; H.blocks = hinge_blocks; H.nh = NH;
-    H.cidx = c_idx; H.cd = c_d; H.cdd = c_dd; H.kappa = P.coll_stiffness; H.d_hat = P.d_hat;
+    H.cidx = c_idx; H.cd = c_d; H.cdd = c_dd; H.cneed = cflag; H.kappa = P.coll_stiffness; H.d_hat = P.d_hat;
     H.aslot = aslot; H.S = S;
     const long long elems_all = (long long)NP + NT + NH;
     // the cluster kernel measured slower than the grid-wide one on the 5k-face stage-2 output (fewer threads
@@ -2857,7 +3090,8 @@ void Stage3::newton_iteration() {
         }
     } else {
         // one cooperative launch: about one thread per element, at most one block per SM (cg_mode 0, 3, 4); or
-        // at least one block per SM (5: 128 threads, 6: 64 threads, two blocks per SM)
+        // at least one block per SM (5: 128 threads, 6: 64 threads, two blocks per SM). Mode 0 stands kCgK threads of the
+        // block for each of the sums' threads once those have more than one element without contacts (k_cg_solve).
         const int bt = cg_mode == 3 ? 256 : cg_mode == 4 ? 512 : cg_mode == 6 ? 64 : 128;
         const long long elems = (long long)NP + NT + NH;
         int g = (int)std::min<long long>((elems + bt - 1) / bt, (long long)n_sm);
@@ -2866,7 +3100,6 @@ void Stage3::newton_iteration() {
         g = std::max(1, std::min(g, std::min(coop_max_blocks, kPartials / 2)));
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(g);
-        cfg.blockDim = dim3(bt);
         cfg.stream = s;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeCooperative;
@@ -2874,18 +3107,17 @@ void Stage3::newton_iteration() {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         CgState* bar = reinterpret_cast<CgState*>(cg_bar);
-        if (bt == 64)
-            cudaLaunchKernelEx(&cfg, k_cg_solve<64>, (const float4*)q, H, (const float4*)grad, (const float4*)hdiag, p, r,
-                               z, v[0], v[1], P.n_cg_iters, sc, partial, bar);
-        else if (bt == 512)
-            cudaLaunchKernelEx(&cfg, k_cg_solve<512>, (const float4*)q, H, (const float4*)grad, (const float4*)hdiag, p, r,
-                               z, v[0], v[1], P.n_cg_iters, sc, partial, bar);
-        else if (bt == 256)
-            cudaLaunchKernelEx(&cfg, k_cg_solve<256>, (const float4*)q, H, (const float4*)grad, (const float4*)hdiag, p, r,
-                               z, v[0], v[1], P.n_cg_iters, sc, partial, bar);
-        else
-            cudaLaunchKernelEx(&cfg, k_cg_solve<128>, (const float4*)q, H, (const float4*)grad, (const float4*)hdiag, p, r,
-                               z, v[0], v[1], P.n_cg_iters, sc, partial, bar);
+        auto solve = [&](auto kernel, int threads) {
+            cfg.blockDim = dim3(threads);
+            cudaLaunchKernelEx(&cfg, kernel, (const float4*)q, H, (const float4*)grad, (const float4*)hdiag, p, r, z, v[0],
+                               v[1], P.n_cg_iters, sc, partial, bar);
+        };
+        if (cg_mode == 6) solve(k_cg_solve<64, 1>, 64);
+        else if (cg_mode == 4) solve(k_cg_solve<512, 1>, 512);
+        else if (cg_mode == 3) solve(k_cg_solve<256, 1>, 256);
+        else if (cg_mode == 5) solve(k_cg_solve<128, 1>, 128);
+        else if (elems > (long long)g * 128) solve(k_cg_solve<128, kCgK>, 128 * kCgK);
+        else solve(k_cg_solve<128, 1>, 128);
         note_launch();
     }
     // step clamp, CCD, line search (system.py:441-459)

@@ -163,6 +163,7 @@ private:
     int* c_cnt = nullptr;    // contact corners per vertex (NP + 1), their offsets and fill cursors
     int* c_off = nullptr;
     int* c_cur = nullptr;
+    int* c_act = nullptr;    // vertices with a contact closer than d_hat
     int* c_tmp = nullptr;    // 4 per contact: the codes filled per vertex, then ranked
     int* c_inv = nullptr;    // 4 per contact: the position of each contact code in its vertex's range
     float4 *gslot = nullptr, *hslot = nullptr, *aslot = nullptr;
@@ -188,7 +189,7 @@ private:
     int graph_key[6] = {0, 0, 0, 0, 0, 0};
 
     void newton_iteration();  // enqueue one Newton iteration (system.py:425-459)
-    void launch_energy(const float4* x, int ls_n = -1);
+    void launch_energy(const float4* x, int ls_n = -1);  // ls_n < 0: also marks c_act
     EnergyArgs energy_args() const;
     int energy_grid() const;  // blocks of the energy sum (k_energy and the line search)
 };
