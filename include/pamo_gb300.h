@@ -321,7 +321,7 @@ const char* pamo_stage3_last_error(const pamo_stage3* s);
  * mesh2gt_dist_stiffness, min_angle_thres (degrees), max_blocks. Execution knobs that leave the method
  * unchanged: use_cuda_graph (0/1), ccd_fp64 (1: float64 CCD step, the default; 0: float32 like the reference),
  * cg_mode (PCG launch shape: 0 cooperative 128-thread blocks, 2 one thread-block cluster, 3/4 256/512-thread
- * blocks, 5/6 at least one/two blocks per SM), ls_mode (1: the line search as one cooperative launch, 0: a
+ * blocks, 5/6 at least one/two blocks per SM), ls_mode (1: the line search's trials side by side, 0: a
  * launch pair per trial). Unknown names: PAMO_ERR_INVALID_ARG. */
 int pamo_stage3_set_param(pamo_stage3* s, const char* name, double value);
 

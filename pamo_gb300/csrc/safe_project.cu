@@ -1065,7 +1065,8 @@ struct ElasticLocal {
     Mat2 F, invDm;
     float W;
 };
-__device__ __forceinline__ ElasticLocal elastic_local(const float4* __restrict__ x, int4 t, float W, float4 inv) {
+template <class X>
+__device__ __forceinline__ ElasticLocal elastic_local(const X& x, int4 t, float W, float4 inv) {
     ElasticLocal L;
     const F3 x0 = f3(x[t.x]), x1 = f3(x[t.y]), x2 = f3(x[t.z]);
     const F3 x01 = x1 - x0, x02 = x2 - x0;
@@ -1113,9 +1114,10 @@ namespace {
 // earlier trial was accepted: q and therefore the energy, distances and contact types are already those of the
 // accepted trial. Every block reads the same flags: the last block writes sc->energy only after all have started.
 // The energy terms of elements first, first + stride, ... of [vertices | triangles | hinges | contacts], summed
-// with compensation in the thread.
-__device__ __forceinline__ CSum energy_elements(const float4* __restrict__ x, const EnergyArgs& A, int nc, long long first,
-                                                long long stride) {
+// with compensation in the thread. x: the positions (TrialPositions: a line-search trial's). kStore = false: the contacts'
+// types and distances are not kept.
+template <bool kStore, class X>
+__device__ __forceinline__ CSum energy_elements(const X& x, const EnergyArgs& A, int nc, long long first, long long stride) {
     const long long e1 = A.np, e2 = e1 + A.nt, e3 = e2 + A.nh, total = e3 + nc;
     CSum acc;
     for (long long g = first; g < total; g += stride) {
@@ -1149,9 +1151,11 @@ __device__ __forceinline__ CSum energy_elements(const float4* __restrict__ x, co
                 t.y = ee_classify(x0, x1, x2, x3, A.ee_thres);
                 d = ee_pair_distance(x0, x1, x2, x3, t.y);
             }
-            A.ctype[b] = t;
-            A.cd[b] = d;
-            if (A.cact && !(d >= A.d_hat)) A.cact[i.x] = A.cact[i.y] = A.cact[i.z] = A.cact[i.w] = 1;
+            if (kStore) {
+                A.ctype[b] = t;
+                A.cd[b] = d;
+            }
+            if (kStore && A.cact && !(d >= A.d_hat)) A.cact[i.x] = A.cact[i.y] = A.cact[i.z] = A.cact[i.w] = 1;
             e = d < A.d_hat ? barrier(d, A.d_hat) * A.kappa : 0.f;
         }
         acc.add(e);
@@ -1164,7 +1168,7 @@ __global__ void __launch_bounds__(kT) k_energy(const float4* __restrict__ x, Ene
     pdl_wait();
     if (sc->abort) return;
     if (ls_n > 0 && sc->energy < sc->energy_prev) return;
-    const CSum acc = energy_elements(x, A, sc->n_contacts, gtid(), gstride());
+    const CSum acc = energy_elements<true>(x, A, sc->n_contacts, gtid(), gstride());
     grid_sum_finish(acc, partial, &sc->red_count, &sc->energy, nullptr);
 }
 
@@ -1791,29 +1795,6 @@ __device__ __forceinline__ void grid_barrier(unsigned* count, int* status, unsig
     __syncthreads();
 }
 
-// Sum of the per-block partials in block order, the same value in every block (after a barrier).
-__device__ __forceinline__ float grid_partials_sum(const float2* partial) {
-    __shared__ float result;
-    CSum a;
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) {
-        CSum t;
-        t.s = __ldcg(&partial[b].x);
-        t.c = __ldcg(&partial[b].y);
-        a.merge(t);
-    }
-    CSum f = block_reduce(a);
-    if (threadIdx.x == 0) result = f.s + f.c;
-    __syncthreads();
-    const float v = result;
-    __syncthreads();
-    return v;
-}
-
-__device__ __forceinline__ void store_partial(CSum acc, float2* partial) {
-    CSum r = block_reduce(acc);
-    if (threadIdx.x == 0) partial[blockIdx.x] = make_float2(r.s, r.c);
-}
-
 struct CgState {
     unsigned count;  // grid_barrier's counter, zeroed before each stage-3 run
 };
@@ -2068,34 +2049,50 @@ __global__ void __launch_bounds__(kThreads* K) k_cg_solve(const float4* __restri
     }
 }
 
-// The line search (system.py:393-409 with line_search_kernel, solver_kernels.py:52-66) as one cooperative
-// launch on k_energy's grid: trial n sets q = q0 + ccd_step 0.5^n p, its energy is summed as k_energy sums it
-// (the same threads, block partials and order, so the same value), and the search stops at the first trial whose
-// energy is below the energy before it. In place of n_trials launches of k_line_search and k_energy, most of
-// which found an earlier trial accepted and returned at once.
-__global__ void __launch_bounds__(kT) k_line_search_coop(const float4* __restrict__ q0, const float4* __restrict__ p,
-                                                         float4* q, EnergyArgs A, int n_trials, SolverScalars* sc,
-                                                         float2* partial, CgState* bar) {
-    if (sc->abort) return;
-    const int nc = sc->n_contacts;
-    const float e_prev = sc->energy_prev, step = sc->ccd_step;
-    const unsigned extra = (unsigned)sc->barrier_extra;
-    float e = sc->energy;
-    for (int n = 0; n < n_trials; ++n) {
-        const float a = step * powf(0.5f, (float)n);
-        for (int i = gtid(); i < A.np; i += gstride()) {
-            const float4 a0 = q0[i], pi = p[i];
-            q[i] = make_float4(a0.x + a * pi.x, a0.y + a * pi.y, a0.z + a * pi.z, 0.f);
-        }
-        grid_barrier(&bar->count, &sc->status, extra);
-        // partials alternate between two buffers trial by trial (rewritten only after the next barrier)
-        float2* part = partial + (size_t)(n & 1) * gridDim.x;
-        store_partial(energy_elements(q, A, nc, gtid(), gstride()), part);
-        grid_barrier(&bar->count, &sc->status, extra);
-        e = grid_partials_sum(part);
-        if (e < e_prev) break;  // the same total in every block
+// The line search (system.py:393-409 with line_search_kernel, solver_kernels.py:52-66): trial n sets q = q0 + ccd_step
+// 0.5^n p, and the search stops at the first trial whose energy is below the energy before it. The trials n0, n0 + 1, ...
+// of one launch (blockIdx.y) run side by side: each forms its own positions where it reads them and sums its energy as
+// k_energy does (the same threads, block partials and order, so the same value); a launch does nothing once an earlier
+// one has a trial that lowers the energy. One after another behind grid barriers (two a trial) the trials took 47 us on
+// 1,534 faces and 112 us on 12,828 faces with 157,922 contacts.
+struct TrialPositions {
+    const float4 *q0, *p;
+    float a;
+    __device__ __forceinline__ float4 operator[](int i) const {
+        const float4 a0 = q0[i], pi = p[i];
+        return make_float4(a0.x + a * pi.x, a0.y + a * pi.y, a0.z + a * pi.z, 0.f);
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) sc->energy = e;
+};
+constexpr int kMaxTrials = 64;    // more fall back to launch pairs (ls_mode 0)
+constexpr int kFirstTrials = 2;   // of the first launch, then kTrialsAtOnce a launch
+constexpr int kTrialsAtOnce = 8;
+struct LineSearch {
+    float energy[kMaxTrials];
+    int counter[kTrialsAtOnce];  // zero between launches
+};
+
+__global__ void __launch_bounds__(kT) k_ls_trials(const float4* __restrict__ q0, const float4* __restrict__ p, EnergyArgs A,
+                                                  int n0, SolverScalars* sc, LineSearch* ls, float2* partial) {
+    pdl_wait();
+    if (sc->abort) return;
+    for (int m = 0; m < n0; ++m)
+        if (ls->energy[m] < sc->energy_prev) return;
+    const int n = n0 + blockIdx.y;
+    const TrialPositions x = {q0, p, sc->ccd_step * powf(0.5f, (float)n)};
+    grid_sum_finish(energy_elements<false>(x, A, sc->n_contacts, gtid(), gstride()),
+                    partial + (size_t)blockIdx.y * gridDim.x, &ls->counter[blockIdx.y], &ls->energy[n], nullptr);
+}
+
+// q of the first trial below the energy before, or of the last one
+__global__ void __launch_bounds__(kT) k_ls_pick(const float4* __restrict__ q0, const float4* __restrict__ p, float4* q,
+                                                int np, int n_trials, SolverScalars* sc, const LineSearch* ls) {
+    pdl_wait();
+    if (sc->abort) return;
+    int n = 0;
+    while (n < n_trials - 1 && !(ls->energy[n] < sc->energy_prev)) ++n;
+    const TrialPositions x = {q0, p, sc->ccd_step * powf(0.5f, (float)n)};
+    for (int i = gtid(); i < np; i += gstride()) q[i] = x[i];
+    if (gtid() == 0) sc->energy = ls->energy[n];
 }
 
 // The same solve inside one thread-block cluster (up to 16 CTAs): the barriers are the hardware cluster
@@ -2555,6 +2552,36 @@ __device__ R ee_pair_distance(T3<R> x0, T3<R> x1, T3<R> x2, T3<R> x3, int t) {
     return Real<R>::c(1e9);
 }
 
+// Whether a contact's first step is certain to go past t = 1, so that it does not bound the step: the distance of the two
+// primitives' boxes is at most theirs, and the relative speed is taken with a margin for rounding (1e-6 of the fastest
+// vertex, whose common motion it leaves out, and 1e-5 of itself). Nearly all contacts of a converging step: their walks
+// in wide arithmetic took 174 us of 157,922 contacts.
+__device__ __forceinline__ bool accd_out_of_reach(const float4* __restrict__ x, const float4* __restrict__ vel, int4 id,
+                                                  bool pt, float slackness, float thickness) {
+    const F3 x0 = f3(x[id.x]), x1 = f3(x[id.y]), x2 = f3(x[id.z]), x3 = f3(x[id.w]);
+    F3 lo0 = x0, hi0 = x0, lo1, hi1;
+    const auto lower = [](F3 a, F3 b) { return F3{fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z)}; };
+    const auto upper = [](F3 a, F3 b) { return F3{fmaxf(a.x, b.x), fmaxf(a.y, b.y), fmaxf(a.z, b.z)}; };
+    lo1 = lower(x2, x3);
+    hi1 = upper(x2, x3);
+    if (pt) {
+        lo1 = lower(lo1, x1);
+        hi1 = upper(hi1, x1);
+    } else {
+        lo0 = lower(x0, x1);
+        hi0 = upper(x0, x1);
+    }
+    const F3 gap = {fmaxf(fmaxf(lo1.x - hi0.x, lo0.x - hi1.x), 0.f), fmaxf(fmaxf(lo1.y - hi0.y, lo0.y - hi1.y), 0.f),
+                    fmaxf(fmaxf(lo1.z - hi0.z, lo0.z - hi1.z), 0.f)};
+    const float d = length(gap);
+    const F3 v0 = f3(vel[id.x]), v1 = f3(vel[id.y]), v2 = f3(vel[id.z]), v3 = f3(vel[id.w]);
+    const F3 va = (v0 + v1 + v2 + v3) * 0.25f;
+    const float l0 = length(v0 - va), l1 = length(v1 - va), l2 = length(v2 - va), l3 = length(v3 - va);
+    const float lv = pt ? l0 + fmaxf(l1, fmaxf(l2, l3)) : fmaxf(l0, l1) + fmaxf(l2, l3);
+    const float vmax = fmaxf(fmaxf(length(v0), length(v1)), fmaxf(length(v2), length(v3)));
+    return slackness * (d * 0.99999f - thickness - 1e-9f) > lv * 1.00001f + 1e-6f * vmax + 1e-12f;
+}
+
 // slackness, thickness and ee_thres as R (the host passes their float values, widened)
 template <class R>
 __global__ void k_accd_wide(const float4* __restrict__ x, const float4* __restrict__ vel, const int4* __restrict__ cidx,
@@ -2569,6 +2596,8 @@ __global__ void k_accd_wide(const float4* __restrict__ x, const float4* __restri
     for (long long bb = spread_first(); bb < n; bb += spread_stride()) {
         const int b = (int)bb;
         const int4 id = cidx[b];
+        const bool pt = ctype[b].x == BLOCK_PT;
+        if (max_iters > 0 && accd_out_of_reach(x, vel, id, pt, slackness_f, thickness_f)) continue;
         T3<R> x0 = t3<R>(x[id.x]), x1 = t3<R>(x[id.y]), x2 = t3<R>(x[id.z]), x3 = t3<R>(x[id.w]);
         T3<R> v0 = t3<R>(vel[id.x]), v1 = t3<R>(vel[id.y]), v2 = t3<R>(vel[id.z]), v3 = t3<R>(vel[id.w]);
         const int type1 = ctype[b].x;
@@ -2686,7 +2715,7 @@ void Stage3::release() {
     if (stream) cudaStreamSynchronize(stream);
     if (pool) cudaMemPoolDestroy(pool);
     pool = nullptr;
-    f(gt_rc); f(tri_rc); f(edge_rc); f(sc); f(d_norm); f(cg_bar); f(partial);
+    f(gt_rc); f(tri_rc); f(edge_rc); f(sc); f(d_norm); f(cg_bar); f(ls_buf); f(partial);
     if (h_sc) cudaFreeHost(h_sc);
     h_sc = nullptr;
     if (ev_in) cudaEventDestroy(ev_in);
@@ -2724,14 +2753,14 @@ int Stage3::ensure(int np, int nt, int ne, int nh, int ngp, int ngt) {
             if (cudaMalloc((void**)&partial, kPartials * sizeof(float2)) != cudaSuccess) return fail(PAMO_ERR_OOM, "cudaMalloc");
             if (cudaMalloc((void**)&cg_bar, 64) != cudaSuccess) return fail(PAMO_ERR_OOM, "cudaMalloc");
             cudaMemset(cg_bar, 0, 64);
+            const size_t ls_bytes = sizeof(LineSearch) + (size_t)kTrialsAtOnce * kRedBlocks * sizeof(float2);
+            if (cudaMalloc((void**)&ls_buf, ls_bytes) != cudaSuccess) return fail(PAMO_ERR_OOM, "cudaMalloc");
+            cudaMemset(ls_buf, 0, ls_bytes);
             int dev = 0, nsm = 0, occ = 0;
             cudaGetDevice(&dev);
             cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_cg_solve<128, 1>, 128, 0);
             coop_max_blocks = std::max(1, nsm * std::max(occ, 0));
-            int occ_ls = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_ls, k_line_search_coop, kT, 0);
-            ls_coop_max_blocks = nsm * std::max(occ_ls, 0);
             n_sm = std::max(1, nsm);
             // largest cluster the device runs k_cg_cluster with (16 needs the non-portable opt-in)
             cluster_size = 1;
@@ -3135,21 +3164,16 @@ void Stage3::newton_iteration() {
         pdl(k_accd, gC, kT, 0, s)(q, p, c_idx, c_type, sc, P.ccd_slackness, P.ccd_thickness, P.ccd_max_iters,
                                 P.ee_classify_thres);
     note_launch();
-    const int g_ls = energy_grid();
-    if (ls_mode == 1 && P.n_line_search_iters > 0 && g_ls <= ls_coop_max_blocks && 2 * g_ls <= kPartials) {
-        // the whole search in one cooperative launch on the energy's grid (co-residency checked at set-up)
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(g_ls);
-        cfg.blockDim = dim3(kT);
-        cfg.stream = s;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeCooperative;
-        attr[0].val.cooperative = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        CgState* ls_bar = reinterpret_cast<CgState*>(static_cast<char*>(cg_bar) + 32);
-        cudaLaunchKernelEx(&cfg, k_line_search_coop, (const float4*)q_prev_newton, (const float4*)p, q, energy_args(),
-                           P.n_line_search_iters, sc, partial, ls_bar);
+    if (ls_mode == 1 && P.n_line_search_iters > 0 && P.n_line_search_iters <= kMaxTrials) {
+        LineSearch* ls = reinterpret_cast<LineSearch*>(ls_buf);
+        float2* ls_partial = reinterpret_cast<float2*>(ls + 1);
+        for (int n0 = 0; n0 < P.n_line_search_iters;) {
+            const int count = std::min(n0 == 0 ? kFirstTrials : kTrialsAtOnce, P.n_line_search_iters - n0);
+            pdl(k_ls_trials, dim3(energy_grid(), count), kT, 0, s)(q_prev_newton, p, energy_args(), n0, sc, ls, ls_partial);
+            note_launch();
+            n0 += count;
+        }
+        pdl(k_ls_pick, grid_for(NP, kT), kT, 0, s)(q_prev_newton, p, q, NP, P.n_line_search_iters, sc, ls);
         note_launch();
     } else {
         for (int n = 0; n < P.n_line_search_iters; ++n) {
@@ -3269,7 +3293,7 @@ int Stage3::run_once(const double* gt_points, const int* gt_tris, int n_gt_point
         vs_host_list.swap(list);
     }
     cudaStream_t s = stream;
-    cudaMemsetAsync(cg_bar, 0, 64, s);  // the barrier counters of the PCG and of the line search
+    cudaMemsetAsync(cg_bar, 0, 64, s);  // the barrier counter of the PCG
     cudaEventRecord(ev_in, caller);
     cudaStreamWaitEvent(s, ev_in, 0);
     std::vector<int4> e4(NE);
@@ -3490,7 +3514,7 @@ int pamo_stage3_set_param(pamo_stage3* s, const char* name, double value) {
         }
         P.ccd_fp64 = (int)value;
     }
-    else if (n == "ls_mode") s->solver.ls_mode = (int)value;  // 1 cooperative line search, 0 launches per trial
+    else if (n == "ls_mode") s->solver.ls_mode = (int)value;  // 1 trials side by side, 0 launches per trial
     else if (n == "cg_mode") s->solver.cg_mode = (int)value;  // 0/1 grid-cooperative (128), 2 cluster, 3 (256), 4 (512), 5 (128, >= 1 block per SM), 6 (64, >= 2 blocks per SM), 7 two ordinary launches per iteration
     else {
         s->solver.err = "unknown stage-3 parameter: " + n;

@@ -86,7 +86,7 @@ public:
     std::string err;
     bool use_graph = true;  // capture one Newton iteration as a CUDA graph and replay it
     int cg_mode = 0;        // PCG kernel: 0/1 grid-wide cooperative, 128 threads; 3: 256 threads; 2: one cluster
-    int ls_mode = 1;        // line search: 1 one cooperative launch, 0 a launch pair per trial
+    int ls_mode = 1;        // line search: 1 trials side by side, 0 a launch pair per trial
     int test_barrier_extra = 0;  // copied to SolverScalars::barrier_extra at each run (tests of the bounded waits)
     int cluster_size = 1;   // CTAs of the cluster kernel (device limit, at most 16)
 
@@ -170,9 +170,9 @@ private:
     size_t cap_slot = 0;
     int* scan_scratch = nullptr;  // two scan scratches (exclusive_scans with two jobs)
     float2* partial = nullptr;  // block partials of the grid-wide sums
+    void* ls_buf = nullptr;     // energies, counters and partials of the line search's trials
     void* cg_bar = nullptr;     // grid-barrier state of the cooperative CG kernel
     int coop_max_blocks = 1, n_sm = 1;
-    int ls_coop_max_blocks = 0;  // co-resident blocks of the cooperative line search
     // LBVHs over the current triangles and edges (built at registration, refitted at every detection)
     BvhBuffers tri_bvh{}, edge_bvh{};
     char *tri_bvh_mem = nullptr, *edge_bvh_mem = nullptr;
