@@ -794,8 +794,8 @@ struct pamo_csr {
         pdl(kb_scatter_costs, grid_for(Eb, kT), kT, 0, s)(rc, slot_mesh.p, mesh.p, vmesh.p, edges.p, cost.p, ecost_reg.p);
         note_launch();
         // selection and collapse
-        launch_collapse(rc, Eb, eorder.p, edges.p, cost.p, collapse_t, vmin.p, nxt.p, spc.p, nt_off, nt.p, tri.p, orig_tri.p, pos.p,
-                        orig_pos.p, occ.p, win.p, s);
+        launch_collapse(rc, Eb, edges.p, cost.p, collapse_t, vmin.p, nxt.p, spc.p, nt_off, nt.p, tri.p, pos.p,
+                        occ.p, win.p, s);
         exclusive_scan(win.p, win.p, &rc->n_edges, 1, &rc->n_win, scan_scratch, s, &rc->status, Eb);
         launch_after_collapse(rc, Eb, Fb, win.p, winners.p, edges.p, nt_off, nt.p, tri.p, pos.p, occ.p, 0, false, s);
         pdl(kb_line_apply, 1, 32, 0, s)(rc, ctl, slot_mesh.p, mesh.p, vmesh.p, edges.p, nt_off, nt.p, tri.p, pos.p, occ.p,

@@ -449,8 +449,8 @@ struct pamo_ctx {
         cudaMemsetAsync(vmin.p, 0xFF, (nP + 1) * sizeof(unsigned long long), s);
         launch_edge_cost(rc, eb, eorder.p, edges.p, nt_off, nt.p, tri.p, pos.p, quad.p, fgeo.p, nxt.p, spc.p, invalid.p, edge_cost.p, vmin.p,
                          d_scale, threshold, 0, s, nullptr, true, skinny_pow);
-        launch_collapse(rc, eb, eorder.p, edges.p, edge_cost.p, collapse_t, vmin.p, nxt.p, spc.p, nt_off, nt.p, tri.p, orig_tri.p, pos.p,
-                        orig_pos.p, occ.p, win.p, s, false);
+        launch_collapse(rc, eb, edges.p, edge_cost.p, collapse_t, vmin.p, nxt.p, spc.p, nt_off, nt.p, tri.p, pos.p,
+                        occ.p, win.p, s, false);
         exclusive_scan(occ.p, pts_map.p, &rc->n_pts, 1, nullptr, scan_scratch, s, &rc->status, nP);
         if ((r = read_counters())) return r;
         if ((r = status_to_error(h_rc->status))) return r;
@@ -545,8 +545,7 @@ struct pamo_ctx {
                              vmin.p, d_scale, threshold, 0, s, &d_ls->is_stuck, false, skinny_pow, precision, nullptr,
                              place_ptr(), qlo_ptr());
             cost_end(s);
-            launch_collapse(rc, eb, eorder.p, edges.p, edge_cost.p, collapse_t, vmin.p, nxt.p, spc.p, nt_off, nt.p, tri.p, orig_tri.p,
-                            pos.p, orig_pos.p, occ.p, win.p, s, true, place_ptr());
+            launch_collapse(rc, eb, edges.p, edge_cost.p, collapse_t, vmin.p, nxt.p, spc.p, nt_off, nt.p, tri.p, pos.p, occ.p, win.p, s, true, place_ptr());
             exclusive_scan(win.p, win.p, &rc->n_edges, 1, &rc->n_win, scan_scratch, s, &rc->status, eb);
             launch_after_collapse(rc, eb, nTb, win.p, collapsed.p, edges.p, nt_off, nt.p, tri.p, pos.p, occ.p,
                                   (int)collapsed.n, true, s);
@@ -719,8 +718,8 @@ struct pamo_ctx {
         cost_end(s);
         prof.end(kPhCost, s);
         prof.begin(kPhCollapse, s);
-        launch_collapse(rc, eb, eorder.p, edges.p, edge_cost.p, collapse_t, vmin.p, nxt.p, spc.p, nt_off, nt.p, tri.p, orig_tri.p, pos.p,
-                        orig_pos.p, occ.p, win.p, s, true, place_ptr());
+        launch_collapse(rc, eb, edges.p, edge_cost.p, collapse_t, vmin.p, nxt.p, spc.p, nt_off, nt.p, tri.p, pos.p,
+                        occ.p, win.p, s, true, place_ptr());
         exclusive_scan(win.p, win.p, &rc->n_edges, 1, &rc->n_win, scan_scratch, s, &rc->status, eb);
         launch_after_collapse(rc, eb, nT, win.p, collapsed.p, edges.p, nt_off, nt.p, tri.p, pos.p, occ.p, (int)collapsed.n,
                               true, s);

@@ -778,82 +778,134 @@ __device__ __forceinline__ bool is_skinny(V3 p, V3 q, V3 r) {  // :617-637
 }
 
 
-__device__ __forceinline__ bool ring_has_skinny(int w, const int* __restrict__ nt_off, const int* __restrict__ nt,
-                                                const int4* tri, const float4* pos) {
-    for (int s = nt_off[w]; s < nt_off[w + 1]; ++s) {
-        const int4 t = tri[nt[s]];
-        if (t.x == -1) continue;
-        if (is_skinny(v3(pos[t.x]), v3(pos[t.y]), v3(pos[t.z]))) return true;
-    }
-    return false;
-}
-
-
 // An edge wins when its key is the least over every face that touches it, that is when no vertex of the rings of u and v
 // has a smaller one in vmin (the least key of its edges; a face's key is the least of its three vertices', and u and v
-// lie in all faces of their rings). vmin[u] and vmin[v] alone reject nearly every edge before a ring is read; the
-// reference's per-face keys (:587-610) are not made. Slots four at a time, their gathers in flight together.
-__device__ __forceinline__ bool ring_keys_at_least(int a, int b, unsigned long long key, const int* __restrict__ nxt,
-                                                   const int2* __restrict__ spc,
-                                                   const unsigned long long* __restrict__ vmin) {
-    for (int s0 = a; s0 < b; s0 += 4) {
-        bool low = false;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int s = min(s0 + k, b - 1);
-            low |= vmin[nxt[s]] < key;
-            low |= vmin[spc[s].x] < key;
-        }
-        if (low) return false;
-    }
-    return true;
-}
-
+// lie in all faces of their rings). vmin[u] and vmin[v] alone reject nearly every edge; the reference's per-face keys
+// (:587-610) are not made.
+// A warp reads its edges in order and keeps those that pass, and takes them four at a time, eight lanes to an edge and a
+// lane to a ring face: the ring's keys, the collapse and the skinny test (kRestore) are chains of two gathers instead of two
+// per face of both rings. Taken by one thread each, where the edge was found, they set the kernel's time (129 us of a mean
+// round of 1.1 ms from 5.24M faces, 17 us of one of 0.14 ms from 1,280).
+// A collapse that leaves a skinny face is undone in the reference; here its faces are not written (the winners' rings
+// share no face, and no winner's ring holds another's endpoint, so no other collapse shows in the test).
 // kRestore = false: CUSimp's collapse (cusimp.cu:512-585), without the skinny-ring restore
 // kOpt (precision mode 2): the collapse places at the edge's precomputed placement instead of the midpoint
-template <bool kRestore, bool kOpt = false>
-__global__ void __launch_bounds__(kT) k_collapse(RoundCounters* rc, const int* __restrict__ eorder,
-                                                 const int2* __restrict__ edges,
+constexpr int kCollapseLanes = 8;
+
+// The face t of the ring of u (side 0) or v (side 1) after the collapse of (u, v) onto u: x = -1 when it dies
+__device__ __forceinline__ int4 collapsed_face(int4 t, int u, int v, int side) {
+    const int other = side ? u : v;
+    if (t.x == other || t.y == other || t.z == other) return make_int4(-1, -1, -1, 0);
+    if (side) {
+        // a face that holds v twice is in the ring twice, and dies at the second visit, which finds u
+        if ((t.x == v) + (t.y == v) + (t.z == v) > 1) return make_int4(-1, -1, -1, 0);
+        if (t.x == v) t.x = u;
+        else if (t.y == v) t.y = u;
+        else if (t.z == v) t.z = u;
+    }
+    return t;
+}
+
+template <bool kRestore, bool kOpt>
+__device__ __forceinline__ void try_collapse(int e, unsigned long long key, int l, unsigned group,
+                                             const int2* __restrict__ edges,
+                                             const unsigned long long* __restrict__ vmin, const int* __restrict__ nxt,
+                                             const int2* __restrict__ spc, const int* __restrict__ nt_off,
+                                             const int* __restrict__ nt, int4* tri, float4* pos, int* occ, int* win,
+                                             const float4* __restrict__ place) {
+    const int2 ed = edges[e];
+    const int u = ed.x, v = ed.y;
+    const int a[2] = {nt_off[u], nt_off[v]}, b[2] = {nt_off[u + 1], nt_off[v + 1]};
+    bool low = false;
+#pragma unroll
+    for (int side = 0; side < 2; ++side)
+        for (int s = a[side] + l; s < b[side]; s += kCollapseLanes) low |= vmin[nxt[s]] < key || vmin[spc[s].x] < key;
+    if (__any_sync(group, low)) return;
+    V3 vm = vdiv(vadd(v3(pos[u]), v3(pos[v])), 2.0f);
+    if constexpr (kOpt) vm = v3(place[e]);
+    if constexpr (kRestore) {
+        // positions as after the collapse: u at vm, v at the origin
+        auto at = [&](int i) { return i == u ? vm : i == v ? V3{0.f, 0.f, 0.f} : v3(pos[i]); };
+        bool skinny = false;
+#pragma unroll
+        for (int side = 0; side < 2; ++side)
+            for (int s = a[side] + l; s < b[side]; s += kCollapseLanes) {
+                const int4 t = collapsed_face(tri[nt[s]], u, v, side);
+                if (t.x != -1 && is_skinny(at(t.x), at(t.y), at(t.z))) skinny = true;
+            }
+        skinny = __any_sync(group, skinny);
+        if (l == 0) win[e] = 1;
+        if (skinny) return;
+    } else {
+        if (l == 0) win[e] = 1;
+    }
+    __syncwarp(group);  // every lane has read what the first one writes
+    if (l == 0) {
+        pos[u] = make_float4(vm.x, vm.y, vm.z, 0.f);
+        pos[v] = make_float4(0.f, 0.f, 0.f, 0.f);
+        occ[v] = 0;
+    }
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+        for (int s = a[side] + l; s < b[side]; s += kCollapseLanes) {
+            const int f = nt[s];
+            const int4 t = tri[f], c = collapsed_face(t, u, v, side);
+            if (t.x != -1 && (c.x != t.x || c.y != t.y || c.z != t.z)) tri[f] = c;
+        }
+        __syncwarp(group);  // the faces of both rings have died before v's ring is read
+    }
+}
+
+template <bool kRestore, bool kOpt>
+__global__ void __launch_bounds__(kT) k_collapse(RoundCounters* rc, const int2* __restrict__ edges,
                                                  const uint32_t* __restrict__ cost, uint32_t collapse_t,
                                                  const unsigned long long* __restrict__ vmin, const int* __restrict__ nxt,
                                                  const int2* __restrict__ spc, const int* __restrict__ nt_off,
-                                                 const int* __restrict__ nt, int4* tri, const int4* __restrict__ orig_tri,
-                                                 float4* pos, const float4* __restrict__ orig_pos, int* occ, int* win,
+                                                 const int* __restrict__ nt, int4* tri, float4* pos, int* occ, int* win,
                                                  const float4* __restrict__ place) {
     pdl_wait();
+    constexpr int kGroups = 32 / kCollapseLanes;
+    __shared__ unsigned long long queue[kT / 32][32 + kGroups];  // keys (cost << 32 | edge) of the warp's candidates
     const int n = rc->n_edges;
+    const int lane = threadIdx.x & 31, l = lane % kCollapseLanes, g = lane / kCollapseLanes;
+    const unsigned group = ((1u << kCollapseLanes) - 1u) << (g * kCollapseLanes);
+    unsigned long long* q = queue[threadIdx.x >> 5];
+    int held = 0;
     if (gtid() == 0) win[n] = 0;
-    for (int i = gtid(); i < n; i += gstride()) {
-        const int e = eorder[i];
-        int w = 0;
-        const uint32_t c = cost[e];
-        if (c <= collapse_t) {
-            const int2 ed = edges[e];
-            const int u = ed.x, v = ed.y;
-            const unsigned long long key = ((unsigned long long)c << 32) | (unsigned)e;
-            if (vmin[u] == key && vmin[v] == key &&
-                ring_keys_at_least(nt_off[u], nt_off[u + 1], key, nxt, spc, vmin) &&
-                ring_keys_at_least(nt_off[v], nt_off[v + 1], key, nxt, spc, vmin)) {
-                w = 1;
-                const V3 v0 = v3(pos[u]), v1 = v3(pos[v]);
-                V3 vm = vdiv(vadd(v0, v1), 2.0f);
-                if constexpr (kOpt) vm = v3(place[e]);
-                pos[u] = make_float4(vm.x, vm.y, vm.z, 0.f);
-                pos[v] = make_float4(0.f, 0.f, 0.f, 0.f);
-                occ[v] = 0;
-                rewire(u, v, nt_off, nt, tri);
-                bool sk = kRestore && ring_has_skinny(u, nt_off, nt, tri, pos);
-                if (kRestore && !sk) sk = ring_has_skinny(v, nt_off, nt, tri, pos);
-                if (sk) {
-                    occ[v] = 1;
-                    pos[u] = orig_pos[u];
-                    pos[v] = orig_pos[v];
-                    restore_ring(u, nt_off, nt, tri, orig_tri);
-                    restore_ring(v, nt_off, nt, tri, orig_tri);
-                }
+    for (int i0 = gtid() - lane; i0 < n; i0 += gstride()) {
+        const int e = i0 + lane;
+        bool candidate = false;
+        unsigned long long key = 0;
+        if (e < n) {
+            win[e] = 0;
+            const uint32_t c = cost[e];
+            if (c <= collapse_t) {
+                const int2 ed = edges[e];
+                key = ((unsigned long long)c << 32) | (unsigned)e;
+                candidate = vmin[ed.x] == key && vmin[ed.y] == key;
             }
         }
-        win[e] = w;
+        const unsigned m = __ballot_sync(0xffffffffu, candidate);
+        if (candidate) q[held + __popc(m & ((1u << lane) - 1u))] = key;
+        held += __popc(m);
+        const bool last = i0 + gstride() >= n;
+        __syncwarp();
+        int done = 0;
+        while (held - done >= (last ? 1 : kGroups)) {
+            if (done + g < held) {
+                const unsigned long long k = q[done + g];
+                try_collapse<kRestore, kOpt>((int)(unsigned)k, k, l, group, edges, vmin, nxt, spc, nt_off, nt, tri, pos,
+                                             occ, win, place);
+            }
+            __syncwarp();
+            done = min(done + kGroups, held);
+        }
+        // the rest, fewer than a warp takes at once, to the front
+        const unsigned long long rest = done + lane < held ? q[done + lane] : 0ull;
+        __syncwarp();
+        if (done + lane < held) q[lane] = rest;
+        __syncwarp();
+        held -= done;
     }
 }
 
@@ -1311,21 +1363,20 @@ void launch_edge_cost_batch(const RoundCounters* rc, int n_edges_bound, const in
                                                         nullptr);
     note_launch();
 }
-void launch_collapse(RoundCounters* rc, int n_edges_bound, const int* eorder, const int2* edges, const uint32_t* cost,
+void launch_collapse(RoundCounters* rc, int n_edges_bound, const int2* edges, const uint32_t* cost,
                      uint32_t collapse_t, const unsigned long long* vmin, const int* nxt, const int2* spc,
-                     const int* nt_off, const int* nt, int4* tri,
-                     const int4* orig_tri, float4* pos, const float4* orig_pos, int* occ, int* win, cudaStream_t s,
+                     const int* nt_off, const int* nt, int4* tri, float4* pos, int* occ, int* win, cudaStream_t s,
                      bool restore, const float4* place) {
+    const int g = grid_for(n_edges_bound, kT);
     if (restore && place)
-        pdl(k_collapse<true, true>, grid_for(n_edges_bound, kT), kT, 0, s)(rc, eorder, edges, cost, collapse_t, vmin, nxt, spc,
-                                                                          nt_off, nt, tri, orig_tri, pos, orig_pos, occ,
-                                                                          win, place);
+        pdl(k_collapse<true, true>, g, kT, 0, s)(rc, edges, cost, collapse_t, vmin, nxt, spc, nt_off, nt, tri, pos, occ, win,
+                                                 place);
     else if (restore)
-        pdl(k_collapse<true>, grid_for(n_edges_bound, kT), kT, 0, s)(rc, eorder, edges, cost, collapse_t, vmin, nxt, spc, nt_off, nt,
-                                                                    tri, orig_tri, pos, orig_pos, occ, win, nullptr);
+        pdl(k_collapse<true, false>, g, kT, 0, s)(rc, edges, cost, collapse_t, vmin, nxt, spc, nt_off, nt, tri, pos, occ,
+                                                  win, nullptr);
     else
-        pdl(k_collapse<false>, grid_for(n_edges_bound, kT), kT, 0, s)(rc, eorder, edges, cost, collapse_t, vmin, nxt, spc, nt_off, nt,
-                                                                     tri, orig_tri, pos, orig_pos, occ, win, nullptr);
+        pdl(k_collapse<false, false>, g, kT, 0, s)(rc, edges, cost, collapse_t, vmin, nxt, spc, nt_off, nt, tri, pos, occ,
+                                                   win, nullptr);
     note_launch();
 }
 void launch_after_collapse(RoundCounters* rc, int n_edges_bound, int n_tris_bound, const int* win_scan, int* collapsed,

@@ -108,10 +108,10 @@ void launch_edge_cost_batch(const RoundCounters* rc, int n_edges_bound, const in
                             unsigned long long* vmin, const float* mesh_scale, const int* mesh_stuck, const int* vmesh,
                             float tres, cudaStream_t s, bool device_pow = false);
 // vmin: the least key (cost << 32 | edge) over the edges of each vertex
-void launch_collapse(RoundCounters* rc, int n_edges_bound, const int* eorder, const int2* edges, const uint32_t* cost,
+// tri and pos are the round's as it began (a collapse that would leave a skinny face is not made)
+void launch_collapse(RoundCounters* rc, int n_edges_bound, const int2* edges, const uint32_t* cost,
                      uint32_t collapse_t, const unsigned long long* vmin, const int* nxt, const int2* spc,
-                     const int* nt_off, const int* nt, int4* tri,
-                     const int4* orig_tri, float4* pos, const float4* orig_pos, int* occ, int* win, cudaStream_t s,
+                     const int* nt_off, const int* nt, int4* tri, float4* pos, int* occ, int* win, cudaStream_t s,
                      bool restore = true, const float4* place = nullptr);
 // After the collapses: the winners' list, the degenerate faces removed and the edges with coincident endpoints counted in
 // rc->n_line; with lines, also collapsed in edge order and appended to the list (up to line_cap), with rc->n_collapsed
