@@ -272,6 +272,52 @@ __device__ __forceinline__ void pair_geom(const float4 c0, const float4 c1, cons
         for (int d = 0; d < 3; ++d) g.cmax = fmaxf(g.cmax, fmaxf(fabsf(g.A.v[v][d]), fabsf(g.B.v[v][d])));
 }
 
+// The translation of both orders of a pair without its divisions: true when the floored means are certain, that is when no
+// mean is within the roundings of its sum (1e-5 of the coordinates, far above the few ulps of either order) of an
+// integer. reach bounds every translated coordinate.
+__device__ __forceinline__ bool pair_translation_fast(const float4 c0, const float4 c1, const float4 c2, const float4 q0,
+                                                      const float4 q1, const float4 q2, float m[3], float& reach) {
+    const float sum[3] = {c0.x + c1.x + c2.x + q0.x + q1.x + q2.x, c0.y + c1.y + c2.y + q0.y + q1.y + q2.y,
+                          c0.z + c1.z + c2.z + q0.z + q1.z + q2.z};
+    const float mag[3] = {fabsf(c0.x) + fabsf(c1.x) + fabsf(c2.x) + fabsf(q0.x) + fabsf(q1.x) + fabsf(q2.x),
+                          fabsf(c0.y) + fabsf(c1.y) + fabsf(c2.y) + fabsf(q0.y) + fabsf(q1.y) + fabsf(q2.y),
+                          fabsf(c0.z) + fabsf(c1.z) + fabsf(c2.z) + fabsf(q0.z) + fabsf(q1.z) + fabsf(q2.z)};
+    bool sure = true;
+    reach = 1.0f;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const float mean = sum[d] * 0.16666667f;
+        m[d] = floorf(mean);
+        const float f = mean - m[d], margin = 1e-5f * (1.0f + mag[d]);
+        sure = sure && f > margin && f < 1.0f - margin;  // false for a coordinate that is not finite or above 1e5
+        reach += mag[d] + fabsf(m[d]);
+    }
+    return sure;
+}
+
+// Whether every vertex of B but `skip` lies strictly on one side of A's plane, by a looser test than strictly_one_side with
+// one normal for the three: the value is n . (b - a1) for the computed n, off by at most 8 roundings (4.8e-7) of the same
+// sum of absolute values, taken as 2e-6; abs_err as in orient_f, with the bound `reach` of the coordinates in place of
+// the largest. True only when it is certain.
+__device__ __forceinline__ bool surely_one_side(const Tri9& A, const Tri9& B, int skip, float reach) {
+    const float e0x = A.v[0][0] - A.v[1][0], e0y = A.v[0][1] - A.v[1][1], e0z = A.v[0][2] - A.v[1][2];
+    const float e1x = A.v[2][0] - A.v[1][0], e1y = A.v[2][1] - A.v[1][1], e1z = A.v[2][2] - A.v[1][2];
+    const float xa = e0y * e1z, xb = e0z * e1y, ya = e0z * e1x, yb = e0x * e1z, za = e0x * e1y, zb = e0y * e1x;
+    const float nx = xa - xb, ny = ya - yb, nz = za - zb;
+    const float px = fabsf(xa) + fabsf(xb), py = fabsf(ya) + fabsf(yb), pz = fabsf(za) + fabsf(zb);
+    const float abs_err = 1e-10f * (fabsf(nx) + fabsf(ny) + fabsf(nz)) * (reach + 1.0f) + 1e-30f;
+    bool above = true, below = true;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float dx = B.v[k][0] - A.v[1][0], dy = B.v[k][1] - A.v[1][1], dz = B.v[k][2] - A.v[1][2];
+        const float d = nx * dx + ny * dy + nz * dz;
+        const float err = 2e-6f * (px * fabsf(dx) + py * fabsf(dy) + pz * fabsf(dz)) + abs_err;
+        above = above && (k == skip || d > err);
+        below = below && (k == skip || d < -err);
+    }
+    return above || below;
+}
+
 // The two grounds on which the reference's decision is certainly "no intersection" without the fp64 path.
 // The faces lie on one side of each other's plane (of either plane, for faces without a common vertex): the same for both
 // orders of a pair.
