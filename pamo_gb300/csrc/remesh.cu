@@ -165,8 +165,10 @@ __device__ __forceinline__ float box_sq(P3f p, float4 lo, float4 hi) {
 // A tree walk per sample in the band (256^3, 327,680 faces) read 60-100 nodes of divergent
 // walks at a quarter of the lanes: 7.99 ms, with 0.83 ms to mark the band and 0.25 ms for the tree. The splat does
 // about 140 M box tests and stays in L2 (the grid's 67 MB). The whole of stage 1, with the bit rows below: 14.8 -> 1.33
-// ms at 256^3 (327,680 faces), 2.58 -> 0.41 ms at 128^3 (20,480 faces).
+// ms at 256^3 (327,680 faces), 2.58 -> 0.41 ms at 128^3 (20,480 faces); with four samples in flight, the fill's early end and
+// the spread of the cells over the warps 1.30 and 0.37 ms.
 constexpr int kSplatMax = 2048;      // samples of one warp's task
+constexpr int kSplatAhead = 4;       // samples of a lane whose values are loaded together
 constexpr int kMaxChunks = 1024;     // tasks of one triangle (larger boxes get larger chunks)
 constexpr int kSplatQueue = 1 << 20; // tasks queued; a triangle that finds no room is done in place
 constexpr float kBoxSlack = 4e-6f;   // of the band: the rounding of a distance computed near coordinate 1
@@ -196,11 +198,12 @@ __device__ __forceinline__ bool splat_box(int4 t, const float4* __restrict__ q, 
     return true;
 }
 
-__device__ __forceinline__ void splat_sample(const SplatBox& s, int x, int y, int z, int R, float inv, float slack,
-                                             unsigned* udf2) {
-    const P3f p = {((float)x + 0.5f) * inv, ((float)y + 0.5f) * inv, ((float)z + 0.5f) * inv};
-    unsigned* at = udf2 + ((size_t)z * R + y) * R + x;
-    const float best = __uint_as_float(__ldcg(at));
+__device__ __forceinline__ P3f splat_point(int x, int y, int z, float inv) {
+    return {((float)x + 0.5f) * inv, ((float)y + 0.5f) * inv, ((float)z + 0.5f) * inv};
+}
+
+// the triangle's offer to the sample at p, whose value was `best` (lowered by others at most)
+__device__ __forceinline__ void splat_sample(const SplatBox& s, P3f p, float best, float slack, unsigned* at) {
     const float bound = box_sq(p, s.lo, s.hi) - slack;
     if (bound >= best) return;
     const float d = point_tri_sq(p, s.a, s.b, s.c);
@@ -213,7 +216,8 @@ __device__ __forceinline__ void splat_range(const SplatBox& s, unsigned i0, unsi
     const unsigned nx = s.nx, nxy = (unsigned)s.nx * (unsigned)s.ny;
     for (unsigned i = i0 + (threadIdx.x & 31); i < i1; i += 32) {
         const unsigned z = i / nxy, r = i - z * nxy, y = r / nx, x = r - y * nx;
-        splat_sample(s, s.x0 + x, s.y0 + y, s.z0 + z, R, inv, slack, udf2);
+        unsigned* at = udf2 + ((size_t)(s.z0 + z) * R + s.y0 + y) * R + s.x0 + x;
+        splat_sample(s, splat_point(s.x0 + x, s.y0 + y, s.z0 + z, inv), __uint_as_float(__ldcg(at)), slack, at);
     }
 }
 
@@ -242,10 +246,20 @@ __global__ void __launch_bounds__(kT) k_splat(const float4* __restrict__ q, cons
         // i / d by a multiplication: exact for i * d < 2^32 (i < 2^11, d <= 2^11; d = 1 apart)
         const unsigned nx = s.nx, nxy = (unsigned)s.nx * (unsigned)s.ny;
         const unsigned mx = nx > 1 ? 0xffffffffu / nx + 1u : 0u, mxy = nxy > 1 ? 0xffffffffu / nxy + 1u : 0u;
-        for (unsigned i = lane; i < n; i += 32) {
-            const unsigned z = nxy > 1 ? __umulhi(i, mxy) : i, r = i - z * nxy, y = nx > 1 ? __umulhi(r, mx) : r,
-                           x = r - y * nx;
-            splat_sample(s, s.x0 + x, s.y0 + y, s.z0 + z, R, inv, slack, udf2);
+        for (unsigned i0 = lane; i0 < n; i0 += 32 * kSplatAhead) {
+            unsigned* at[kSplatAhead];
+            float best[kSplatAhead];
+            P3f p[kSplatAhead];
+#pragma unroll
+            for (int k = 0; k < kSplatAhead; ++k) {
+                const unsigned i = i0 + 32 * k, z = nxy > 1 ? __umulhi(i, mxy) : i, r = i - z * nxy,
+                               y = nx > 1 ? __umulhi(r, mx) : r, x = r - y * nx;
+                p[k] = splat_point(s.x0 + x, s.y0 + y, s.z0 + z, inv);
+                at[k] = udf2 + ((size_t)(s.z0 + z) * R + s.y0 + y) * R + s.x0 + x;
+                best[k] = i < n ? __uint_as_float(__ldcg(at[k])) : -1.f;  // past the end: no offer is below
+            }
+#pragma unroll
+            for (int k = 0; k < kSplatAhead; ++k) splat_sample(s, p[k], best[k], slack, at[k]);
         }
     }
 }
@@ -389,8 +403,19 @@ __global__ void __launch_bounds__(kFillThreads) k_fill(const unsigned* __restric
                 diff = 1;
             }
         }
-        // a tile that the rows leave as they are has been through the doubling steps of the pass before (or of none)
-        if (!__syncthreads_or(diff) && it > 0) break;
+        // a tile whose rows stay as they are and have nothing to give to the rows beside them is done: the doubling steps
+        // are for those that have (the last passes of a fill change nothing anywhere)
+        if (!__syncthreads_or(diff)) {
+            int grows = 0;
+#pragma unroll
+            for (int j = 0; j < kFillItems; ++j) {
+                const int i = threadIdx.x + j * kFillThreads;
+                if (i >= n) continue;
+                const unsigned beside = (i >= W ? sg[i - W] : 0u) | (i + W < n ? sg[i + W] : 0u);
+                grows |= (p[j] & beside & ~sg[i]) != 0u;
+            }
+            if (!__syncthreads_or(grows)) break;
+        }
         diff = 0;
         for (int dir = 0; dir < 2; ++dir) {
             for (int k = W; k < n; k *= 2) {
@@ -505,8 +530,9 @@ __global__ void k_surface_counts(const unsigned* __restrict__ neg, int R, int W,
 __constant__ int kEdgeCorners[12][2] = {{0, 1}, {2, 3}, {4, 5}, {6, 7}, {0, 2}, {1, 3}, {4, 6}, {5, 7},
                                         {0, 4}, {1, 5}, {2, 6}, {3, 7}};
 
-// the vertex of each active cell at the mean of its edge crossings, in cell order; a warp takes 32 words and its lanes
-// the cells of each word that has some
+// the vertex of each active cell at the mean of its edge crossings, in cell order; a warp looks at 32 words at a time, far
+// apart (the words with cells lie together: 32 in a row were up to 32 turns for one warp), and its lanes take the cells of
+// each word that has some
 __global__ void __launch_bounds__(kT) k_cell_vertices(const unsigned* __restrict__ udf2, const unsigned* __restrict__ neg,
                                                       const unsigned* __restrict__ cells, int R, int W, float iso,
                                                       const int* __restrict__ cscan, float band, float margin,
@@ -515,13 +541,14 @@ __global__ void __launch_bounds__(kT) k_cell_vertices(const unsigned* __restrict
     const float t0 = unord(ext[0]), t1 = unord(ext[1]), t2 = unord(ext[2]), tmax = extent_max(ext);
     const int lane = threadIdx.x & 31;
     const long long words = (long long)R * R * W, RR = (long long)R * R;
-    for (long long w0 = 32ll * (gtid() >> 5); w0 < words; w0 += gstride()) {
-        const unsigned mine = w0 + lane < words ? cells[w0 + lane] : 0u;
+    const long long warp = gtid() >> 5, warps = gstride() >> 5;
+    for (long long w0 = warp; w0 < words; w0 += 32 * warps) {
+        const unsigned mine = w0 + lane * warps < words ? cells[w0 + lane * warps] : 0u;
         for (unsigned todo = __ballot_sync(0xffffffffu, mine != 0u); todo; todo &= todo - 1u) {
             const int k = __ffs(todo) - 1;
             const unsigned act = __shfl_sync(0xffffffffu, mine, k);
             if (!((act >> lane) & 1u)) continue;
-            const long long i = w0 + k, row = i / W;
+            const long long i = w0 + k * warps, row = i / W;
             const int w = (int)(i - row * W), y = (int)(row % R), z = (int)(row / R), x = 32 * w + lane;
             float v[8];
             for (int c = 0; c < 8; ++c) {
@@ -565,10 +592,12 @@ __global__ void __launch_bounds__(kT) k_quads(const unsigned* __restrict__ neg, 
         const long long i = ((long long)cz * R + cy) * W + (cx >> 5);
         return cscan[i] + __popc(cells[i] & ((1u << (cx & 31)) - 1u));
     };
-    for (long long w0 = 32ll * (gtid() >> 5); w0 < words; w0 += gstride()) {
-        const bool on = w0 + lane < words && qscan[w0 + lane + 1] != qscan[w0 + lane];
+    const long long warp = gtid() >> 5, warps = gstride() >> 5;
+    for (long long w0 = warp; w0 < words; w0 += 32 * warps) {
+        const long long mine = w0 + lane * warps;
+        const bool on = mine < words && qscan[mine + 1] != qscan[mine];
         for (unsigned todo = __ballot_sync(0xffffffffu, on); todo; todo &= todo - 1u) {
-            const long long i = w0 + __ffs(todo) - 1, row = i / W;
+            const long long i = w0 + (__ffs(todo) - 1) * warps, row = i / W;
             const int w = (int)(i - row * W), y = (int)(row % R), z = (int)(row / R), x = 32 * w + lane;
             unsigned e[3];
             edge_bits(neg, i, R, W, w, y, z, e);
