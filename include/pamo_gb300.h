@@ -362,6 +362,13 @@ int pamo_point_mesh_sqdist(const double* points, int32_t n_points, const double*
                            const int32_t* triangles, int32_t n_triangles, double* out_sqdist, int32_t* out_face,
                            pamo_stream stream);
 
+/* The same in the caller's device memory: workspace of at least the bytes that pamo_point_mesh_workspace gives for the
+ * mesh, any contents, free again when the call returns (the other form allocates and frees it on each call). */
+int pamo_point_mesh_workspace(int32_t n_vertices, int32_t n_triangles, int64_t* bytes);
+int pamo_point_mesh_sqdist_ws(const double* points, int32_t n_points, const double* vertices, int32_t n_vertices,
+                              const int32_t* triangles, int32_t n_triangles, double* out_sqdist, int32_t* out_face,
+                              void* workspace, int64_t workspace_bytes, pamo_stream stream);
+
 /* Per-face minimum angles in radians (metrics.py:55-107): out_edge_form as compute_min_angle_VF computes
  * the corner angles (from the face's edge vectors, cosines clipped to [-1, 1]), out_igl_form as
  * igl.internal_angles does (law of cosines on the edge lengths), NaN for a face with a repeated index. Either

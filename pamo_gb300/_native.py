@@ -41,6 +41,8 @@ SIGNATURES = {
     "pamo_forward_round": (ctypes.c_int, [_P, _P, _P, _P, _I32, _I32, _I32, _F32, _F32, _I32, _I32, _P]),
     "pamo_legacy_round": (ctypes.c_int, [_P, _P, _P, _I32, _I32, _F32, _F32, _I32, _P]),
     "pamo_point_mesh_sqdist": (ctypes.c_int, [_P, _I32, _P, _I32, _P, _I32, _P, _P, _P]),
+    "pamo_point_mesh_workspace": (ctypes.c_int, [_I32, _I32, ctypes.POINTER(ctypes.c_int64)]),
+    "pamo_point_mesh_sqdist_ws": (ctypes.c_int, [_P, _I32, _P, _I32, _P, _I32, _P, _P, _P, ctypes.c_int64, _P]),
     "pamo_face_min_angles": (ctypes.c_int, [_P, _P, _I32, _P, _P, _P]),
     "pamo_remesher_create": (ctypes.c_int, [ctypes.POINTER(ctypes.c_void_p), _I32]),
     "pamo_remesher_destroy": (ctypes.c_int, [_P]),

@@ -15,6 +15,7 @@
 #include "../../include/pamo_gb300.h"
 #include "lbvh.cuh"
 #include "pamo_common.cuh"
+#include "scan.cuh"
 
 namespace {
 
@@ -306,11 +307,61 @@ __global__ void k_face_min_angles(const double* __restrict__ V, const int* __res
     }
 }
 
+size_t up256(size_t x) { return (x + 255) & ~size_t(255); }
+
 int cuda_status(cudaError_t e) { return e == cudaSuccess ? PAMO_OK : PAMO_ERR_CUDA; }
 
 }  // namespace
 
 extern "C" {
+
+int pamo_point_mesh_workspace(int32_t n_vertices, int32_t n_triangles, int64_t* bytes) {
+    if (n_vertices < 1 || n_triangles < 1 || !bytes) return PAMO_ERR_INVALID_ARG;
+    *bytes = (int64_t)(256 + up256(sizeof(RoundCounters)) + up256((size_t)n_vertices * sizeof(float4)) +
+                       up256(((size_t)n_triangles + 1) * sizeof(int4)) + bvh_bytes(n_triangles));
+    return PAMO_OK;
+}
+
+int pamo_point_mesh_sqdist_ws(const double* points, int32_t n_points, const double* vertices, int32_t n_vertices,
+                              const int32_t* triangles, int32_t n_triangles, double* out_sqdist, int32_t* out_face,
+                              void* workspace, int64_t workspace_bytes, pamo_stream stream) {
+    if (!points || !vertices || !triangles || !out_sqdist || n_points < 0 || n_vertices < 1 || n_triangles < 1)
+        return PAMO_ERR_INVALID_ARG;
+    if (n_points == 0) return PAMO_OK;
+    int64_t need = 0;
+    pamo_point_mesh_workspace(n_vertices, n_triangles, &need);
+    if (!workspace || workspace_bytes < need) return PAMO_ERR_INVALID_ARG;
+    cudaStream_t s = (cudaStream_t)stream;
+    char* at = reinterpret_cast<char*>(up256(reinterpret_cast<uintptr_t>(workspace)));
+    auto take = [&](size_t bytes) {
+        char* p = at;
+        at += up256(bytes);
+        return p;
+    };
+    RoundCounters* rc = reinterpret_cast<RoundCounters*>(take(sizeof(RoundCounters)));
+    float4* pos = reinterpret_cast<float4*>(take((size_t)n_vertices * sizeof(float4)));
+    int4* tri = reinterpret_cast<int4*>(take(((size_t)n_triangles + 1) * sizeof(int4)));
+    BvhBuffers b;
+    bvh_carve(b, n_triangles, at, false);
+    cudaMemsetAsync(b.scan_scratch, 0, scan_scratch_ints() * sizeof(int), s);
+    RoundCounters h{};
+    h.n_pts = n_vertices;
+    h.n_tris = n_triangles;
+    cudaMemcpyAsync(rc, &h, sizeof(h), cudaMemcpyHostToDevice, s);
+    pdl(k_to_float4, grid_for(n_vertices, kT), kT, 0, s)(vertices, n_vertices, pos);
+    pdl(k_to_int4, grid_for(n_triangles, kT), kT, 0, s)(triangles, n_triangles, n_vertices, tri, &rc->status);
+    note_launches(2);
+    bvh_build(b, tri, pos, rc, n_triangles, s, false, BvhQuery(), false);
+    pdl(k_point_mesh, grid_for(n_points, kQT, 16), kQT, 0, s)(points, n_points, vertices, pos, tri, b.packed, b.scene,
+                                                             b.vals[0], rc, out_sqdist, out_face, &rc->status);
+    note_launch();
+    int st = 0;
+    cudaMemcpyAsync(&st, &rc->status, sizeof(int), cudaMemcpyDeviceToHost, s);
+    int r = cuda_status(cudaStreamSynchronize(s));
+    if (r == PAMO_OK && (st & kErrBadIndex)) r = PAMO_ERR_INVALID_ARG;
+    else if (r == PAMO_OK && st) r = PAMO_ERR_ITER_LIMIT;
+    return r;
+}
 
 int pamo_point_mesh_sqdist(const double* points, int32_t n_points, const double* vertices, int32_t n_vertices,
                            const int32_t* triangles, int32_t n_triangles, double* out_sqdist, int32_t* out_face,
@@ -318,44 +369,13 @@ int pamo_point_mesh_sqdist(const double* points, int32_t n_points, const double*
     if (!points || !vertices || !triangles || !out_sqdist || n_points < 0 || n_vertices < 1 || n_triangles < 1)
         return PAMO_ERR_INVALID_ARG;
     if (n_points == 0) return PAMO_OK;
-    cudaStream_t s = (cudaStream_t)stream;
-    float4* pos = nullptr;
-    int4* tri = nullptr;
-    RoundCounters* rc = nullptr;
-    char* bvh_mem = nullptr;
-    int r = PAMO_OK;
-    if (cudaMalloc((void**)&pos, (size_t)n_vertices * sizeof(float4)) != cudaSuccess ||
-        cudaMalloc((void**)&tri, ((size_t)n_triangles + 1) * sizeof(int4)) != cudaSuccess ||
-        cudaMalloc((void**)&rc, sizeof(RoundCounters)) != cudaSuccess ||
-        cudaMalloc((void**)&bvh_mem, bvh_bytes(n_triangles)) != cudaSuccess) {
-        r = PAMO_ERR_OOM;
-    }
-    if (r == PAMO_OK) {
-        BvhBuffers b;
-        bvh_carve(b, n_triangles, bvh_mem);
-        RoundCounters h{};
-        h.n_pts = n_vertices;
-        h.n_tris = n_triangles;
-        cudaMemcpyAsync(rc, &h, sizeof(h), cudaMemcpyHostToDevice, s);
-        pdl(k_to_float4, grid_for(n_vertices, kT), kT, 0, s)(vertices, n_vertices, pos);
-        pdl(k_to_int4, grid_for(n_triangles, kT), kT, 0, s)(triangles, n_triangles, n_vertices, tri, &rc->status);
-        note_launches(2);
-        bvh_build(b, tri, pos, rc, n_triangles, s, false, BvhQuery(), false);
-        pdl(k_point_mesh, grid_for(n_points, kQT, 16), kQT, 0, s)(points, n_points, vertices, pos, tri, b.packed, b.scene,
-                                                                b.vals[0], rc, out_sqdist, out_face, &rc->status);
-        note_launch();
-        r = cuda_status(cudaStreamSynchronize(s));
-        if (r == PAMO_OK) {
-            int st = 0;
-            r = cuda_status(cudaMemcpy(&st, &rc->status, sizeof(int), cudaMemcpyDeviceToHost));
-            if (r == PAMO_OK && (st & kErrBadIndex)) r = PAMO_ERR_INVALID_ARG;
-            else if (r == PAMO_OK && st) r = PAMO_ERR_ITER_LIMIT;
-        }
-    }
-    cudaFree(pos);
-    cudaFree(tri);
-    cudaFree(rc);
-    cudaFree(bvh_mem);
+    int64_t bytes = 0;
+    pamo_point_mesh_workspace(n_vertices, n_triangles, &bytes);
+    void* workspace = nullptr;
+    if (cudaMalloc(&workspace, (size_t)bytes) != cudaSuccess) return PAMO_ERR_OOM;
+    const int r = pamo_point_mesh_sqdist_ws(points, n_points, vertices, n_vertices, triangles, n_triangles, out_sqdist,
+                                            out_face, workspace, bytes, stream);
+    cudaFree(workspace);
     return r;
 }
 

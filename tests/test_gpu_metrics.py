@@ -65,6 +65,38 @@ def test_point_mesh_sqdist_over_scales_and_shapes(scale, shift, thin, far, faces
     assert (np.abs(all_d2[fi, np.arange(len(P))] - want) <= bound).all()
 
 
+def test_point_mesh_sqdist_in_the_callers_memory():
+    """The form that allocates gives the same as the one with a workspace, and a workspace that is too small is refused."""
+    import ctypes
+
+    import torch
+
+    from pamo_gb300 import _native
+
+    V, F = meshes.sphere(6)
+    V = torch.tensor(V, dtype=torch.float64, device="cuda")
+    F = torch.tensor(np.asarray(F, np.int32), device="cuda")
+    P = 1.1 * V[:77].contiguous()
+    lib, need = _native.load(), ctypes.c_int64(0)
+    assert lib.pamo_point_mesh_workspace(len(V), len(F), ctypes.byref(need)) == _native.PAMO_OK
+    out = []
+    for size in (0, need.value, need.value - 1):
+        d2, fi = torch.empty(77, dtype=torch.float64, device="cuda"), torch.empty(77, dtype=torch.int32, device="cuda")
+        args = [ctypes.c_void_p(P.data_ptr()), 77, ctypes.c_void_p(V.data_ptr()), len(V), ctypes.c_void_p(F.data_ptr()), len(F),
+                ctypes.c_void_p(d2.data_ptr()), ctypes.c_void_p(fi.data_ptr())]
+        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        if size == 0:
+            assert lib.pamo_point_mesh_sqdist(*args, stream) == _native.PAMO_OK
+        else:
+            work = torch.full((size,), 255, dtype=torch.uint8, device="cuda")
+            r = lib.pamo_point_mesh_sqdist_ws(*args, ctypes.c_void_p(work.data_ptr()), size, stream)
+            assert (r == _native.PAMO_OK) == (size >= need.value)
+            if r != _native.PAMO_OK:
+                continue
+        out.append((d2.cpu(), fi.cpu()))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
 def test_face_min_angles_match_the_reference_formulas():
     V, F = meshes.with_degenerate_face()
     V = V.astype(np.float64)
