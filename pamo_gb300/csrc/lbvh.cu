@@ -18,6 +18,8 @@ namespace {
 constexpr int kSortTiles = 4 * kNumSM;
 constexpr size_t kExactQueue = 1 << 20;  // pairs queued for the float64 pass (the rest are decided in place)
 constexpr int kSortThreads = 256;
+constexpr int kFusedTiles = 16;   // tiles up to which a sort pass is one launch (k_rs_pass)
+constexpr int kSortCtl = 4 * 256 + 4 * (1 + kFusedTiles);  // the digit totals, then each pass's ticket and flags
 constexpr int kQueryThreads = 128;
 constexpr int kStackDepth = 64;  // enough for any tree (depth <= 62 + 1)
 constexpr int kShortStack = 24;  // first walk: deeper queries are handed to the second walk
@@ -48,8 +50,10 @@ __device__ __forceinline__ unsigned expand10(unsigned v) {
 __global__ void __launch_bounds__(256) k_boxes(const int4* __restrict__ tri, const float4* __restrict__ pos,
                                                 RoundCounters* rc, float4* box_lo, float4* box_hi, int* live,
                                                 unsigned* scene, int all_faces, BvhQuery q, int* xq_count, int* visit,
-                                                const int* leaves) {
+                                                const int* leaves, int* sort_ctl) {
     pdl_wait();
+    if (!leaves)
+        for (int i = gtid(); i < kSortCtl; i += gstride()) sort_ctl[i] = 0;
     if (gtid() == 0) {
         rc->pad[1] = rc->pad[2] = rc->pad[3] = 0;  // pair list length, query count, redo count
         *xq_count = 0;
@@ -156,10 +160,10 @@ __global__ void __launch_bounds__(256) k_morton(const RoundCounters* rc, const i
 }
 
 // ---------------------------------------------------------------- stable LSD radix sort
-__device__ __forceinline__ void sort_chunk(int n, int& lo, int& hi) {
-    long long chunk = ((long long)n + gridDim.x - 1) / gridDim.x;
+__device__ __forceinline__ void sort_chunk(int n, int tile, int tiles, int& lo, int& hi) {
+    long long chunk = ((long long)n + tiles - 1) / tiles;
     chunk = (chunk + kSortThreads - 1) / kSortThreads * kSortThreads;
-    long long a = chunk * blockIdx.x, b = a + chunk;
+    long long a = chunk * tile, b = a + chunk;
     lo = (int)(a < n ? a : n);
     hi = (int)(b < n ? b : n);
 }
@@ -171,28 +175,24 @@ __global__ void __launch_bounds__(kSortThreads) k_rs_hist(const unsigned* __rest
     h[threadIdx.x] = 0;
     __syncthreads();
     int lo, hi;
-    sort_chunk(*d_n, lo, hi);
+    sort_chunk(*d_n, blockIdx.x, gridDim.x, lo, hi);
     for (int i = lo + threadIdx.x; i < hi; i += kSortThreads) atomicAdd(&h[(keys[i] >> shift) & 0xFF], 1);
     __syncthreads();
     hist[threadIdx.x * gridDim.x + blockIdx.x] = h[threadIdx.x];
 }
 
-// Each tile of 256 keys is ranked stably: lanes of a warp with the same digit find each other with
+// Scatters keys [lo, hi) by the digit at `shift`, base[d] being the place of the first one with digit d (shared; it moves on
+// with the keys). Each tile of 256 keys is ranked stably: lanes of a warp with the same digit find each other with
 // __match_any_sync, warps are ordered through per-warp digit counts in shared memory.
-__global__ void __launch_bounds__(kSortThreads) k_rs_scatter(const unsigned* __restrict__ kin, const int* __restrict__ vin,
-                                                             unsigned* kout, int* vout, const int* d_n, int shift,
-                                                             const int* hist) {
-    pdl_wait();
+struct SortShared {
+    int base[256], wcnt[kSortThreads / 32][256], tot[256];
+};
+__device__ __forceinline__ void sort_scatter(const unsigned* kin, const int* vin, unsigned* kout, int* vout, int lo, int hi,
+                                             int shift, SortShared& S) {
     constexpr int W = kSortThreads / 32;
-    __shared__ int base[256];
-    __shared__ int wcnt[W][256];
-    __shared__ int tot[256];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    base[threadIdx.x] = hist[threadIdx.x * gridDim.x + blockIdx.x];
-    for (int w = 0; w < W; ++w) wcnt[w][threadIdx.x] = 0;
+    for (int w = 0; w < W; ++w) S.wcnt[w][threadIdx.x] = 0;
     __syncthreads();
-    int lo, hi;
-    sort_chunk(*d_n, lo, hi);
     for (int t0 = lo; t0 < hi; t0 += kSortThreads) {
         const int i = t0 + threadIdx.x;
         const bool valid = i < hi;
@@ -201,26 +201,118 @@ __global__ void __launch_bounds__(kSortThreads) k_rs_scatter(const unsigned* __r
         const int dig = valid ? (int)((key >> shift) & 0xFF) : 256;
         const unsigned peers = __match_any_sync(0xffffffffu, dig);
         const int rank = __popc(peers & ((1u << lane) - 1u));
-        if (valid && rank == 0) wcnt[warp][dig] = __popc(peers);
+        if (valid && rank == 0) S.wcnt[warp][dig] = __popc(peers);
         __syncthreads();
         {
             int run = 0;
             for (int w = 0; w < W; ++w) {
-                int c = wcnt[w][threadIdx.x];
-                wcnt[w][threadIdx.x] = run;
+                int c = S.wcnt[w][threadIdx.x];
+                S.wcnt[w][threadIdx.x] = run;
                 run += c;
             }
-            tot[threadIdx.x] = run;
+            S.tot[threadIdx.x] = run;
         }
         __syncthreads();
         if (valid) {
-            const int dst = base[dig] + wcnt[warp][dig] + rank;
+            const int dst = S.base[dig] + S.wcnt[warp][dig] + rank;
             kout[dst] = key;
             vout[dst] = val;
         }
         __syncthreads();
-        base[threadIdx.x] += tot[threadIdx.x];
-        for (int w = 0; w < W; ++w) wcnt[w][threadIdx.x] = 0;
+        S.base[threadIdx.x] += S.tot[threadIdx.x];
+        for (int w = 0; w < W; ++w) S.wcnt[w][threadIdx.x] = 0;
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(kSortThreads) k_rs_scatter(const unsigned* __restrict__ kin, const int* __restrict__ vin,
+                                                             unsigned* kout, int* vout, const int* d_n, int shift,
+                                                             const int* hist) {
+    pdl_wait();
+    __shared__ SortShared S;
+    S.base[threadIdx.x] = hist[threadIdx.x * gridDim.x + blockIdx.x];
+    int lo, hi;
+    sort_chunk(*d_n, blockIdx.x, gridDim.x, lo, hi);
+    sort_scatter(kin, vin, kout, vout, lo, hi, shift, S);
+}
+
+// Up to kFusedTiles tiles: one kernel counts the digits of all four passes (ctl's first 1024 words, zeroed by k_boxes), and a
+// pass is one launch: a tile publishes its own digit counts, waits for the tiles before it, and adds theirs up. Tiles are
+// taken in the order the blocks start, so a tile only waits for blocks that run already; the wait is bounded
+// (kErrIterLimit). In place of a count, a scan and a scatter launch a pass; with more tiles the sums over them (256 tiles^2
+// / 2 words) cost more than the scan (one intersection check of 327,680 faces, 160 tiles: 515 -> 532 us). One tile (up to
+// 2048 keys): all passes in one block. Twelve launches to five, to one for one tile: a stage-2 run from 1,280 faces 4.44 ->
+// 4.33 ms, from 20,480 faces 14.25 -> 14.02 ms.
+__global__ void __launch_bounds__(kSortThreads) k_rs_digits(const unsigned* __restrict__ keys, const int* d_n, int* total) {
+    pdl_wait();
+    __shared__ int h[4][256];
+    for (int k = 0; k < 4; ++k) h[k][threadIdx.x] = 0;
+    __syncthreads();
+    int lo, hi;
+    sort_chunk(*d_n, blockIdx.x, gridDim.x, lo, hi);
+    for (int i = lo + threadIdx.x; i < hi; i += kSortThreads) {
+        const unsigned key = keys[i];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) atomicAdd(&h[k][(key >> (8 * k)) & 0xFF], 1);
+    }
+    __syncthreads();
+    for (int k = 0; k < 4; ++k)
+        if (h[k][threadIdx.x]) atomicAdd(&total[256 * k + threadIdx.x], h[k][threadIdx.x]);
+}
+
+__global__ void __launch_bounds__(kSortThreads) k_rs_pass(const unsigned* __restrict__ kin, const int* __restrict__ vin,
+                                                          unsigned* kout, int* vout, const int* d_n, int shift,
+                                                          const int* __restrict__ total, int* ticket, int* ready,
+                                                          int* hist, int* err) {
+    pdl_wait();
+    __shared__ SortShared S;
+    __shared__ int h[256], sm[33], s_tile;
+    if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1);
+    h[threadIdx.x] = 0;
+    __syncthreads();
+    const int tile = s_tile;
+    int lo, hi;
+    sort_chunk(*d_n, tile, gridDim.x, lo, hi);
+    for (int i = lo + threadIdx.x; i < hi; i += kSortThreads) atomicAdd(&h[(kin[i] >> shift) & 0xFF], 1);
+    __syncthreads();
+    __stcg(&hist[256 * tile + threadIdx.x], h[threadIdx.x]);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        asm volatile("st.release.gpu.global.s32 [%0], 1;" ::"l"(&ready[tile]) : "memory");
+    }
+    if ((int)threadIdx.x < tile) {  // at most kFusedTiles - 1 < kSortThreads
+        int there = 0;
+        for (int spins = 0; !there; ++spins) {
+            asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(there) : "l"(&ready[threadIdx.x]) : "memory");
+            if (spins > (1 << 22)) {
+                atomicOr(err, kErrIterLimit);
+                break;
+            }
+        }
+    }
+    int all;
+    int at = block_exclusive_scan(total[threadIdx.x], &all, sm);  // its barriers follow the waits
+#pragma unroll 8
+    for (int k = 0; k < tile; ++k) at += __ldcg(&hist[256 * k + threadIdx.x]);
+    S.base[threadIdx.x] = at;
+    if (hi > lo) sort_scatter(kin, vin, kout, vout, lo, hi, shift, S);
+}
+
+__global__ void __launch_bounds__(kSortThreads) k_rs_one_tile(unsigned* k0, int* v0, unsigned* k1, int* v1, const int* d_n) {
+    pdl_wait();
+    __shared__ SortShared S;
+    __shared__ int h[256], sm[33];
+    const int n = *d_n;
+    for (int pass = 0; pass < 4; ++pass) {
+        const unsigned* kin = pass & 1 ? k1 : k0;
+        h[threadIdx.x] = 0;
+        __syncthreads();
+        for (int i = threadIdx.x; i < n; i += kSortThreads) atomicAdd(&h[(kin[i] >> (8 * pass)) & 0xFF], 1);
+        __syncthreads();
+        int all;
+        S.base[threadIdx.x] = block_exclusive_scan(h[threadIdx.x], &all, sm);
+        sort_scatter(kin, pass & 1 ? v1 : v0, pass & 1 ? k0 : k1, pass & 1 ? v0 : v1, 0, n, 8 * pass, S);
         __syncthreads();
     }
 }
@@ -982,6 +1074,7 @@ size_t bvh_bytes(int cap) {
     b += 2 * align256(4 * c);               // keys
     b += 2 * align256(4 * c);               // vals
     b += align256(4 * (256 * (size_t)kSortTiles + 1));
+    b += align256(4 * kSortCtl);
     b += align256(8 * c);                   // child
     b += align256(8 * c);                   // range
     b += 2 * align256(4 * c);               // iparent, lparent
@@ -1013,6 +1106,7 @@ void bvh_carve(BvhBuffers& b, int cap, char* base, bool clear_scan_scratch) {
     b.vals[0] = (int*)take(4 * c);
     b.vals[1] = (int*)take(4 * c);
     b.hist = (int*)take(4 * (256 * (size_t)kSortTiles + 1));
+    b.sort_ctl = (int*)take(4 * kSortCtl);
     b.child = (int2*)take(8 * c);
     b.range = (int2*)take(8 * c);
     b.iparent = (int*)take(4 * c);
@@ -1039,7 +1133,7 @@ void bvh_build(BvhBuffers& b, const int4* tri, const float4* pos, RoundCounters*
     cudaMemsetAsync(b.scene + 3, 0x00, 3 * sizeof(unsigned), s);
     const int gF = grid_for(n_tris_bound, 256);
     pdl(k_boxes, gF, 256, 0, s)(tri, pos, rc, b.box_lo, b.box_hi, b.live_scan, b.scene, all_faces ? 1 : 0, query,
-                                   b.xq_count, b.visit, nullptr); note_launch();
+                                   b.xq_count, b.visit, nullptr, b.sort_ctl); note_launch();
     exclusive_scan(b.live_scan, b.live_scan, &rc->n_tris, 1, &rc->n_live, b.scan_scratch, s, &rc->status, n_tris_bound);
     pdl(k_morton, gF, 256, 0, s)(rc, b.live_scan, b.box_lo, b.box_hi, b.scene, b.keys[0], b.vals[0],
                                 meshes ? meshes->fmesh : nullptr, meshes ? meshes->bits : 0, b.visit); note_launch();
@@ -1048,12 +1142,25 @@ void bvh_build(BvhBuffers& b, const int4* tri, const float4* pos, RoundCounters*
     // digit-major over the tiles, so its scan gives each tile's output offset per digit
     long long st = n_tris_bound >= (1 << 19) ? kSortTiles : ((long long)n_tris_bound + 2047) / 2048;
     const int sort_tiles = (int)(st < 1 ? 1 : (st > kSortTiles ? kSortTiles : st));
-    for (int pass = 0; pass < 4; ++pass) {
-        const int in = pass & 1, out = in ^ 1;
-        pdl(k_rs_hist, sort_tiles, kSortThreads, 0, s)(b.keys[in], &rc->n_live, 8 * pass, b.hist); note_launch();
-        exclusive_scan(b.hist, b.hist, nullptr, 256 * sort_tiles, nullptr, b.scan_scratch, s, &rc->status, 0);
-        pdl(k_rs_scatter, sort_tiles, kSortThreads, 0, s)(b.keys[in], b.vals[in], b.keys[out], b.vals[out], &rc->n_live,
-                                                         8 * pass, b.hist); note_launch();
+    if (sort_tiles == 1) {
+        pdl(k_rs_one_tile, 1, kSortThreads, 0, s)(b.keys[0], b.vals[0], b.keys[1], b.vals[1], &rc->n_live); note_launch();
+    } else if (sort_tiles <= kFusedTiles) {
+        pdl(k_rs_digits, sort_tiles, kSortThreads, 0, s)(b.keys[0], &rc->n_live, b.sort_ctl); note_launch();
+        for (int pass = 0; pass < 4; ++pass) {
+            const int in = pass & 1, out = in ^ 1;
+            int* ticket = b.sort_ctl + 1024 + pass * (1 + kFusedTiles);
+            pdl(k_rs_pass, sort_tiles, kSortThreads, 0, s)(b.keys[in], b.vals[in], b.keys[out], b.vals[out], &rc->n_live,
+                                                          8 * pass, b.sort_ctl + 256 * pass, ticket, ticket + 1, b.hist,
+                                                          &rc->status); note_launch();
+        }
+    } else {
+        for (int pass = 0; pass < 4; ++pass) {
+            const int in = pass & 1, out = in ^ 1;
+            pdl(k_rs_hist, sort_tiles, kSortThreads, 0, s)(b.keys[in], &rc->n_live, 8 * pass, b.hist); note_launch();
+            exclusive_scan(b.hist, b.hist, nullptr, 256 * sort_tiles, nullptr, b.scan_scratch, s, &rc->status, 0);
+            pdl(k_rs_scatter, sort_tiles, kSortThreads, 0, s)(b.keys[in], b.vals[in], b.keys[out], b.vals[out], &rc->n_live,
+                                                             8 * pass, b.hist); note_launch();
+        }
     }
     pdl(k_karras, gF, 256, 0, s)(rc, b.keys[0], b.child, b.iparent, b.lparent, b.range); note_launch();
     if (meshes) {
@@ -1090,7 +1197,7 @@ void bvh_refit(BvhBuffers& b, const int4* tri, const float4* pos, RoundCounters*
 void bvh_refit_faces(BvhBuffers& b, const int4* tri, const float4* pos, RoundCounters* rc, int n_tris_bound,
                      cudaStream_t s, bool next_round, const BvhQuery& query) {
     pdl(k_boxes, grid_for(n_tris_bound, 256), 256, 0, s)(tri, pos, rc, b.box_lo, b.box_hi, b.live_scan, b.scene, 1, query,
-                                                       b.xq_count, b.visit, b.meta); note_launch();
+                                                       b.xq_count, b.visit, b.meta, nullptr); note_launch();
     bottom_up<true, false, kLeafReuse>(b, rc, n_tris_bound, next_round ? (const int*)b.keys[1] : nullptr, query.flags,
                                        nullptr, s);
 }

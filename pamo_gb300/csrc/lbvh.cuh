@@ -14,6 +14,7 @@ struct BvhBuffers {
     unsigned* keys[2] = {nullptr, nullptr};  // Morton codes, sort ping-pong
     int* vals[2] = {nullptr, nullptr};       // face ids, sort ping-pong
     int* hist = nullptr;               // radix histograms [256 * kSortTiles + 1]
+    int* sort_ctl = nullptr;           // the sort's digit totals, tickets and flags
     int2* child = nullptr;             // internal node children; v < 0 encodes leaf ~v
     int2* range = nullptr;             // internal node leaf range [lo, hi] (the node index is one end)
     int* iparent = nullptr;            // parent of internal node

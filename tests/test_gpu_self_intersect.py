@@ -33,6 +33,17 @@ def test_flags_at_the_edges_of_tiles_and_warps(faces):
     assert np.array_equal(got, ref)
 
 
+@pytest.mark.parametrize("n", [40, 41])
+def test_flags_at_the_edge_of_the_sort_rule(n):
+    """32,000 and 33,620 faces: 16 tiles of the radix sort (a launch a pass) and 17 (a count, a scan and a scatter)."""
+    import pamo_gb300
+
+    v, f = meshes.tangled(n, seed=n, frac=0.02, amp=0.05)
+    ref, _ = orc.Oracle().self_intersect(v, f)
+    got = pamo_gb300.self_intersect(torch.from_numpy(v).cuda(), torch.from_numpy(f).cuda()).cpu().numpy()
+    assert ref.sum() > 0 and np.array_equal(got, ref)
+
+
 def test_star_shaped_input_is_clean():
     import pamo_gb300
     from pamo_gb300 import synth
