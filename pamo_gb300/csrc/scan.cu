@@ -74,6 +74,24 @@ __global__ void __launch_bounds__(kThreads) k_scan(ScanJobs jobs, int* err) {
     __shared__ int s_tile, s_prefix;
     unsigned long long* status = reinterpret_cast<unsigned long long*>(scratch + kHeader);
     const int n = (d_n ? *d_n : 0) + n_add;
+    if (gridDim.x == 1) {  // one tile: no tickets, no look-back, each element read once (four scans a round from 1,280
+                           // faces, 4.40 -> 4.24 ms with the fill's ranks)
+        int carry = 0;
+        for (int base = 0; base < n; base += kPass) {
+            const int idx = base + threadIdx.x * kItems;
+            int v[kItems], tot;
+            load4(in, idx, n, v);
+            int run = carry + block_exclusive_scan(v[0] + v[1] + v[2] + v[3], &tot, sm);
+#pragma unroll
+            for (int k = 0; k < kItems; ++k) {
+                if (idx + k < n) out[idx + k] = run;
+                run += v[k];
+            }
+            carry += tot;
+        }
+        if (d_total && threadIdx.x == 0) *d_total = carry;
+        return;
+    }
     if (threadIdx.x == 0) s_tile = atomicAdd(&scratch[kNext], 1);
     __syncthreads();
     const int t = s_tile;
