@@ -572,7 +572,7 @@ struct pamo_csr {
 
     // per vertex / face / edge of a round
     Buf<float4> pos, orig_pos, pos_in, pos_next, res_pos;
-    Buf<int> occ, valence, cursor, vedges, vcursor, vmesh, vscan;
+    Buf<int> occ, valence, vedges, vmesh, vscan;
     Buf<Quadric> quad;
     Buf<unsigned long long> vmin;
     Buf<unsigned char> invalid;
@@ -661,7 +661,7 @@ struct pamo_csr {
         cudaSetDevice(device);
         cudaDeviceSynchronize();
         release(pos); release(orig_pos); release(pos_in); release(pos_next); release(res_pos);
-        release(occ); release(valence); release(cursor); release(vedges); release(vcursor); release(vmesh);
+        release(occ); release(valence); release(vedges); release(vmesh);
         release(vscan); release(quad); release(vmin); release(invalid); release(tri); release(orig_tri);
         release(tri_in); release(tri_next); release(res_tri); release(tri_load); release(ecount); release(qflag);
         release(fflags); release(nt); release(nxt); release(spc); release(fmesh); release(shuffle_flags);
@@ -686,7 +686,7 @@ struct pamo_csr {
         int r;
         if ((r = grow(pos, vc)) || (r = grow(orig_pos, vc)) || (r = grow(pos_in, vc)) || (r = grow(pos_next, vc)) ||
             (r = grow(res_pos, vc)) || (r = grow(occ, vc + 1)) || (r = grow(valence, vc + 1)) ||
-            (r = grow(cursor, vc + 1)) || (r = grow(vedges, vc + 1)) || (r = grow(vcursor, vc + 1)) ||
+            (r = grow(vedges, vc + 1)) || 
             (r = grow(vmesh, vc)) || (r = grow(vscan, vc + 1)) || (r = grow(quad, vc)) || (r = grow(vmin, vc + 1)) ||
             (r = grow(invalid, vc)))
             return r;
@@ -769,11 +769,11 @@ struct pamo_csr {
         rs.rc = rc;
         rs.pts_in = pos_in.p; rs.pos = pos.p; rs.orig_pos = orig_pos.p; rs.occ = occ.p;
         rs.tri_in = tri_in.p; rs.tri = tri.p; rs.orig_tri = orig_tri.p;
-        rs.valence = valence.p; rs.cursor = cursor.p; rs.vedges = vedges.p; rs.vcursor = vcursor.p;
+        rs.valence = valence.p; rs.vedges = vedges.p;
         rs.qflag = qflag.p; rs.vmin = vmin.p;
         launch_round_prologue_dev(rs, Vb, Fb, s);
         // adjacency, quadrics (per element: rings never leave a mesh)
-        launch_face_counts(tri.p, rc, Fb, valence.p, ecount.p, vedges.p, s, pos.p, fgeo.p);
+        launch_face_counts(tri.p, rc, Fb, valence.p, ecount.p, vedges.p, s, pos.p, fgeo.p, spc.p);
         {
             const size_t sz = scan_scratch_ints();
             const ScanJob jobs[3] = {{valence.p, valence.p, &rc->n_pts, 1, nullptr, scan_scratch},
@@ -781,7 +781,7 @@ struct pamo_csr {
                                      {vedges.p, vedges.p, &rc->n_pts, 1, nullptr, scan_scratch + 2 * sz}};
             exclusive_scans(jobs, 3, s, &rc->status, std::max(Vb, Fb));
         }
-        launch_fill_adjacency(tri.p, rc, Fb, valence.p, cursor.p, nt.p, ecount.p, edges.p, vedges.p, vcursor.p,
+        launch_fill_adjacency(tri.p, rc, Fb, valence.p, spc.p, nt.p, ecount.p, edges.p, vedges.p,
                               eorder.p, s);
         const int* nt_off = valence.p;
         launch_ring_quadrics(rc, Vb, nt_off, nt.p, tri.p, fgeo.p, quad.p, nxt.p, spc.p, s);

@@ -105,8 +105,8 @@ struct pamo_ctx {
 
     // ---- per-vertex working buffers ----
     DevBuf<float4> pos, orig_pos, pos_in, pos_out;
-    DevBuf<int> occ, valence, cursor;
-    DevBuf<int> vedges, vcursor;  // edges per lower endpoint (offsets) and fill cursors
+    DevBuf<int> occ, valence;
+    DevBuf<int> vedges;  // edges per lower endpoint (offsets)
     DevBuf<Quadric> quad;
     DevBuf<Quadric> quad_lo;  // precision modes: the quadrics' lo parts (q = quad + quad_lo in double-float)
     DevBuf<unsigned long long> vmin;
@@ -285,9 +285,9 @@ struct pamo_ctx {
             b.n = 0;
         };
         fr(edge_cost); fr(invalid); fr(pts_map); fr(pts_map_prev); fr(undo_list); fr(tmp_undo);
-        fr(pos); fr(orig_pos); fr(pos_in); fr(pos_out); fr(occ); fr(valence); fr(cursor); fr(quad); fr(quad_lo); fr(vmin); fr(undo_in);
+        fr(pos); fr(orig_pos); fr(pos_in); fr(pos_out); fr(occ); fr(valence); fr(quad); fr(quad_lo); fr(vmin); fr(undo_in);
         fr(nxt); fr(spc); fr(fgeo); fr(tri); fr(orig_tri); fr(tri_in); fr(tri_out); fr(ecount); fr(qflag); fr(fflags); fr(nt);
-        fr(shuffle_flags); fr(eorder); fr(vedges); fr(vcursor); fr(hit); fr(edges); fr(win); fr(collapsed); fr(uflag); fr(face_mean); fr(exact_list); fr(place); fr(probe_raw);
+        fr(shuffle_flags); fr(eorder); fr(vedges); fr(hit); fr(edges); fr(win); fr(collapsed); fr(uflag); fr(face_mean); fr(exact_list); fr(place); fr(probe_raw);
         if (bvh_mem) cudaFree(bvh_mem);
         bvh_mem = nullptr;
         prof.destroy();
@@ -356,7 +356,7 @@ struct pamo_ctx {
     size_t device_bytes() const {
         size_t b = 0;
         b += pos.bytes() + orig_pos.bytes() + pos_in.bytes() + pos_out.bytes() + occ.bytes() + valence.bytes() +
-             cursor.bytes() + vedges.bytes() + vcursor.bytes() + quad.bytes() + quad_lo.bytes() + vmin.bytes() +
+             vedges.bytes() + quad.bytes() + quad_lo.bytes() + vmin.bytes() +
              undo_in.bytes();
         b += nxt.bytes() + spc.bytes() + fgeo.bytes();
         b += tri.bytes() + orig_tri.bytes() + tri_in.bytes() + tri_out.bytes() + ecount.bytes() + qflag.bytes() +
@@ -375,7 +375,7 @@ struct pamo_ctx {
         const size_t nc = c + c / 5;
         int r;
         if ((r = grow(pos, nc)) || (r = grow(orig_pos, nc)) || (r = grow(pos_out, nc)) || (r = grow(occ, nc + 1)) ||
-            (r = grow(valence, nc + 1)) || (r = grow(cursor, nc)) || (r = grow(vedges, nc + 1)) || (r = grow(vcursor, nc)) || (r = grow(quad, nc)) || (r = grow(vmin, nc)) ||
+            (r = grow(valence, nc + 1)) || (r = grow(vedges, nc + 1)) ||  (r = grow(quad, nc)) || (r = grow(vmin, nc)) ||
             (r = grow(pos_in, nc)))
             return r;
         cap_v = nc;
@@ -435,12 +435,10 @@ struct pamo_ctx {
             if (nT > 0) launch_shuffle_tris(fb, shuffle_flags.p, scan_scratch, tri_src, tri.p, nT, s, &rc->status);
         }
         cudaMemsetAsync(valence.p, 0, (nP + 1) * sizeof(int), s);
-        cudaMemsetAsync(cursor.p, 0, (nP + 1) * sizeof(int), s);
         cudaMemsetAsync(vedges.p, 0, (nP + 1) * sizeof(int), s);
-        cudaMemsetAsync(vcursor.p, 0, (nP + 1) * sizeof(int), s);
-        launch_face_counts(tri.p, rc, nT, valence.p, ecount.p, vedges.p, s, pos.p, fgeo.p);
+        launch_face_counts(tri.p, rc, nT, valence.p, ecount.p, vedges.p, s, pos.p, fgeo.p, spc.p);
         scan_adjacency_counts(s, std::max(nP, nT));
-        launch_fill_adjacency(tri.p, rc, nT, valence.p, cursor.p, nt.p, ecount.p, edges.p, vedges.p, vcursor.p, eorder.p, s,
+        launch_fill_adjacency(tri.p, rc, nT, valence.p, spc.p, nt.p, ecount.p, edges.p, vedges.p, eorder.p, s,
                               d_ecap);
         const int* nt_off = valence.p;
         const int eb = 2 * nT;
@@ -478,13 +476,11 @@ struct pamo_ctx {
         launch_load_points(pts3, nP, pos.p, orig_pos.p, occ.p, s);
         launch_load_tris(tris3, nT, nP, tri.p, rc, s);
         cudaMemsetAsync(valence.p, 0, (nP + 1) * sizeof(int), s);
-        cudaMemsetAsync(cursor.p, 0, (nP + 1) * sizeof(int), s);
         cudaMemsetAsync(vedges.p, 0, (nP + 1) * sizeof(int), s);
-        cudaMemsetAsync(vcursor.p, 0, (nP + 1) * sizeof(int), s);
         cudaMemsetAsync(invalid.p, 0, invalid.n, s);
-        launch_face_counts(tri.p, rc, nT, valence.p, ecount.p, vedges.p, s, pos.p, fgeo.p, mode > 0);
+        launch_face_counts(tri.p, rc, nT, valence.p, ecount.p, vedges.p, s, pos.p, fgeo.p, spc.p, mode > 0);
         scan_adjacency_counts(s, std::max(nP, nT));
-        launch_fill_adjacency(tri.p, rc, nT, valence.p, cursor.p, nt.p, ecount.p, edges.p, vedges.p, vcursor.p, eorder.p, s);
+        launch_fill_adjacency(tri.p, rc, nT, valence.p, spc.p, nt.p, ecount.p, edges.p, vedges.p, eorder.p, s);
         Quadric* qlo = mode > 0 ? quad_lo.p : nullptr;
         launch_ring_quadrics(rc, nP, valence.p, nt.p, tri.p, fgeo.p, quad.p, nxt.p, spc.p, s, qlo);
         cudaMemsetAsync(vmin.p, 0xFF, (nP + 1) * sizeof(unsigned long long), s);
@@ -527,16 +523,16 @@ struct pamo_ctx {
             rs.pts_map = pts_map.p; rs.pts_map_prev = pts_map_prev.p;
             rs.pts_in = pos_in.p; rs.pos = pos.p; rs.orig_pos = orig_pos.p; rs.occ = occ.p;
             rs.tri_in = tri_in.p; rs.tri = tri.p; rs.orig_tri = orig_tri.p;
-            rs.valence = valence.p; rs.cursor = cursor.p; rs.vedges = vedges.p; rs.vcursor = vcursor.p;
+            rs.valence = valence.p; rs.vedges = vedges.p;
             rs.qflag = qflag.p; rs.vmin = vmin.p;
             launch_round_prologue_dev(rs, nPb, nTb, s);
             UndoBook book;
             book.ls = d_ls; book.verts_undo = undo_in.p; book.tmp_undo = tmp_undo.p; book.undo_list = undo_list.p;
             book.pts_map = pts_map.p; book.map_len = (int)pts_map.n;
             book.invalid = invalid.p; book.invalid_len = (int)invalid.n;
-            launch_face_counts(tri.p, rc, nTb, valence.p, ecount.p, vedges.p, s, pos.p, fgeo.p, precision > 0, book);
+            launch_face_counts(tri.p, rc, nTb, valence.p, ecount.p, vedges.p, s, pos.p, fgeo.p, spc.p, precision > 0, book);
             scan_adjacency_counts(s, std::max(nPb, nTb));
-            launch_fill_adjacency(tri.p, rc, nTb, valence.p, cursor.p, nt.p, ecount.p, edges.p, vedges.p, vcursor.p,
+            launch_fill_adjacency(tri.p, rc, nTb, valence.p, spc.p, nt.p, ecount.p, edges.p, vedges.p,
                                   eorder.p, s, d_ecap);
             launch_ring_quadrics(rc, nPb, nt_off, nt.p, tri.p, fgeo.p, quad.p, nxt.p, spc.p, s, qlo_ptr(), edge_cost.p,
                                  (int)edge_cost.n);
@@ -693,12 +689,10 @@ struct pamo_ctx {
         // adjacency
         prof.begin(kPhAdj, s);
         cudaMemsetAsync(valence.p, 0, (nP + 1) * sizeof(int), s);
-        cudaMemsetAsync(cursor.p, 0, (nP + 1) * sizeof(int), s);
         cudaMemsetAsync(vedges.p, 0, (nP + 1) * sizeof(int), s);
-        cudaMemsetAsync(vcursor.p, 0, (nP + 1) * sizeof(int), s);
-        launch_face_counts(tri.p, rc, nT, valence.p, ecount.p, vedges.p, s, pos.p, fgeo.p, precision > 0);
+        launch_face_counts(tri.p, rc, nT, valence.p, ecount.p, vedges.p, s, pos.p, fgeo.p, spc.p, precision > 0);
         scan_adjacency_counts(s, std::max(nP, nT));
-        launch_fill_adjacency(tri.p, rc, nT, valence.p, cursor.p, nt.p, ecount.p, edges.p, vedges.p, vcursor.p, eorder.p, s,
+        launch_fill_adjacency(tri.p, rc, nT, valence.p, spc.p, nt.p, ecount.p, edges.p, vedges.p, eorder.p, s,
                               d_ecap);
         const int* nt_off = valence.p;
         const int eb = 2 * nT;

@@ -202,7 +202,7 @@ __device__ __forceinline__ float acc_value(const CSum& a) { return a.value(); }
 // plane_df (precision mode): the planes as double-float pairs, fgeo[4n + 2f] (hi) and fgeo[4n + 2f + 1] (lo)
 __global__ void __launch_bounds__(kT) k_face_counts(const int4* __restrict__ tri, const RoundCounters* rc, int* valence,
                                                     int* ecount, int* vedges, const float4* __restrict__ pos,
-                                                    float4* fgeo, int plane_df, UndoBook book) {
+                                                    float4* fgeo, int plane_df, int2* rank, UndoBook book) {
     pdl_wait();
     const int n = rc->n_tris;
     if (book.ls) {
@@ -245,14 +245,16 @@ __global__ void __launch_bounds__(kT) k_face_counts(const int4* __restrict__ tri
                 fgeo[4 * (size_t)n + f] = make_float4(pl[0], pl[1], pl[2], pl[3]);
             }
         }
-        atomicAdd(&valence[t.x], 1);
-        atomicAdd(&valence[t.y], 1);
-        atomicAdd(&valence[t.z], 1);
         ecount[f] = (t.x > t.y) + (t.y > t.z) + (t.z > t.x);  // count_edge_kernel, :306-316
-        // edges per lower endpoint, for the vertex-grouped processing order
-        if (t.x > t.y) atomicAdd(&vedges[t.y], 1);
-        if (t.y > t.z) atomicAdd(&vedges[t.z], 1);
-        if (t.z > t.x) atomicAdd(&vedges[t.x], 1);
+        // each count's old value is the corner's place in its ring (and the edge's among those of its lower endpoint, for
+        // the vertex-grouped processing order), kept for the fill, which then needs no counters of its own
+        const int2 r0 = {atomicAdd(&valence[t.x], 1), t.x > t.y ? atomicAdd(&vedges[t.y], 1) : -1};
+        const int2 r1 = {atomicAdd(&valence[t.y], 1), t.y > t.z ? atomicAdd(&vedges[t.z], 1) : -1};
+        const int2 r2 = {atomicAdd(&valence[t.z], 1), t.z > t.x ? atomicAdd(&vedges[t.x], 1) : -1};
+        int2* at = rank + 3 * (size_t)f;
+        at[0] = r0;
+        at[1] = r1;
+        at[2] = r2;
     }
     if (gtid() == 0) ecount[n] = 0;
 }
@@ -260,10 +262,9 @@ __global__ void __launch_bounds__(kT) k_face_counts(const int4* __restrict__ tri
 // d_cap (or null): the length of the edge costs as the reference sizes them; rc->pad[0] says whether it grew, and then the
 // costs start from zero (k_ring_quadrics)
 __global__ void __launch_bounds__(kT) k_fill_adjacency(const int4* __restrict__ tri, RoundCounters* rc,
-                                                       const int* __restrict__ nt_off, int* cursor, int* nt,
-                                                       const int* __restrict__ edge_off, int2* edges,
-                                                       const int* __restrict__ voff, int* vcursor, int* eorder,
-                                                       int* d_cap) {
+                                                       const int* __restrict__ nt_off, const int2* __restrict__ rank,
+                                                       int* nt, const int* __restrict__ edge_off, int2* edges,
+                                                       const int* __restrict__ voff, int* eorder, int* d_cap) {
     pdl_wait();
     const int n = rc->n_tris;
     if (d_cap && gtid() == 0) {
@@ -275,20 +276,21 @@ __global__ void __launch_bounds__(kT) k_fill_adjacency(const int4* __restrict__ 
     for (int f = gtid(); f < n; f += gstride()) {
         const int4 t = tri[f];
         if (face_killed(t)) continue;
-        nt[nt_off[t.x] + atomicAdd(&cursor[t.x], 1)] = f;
-        nt[nt_off[t.y] + atomicAdd(&cursor[t.y], 1)] = f;
-        nt[nt_off[t.z] + atomicAdd(&cursor[t.z], 1)] = f;
+        const int2 r0 = rank[3 * (size_t)f], r1 = rank[3 * (size_t)f + 1], r2 = rank[3 * (size_t)f + 2];
+        nt[nt_off[t.x] + r0.x] = f;
+        nt[nt_off[t.y] + r1.x] = f;
+        nt[nt_off[t.z] + r2.x] = f;
         int e = edge_off[f];  // create_edge_kernel, :318-335
         if (t.x > t.y) {
-            eorder[voff[t.y] + atomicAdd(&vcursor[t.y], 1)] = e;
+            eorder[voff[t.y] + r0.y] = e;
             edges[e++] = make_int2(t.y, t.x);
         }
         if (t.y > t.z) {
-            eorder[voff[t.z] + atomicAdd(&vcursor[t.z], 1)] = e;
+            eorder[voff[t.z] + r1.y] = e;
             edges[e++] = make_int2(t.z, t.y);
         }
         if (t.z > t.x) {
-            eorder[voff[t.x] + atomicAdd(&vcursor[t.x], 1)] = e;
+            eorder[voff[t.x] + r2.y] = e;
             edges[e++] = make_int2(t.x, t.z);
         }
     }
@@ -1182,7 +1184,7 @@ __global__ void k_round_prologue_dev(RoundStart r) {
             r.occ[np] = 0;
         }
         if (i <= np) {
-            r.valence[i] = r.cursor[i] = r.vedges[i] = r.vcursor[i] = 0;
+            r.valence[i] = r.vedges[i] = 0;
             r.vmin[i] = ~0ull;
         }
         if (i < nf) {
@@ -1272,17 +1274,17 @@ void launch_shuffle_tris(const Feistel& fb, int* flags, int* scan_scratch, int4*
 }
 
 void launch_face_counts(const int4* tri, const RoundCounters* rc, int n_tris_bound, int* valence, int* ecount,
-                        int* vedges, cudaStream_t s, const float4* pos, float4* fgeo, bool plane_df,
+                        int* vedges, cudaStream_t s, const float4* pos, float4* fgeo, int2* rank, bool plane_df,
                         const UndoBook& book) {
     pdl(k_face_counts, grid_for(n_tris_bound, kT), kT, 0, s)(tri, rc, valence, ecount, vedges, pos, fgeo,
-                                                            plane_df ? 1 : 0, book);
+                                                            plane_df ? 1 : 0, rank, book);
     note_launch();
 }
-void launch_fill_adjacency(const int4* tri, RoundCounters* rc, int n_tris_bound, const int* nt_off, int* cursor,
-                           int* nt, const int* edge_off, int2* edges, const int* voff, int* vcursor, int* eorder,
-                           cudaStream_t s, int* d_cap) {
-    pdl(k_fill_adjacency, grid_for(n_tris_bound, kT), kT, 0, s)(tri, rc, nt_off, cursor, nt, edge_off, edges, voff, vcursor,
-                                                               eorder, d_cap);
+void launch_fill_adjacency(const int4* tri, RoundCounters* rc, int n_tris_bound, const int* nt_off, const int2* rank,
+                           int* nt, const int* edge_off, int2* edges, const int* voff, int* eorder, cudaStream_t s,
+                           int* d_cap) {
+    pdl(k_fill_adjacency, grid_for(n_tris_bound, kT), kT, 0, s)(tri, rc, nt_off, rank, nt, edge_off, edges, voff, eorder,
+                                                               d_cap);
     note_launch();
 }
 void launch_ring_quadrics(const RoundCounters* rc, int n_pts_bound, const int* nt_off, int* nt, const int4* tri,

@@ -73,13 +73,15 @@ struct UndoBook {
 // with fgeo: also the per-face geometry the rings read (from pos; room for six float4 per face): a 64-byte record per
 // face (fgeo[4f .. 4f + 3]: edge lengths, normal, corner positions), then the planes after all n faces' records, one
 // float4 per face (fgeo[4n + f]) or, with plane_df (precision mode), a double-float pair (fgeo[4n + 2f], +1)
+// rank: per face, its place in each corner's ring and its edges' places among those of their lower endpoints (three
+// pairs), for launch_fill_adjacency
 void launch_face_counts(const int4* tri, const RoundCounters* rc, int n_tris_bound, int* valence, int* ecount,
-                        int* vedges, cudaStream_t s, const float4* pos = nullptr, float4* fgeo = nullptr,
-                        bool plane_df = false, const UndoBook& book = UndoBook());
+                        int* vedges, cudaStream_t s, const float4* pos, float4* fgeo, int2* rank, bool plane_df = false,
+                        const UndoBook& book = UndoBook());
 // d_cap (or null): the length of the edge costs as the reference sizes them, grown to the round's edges
-void launch_fill_adjacency(const int4* tri, RoundCounters* rc, int n_tris_bound, const int* nt_off, int* cursor,
-                           int* nt, const int* edge_off, int2* edges, const int* voff, int* vcursor, int* eorder,
-                           cudaStream_t s, int* d_cap = nullptr);
+void launch_fill_adjacency(const int4* tri, RoundCounters* rc, int n_tris_bound, const int* nt_off, const int2* rank,
+                           int* nt, const int* edge_off, int2* edges, const int* voff, int* eorder, cudaStream_t s,
+                           int* d_cap = nullptr);
 
 // ---- cost, selection, collapse ----
 // The rings sorted by face, and the quadrics.
@@ -173,7 +175,7 @@ void launch_after_check(RoundCounters* rc, cudaStream_t s);
 
 // ---- device-driven rounds: sizes from LoopState / RoundCounters, host values only bound the grids ----
 // The start of a round in one launch: pos = orig_pos = the round's points, occ = 1 and occ[n_pts] = 0; tri = orig_tri = the
-// round's faces; valence, cursor, vedges, vcursor = 0 and vmin = ~0 over n_pts + 1 entries; qflag = 0 over n_tris + 1
+// round's faces; valence, vedges = 0 and vmin = ~0 over n_pts + 1 entries; qflag = 0 over n_tris + 1
 // entries. With next (device-driven rounds; null: the sizes are rc's and the rest is not touched) also *ls = *next, rc as
 // forward() sets it, the invalid table cleared where undo vertices are carried into a round that is not stuck, and
 // pts_map_prev[0, n_pts) = pts_map (the previous round's map, read by this round's undo passes).
@@ -190,7 +192,7 @@ struct RoundStart {
     int* occ = nullptr;
     const int4* tri_in = nullptr;
     int4 *tri = nullptr, *orig_tri = nullptr;
-    int *valence = nullptr, *cursor = nullptr, *vedges = nullptr, *vcursor = nullptr, *qflag = nullptr;
+    int *valence = nullptr, *vedges = nullptr, *qflag = nullptr;
     unsigned long long* vmin = nullptr;
 };
 void launch_round_prologue_dev(const RoundStart& r, int n_pts_bound, int n_tris_bound, cudaStream_t s);
