@@ -480,69 +480,96 @@ __device__ __forceinline__ float skinny_term(float k4s3, float area, float l01, 
     return 1.0f - rclamp(e, 0.0f, 1.0f);
 }
 
-// One pass over the ring of w (slots in face-index order) for both ring sums of the edge (w, other):
-// * the edge-length term (:449-484): every ring face adds the lengths of its edges whose first vertex is the larger
-//   (t.x > t.y, t.y > t.z, t.z > t.x), to len and their count to cnt;
-// * the flip test and the skinny term with w moved to vm, over the ring faces without `other`: false as soon as a
-//   face's normal flips (the edge is invalid), else each face adds its skinny term to qa and 1 to ntri.
-// Called for the ring of u, then of v, each sum runs in the order of the two separate loops of the reference. The face
-// t is rebuilt from w, nxt[s] and spc[s], and its corners come from the face record, so a slot costs two aligned
+// What one ring slot gives to the two ring sums of the edge (w, other):
+// * the edge-length term (:449-484): the lengths g.x, g.y, g.z of the face's edges whose first vertex is the larger (t.x >
+//   t.y, t.y > t.z, t.z > t.x: longer's bits 0, 1, 2);
+// * the flip test and the skinny term q with w moved to vm, for a face without `other` (counted); ok = false where the
+//   face's normal flips (the edge is invalid).
+// The face t is rebuilt from w, nxt[s] and spc[s], and its corners come from the face record, so a slot costs two aligned
 // 32-byte sectors of the record and contiguous per-slot words.
 // The flip test dot(n_old/|n_old|, n_new/|n_new|) < 0 takes its sign from the unnormalised normals when a
 // float bound proves it (|dot| > 1e-5 |n_old|_1 |n_new|_1, far above the ~1e-6 relative rounding of the
 // normalised form); otherwise the normalised form is evaluated exactly as the reference does.
+struct SlotTerms {
+    float4 g;
+    unsigned longer;
+    bool counted, ok;
+    float q;
+};
+template <bool kLegacy, bool kPow>
+__device__ __forceinline__ SlotTerms slot_terms(int w, int other, V3 vm, int s, const int* __restrict__ nt,
+                                                const int* __restrict__ nxt, const int2* __restrict__ spc,
+                                                const float4* __restrict__ fgeo) {
+    const float k4s3 = 4.0f * sqrtf(3.0f);
+    const float4* r = fgeo + 4 * (size_t)nt[s];
+    const int nx = nxt[s];
+    const int2 pc = spc[s];
+    const int4 t = pc.y == 0 ? make_int4(w, nx, pc.x, 0) : (pc.y == 1 ? make_int4(pc.x, w, nx, 0)
+                                                                      : make_int4(nx, pc.x, w, 0));
+    SlotTerms T;
+    T.g = r[0];
+    T.longer = (t.x > t.y ? 1u : 0u) | (t.y > t.z ? 2u : 0u) | (t.z > t.x ? 4u : 0u);
+    T.counted = !(t.x == other || t.y == other || t.z == other);
+    T.ok = true;
+    T.q = 0.0f;
+    if (!T.counted) return T;
+    T.ok = false;
+    const float4 r1 = r[1], r2 = r[2], r3 = r[3];
+    const bool wx = t.x == w, wy = t.y == w, wz = t.z == w;
+    const V3 n0 = wx ? vm : V3{r1.w, r2.x, r2.y}, n1 = wy ? vm : V3{r2.z, r2.w, r3.x},
+             n2 = wz ? vm : V3{r3.y, r3.z, r3.w};
+    const V3 ou = {r1.x, r1.y, r1.z};
+    const V3 nu = vcross(vsub(n1, n0), vsub(n2, n0));
+    const float du = vdot(ou, nu);
+    const float bound = 1e-5f * T.g.w * (fabsf(nu.x) + fabsf(nu.y) + fabsf(nu.z));
+    if (du < -bound) return T;
+    if (!(du > bound)) {
+        const V3 on = vdiv(ou, vnorm(ou));
+        const V3 nn = vdiv(nu, vnorm(nu));
+        if (vdot(on, nn) < 0) return T;
+    }
+    // an edge without w keeps its length (same operations as the per-face value)
+    const float l01 = (wx || wy) ? vnorm(vsub(n0, n1)) : T.g.x;
+    const float l12 = (wy || wz) ? vnorm(vsub(n1, n2)) : T.g.y;
+    const float l20 = (wz || wx) ? vnorm(vsub(n2, n0)) : T.g.z;
+    const float sh = (l01 + l12 + l20) / 2;  // triangle_area (Heron), :368-375
+    const float heron = sh * (sh - l01) * (sh - l12) * (sh - l20);
+    // A face with area >= l01^2 / (4 sqrt 3) makes the first quotient of the skinny sum at least 1, so the clamped
+    // sum is 1 and the term exactly 0. Most faces are that fat; it is proven here from Heron's product against
+    // (l01^2 / (4 sqrt 3))^2 with a 1e-4 relative margin (far above the few ulps of rounding on either side, the
+    // 2-ulp difference of the device's pow and the double-precision constant of the legacy sum), which skips the
+    // square root and the division. A bound that is not a normal positive number, or a NaN, takes the full path.
+    const float tb = l01 * l01 * 0.144337567f;  // l01^2 / (4 sqrt 3)
+    const float tb2 = tb * tb;
+    if (tb2 > 1e-30f && tb2 < 1e30f && heron >= tb2 * 1.0001f) {
+        T.q = 0.0f;  // the saturated term
+    } else {
+        const float area = sqrtf(heron);
+        T.q = skinny_term<kLegacy, kPow>(k4s3, area, l01, l12, l20);
+    }
+    T.ok = true;
+    return T;
+}
+
+// One pass over the ring of w (slots in face-index order) for both ring sums of the edge (w, other): lengths to len and
+// their count to cnt, skinny terms to qa and the faces to ntri; false as soon as a face flips.
+// Called for the ring of u, then of v, each sum runs in the order of the two separate loops of the reference.
 template <bool kLegacy, bool kPow, class Acc>
 __device__ __forceinline__ bool ring_pass(int w, int other, V3 vm, const int* __restrict__ nt_off,
                                           const int* __restrict__ nt, const int* __restrict__ nxt,
                                           const int2* __restrict__ spc, const float4* __restrict__ fgeo, Acc& len,
                                           int& cnt, Acc& qa, int& ntri) {
-    const float k4s3 = 4.0f * sqrtf(3.0f);
     const int b = nt_off[w + 1];
     for (int s = nt_off[w]; s < b; ++s) {
-        const float4* r = fgeo + 4 * (size_t)nt[s];
-        const int nx = nxt[s];
-        const int2 pc = spc[s];
-        const int4 t = pc.y == 0 ? make_int4(w, nx, pc.x, 0) : (pc.y == 1 ? make_int4(pc.x, w, nx, 0)
-                                                                          : make_int4(nx, pc.x, w, 0));
-        const float4 g = r[0];
-        if (t.x > t.y) { acc_add(len, g.x); cnt++; }
-        if (t.y > t.z) { acc_add(len, g.y); cnt++; }
-        if (t.z > t.x) { acc_add(len, g.z); cnt++; }
-        if (t.x == other || t.y == other || t.z == other) continue;
-        const float4 r1 = r[1], r2 = r[2], r3 = r[3];
-        const bool wx = t.x == w, wy = t.y == w, wz = t.z == w;
-        const V3 n0 = wx ? vm : V3{r1.w, r2.x, r2.y}, n1 = wy ? vm : V3{r2.z, r2.w, r3.x},
-                 n2 = wz ? vm : V3{r3.y, r3.z, r3.w};
-        const V3 ou = {r1.x, r1.y, r1.z};
-        const V3 nu = vcross(vsub(n1, n0), vsub(n2, n0));
-        const float du = vdot(ou, nu);
-        const float bound = 1e-5f * g.w * (fabsf(nu.x) + fabsf(nu.y) + fabsf(nu.z));
-        if (du < -bound) return false;
-        if (!(du > bound)) {
-            const V3 on = vdiv(ou, vnorm(ou));
-            const V3 nn = vdiv(nu, vnorm(nu));
-            if (vdot(on, nn) < 0) return false;
+        const SlotTerms T = slot_terms<kLegacy, kPow>(w, other, vm, s, nt, nxt, spc, fgeo);
+        if (!T.ok) return false;
+        if (T.longer & 1u) { acc_add(len, T.g.x); cnt++; }
+        if (T.longer & 2u) { acc_add(len, T.g.y); cnt++; }
+        if (T.longer & 4u) { acc_add(len, T.g.z); cnt++; }
+        if (T.counted) {
+            acc_add(qa, T.q);
+            ntri++;
         }
-        // an edge without w keeps its length (same operations as the per-face value)
-        const float l01 = (wx || wy) ? vnorm(vsub(n0, n1)) : g.x;
-        const float l12 = (wy || wz) ? vnorm(vsub(n1, n2)) : g.y;
-        const float l20 = (wz || wx) ? vnorm(vsub(n2, n0)) : g.z;
-        const float sh = (l01 + l12 + l20) / 2;  // triangle_area (Heron), :368-375
-        const float heron = sh * (sh - l01) * (sh - l12) * (sh - l20);
-        // A face with area >= l01^2 / (4 sqrt 3) makes the first quotient of the skinny sum at least 1, so the clamped
-        // sum is 1 and the term exactly 0. Most faces are that fat; it is proven here from Heron's product against
-        // (l01^2 / (4 sqrt 3))^2 with a 1e-4 relative margin (far above the few ulps of rounding on either side, the
-        // 2-ulp difference of the device's pow and the double-precision constant of the legacy sum), which skips the
-        // square root and the division. A bound that is not a normal positive number, or a NaN, takes the full path.
-        const float tb = l01 * l01 * 0.144337567f;  // l01^2 / (4 sqrt 3)
-        const float tb2 = tb * tb;
-        if (tb2 > 1e-30f && tb2 < 1e30f && heron >= tb2 * 1.0001f) {
-            acc_add(qa, 0.0f);  // the saturated term
-        } else {
-            const float area = sqrtf(heron);
-            acc_add(qa, skinny_term<kLegacy, kPow>(k4s3, area, l01, l12, l20));
-        }
-        ntri++;
     }
     return true;
 }
@@ -613,6 +640,62 @@ __device__ __forceinline__ void edge_quadric(int u, int v, const Quadric* __rest
     }
 }
 
+// The cost from the two ring sums (cusimp_free.cu:449-585): the mean ring length, the quadric's value at the placement and
+// the mean skinny term.
+template <bool kLegacy, int kMode>
+__device__ __forceinline__ uint32_t cost_of_sums(int u, int v, V3 v0, V3 v1, V3 vm, float len, int cnt, float qa, int ntri,
+                                                 const Quadric* __restrict__ q, const Quadric* __restrict__ qlo, float scale,
+                                                 float tres, float& raw) {
+    len = len / (float)cnt / scale * tres;
+    if (kLegacy) len = len + (len + vnorm(vsub(v0, v1)) / scale * tres);
+    else len = len + vnorm(vsub(v0, v1)) / scale * tres;
+    float m[10], mlo[10];
+    edge_quadric<kMode>(u, v, q, qlo, m, mlo);  // after the ring passes: not live across them
+    if (!kLegacy) qa = 5.0f * qa;  // SKINNY_TRIANGLE_PENALTY
+    const float x = vm.x, y = vm.y, z = vm.z, w = 1.0f;
+    float qem;
+    if constexpr (kMode == 0) {
+        const float m00 = m[0], m01 = m[1], m02 = m[2], m03 = m[3], m11 = m[4], m12 = m[5], m13 = m[6], m22 = m[7],
+                    m23 = m[8], m33 = m[9];
+        // Mat4x4::vTMv (cusimp_free.h:145-152) on the symmetric matrix
+        const float c0 = m00 * x + m01 * y + m02 * z + m03 * w;
+        const float c1 = m01 * x + m11 * y + m12 * z + m13 * w;
+        const float c2 = m02 * x + m12 * y + m22 * z + m23 * w;
+        const float c3 = m03 * x + m13 * y + m23 * z + m33 * w;
+        qem = c0 * x + c1 * y + c2 * z + c3 * w;
+    } else {
+        // the same products with the matrix as hi + lo, each dot compensated
+        const int row[4][4] = {{0, 1, 2, 3}, {1, 4, 5, 6}, {2, 5, 7, 8}, {3, 6, 8, 9}};
+        const float vv[4] = {x, y, z, w};
+        CSum outer;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            CSum inner;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                inner.add_prod(m[row[r][c]], vv[c]);
+                inner.add_prod(mlo[row[r][c]], vv[c]);
+            }
+            outer.add_prod(inner.s, vv[r]);
+            outer.add_prod(inner.c, vv[r]);
+        }
+        qem = outer.value();
+    }
+    const float cost = qem / (scale * scale);
+    float tot;
+    if constexpr (kMode == 0) {
+        tot = cost + len + qa / (float)ntri * tres;
+    } else {
+        CSum t;
+        t.add(cost);
+        t.add(len);
+        t.add(qa / (float)ntri * tres);
+        tot = t.value();
+    }
+    raw = tot;
+    return f2u_sat(rclamp(tot, 0.0f, kCostRange) / kCostRange * kU32MaxF);
+}
+
 // returns false when the reference leaves the stale cost in place. kLegacy: the cost of CUSimp
 // (cusimp.cu:270-471): the mean ring length is counted twice (`edge_len += edge_len + |e|`) and the skinny term
 // has no penalty factor. kMode (precision mode, not the reference's arithmetic): 0 the reference's float order;
@@ -658,56 +741,116 @@ __device__ __forceinline__ bool edge_cost_value(int u, int v, const int* __restr
         out = 0xFFFFFFFFu;
         return true;
     }
-    float len = acc_value(lacc);
-    len = len / (float)cnt / scale * tres;
-    if (kLegacy) len = len + (len + vnorm(vsub(v0, v1)) / scale * tres);
-    else len = len + vnorm(vsub(v0, v1)) / scale * tres;
-    edge_quadric<kMode>(u, v, q, qlo, m, mlo);  // after the ring passes: not live across them
-    float qa = acc_value(qacc);
-    if (!kLegacy) qa = 5.0f * qa;  // SKINNY_TRIANGLE_PENALTY
-    const float x = vm.x, y = vm.y, z = vm.z, w = 1.0f;
-    float qem;
-    if constexpr (kMode == 0) {
-        const float m00 = m[0], m01 = m[1], m02 = m[2], m03 = m[3], m11 = m[4], m12 = m[5], m13 = m[6], m22 = m[7],
-                    m23 = m[8], m33 = m[9];
-        // Mat4x4::vTMv (cusimp_free.h:145-152) on the symmetric matrix
-        const float c0 = m00 * x + m01 * y + m02 * z + m03 * w;
-        const float c1 = m01 * x + m11 * y + m12 * z + m13 * w;
-        const float c2 = m02 * x + m12 * y + m22 * z + m23 * w;
-        const float c3 = m03 * x + m13 * y + m23 * z + m33 * w;
-        qem = c0 * x + c1 * y + c2 * z + c3 * w;
-    } else {
-        // the same products with the matrix as hi + lo, each dot compensated
-        const int row[4][4] = {{0, 1, 2, 3}, {1, 4, 5, 6}, {2, 5, 7, 8}, {3, 6, 8, 9}};
-        const float vv[4] = {x, y, z, w};
-        CSum outer;
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            CSum inner;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                inner.add_prod(m[row[r][c]], vv[c]);
-                inner.add_prod(mlo[row[r][c]], vv[c]);
-            }
-            outer.add_prod(inner.s, vv[r]);
-            outer.add_prod(inner.c, vv[r]);
-        }
-        qem = outer.value();
-    }
-    const float cost = qem / (scale * scale);
-    float tot;
-    if constexpr (kMode == 0) {
-        tot = cost + len + qa / (float)ntri * tres;
-    } else {
-        CSum t;
-        t.add(cost);
-        t.add(len);
-        t.add(qa / (float)ntri * tres);
-        tot = t.value();
-    }
-    raw = tot;
-    out = f2u_sat(rclamp(tot, 0.0f, kCostRange) / kCostRange * kU32MaxF);
+    out = cost_of_sums<kLegacy, kMode>(u, v, v0, v1, vm, acc_value(lacc), cnt, acc_value(qacc), ntri, q, qlo, scale, tres, raw);
     return true;
+}
+
+// The same cost (the reference's arithmetic) by eight lanes an edge, a lane to a ring slot: the slots' terms are made side by
+// side, and every lane adds them in slot order, so the bits are the same. For rounds whose edges leave the GPU idle: there a
+// thread's chain over a dozen slots, two gathers each, set the time. It costs about 1.4 times the instructions. 1,280 faces
+// 4.26 -> 3.84 ms, 20,480 faces 13.95 -> 12.90 ms, a height field of 286k 15.6 -> 14.8 ms.
+constexpr int kCostLanes = 8;
+constexpr int kCostLanesEdges = 1 << 17;  // largest edge bound that takes it
+
+template <bool kPow>
+__device__ __forceinline__ bool ring_pass_lanes(int w, int other, V3 vm, int l, unsigned group, const int* __restrict__ nt_off,
+                                                const int* __restrict__ nt, const int* __restrict__ nxt,
+                                                const int2* __restrict__ spc, const float4* __restrict__ fgeo, float& len,
+                                                int& cnt, float& qa, int& ntri) {
+    const int a = nt_off[w], b = nt_off[w + 1];
+    for (int s0 = a; s0 < b; s0 += kCostLanes) {
+        SlotTerms T;
+        T.g = make_float4(0.f, 0.f, 0.f, 0.f);
+        T.longer = 0;
+        T.counted = false;
+        T.ok = true;
+        T.q = 0.f;
+        if (s0 + l < b) T = slot_terms<false, kPow>(w, other, vm, s0 + l, nt, nxt, spc, fgeo);
+        if (__any_sync(group, !T.ok)) return false;
+        const unsigned bits = T.longer | (T.counted ? 8u : 0u);
+        const int m = min(kCostLanes, b - s0);
+        for (int k = 0; k < m; ++k) {
+            const unsigned f = __shfl_sync(group, bits, k, kCostLanes);
+            const float x = __shfl_sync(group, T.g.x, k, kCostLanes), y = __shfl_sync(group, T.g.y, k, kCostLanes),
+                        z = __shfl_sync(group, T.g.z, k, kCostLanes), q = __shfl_sync(group, T.q, k, kCostLanes);
+            if (f & 1u) len += x;
+            if (f & 2u) len += y;
+            if (f & 4u) len += z;
+            cnt += __popc(f & 7u);
+            if (f & 8u) {
+                qa += q;
+                ntri++;
+            }
+        }
+    }
+    return true;
+}
+
+template <bool kPow>
+__device__ __forceinline__ bool edge_cost_lanes(int u, int v, int l, unsigned group, const int* __restrict__ nt_off,
+                                                const int* __restrict__ nt, const float4* __restrict__ pos,
+                                                const Quadric* __restrict__ q, const float4* __restrict__ fgeo,
+                                                const int* __restrict__ nxt, const int2* __restrict__ spc, float scale,
+                                                float tres, uint32_t& out) {
+    const int ua = nt_off[u], ub = nt_off[u + 1], va = nt_off[v], vb = nt_off[v + 1];
+    int dup = 0;
+    for (int a = ua + l; a < ub; a += kCostLanes) {
+        const int iu = nxt[a];
+        for (int b = va; b < vb; ++b) dup += iu == nxt[b];
+    }
+    for (int o = kCostLanes / 2; o > 0; o >>= 1) dup += __shfl_xor_sync(group, dup, o);
+    if (dup > 2) {
+        out = 0xFFFFFFFFu;
+        return true;
+    }
+    if (dup != 2) return false;
+    const V3 v0 = v3(pos[u]), v1 = v3(pos[v]);
+    const V3 vm = vdiv(vadd(v0, v1), 2.0f);
+    float len = 0.f, qa = 0.f;
+    int cnt = 0, ntri = 0;
+    if (!ring_pass_lanes<kPow>(u, v, vm, l, group, nt_off, nt, nxt, spc, fgeo, len, cnt, qa, ntri) ||
+        !ring_pass_lanes<kPow>(v, u, vm, l, group, nt_off, nt, nxt, spc, fgeo, len, cnt, qa, ntri)) {
+        out = 0xFFFFFFFFu;
+        return true;
+    }
+    float raw;
+    out = cost_of_sums<false, 0>(u, v, v0, v1, vm, len, cnt, qa, ntri, q, nullptr, scale, tres, raw);
+    return true;
+}
+
+template <bool kPow>
+__global__ void __launch_bounds__(kT) k_edge_cost_lanes(const RoundCounters* rc, const int* __restrict__ eorder,
+                                                        const int2* __restrict__ edges, const int* __restrict__ nt_off,
+                                                        const int* __restrict__ nt, const float4* __restrict__ pos,
+                                                        const Quadric* __restrict__ q, const float4* __restrict__ fgeo,
+                                                        const int* __restrict__ nxt, const int2* __restrict__ spc,
+                                                        const unsigned char* __restrict__ invalid, uint32_t* cost,
+                                                        unsigned long long* vmin, const float* d_scale, float tres,
+                                                        int is_stuck_host, const int* is_stuck_dev) {
+    pdl_wait();
+    const int is_stuck = is_stuck_dev ? *is_stuck_dev : is_stuck_host;
+    const float scale = *d_scale;
+    const int n = rc->n_edges, lane = threadIdx.x & 31, l = lane % kCostLanes;
+    const unsigned group = ((1u << kCostLanes) - 1u) << (lane - l);
+    for (long long i = gtid() / kCostLanes; i < n; i += gstride() / kCostLanes) {
+        const int e = eorder[i];
+        const int2 ed = edges[e];
+        const int u = ed.x, v = ed.y;
+        uint32_t c = 0;
+        bool write = false;
+        if (invalid[u] && invalid[v]) {
+            c = 0xFFFFFFFFu;
+            write = true;
+        } else if (!is_stuck) {
+            write = edge_cost_lanes<kPow>(u, v, l, group, nt_off, nt, pos, q, fgeo, nxt, spc, scale, tres, c);
+        }
+        if (l != 0) continue;
+        if (write) cost[e] = c;
+        else c = cost[e];  // stale value of an earlier round
+        const unsigned long long key = ((unsigned long long)c << 32) | (unsigned)e;
+        atomicMin(&vmin[u], key);
+        atomicMin(&vmin[v], key);
+    }
 }
 
 // kBatch: many meshes in one vertex numbering; the scale and is_stuck of an edge's mesh come from per-mesh arrays
@@ -1301,6 +1444,13 @@ void launch_edge_cost(const RoundCounters* rc, int n_edges_bound, const int* eor
                       unsigned long long* vmin,
                       const float* d_scale, float tres, int is_stuck, cudaStream_t s, const int* is_stuck_dev, bool legacy,
                       bool device_pow, int mode, float* raw, float4* place, const Quadric* qlo) {
+    if (!legacy && mode == 0 && !raw && !place && n_edges_bound <= kCostLanesEdges) {
+        const int gl = grid_for((long long)kCostLanes * n_edges_bound, kT);
+        pdl(device_pow ? k_edge_cost_lanes<true> : k_edge_cost_lanes<false>, gl, kT, 0, s)(
+            rc, eorder, edges, nt_off, nt, pos, q, fgeo, nxt, spc, invalid, cost, vmin, d_scale, tres, is_stuck, is_stuck_dev);
+        note_launch();
+        return;
+    }
     const int g = grid_for(n_edges_bound, kT);
 #define PAMO_COST_MODE(M, P, O)                                                                                      \
     pdl(k_edge_cost<false, P, false, M, O>, g, kT, 0, s)(rc, eorder, edges, nt_off, nt, tri, pos, q, fgeo, nxt,       \
