@@ -750,7 +750,9 @@ __device__ __forceinline__ bool edge_cost_value(int u, int v, const int* __restr
 // thread's chain over a dozen slots, two gathers each, set the time. It costs about 1.4 times the instructions. 1,280 faces
 // 4.26 -> 3.84 ms, 20,480 faces 13.95 -> 12.90 ms, a height field of 286k 15.6 -> 14.8 ms.
 constexpr int kCostLanes = 8;
-constexpr int kCostLanesEdges = 1 << 17;  // largest edge bound that takes it
+// largest edge bound that takes it: against 2^15, 2^16, 2^18 and 2^19 the height field of 286k ran 1.04, 1.01, 1.02 and 1.08 times
+// as fast, the others the same or less so
+constexpr int kCostLanesEdges = 1 << 17;
 
 template <bool kPow>
 __device__ __forceinline__ bool ring_pass_lanes(int w, int other, V3 vm, int l, unsigned group, const int* __restrict__ nt_off,
@@ -1117,22 +1119,19 @@ __global__ void __launch_bounds__(kT) k_after_collapse(RoundCounters* rc, const 
 }
 
 // ------------------------------------------------------------------ rollback
+// Eight lanes a collapsed edge, a lane to a slot of each ring: one thread an edge was a chain over a dozen slots (a height
+// field of 286k 14.8 -> 14.7 ms, 20,480 faces 12.9 -> 12.8 ms)
+constexpr int kRingLanes = 8;
+
 __global__ void k_mark_query(const RoundCounters* rc, const int* __restrict__ collapsed, const int2* __restrict__ edges,
                              const int* __restrict__ nt_off, const int* __restrict__ nt, int* qflag) {
     pdl_wait();
     const int n = rc->n_considered;
-    for (int c = gtid(); c < n; c += gstride()) {
+    const int l = threadIdx.x % kRingLanes;
+    for (long long c = gtid() / kRingLanes; c < n; c += gstride() / kRingLanes) {
         const int2 ed = edges[collapsed[c]];
-        for (int side = 0; side < 2; ++side) {
-            const int w = side ? ed.y : ed.x, b = nt_off[w + 1];
-            for (int s0 = nt_off[w]; s0 < b; s0 += 4) {  // four slots at a time: their loads are in flight together
-                int f[4];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) f[k] = nt[min(s0 + k, b - 1)];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) qflag[f[k]] = 1;
-            }
-        }
+        for (int s = nt_off[ed.x] + l; s < nt_off[ed.x + 1]; s += kRingLanes) qflag[nt[s]] = 1;
+        for (int s = nt_off[ed.y] + l; s < nt_off[ed.y + 1]; s += kRingLanes) qflag[nt[s]] = 1;
     }
 }
 
@@ -1148,16 +1147,15 @@ __global__ void k_undo_check(RoundCounters* rc, const int* __restrict__ collapse
     }
     const int n = rc->n_considered;
     if (gtid() == 0) uflag[n] = 0;
-    for (int c = gtid(); c < n; c += gstride()) {
+    const int l = threadIdx.x % kRingLanes;
+    const unsigned group = ((1u << kRingLanes) - 1u) << ((threadIdx.x & 31) - l);
+    for (long long c = gtid() / kRingLanes; c < n; c += gstride() / kRingLanes) {
         const int2 ed = edges[collapsed[c]];
         int f = 0;
-        for (int side = 0; side < 2 && !f; ++side) {
-            const int w = side ? ed.y : ed.x, b = nt_off[w + 1];
-            for (int s0 = nt_off[w]; s0 < b && !f; s0 += 4)
-#pragma unroll
-                for (int k = 0; k < 4; ++k) f |= hit[nt[min(s0 + k, b - 1)]];
-        }
-        uflag[c] = f ? 1 : 0;
+        for (int s = nt_off[ed.x] + l; s < nt_off[ed.x + 1]; s += kRingLanes) f |= hit[nt[s]];
+        for (int s = nt_off[ed.y] + l; s < nt_off[ed.y + 1]; s += kRingLanes) f |= hit[nt[s]];
+        f = __any_sync(group, f);
+        if (l == 0) uflag[c] = f ? 1 : 0;
     }
 }
 
