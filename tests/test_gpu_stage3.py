@@ -251,3 +251,22 @@ def test_two_launch_pcg_equals_cooperative_pcg():
         s.set("cg_mode", mode)
         outs.append(s.project(GV, GF, V, F, 3).cpu().numpy())
     assert np.array_equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("n", [25, 26])
+def test_two_threads_for_one_of_the_sums_threads_give_the_same_bits(n):
+    """12,500 and 13,520 faces: more elements than the default PCG's grid has threads, so that two threads stand for each
+    of the sums' threads. cg_mode 7 has one thread for each, in the same grid; the contacts without a barrier term are left
+    out of both."""
+    from pamo_gb300 import safe_project
+    from tests import meshes
+
+    GV, GF = meshes.sphere(40, seed=3)
+    V, F = meshes.sphere(n, seed=4)
+    out = []
+    for mode in (0, 7):
+        s = safe_project.Stage3System(safe_project.Stage3Config(), "cuda:0")
+        s.set("cg_mode", mode)
+        out.append(s.project(GV.astype(np.float64), GF, V.astype(np.float64), F, 1).cpu().numpy())
+        assert s.stats()["max_contacts"] > 0
+    assert np.isfinite(out[0]).all() and np.array_equal(out[0], out[1])
