@@ -238,9 +238,11 @@ __global__ void __launch_bounds__(kSortThreads) k_rs_scatter(const unsigned* __r
 
 // Up to kFusedTiles tiles: one kernel counts the digits of all four passes (ctl's first 1024 words, zeroed by k_boxes), and a
 // pass is one launch: a tile publishes its own digit counts, waits for the tiles before it, and adds theirs up. Tiles are
-// taken in the order the blocks start, so a tile only waits for blocks that run already; the wait is bounded
-// (kErrIterLimit). In place of a count, a scan and a scatter launch a pass; with more tiles the sums over them (256 tiles^2
-// / 2 words) cost more than the scan (one intersection check of 327,680 faces, 160 tiles: 515 -> 532 us). One tile (up to
+// taken in the order the blocks start, so a tile only waits for blocks that run already; the wait is bounded, and a tile
+// whose counts have not come by then is counted again by the one that waits, from the pass's keys, so that no place is
+// ever formed from counts that were not published. In place of a count, a scan and a scatter launch a pass; with more
+// tiles the sums over them (256 tiles^2 / 2 words) cost more than the scan (one intersection check of 327,680 faces, 160
+// tiles: 515 -> 532 us). One tile (up to
 // 2048 keys): all passes in one block. Twelve launches to five, to one for one tile: a stage-2 run from 1,280 faces 4.44 ->
 // 4.33 ms, from 20,480 faces 14.25 -> 14.02 ms.
 __global__ void __launch_bounds__(kSortThreads) k_rs_digits(const unsigned* __restrict__ keys, const int* d_n, int* total) {
@@ -263,16 +265,17 @@ __global__ void __launch_bounds__(kSortThreads) k_rs_digits(const unsigned* __re
 __global__ void __launch_bounds__(kSortThreads) k_rs_pass(const unsigned* __restrict__ kin, const int* __restrict__ vin,
                                                           unsigned* kout, int* vout, const int* d_n, int shift,
                                                           const int* __restrict__ total, int* ticket, int* ready,
-                                                          int* hist, int* err) {
+                                                          int* hist, int wait_limit) {
     pdl_wait();
     __shared__ SortShared S;
     __shared__ int h[256], sm[33], s_tile;
+    __shared__ unsigned s_late;  // the tiles before this one whose counts have not come
     if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1);
     h[threadIdx.x] = 0;
     __syncthreads();
-    const int tile = s_tile;
+    const int tile = s_tile, n = *d_n;
     int lo, hi;
-    sort_chunk(*d_n, tile, gridDim.x, lo, hi);
+    sort_chunk(n, tile, gridDim.x, lo, hi);
     for (int i = lo + threadIdx.x; i < hi; i += kSortThreads) atomicAdd(&h[(kin[i] >> shift) & 0xFF], 1);
     __syncthreads();
     __stcg(&hist[256 * tile + threadIdx.x], h[threadIdx.x]);
@@ -281,20 +284,36 @@ __global__ void __launch_bounds__(kSortThreads) k_rs_pass(const unsigned* __rest
     if (threadIdx.x == 0) {
         asm volatile("st.release.gpu.global.s32 [%0], 1;" ::"l"(&ready[tile]) : "memory");
     }
-    if ((int)threadIdx.x < tile) {  // at most kFusedTiles - 1 < kSortThreads
-        int there = 0;
-        for (int spins = 0; !there; ++spins) {
+    if (threadIdx.x < 32) {  // a lane to an earlier tile (at most kFusedTiles - 1)
+        int there = (int)threadIdx.x >= tile;
+        for (int spins = 0; !there && spins < wait_limit; ++spins)
             asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(there) : "l"(&ready[threadIdx.x]) : "memory");
-            if (spins > (1 << 22)) {
-                atomicOr(err, kErrIterLimit);
-                break;
+        const unsigned late = __ballot_sync(0xffffffffu, !there);
+        if (threadIdx.x == 0) s_late = late;
+    }
+    __syncthreads();
+    const unsigned late = s_late;
+    int all;
+    int at = block_exclusive_scan(total[threadIdx.x], &all, sm);
+    if (late == 0u) {
+#pragma unroll 8
+        for (int k = 0; k < tile; ++k) at += __ldcg(&hist[256 * k + threadIdx.x]);
+    } else {
+        for (int k = 0; k < tile; ++k) {
+            if (!((late >> k) & 1u)) {
+                at += __ldcg(&hist[256 * k + threadIdx.x]);
+                continue;
             }
+            __syncthreads();  // the counts of the tile before are no longer read
+            h[threadIdx.x] = 0;
+            __syncthreads();
+            int klo, khi;
+            sort_chunk(n, k, gridDim.x, klo, khi);
+            for (int i = klo + threadIdx.x; i < khi; i += kSortThreads) atomicAdd(&h[(kin[i] >> shift) & 0xFF], 1);
+            __syncthreads();
+            at += h[threadIdx.x];
         }
     }
-    int all;
-    int at = block_exclusive_scan(total[threadIdx.x], &all, sm);  // its barriers follow the waits
-#pragma unroll 8
-    for (int k = 0; k < tile; ++k) at += __ldcg(&hist[256 * k + threadIdx.x]);
     S.base[threadIdx.x] = at;
     if (hi > lo) sort_scatter(kin, vin, kout, vout, lo, hi, shift, S);
 }
@@ -1151,7 +1170,7 @@ void bvh_build(BvhBuffers& b, const int4* tri, const float4* pos, RoundCounters*
             int* ticket = b.sort_ctl + 1024 + pass * (1 + kFusedTiles);
             pdl(k_rs_pass, sort_tiles, kSortThreads, 0, s)(b.keys[in], b.vals[in], b.keys[out], b.vals[out], &rc->n_live,
                                                           8 * pass, b.sort_ctl + 256 * pass, ticket, ticket + 1, b.hist,
-                                                          &rc->status); note_launch();
+                                                          b.sort_wait); note_launch();
         }
     } else {
         for (int pass = 0; pass < 4; ++pass) {

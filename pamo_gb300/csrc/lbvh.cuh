@@ -15,6 +15,7 @@ struct BvhBuffers {
     int* vals[2] = {nullptr, nullptr};       // face ids, sort ping-pong
     int* hist = nullptr;               // radix histograms [256 * kSortTiles + 1]
     int* sort_ctl = nullptr;           // the sort's digit totals, tickets and flags
+    int sort_wait = 1 << 22;           // polls of a sort tile before it counts an earlier one itself
     int2* child = nullptr;             // internal node children; v < 0 encodes leaf ~v
     int2* range = nullptr;             // internal node leaf range [lo, hi] (the node index is one end)
     int* iparent = nullptr;            // parent of internal node

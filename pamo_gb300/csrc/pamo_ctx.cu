@@ -850,6 +850,10 @@ int pamo_ctx_set_option(pamo_ctx* ctx, const char* name, int64_t value) {
     } else if (n == "pair_cap") {
         ctx->pair_cap_limit = value;
         ctx->drop_graphs();
+    } else if (n == "test_sort_wait") {  // tests: the sort's waits run out after this many polls
+        if (value < 0 || value > (1 << 22)) return ctx->fail(PAMO_ERR_INVALID_ARG, "test_sort_wait is 0 to 2^22");
+        ctx->bvh.sort_wait = (int)value;
+        ctx->drop_graphs();
     } else return ctx->fail(PAMO_ERR_INVALID_ARG, "unknown option %s", name);
     return PAMO_OK;
 }
