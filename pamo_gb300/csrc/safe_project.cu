@@ -2656,8 +2656,10 @@ __global__ void k_line_search(const float4* __restrict__ q0, const float4* __res
     }
 }
 
-__global__ void k_iter_end(SolverScalars* sc) {
+// A build or refit that gave up says so in its own tree's counters; the host reads only the solver's (bit 1: a tree's limit)
+__global__ void k_iter_end(SolverScalars* sc, const RoundCounters* gt, const RoundCounters* tri, const RoundCounters* edge) {
     pdl_wait();
+    if (gt->status | tri->status | edge->status) sc->status |= 2;
     if (sc->abort) return;
     sc->iters_done += 1;
 }
@@ -3189,7 +3191,7 @@ void Stage3::newton_iteration() {
             launch_energy(q, n);
         }
     }
-    pdl(k_iter_end, 1, 1, 0, s)(sc);
+    pdl(k_iter_end, 1, 1, 0, s)(sc, gt_rc, tri_rc, edge_rc);
     note_launch();
 }
 
@@ -3340,6 +3342,7 @@ int Stage3::run_once(const double* gt_points, const int* gt_tris, int n_gt_point
         RoundCounters h{};
         h.n_pts = NGP;
         h.n_tris = NGT;
+        h.status = test_tree_status;
         cudaMemcpyAsync(gt_rc, &h, sizeof(h), cudaMemcpyHostToDevice, s);
         bvh_build(gt_bvh, gt_tri, gt_pos, gt_rc, NGT, s, false, BvhQuery(), false);
         h.n_pts = NP;
@@ -3449,7 +3452,7 @@ int Stage3::run_once(const double* gt_points, const int* gt_tris, int n_gt_point
         barrier_gave_up = true;
         return fail(PAMO_ERR_ITER_LIMIT, "grid barrier of the PCG timed out");
     }
-    if (h_sc->status & 6) return fail(PAMO_ERR_ITER_LIMIT, "BVH traversal limit in stage 3");
+    if (h_sc->status & 6) return fail(PAMO_ERR_ITER_LIMIT, "BVH build or traversal limit in stage 3");
     stats.last_energy = h_sc->energy;
     stats.max_contacts = h_sc->max_contacts;
     stats.total_contacts = h_sc->total_contacts;
@@ -3513,6 +3516,7 @@ int pamo_stage3_set_param(pamo_stage3* s, const char* name, double value) {
     else if (n == "max_blocks") P.max_blocks = (long long)value;
     else if (n == "use_cuda_graph") s->solver.use_graph = value != 0.0;
     else if (n == "test_barrier_extra") s->solver.test_barrier_extra = (int)value;  // tests: grid barriers run out
+    else if (n == "test_tree_status") s->solver.test_tree_status = (int)value;  // tests: a tree's build gave up
     else if (n == "ccd_fp64") {  // 0 float32 (Warp's kernels), 1 float64, 2 double-float (default)
         if (value != 0.0 && value != 1.0 && value != 2.0) {
             s->solver.err = "ccd_fp64 is 0, 1 or 2";

@@ -87,6 +87,7 @@ public:
     bool use_graph = true;  // capture one Newton iteration as a CUDA graph and replay it
     int cg_mode = 0;        // PCG kernel: 0/1 grid-wide cooperative, 128 threads; 3: 256 threads; 2: one cluster
     int ls_mode = 1;        // line search: 1 trials side by side, 0 a launch pair per trial
+    int test_tree_status = 0;    // the trees' status words at the start of a run (tests of their reporting)
     int test_barrier_extra = 0;  // copied to SolverScalars::barrier_extra at each run (tests of the bounded waits)
     int cluster_size = 1;   // CTAs of the cluster kernel (device limit, at most 16)
 
