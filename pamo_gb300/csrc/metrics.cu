@@ -7,7 +7,8 @@
 // first, all in float, gives an upper bound of the distance; the second collects the triangles that may be as near, and
 // those few take the exact float64 point-triangle distance (Ericson, Real-Time Collision Detection, 5.1.5), the lanes
 // of a warp together. The nearest triangle and the smallest index of equally near ones are the same as by trying every
-// triangle in float64; the margins below hold what float adds.
+// triangle in float64; the margins below hold what float adds. Points that float cannot serve (very far away, or with a
+// thousand triangles that it cannot tell apart) are left to a walk in float64.
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -85,61 +86,96 @@ __device__ __forceinline__ F3 f3(float4 v) { return {v.x, v.y, v.z}; }
 
 __device__ __forceinline__ float unit(float x) { return fminf(fmaxf(x, 0.f), 1.f); }  // a NaN counts as 0
 
-// Distance in float from p to the triangle, and its scale: the largest of |ab|, |ac| and the distance. The point that it
-// is taken to lies in the triangle whatever the rounding did (the parameters are clamped), so the distance is an upper
-// bound of the true one up to the rounding of that point. slim: it is no lower bound to rely on. The parameters come from
-// differences of products of size (side * scale)^2, rounded to about 1e-6 of that and divided by n2 = |ab x ac|^2, so the
-// point is off by up to 1e-6 side^3 scale^2 / n2, within kLower * scale (with a factor of 4) if side^3 scale <= 25 n2.
-__device__ __forceinline__ float tri_distance(F3 p, F3 a, F3 b, F3 c, float& scale, bool& slim) {
-    const F3 ab = fsub(b, a), ac = fsub(c, a), ap = fsub(p, a);
+__device__ __forceinline__ F3 fabs3(F3 a) { return {fabsf(a.x), fabsf(a.y), fabsf(a.z)}; }
+
+// What the float walks compare. For a point p let c be a float point near it, the nearest of the mesh's box, and w = p - c.
+// With y = x - c, |p - x|^2 = |w|^2 + 2 g(x), g(x) = sum over the axes of y (y / 2 - w). |w|^2 is the point's own, so g orders
+// the mesh as the distance does, and from far away it is made of small numbers: its rounding is about 1e-6 of |y| in the
+// distance, however far the point is, where the distance itself is rounded by 1e-7 of its value. From within the mesh's
+// box w is the rounding of p's float copy (which it takes out) and g half the squared distance.
+//
+// The margins, each of the numbers that it comes from, so that one far vertex or point widens nothing else (u = 2^-24 is
+// float's rounding of a value):
+//  * a term y (y / 2 - w) with y, w and each operation rounded is off by at most 6 u |y| (|y| + |w|), with the sum of the
+//    three terms: kTerm of the sum of |y| (|y| + |w|);
+//  * a box's coordinates are those of float copies, off by u of the larger of an axis's two: kBox of it, by which the box is
+//    widened;
+//  * a point of a triangle is y = (a - c) + v ab + w ac, off by at most u (|a| + 10 side + 2 |y|) in an axis, vertices' copies
+//    included, which counts |r| times, r = y - w being the slope of g: kVert of |r| |a|, kSide of |r| side (side: the longer
+//    of |ab| and |ac|; its share of the corner test below included), and the square of both where r vanishes;
+//  * kTiny: products that underflow.
+constexpr float kTerm = 1e-6f, kBox = 2.5e-7f, kVert = 1.5e-7f, kSide = 1.5e-6f, kTiny = 1e-36f;
+
+// g at its least in a box (the exact vertices'), less its margin
+__device__ __forceinline__ void box_axis(float c, float w, float lo, float hi, float& g, float& size) {
+    const float grow = kBox * fmaxf(fabsf(lo), fabsf(hi));
+    const float y = fminf(fmaxf(w, (lo - c) - grow), (hi - c) + grow), m = fabsf(y);
+    g += y * (0.5f * y - w);
+    size += m * (m + fabsf(w));
+}
+__device__ __forceinline__ float box_g(F3 c, F3 w, float4 lo, float4 hi) {
+    float g = 0.f, size = 0.f;
+    box_axis(c.x, w.x, lo.x, hi.x, g, size);
+    box_axis(c.y, w.y, lo.y, hi.y, g, size);
+    box_axis(c.z, w.z, lo.z, hi.z, g, size);
+    return g - kTerm * size;
+}
+
+// g at the triangle's nearest point as float finds it, and its margin err: g + err is an upper bound of the triangle's
+// least g, since the point lies in the triangle whatever the rounding did (the parameters are clamped). With kLow, low is
+// a lower bound: g is convex, so over the triangle it is at least its tangent at that point, which is least at a corner.
+// (For the true nearest point the corners all lie on the far side; how far the parameters are off shows in it.)
+template <bool kLow>
+__device__ __forceinline__ float tri_g(F3 c, F3 w, F3 a, F3 b, F3 d, float& err, float& low) {
+    const F3 ya = fsub(a, c), ab = fsub(b, a), ac = fsub(d, a), ap = fsub(w, ya);
     const float d1 = fdot(ab, ap), d2 = fdot(ac, ap);
-    const float bb = fdot(ab, ab), cc = fdot(ac, ac), bc = fdot(ab, ac);
-    float v = 0.f, w = 0.f;
+    const float bb = fdot(ab, ab), cc = fdot(ac, ac);
+    float s = 0.f, t = 0.f;
     if (!(d1 <= 0.f && d2 <= 0.f)) {
-        const F3 bp = fsub(p, b), cp = fsub(p, c);
+        const F3 bp = fsub(ap, ab), cp = fsub(ap, ac);
         const float d3 = fdot(ab, bp), d4 = fdot(ac, bp), d5 = fdot(ab, cp), d6 = fdot(ac, cp);
         const float vc = d1 * d4 - d3 * d2, vb = d5 * d2 - d1 * d6, va = d3 * d6 - d5 * d4;
-        if (d3 >= 0.f && d4 <= d3) v = 1.f;
-        else if (vc <= 0.f && d1 >= 0.f && d3 <= 0.f) v = unit(d1 / (d1 - d3));
-        else if (d6 >= 0.f && d5 <= d6) w = 1.f;
-        else if (vb <= 0.f && d2 >= 0.f && d6 <= 0.f) w = unit(d2 / (d2 - d6));
+        if (d3 >= 0.f && d4 <= d3) s = 1.f;
+        else if (vc <= 0.f && d1 >= 0.f && d3 <= 0.f) s = unit(d1 / (d1 - d3));
+        else if (d6 >= 0.f && d5 <= d6) t = 1.f;
+        else if (vb <= 0.f && d2 >= 0.f && d6 <= 0.f) t = unit(d2 / (d2 - d6));
         else if (va <= 0.f && (d4 - d3) >= 0.f && (d5 - d6) >= 0.f) {
-            w = unit((d4 - d3) / ((d4 - d3) + (d5 - d6)));
-            v = 1.f - w;
+            t = unit((d4 - d3) / ((d4 - d3) + (d5 - d6)));
+            s = 1.f - t;
         } else {
             const float den = 1.f / (va + vb + vc);
-            v = unit(vb * den);
-            w = fminf(unit(vc * den), 1.f - v);
+            s = unit(vb * den);
+            t = fminf(unit(vc * den), 1.f - s);
         }
     }
-    const F3 r = {ab.x * v + ac.x * w - ap.x, ab.y * v + ac.y * w - ap.y, ab.z * v + ac.z * w - ap.z};
-    const float d = sqrtf(fdot(r, r));
-    const float side = sqrtf(fmaxf(bb, cc)), n2 = bb * cc - bc * bc;
-    scale = fmaxf(side, d);
-    slim = !(n2 > 1e-30f && n2 < 1e30f && side * side * side * scale <= 25.f * n2);
-    return d;
+    const F3 e = {ab.x * s + ac.x * t, ab.y * s + ac.y * t, ab.z * s + ac.z * t};
+    const F3 y = {ya.x + e.x, ya.y + e.y, ya.z + e.z}, r = fsub(y, w);
+    const F3 ma = fabs3(a), my = fabs3(y), mr = fabs3(r), mw = fabs3(w);
+    const float g = y.x * (0.5f * y.x - w.x) + y.y * (0.5f * y.y - w.y) + y.z * (0.5f * y.z - w.z);
+    const float side = sqrtf(fmaxf(bb, cc));
+    const float still = kVert * fmaxf(ma.x, fmaxf(ma.y, ma.z)) + kSide * side;
+    err = kTerm * fdot(my, F3{my.x + mw.x, my.y + mw.y, my.z + mw.z}) + kVert * fdot(mr, ma) +
+          kSide * side * (mr.x + mr.y + mr.z) + still * still;
+    if (kLow) {
+        const F3 eb = fsub(e, ab), ec = fsub(e, ac);
+        low = g - fmaxf(fmaxf(fdot(r, e), fdot(r, eb)), fmaxf(fdot(r, ec), 0.f)) - err;
+    }
+    return g;
 }
 
-// The margins. kCoord of the largest coordinate covers the float copies of a vertex and of the point (2^-24 of it for
-// each of three coordinates, twice) and kTiny squares that underflow; a distance to a point of a triangle is computed
-// within kUpper of the triangle's scale, and the nearest point of a triangle that is not slim is found within kLower of
-// it.
-constexpr float kCoord = 5e-7f, kTiny = 1e-18f, kUpper = 2e-6f, kLower = 1e-4f;
-
-__device__ __forceinline__ float box_sq(F3 p, float4 lo, float4 hi) {
-    const float dx = fmaxf(fmaxf(lo.x - p.x, 0.f), p.x - hi.x), dy = fmaxf(fmaxf(lo.y - p.y, 0.f), p.y - hi.y),
-                dz = fmaxf(fmaxf(lo.z - p.z, 0.f), p.z - hi.z);
-    return dx * dx + dy * dy + dz * dz;
-}
-// squared distances above this are above `upper` for certain
-__device__ __forceinline__ float above(float upper, float margin) {
-    const float u = upper + margin;
-    return u * u * 1.00001f;
-}
+// A point farther from the mesh's box than kFar of its extents is left to the float64 walk at once, one with more than kMaxNear
+// triangles to evaluate when it has that many: from there on the float walk no longer tells what it is for (a flat mesh of 286k
+// faces seen from 1,000 of its extents: thousands of triangles within the rounding of a float).
+constexpr float kFar = 100.f;
+constexpr int kMaxNear = 1024;
 
 // One walk per point in float64 with a float64 box bound took 1.97 ms for 20,000 points and 327,680 faces: the float64
 // pipes (1/64 of the float32 rate) and three dependent loads a node set its time. The whole call, with its copies from and
-// to NumPy arrays, went from 2.94 to 1.16 ms.
+// to NumPy arrays, went from 2.94 to 1.16 ms, and to 0.62 ms with the caller's workspace.
+// With margins of the whole scene's coordinates and of the distance itself, that case kept its time but a vertex at 1e6
+// took 1,079 ms (the float64 walk: 32 ms), 2,000 points at 1e5 1,033 ms (72 ms) and 2,000 points 50 to 100 extents above a
+// flat mesh of 286k faces 1,053 ms (1.25 ms): nearly every triangle was a candidate. With g and its margins they take 4.7,
+// 46 and 0.56 ms, and 2,000 points at 3 to 100 radii of the mesh 11 to 16 ms (20 to 30; 48 to 72).
 __global__ void __launch_bounds__(kQT) k_point_mesh(const double* __restrict__ pts, int np, const double* __restrict__ V,
                                                     const float4* __restrict__ pos, const int4* __restrict__ tri,
                                                     const float4* __restrict__ packed, const unsigned* __restrict__ scene,
@@ -150,18 +186,23 @@ __global__ void __launch_bounds__(kQT) k_point_mesh(const double* __restrict__ p
     __shared__ float s_dist[kStack][kQT];
     __shared__ int s_list[kList][kQT];
     const int nl = rc->n_live, me = threadIdx.x;
-    float extent = 0.f;
+    float ends[6];
     for (int d = 0; d < 6; ++d) {
         const unsigned u = scene[d];
-        extent = fmaxf(extent, fabsf(__uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u)));
+        ends[d] = __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
     }
+    const float extent = fmaxf(ends[3] - ends[0], fmaxf(ends[4] - ends[1], ends[5] - ends[2]));
     // all lanes of a warp make the same number of rounds (the walks end in warp votes)
     for (int i0 = gtid() & ~31; i0 < np; i0 += gstride()) {
         const int i = i0 + (me & 31);
         const bool on = i < np;
         const D3 pd = on ? dload(pts, i) : D3{0.0, 0.0, 0.0};
-        const F3 p = {(float)pd.x, (float)pd.y, (float)pd.z};
-        const float margin = kCoord * fmaxf(extent, fmaxf(fabsf(p.x), fmaxf(fabsf(p.y), fabsf(p.z)))) + kTiny;
+        const F3 c = {fminf(fmaxf((float)pd.x, ends[0]), ends[3]), fminf(fmaxf((float)pd.y, ends[1]), ends[4]),
+                      fminf(fmaxf((float)pd.z, ends[2]), ends[5])};
+        const D3 wd = {pd.x - c.x, pd.y - c.y, pd.z - c.z};
+        const F3 w = {(float)wd.x, (float)wd.y, (float)wd.z};
+        bool left = nl >= 2 && fmaxf(fabsf(w.x), fmaxf(fabsf(w.y), fabsf(w.z))) > kFar * extent;
+        int near = 0;
         float upper = INFINITY;
         double best = INFINITY;
         int bf = -1;
@@ -186,8 +227,7 @@ __global__ void __launch_bounds__(kQT) k_point_mesh(const double* __restrict__ p
         if (nl >= 2) {
             // pass 0: the upper bound; pass 1: the triangles that may be nearest
             for (int pass = 0; pass < 2; ++pass) {
-                int sp = 0, node = on ? 0 : -1, guard = 0, count = 0;
-                float limit = above(upper, margin);
+                int sp = 0, node = on && !left ? 0 : -1, guard = 0, count = 0;
                 while (__any_sync(0xffffffffu, node >= 0)) {
                     if (node >= 0 && ++guard > (1 << 22)) {
                         atomicOr(status, kErrIterLimit);
@@ -196,7 +236,7 @@ __global__ void __launch_bounds__(kQT) k_point_mesh(const double* __restrict__ p
                     if (node >= 0) {
                         const float4* rec = packed + 4 * (size_t)node;
                         const float4 lo0 = __ldg(rec), hi0 = __ldg(rec + 1), lo1 = __ldg(rec + 2), hi1 = __ldg(rec + 3);
-                        float b0 = box_sq(p, lo0, hi0), b1 = box_sq(p, lo1, hi1);
+                        float b0 = box_g(c, w, lo0, hi0), b1 = box_g(c, w, lo1, hi1);
                         int c0 = __float_as_int(lo0.w), c1 = __float_as_int(lo1.w);
                         int g0 = __float_as_int(hi0.w), g1 = __float_as_int(hi1.w);
                         if (b1 < b0) {  // the nearer child first
@@ -208,7 +248,7 @@ __global__ void __launch_bounds__(kQT) k_point_mesh(const double* __restrict__ p
 #pragma unroll
                         for (int side = 0; side < 2; ++side) {
                             const float bd = side ? b1 : b0;
-                            if (bd > limit) continue;
+                            if (bd > upper) continue;
                             const int x = side ? c1 : c0, f = side ? g1 : g0;
                             if (x >= 0) {
                                 if (side) n1 = x;
@@ -216,16 +256,14 @@ __global__ void __launch_bounds__(kQT) k_point_mesh(const double* __restrict__ p
                                 continue;
                             }
                             const int4 t = tri[f];
-                            float scale;
-                            bool slim;
-                            const float d = tri_distance(p, f3(pos[t.x]), f3(pos[t.y]), f3(pos[t.z]), scale, slim);
+                            float err, low = 0.f;
                             if (pass == 0) {
-                                const float u = d + (kUpper * scale + margin);
-                                if (u < upper) {
-                                    upper = u;
-                                    limit = above(upper, margin);
-                                }
-                            } else if (slim || !(d - (kLower * scale + margin) > upper)) {
+                                const float u = tri_g<false>(c, w, f3(pos[t.x]), f3(pos[t.y]), f3(pos[t.z]), err, low) + err + kTiny;
+                                if (u < upper) upper = u;
+                                continue;
+                            }
+                            tri_g<true>(c, w, f3(pos[t.x]), f3(pos[t.y]), f3(pos[t.z]), err, low);
+                            if (!(low > upper)) {  // also where low is not a number
                                 s_list[count++][me] = f;
                             }
                         }
@@ -244,21 +282,109 @@ __global__ void __launch_bounds__(kQT) k_point_mesh(const double* __restrict__ p
                         }
                         while (node < 0 && sp > 0) {
                             --sp;
-                            if (!(s_dist[sp][me] > limit)) node = s_node[sp][me];
+                            if (!(s_dist[sp][me] > upper)) node = s_node[sp][me];
                         }
                     }
                     if (__any_sync(0xffffffffu, count > kList - 2)) {
                         evaluate(count);
+                        near += count;
                         count = 0;
+                        if (near > kMaxNear) {
+                            left = true;
+                            node = -1;
+                            sp = 0;
+                        }
                     }
                 }
                 evaluate(count);
             }
         }
-        if (on) {
+        if (on && left) {
+            // a negative value: the walk in float64 is to find it, from this bound
+            const double bound = ddot(wd, wd) + 2.0 * (double)upper;
+            out_d2[i] = -(fmin(bound, best) * (1.0 + 1e-12) + 1e-300);
+        } else if (on) {
             out_d2[i] = best;
             if (out_face) out_face[i] = bf;
         }
+    }
+}
+
+// squared distance from p to a box widened by a relative 2^-22 (so that it bounds the float64 geometry the float box was
+// rounded from, by 2^-24 of it), as a lower bound for pruning
+__device__ __forceinline__ double box_lower_bound(D3 p, float4 lo, float4 hi) {
+    const double e = 2.384185791015625e-07;  // 2^-22
+    auto axis = [&](double x, float l, float h) {
+        const double dl = (double)l - e * fabs((double)l) - 1e-30, dh = (double)h + e * fabs((double)h) + 1e-30;
+        return x < dl ? dl - x : (x > dh ? x - dh : 0.0);
+    };
+    const double dx = axis(p.x, lo.x, hi.x), dy = axis(p.y, lo.y, hi.y), dz = axis(p.z, lo.z, hi.z);
+    return dx * dx + dy * dy + dz * dz;
+}
+
+// The points that k_point_mesh left, one thread each and all in float64: far away (a float is coarser than the mesh's
+// features there) or with very many triangles at nearly the same distance.
+__global__ void __launch_bounds__(kQT) k_point_mesh_wide(const double* __restrict__ pts, int np, const double* __restrict__ V,
+                                                         const int4* __restrict__ tri, const float4* __restrict__ packed,
+                                                         const RoundCounters* rc, double* out_d2, int* out_face,
+                                                         int* status) {
+    pdl_wait();
+    __shared__ int s_node[kStack][kQT];
+    __shared__ double s_dist[kStack][kQT];
+    if (rc->n_live < 2) return;  // no point is left then
+    const int me = threadIdx.x;
+    for (int i = gtid(); i < np; i += gstride()) {
+        double best = -out_d2[i];
+        if (!(best > 0.0)) continue;
+        const D3 p = dload(pts, i);
+        int bf = -1, sp = 0, node = 0, guard = 0;
+        while (node >= 0) {
+            if (++guard > (1 << 22)) {
+                atomicOr(status, kErrIterLimit);
+                break;
+            }
+            const float4* rec = packed + 4 * (size_t)node;
+            const float4 lo[2] = {__ldg(rec), __ldg(rec + 2)}, hi[2] = {__ldg(rec + 1), __ldg(rec + 3)};
+            int n[2] = {-1, -1};
+            double nd[2];
+#pragma unroll
+            for (int side = 0; side < 2; ++side) {
+                nd[side] = box_lower_bound(p, lo[side], hi[side]);
+                if (nd[side] > best) continue;
+                const int x = __float_as_int(lo[side].w);
+                if (x >= 0) {
+                    n[side] = x;
+                    continue;
+                }
+                const int f = __float_as_int(hi[side].w);
+                const int4 t = tri[f];
+                const D3 c = closest_point_triangle(p, dload(V, t.x), dload(V, t.y), dload(V, t.z));
+                const D3 d = dsub(c, p);
+                const double d2 = ddot(d, d);
+                if (d2 < best || (d2 == best && f < bf)) {
+                    best = d2;
+                    bf = f;
+                }
+            }
+            if (n[0] >= 0 && n[1] >= 0) {
+                if (sp >= kStack) {
+                    atomicOr(status, kErrStackOverflow);
+                    break;
+                }
+                const bool swap = nd[1] < nd[0];
+                s_node[sp][me] = swap ? n[0] : n[1];
+                s_dist[sp++][me] = swap ? nd[0] : nd[1];
+                node = swap ? n[1] : n[0];
+            } else {
+                node = n[0] >= 0 ? n[0] : n[1];
+            }
+            while (node < 0 && sp > 0) {
+                --sp;
+                if (!(s_dist[sp][me] > best)) node = s_node[sp][me];
+            }
+        }
+        out_d2[i] = bf >= 0 ? best : INFINITY;
+        if (out_face) out_face[i] = bf;
     }
 }
 
@@ -354,7 +480,9 @@ int pamo_point_mesh_sqdist_ws(const double* points, int32_t n_points, const doub
     bvh_build(b, tri, pos, rc, n_triangles, s, false, BvhQuery(), false);
     pdl(k_point_mesh, grid_for(n_points, kQT, 16), kQT, 0, s)(points, n_points, vertices, pos, tri, b.packed, b.scene,
                                                              b.vals[0], rc, out_sqdist, out_face, &rc->status);
-    note_launch();
+    pdl(k_point_mesh_wide, grid_for(n_points, kQT, 16), kQT, 0, s)(points, n_points, vertices, tri, b.packed, rc, out_sqdist,
+                                                                  out_face, &rc->status);
+    note_launches(2);
     int st = 0;
     cudaMemcpyAsync(&st, &rc->status, sizeof(int), cudaMemcpyDeviceToHost, s);
     int r = cuda_status(cudaStreamSynchronize(s));
