@@ -1532,6 +1532,125 @@ struct HvpElement {
     float e[kHingeStride];
 };
 
+// The parts of load_element and apply_element by kind. The kernels that do not keep an element join a kind's two parts in
+// one branch (product_element): through the struct of any kind a cluster thread's 64 registers spilled 292 bytes.
+__device__ __forceinline__ void load_tri(HvpElement& E, const float4* __restrict__ x, const HvpArgs& A, long long f) {
+    E.kind = kElTri;
+    const ElasticLocal L = elastic_local(x, E.ids, A.area[f], A.invDm[f]);
+    const Mat2 I = {1.f, 0.f, 0.f, 1.f};
+    const Mat2 S = mscale(0.5f, madd(mmul(mtr(L.F), L.F), mscale(-1.f, I)));
+    const Mat2 M = madd(mscale(2.f * A.mu, S), mscale(A.la * mtrace(S), I));
+    E.e[0] = L.b1.x; E.e[1] = L.b1.y; E.e[2] = L.b1.z;
+    E.e[3] = L.b2.x; E.e[4] = L.b2.y; E.e[5] = L.b2.z;
+    E.e[6] = L.F.a; E.e[7] = L.F.b; E.e[8] = L.F.c; E.e[9] = L.F.d;
+    E.e[10] = L.invDm.a; E.e[11] = L.invDm.b; E.e[12] = L.invDm.c; E.e[13] = L.invDm.d;
+    E.e[14] = M.a; E.e[15] = M.b; E.e[16] = M.c; E.e[17] = M.d;
+    E.e[18] = L.W;
+}
+
+__device__ __forceinline__ void load_hinge(HvpElement& E, const HvpArgs& A, long long h) {
+    E.kind = kElHinge;
+    const float4* B4 = reinterpret_cast<const float4*>(A.blocks + (size_t)h * kHingeStride);
+#pragma unroll
+    for (int k = 0; k < kHingeStride / 4; ++k) {
+        const float4 b = B4[k];
+        E.e[4 * k] = b.x; E.e[4 * k + 1] = b.y; E.e[4 * k + 2] = b.z; E.e[4 * k + 3] = b.w;
+    }
+}
+
+__device__ __forceinline__ void load_contact(HvpElement& E, const HvpArgs& A, long long b) {
+    const float dist = A.cd[b];
+    if (dist >= A.d_hat) {  // no barrier term: zero parts, at the vertices that have others
+        E.kind = kElContactOff;
+        if (!A.S.cact[E.ids.x]) E.at.x = -1;
+        if (!A.S.cact[E.ids.y]) E.at.y = -1;
+        if (!A.S.cact[E.ids.z]) E.at.z = -1;
+        if (!A.S.cact[E.ids.w]) E.at.w = -1;
+        return;
+    }
+    E.kind = kElContact;
+    E.e[12] = barrier_d2(dist, A.d_hat) * A.kappa;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float4 d = A.cdd[4 * (size_t)b + k];
+        E.e[3 * k] = d.x; E.e[3 * k + 1] = d.y; E.e[3 * k + 2] = d.z;
+    }
+}
+
+__device__ __forceinline__ float apply_tri(const HvpElement& E, const HvpArgs& A, const float4* __restrict__ z,
+                                           const float4* __restrict__ vprev, float s) {
+    const F3 v0 = cg_dir(z, vprev, s, E.ids.x), v1 = cg_dir(z, vprev, s, E.ids.y), v2 = cg_dir(z, vprev, s, E.ids.z);
+    const F3 b1 = {E.e[0], E.e[1], E.e[2]}, b2 = {E.e[3], E.e[4], E.e[5]};
+    const Mat2 F = {E.e[6], E.e[7], E.e[8], E.e[9]}, invDm = {E.e[10], E.e[11], E.e[12], E.e[13]},
+               M = {E.e[14], E.e[15], E.e[16], E.e[17]};
+    const Mat2 I = {1.f, 0.f, 0.f, 1.f};
+    const F3 dx01 = v1 - v0, dx02 = v2 - v0;
+    const Mat2 dDs = {dot(b1, dx01), dot(b1, dx02), dot(b2, dx01), dot(b2, dx02)};
+    const Mat2 dF = mmul(dDs, invDm);
+    const Mat2 dE = mscale(0.5f, madd(mmul(mtr(dF), F), mmul(mtr(F), dF)));
+    const float trdE = mtrace(dE);
+    const Mat2 dP = madd(mmul(dF, M), mmul(F, madd(mscale(2.f * A.mu, dE), mscale(A.la * trdE, I))));
+    const Mat2 dH = mmul(mscale(E.e[18], dP), mtr(invDm));
+    const F3 df1 = dH.a * b1 + dH.c * b2;
+    const F3 df2 = dH.b * b1 + dH.d * b2;
+    const F3 df0 = -df1 - df2;
+    A.aslot[E.at.x] = f4(df0);
+    A.aslot[E.at.y] = f4(df1);
+    A.aslot[E.at.z] = f4(df2);
+    return dot(v0, df0) + dot(v1, df1) + dot(v2, df2);
+}
+
+__device__ __forceinline__ float apply_hinge(const HvpElement& E, const HvpArgs& A, const float4* __restrict__ z,
+                                             const float4* __restrict__ vprev, float s) {
+    const int ids[4] = {E.ids.x, E.ids.y, E.ids.z, E.ids.w}, at[4] = {E.at.x, E.at.y, E.at.z, E.at.w};
+    // H v with the fourth block row/column minus the sums of the first three: for w_a = v_a - v_3,
+    // (H v)_a = sum_b A_ab w_b (a < 3), (H v)_3 = -sum_a (H v)_a, and v.H v = w.A w
+    const F3 d3 = cg_dir(z, vprev, s, ids[3]);
+    float w[9];
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+        const F3 wb = cg_dir(z, vprev, s, ids[b]) - d3;
+        w[3 * b] = wb.x; w[3 * b + 1] = wb.y; w[3 * b + 2] = wb.z;
+    }
+    float u[9];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+        float t = 0.f;
+#pragma unroll
+        for (int j = 0; j < 9; ++j) t += E.e[sym9(i, j)] * w[j];
+        u[i] = t;
+    }
+    float vhv = 0.f;
+    F3 sum = {0.f, 0.f, 0.f};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const F3 ua = {u[3 * a], u[3 * a + 1], u[3 * a + 2]};
+        A.aslot[at[a]] = f4(ua);
+        sum = sum + ua;
+        vhv += w[3 * a] * ua.x + w[3 * a + 1] * ua.y + w[3 * a + 2] * ua.z;
+    }
+    A.aslot[at[3]] = f4(-sum);
+    return vhv;
+}
+
+__device__ __forceinline__ float apply_contact(const HvpElement& E, const HvpArgs& A, const float4* __restrict__ z,
+                                               const float4* __restrict__ vprev, float s) {
+    const int ids[4] = {E.ids.x, E.ids.y, E.ids.z, E.ids.w}, at[4] = {E.at.x, E.at.y, E.at.z, E.at.w};
+    if (E.kind == kElContactOff) {
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k = 0; k < 4; ++k)
+            if (at[k] >= 0) A.aslot[at[k]] = zero;
+        return 0.f;
+    }
+    float sd = 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) sd += dot(F3{E.e[3 * k], E.e[3 * k + 1], E.e[3 * k + 2]}, cg_dir(z, vprev, s, ids[k]));
+    const float c = E.e[12];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) A.aslot[at[k]] = f4(F3{E.e[3 * k], E.e[3 * k + 1], E.e[3 * k + 2]} * (sd * c));
+    return sd * sd * c;
+}
+
 __device__ __forceinline__ HvpElement load_element(const float4* __restrict__ x, const HvpArgs& A, int nc, long long g) {
     const long long e1 = A.np, e2 = e1 + A.nt, e3 = e2 + A.nh, total = e3 + nc;
     HvpElement E;
@@ -1548,47 +1667,17 @@ __device__ __forceinline__ HvpElement load_element(const float4* __restrict__ x,
     if (g >= e3 && !A.cneed[g - e3]) return E;  // no parts
     E.ids = element_ids(A, nc, g);
     E.at = element_slots(A, nc, g);
-    if (g < e2) {
-        const int f = (int)(g - e1);
-        E.kind = kElTri;
-        const ElasticLocal L = elastic_local(x, E.ids, A.area[f], A.invDm[f]);
-        const Mat2 I = {1.f, 0.f, 0.f, 1.f};
-        const Mat2 S = mscale(0.5f, madd(mmul(mtr(L.F), L.F), mscale(-1.f, I)));
-        const Mat2 M = madd(mscale(2.f * A.mu, S), mscale(A.la * mtrace(S), I));
-        E.e[0] = L.b1.x; E.e[1] = L.b1.y; E.e[2] = L.b1.z;
-        E.e[3] = L.b2.x; E.e[4] = L.b2.y; E.e[5] = L.b2.z;
-        E.e[6] = L.F.a; E.e[7] = L.F.b; E.e[8] = L.F.c; E.e[9] = L.F.d;
-        E.e[10] = L.invDm.a; E.e[11] = L.invDm.b; E.e[12] = L.invDm.c; E.e[13] = L.invDm.d;
-        E.e[14] = M.a; E.e[15] = M.b; E.e[16] = M.c; E.e[17] = M.d;
-        E.e[18] = L.W;
-    } else if (g < e3) {
-        E.kind = kElHinge;
-        const float4* B4 = reinterpret_cast<const float4*>(A.blocks + (size_t)(g - e2) * kHingeStride);
-#pragma unroll
-        for (int k = 0; k < kHingeStride / 4; ++k) {
-            const float4 b = B4[k];
-            E.e[4 * k] = b.x; E.e[4 * k + 1] = b.y; E.e[4 * k + 2] = b.z; E.e[4 * k + 3] = b.w;
-        }
-    } else {
-        const int b = (int)(g - e3);
-        const float dist = A.cd[b];
-        if (dist >= A.d_hat) {  // no barrier term: zero parts, at the vertices that have others
-            E.kind = kElContactOff;
-            if (!A.S.cact[E.ids.x]) E.at.x = -1;
-            if (!A.S.cact[E.ids.y]) E.at.y = -1;
-            if (!A.S.cact[E.ids.z]) E.at.z = -1;
-            if (!A.S.cact[E.ids.w]) E.at.w = -1;
-            return E;
-        }
-        E.kind = kElContact;
-        E.e[12] = barrier_d2(dist, A.d_hat) * A.kappa;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float4 d = A.cdd[4 * (size_t)b + k];
-            E.e[3 * k] = d.x; E.e[3 * k + 1] = d.y; E.e[3 * k + 2] = d.z;
-        }
-    }
+    if (g < e2) load_tri(E, x, A, g - e1);
+    else if (g < e3) load_hinge(E, A, g - e2);
+    else load_contact(E, A, g - e3);
     return E;
+}
+
+__device__ __forceinline__ float apply_vertex(int i, float w, const float4* __restrict__ z, const float4* __restrict__ vprev,
+                                              float4* vout, float s) {
+    const F3 vi = cg_dir(z, vprev, s, i);
+    vout[i] = f4(vi);
+    return dot(vi, vi * w);
 }
 
 // The corners' parts of H v of one element into A.aslot; returns its part of v.Av. The direction is v = z + s v_prev,
@@ -1596,87 +1685,46 @@ __device__ __forceinline__ HvpElement load_element(const float4* __restrict__ x,
 __device__ __forceinline__ float apply_element(const HvpElement& E, const HvpArgs& A, const float4* __restrict__ z,
                                                const float4* __restrict__ vprev, float4* vout, float s) {
     if (E.kind == kElNone) return 0.f;
-    if (E.kind == kElVertex) {
-        const F3 vi = cg_dir(z, vprev, s, E.index);
-        vout[E.index] = f4(vi);
-        return dot(vi, vi * E.e[0]);
+    if (E.kind == kElVertex) return apply_vertex(E.index, E.e[0], z, vprev, vout, s);
+    if (E.kind == kElTri) return apply_tri(E, A, z, vprev, s);
+    if (E.kind == kElHinge) return apply_hinge(E, A, z, vprev, s);
+    return apply_contact(E, A, z, vprev, s);
+}
+
+// apply_element(load_element(g)), the vertex ids and slots given (they are fixed during a solve)
+__device__ __forceinline__ float product_element(const float4* __restrict__ x, const HvpArgs& A, const float4* __restrict__ z,
+                                                 const float4* __restrict__ vprev, float4* vout, float s, int nc,
+                                                 long long g, int4 ids, int4 at) {
+    const long long e1 = A.np, e2 = e1 + A.nt, e3 = e2 + A.nh;
+    if (g < e1) return apply_vertex((int)g, A.w[g] * A.m2gt_k, z, vprev, vout, s);
+    HvpElement E;
+    E.ids = ids;
+    E.at = at;
+    if (g < e2) {
+        load_tri(E, x, A, g - e1);
+        return apply_tri(E, A, z, vprev, s);
     }
-    if (E.kind == kElTri) {
-        const F3 v0 = cg_dir(z, vprev, s, E.ids.x), v1 = cg_dir(z, vprev, s, E.ids.y), v2 = cg_dir(z, vprev, s, E.ids.z);
-        const F3 b1 = {E.e[0], E.e[1], E.e[2]}, b2 = {E.e[3], E.e[4], E.e[5]};
-        const Mat2 F = {E.e[6], E.e[7], E.e[8], E.e[9]}, invDm = {E.e[10], E.e[11], E.e[12], E.e[13]},
-                   M = {E.e[14], E.e[15], E.e[16], E.e[17]};
-        const Mat2 I = {1.f, 0.f, 0.f, 1.f};
-        const F3 dx01 = v1 - v0, dx02 = v2 - v0;
-        const Mat2 dDs = {dot(b1, dx01), dot(b1, dx02), dot(b2, dx01), dot(b2, dx02)};
-        const Mat2 dF = mmul(dDs, invDm);
-        const Mat2 dE = mscale(0.5f, madd(mmul(mtr(dF), F), mmul(mtr(F), dF)));
-        const float trdE = mtrace(dE);
-        const Mat2 dP = madd(mmul(dF, M), mmul(F, madd(mscale(2.f * A.mu, dE), mscale(A.la * trdE, I))));
-        const Mat2 dH = mmul(mscale(E.e[18], dP), mtr(invDm));
-        const F3 df1 = dH.a * b1 + dH.c * b2;
-        const F3 df2 = dH.b * b1 + dH.d * b2;
-        const F3 df0 = -df1 - df2;
-        A.aslot[E.at.x] = f4(df0);
-        A.aslot[E.at.y] = f4(df1);
-        A.aslot[E.at.z] = f4(df2);
-        return dot(v0, df0) + dot(v1, df1) + dot(v2, df2);
+    if (g < e3) {
+        load_hinge(E, A, g - e2);
+        return apply_hinge(E, A, z, vprev, s);
     }
-    const int ids[4] = {E.ids.x, E.ids.y, E.ids.z, E.ids.w}, at[4] = {E.at.x, E.at.y, E.at.z, E.at.w};
-    if (E.kind == kElHinge) {
-        // H v with the fourth block row/column minus the sums of the first three: for w_a = v_a - v_3,
-        // (H v)_a = sum_b A_ab w_b (a < 3), (H v)_3 = -sum_a (H v)_a, and v.H v = w.A w
-        const F3 d3 = cg_dir(z, vprev, s, ids[3]);
-        float w[9];
-#pragma unroll
-        for (int b = 0; b < 3; ++b) {
-            const F3 wb = cg_dir(z, vprev, s, ids[b]) - d3;
-            w[3 * b] = wb.x; w[3 * b + 1] = wb.y; w[3 * b + 2] = wb.z;
-        }
-        float u[9];
-#pragma unroll
-        for (int i = 0; i < 9; ++i) {
-            float t = 0.f;
-#pragma unroll
-            for (int j = 0; j < 9; ++j) t += E.e[sym9(i, j)] * w[j];
-            u[i] = t;
-        }
-        float vhv = 0.f;
-        F3 sum = {0.f, 0.f, 0.f};
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            const F3 ua = {u[3 * a], u[3 * a + 1], u[3 * a + 2]};
-            A.aslot[at[a]] = f4(ua);
-            sum = sum + ua;
-            vhv += w[3 * a] * ua.x + w[3 * a + 1] * ua.y + w[3 * a + 2] * ua.z;
-        }
-        A.aslot[at[3]] = f4(-sum);
-        return vhv;
-    }
-    if (E.kind == kElContactOff) {
-        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int k = 0; k < 4; ++k)
-            if (at[k] >= 0) A.aslot[at[k]] = zero;
-        return 0.f;
-    }
-    float sd = 0.f;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) sd += dot(F3{E.e[3 * k], E.e[3 * k + 1], E.e[3 * k + 2]}, cg_dir(z, vprev, s, ids[k]));
-    const float c = E.e[12];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) A.aslot[at[k]] = f4(F3{E.e[3 * k], E.e[3 * k + 1], E.e[3 * k + 2]} * (sd * c));
-    return sd * sd * c;
+    load_contact(E, A, g - e3);
+    return apply_contact(E, A, z, vprev, s);
 }
 
 // The corners' parts of H v over the elements first, first + stride, ... into A.aslot; returns this thread's part of
-// v.Av.
+// v.Av. ids0 = element_ids(first), at0 = element_slots(first): a thread of a solve loads them once.
 __device__ __forceinline__ CSum hvp_elements(const float4* __restrict__ x, const HvpArgs& A, const float4* __restrict__ z,
                                              const float4* __restrict__ vprev, float4* vout, float s, int nc,
-                                             long long first, long long stride) {
-    const long long total = (long long)A.np + A.nt + A.nh + nc;
+                                             long long first, long long stride, int4 ids0, int4 at0) {
+    const long long e3 = (long long)A.np + A.nt + A.nh, total = e3 + nc;
     CSum acc;
-    for (long long g = first; g < total; g += stride)
-        acc.add(apply_element(load_element(x, A, nc, g), A, z, vprev, vout, s));
+    for (long long g = first; g < total; g += stride) {
+        if (g >= e3 && !A.cneed[g - e3]) continue;  // no parts
+        const bool own = g == first;
+        acc.add(product_element(x, A, z, vprev, vout, s, nc, g, own ? ids0 : element_ids(A, nc, g),
+                                own ? at0 : element_slots(A, nc, g)));
+    }
     return acc;
 }
 
@@ -1885,7 +1933,8 @@ __global__ void __launch_bounds__(kThreads) k_cg_product(const float4* __restric
     const int nc = sc->n_contacts;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
     const float s_dir = it == 0 ? 0.f : sc->z_r / sc->z_r_last;
-    grid_sum_finish(hvp_elements(x, A, z, vin, vout, s_dir, nc, tid, nthreads), partial, &sc->red_count,
+    grid_sum_finish(hvp_elements(x, A, z, vin, vout, s_dir, nc, tid, nthreads, element_ids(A, nc, tid),
+                                 element_slots(A, nc, tid)), partial, &sc->red_count,
                     &sc->v_A_v, nullptr);
 }
 
@@ -2144,6 +2193,7 @@ __global__ void __launch_bounds__(kClusterThreads) k_cg_cluster(const float4* __
         __syncthreads();
         return v;
     };
+    const int4 ids0 = element_ids(A, nc, tid), at0 = element_slots(A, nc, tid);
     const PrzLanes L = prz_lanes(tid, nthreads, A.np);
     const VRange R0 = vertex_range(A.S, L.group < A.np ? L.group : 0, L.group < A.np);  // the group's first vertex
     float zr = cluster_total(cg_init_vertices(grad, hd, A.np, p, r, z, v0, tid, nthreads)), zr_last = zr;
@@ -2152,7 +2202,7 @@ __global__ void __launch_bounds__(kClusterThreads) k_cg_cluster(const float4* __
         const float4* vin = (it & 1) ? v1 : v0;
         float4* vout = (it & 1) ? v0 : v1;
         const float s_dir = it == 0 ? 0.f : zr / zr_last;
-        vAv = cluster_total(hvp_elements(x, A, z, vin, vout, s_dir, nc, tid, nthreads));
+        vAv = cluster_total(hvp_elements(x, A, z, vin, vout, s_dir, nc, tid, nthreads, ids0, at0));
         const PrzVertex pre = prz_load(A, vout, hd, p, r, L.group < A.np ? L.group : 0, L.group < A.np, L, R0);
         const float zr_new = cluster_total(cg_prz_vertices(A, vout, hd, p, r, z, zr, vAv, L, pre));
         zr_last = zr;
