@@ -701,7 +701,7 @@ __device__ __forceinline__ uint32_t cost_of_sums(int u, int v, V3 v0, V3 v1, V3 
 // has no penalty factor. kMode (precision mode, not the reference's arithmetic): 0 the reference's float order;
 // 1 quadric, ring-length, skinny and cost sums compensated (TwoSum/TwoProd, rounded once); 2 as 1 with the
 // placement at the quadric's minimiser (qem_optimum) instead of the midpoint. raw: the cost before its clamp and
-// quantisation; place: the placement.
+// quantisation; place: the placement, left as it is where there is none (no link of two vertices).
 template <bool kLegacy, bool kPow, int kMode>
 __device__ __forceinline__ bool edge_cost_value(int u, int v, const int* __restrict__ nt_off, const int* __restrict__ nt,
                                                 const int4* __restrict__ tri, const float4* __restrict__ pos,
@@ -890,6 +890,10 @@ __global__ void __launch_bounds__(kT) k_edge_cost(const RoundCounters* rc, const
         }
         uint32_t c = 0;
         bool write;
+        V3 place;
+        // an edge that may collapse by the stale cost of an earlier round (no link of two, a stuck round) has no placement
+        // of its own: the midpoint
+        if constexpr (kOut) place = vdiv(vadd(v3(pos[u]), v3(pos[v])), 2.0f);
         if (!kLegacy && invalid[u] && invalid[v]) {
             c = 0xFFFFFFFFu;
             write = true;
@@ -897,13 +901,14 @@ __global__ void __launch_bounds__(kT) k_edge_cost(const RoundCounters* rc, const
             write = false;
         } else {
             float raw;
-            V3 place;
             write = edge_cost_value<kLegacy, kPow, kMode>(u, v, nt_off, nt, tri, pos, q, fgeo, nxt, spc, scale, tres, c,
                                                           raw, place, qlo);
             if constexpr (kOut) {
                 if (raw_out) raw_out[e] = write ? raw : __int_as_float(0x7fc00000);
-                if (place_out) place_out[e] = make_float4(place.x, place.y, place.z, 0.f);
             }
+        }
+        if constexpr (kOut) {
+            if (place_out) place_out[e] = make_float4(place.x, place.y, place.z, 0.f);
         }
         if (write) cost[e] = c;
         else c = cost[e];  // stale value of an earlier round
