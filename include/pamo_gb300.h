@@ -319,10 +319,11 @@ const char* pamo_stage3_last_error(const pamo_stage3* s);
  * n_line_search_iters, d_hat, coll_stiffness, contact_detection_radius, ee_classify_thres, ccd_slackness,
  * ccd_thickness, ccd_max_iters, spd_max_iters, elas_young_modulus, elas_poisson_ratio, hinge_stiffness,
  * mesh2gt_dist_stiffness, min_angle_thres (degrees), max_blocks. Execution knobs that leave the method
- * unchanged: use_cuda_graph (0/1), ccd_fp64 (1: float64 CCD step, the default; 0: float32 like the reference),
- * cg_mode (PCG launch shape: 0 cooperative 128-thread blocks, 2 one thread-block cluster, 3/4 256/512-thread
- * blocks, 5/6 at least one/two blocks per SM), ls_mode (1: the line search's trials side by side, 0: a
- * launch pair per trial). Unknown names: PAMO_ERR_INVALID_ARG. */
+ * unchanged: use_cuda_graph (0/1), ccd_fp64 (2: CCD step in double-float pairs, the default; 1: float64; 0: float32
+ * like the reference), cg_mode (PCG launch shape: 0 cooperative, 128 threads a block, or 256 of which two stand for
+ * one on meshes with more elements than that grid has threads; 2 one thread-block cluster, 3/4 cooperative 256/512-thread
+ * blocks, 5/6 at least one/two blocks per SM, 7 two ordinary launches per iteration), ls_mode (1: the line search's
+ * trials side by side, 0: a launch pair per trial). Unknown names: PAMO_ERR_INVALID_ARG. */
 int pamo_stage3_set_param(pamo_stage3* s, const char* name, double value);
 
 /*

@@ -645,13 +645,16 @@ void bottom_up(BvhBuffers& b, RoundCounters* rc, int n_bound, const int* new_ids
 }
 
 // ---------------------------------------------------------------- localized query
-// 1. k_query_order: the query faces in leaf (Morton) order, so that neighbouring threads walk the same
+// 1. k_query_gather: the query faces in leaf (Morton) order, so that neighbouring lanes walk the same
 //    part of the tree and test neighbouring faces.
-// 2. k_traverse_list: one thread per query face walks the tree with a short stack in shared memory and emits
-//    every overlapping leaf g as a candidate pair (f, g); a pair of two query faces is emitted only by the lower
-//    face index. Queries that overflow the list or the stack walk again (k_traverse_redo) and decide in place.
-// 3. k_pairs: one thread per candidate pair runs the reference's decision in both orders (float
-//    certificates first, the fp64 path only for undecided pairs) and flags both faces when it holds.
+// 2. k_traverse_list: the lanes of a warp walk the tree for its query faces with short stacks in shared memory, an idle
+//    lane taking a subtree of another's walk, and list every overlapping leaf g as a candidate pair (f, g); a pair of two
+//    query faces is listed only by the lower face index. Queries that overflow the list or the stack walk again
+//    (redo_walks) and decide in place.
+// 3. k_pairs: one thread per candidate pair decides it in both orders by float certificates, and queues the orders that
+//    they leave open.
+// 4. k_pairs_exact: one thread per queued order runs the reference's fp64 decision; then the walks of 2. that are to be
+//    done again.
 __device__ __forceinline__ bool decide_pair(int f, int g, const int4* __restrict__ tri, const float4* __restrict__ pos,
                                             float eps, unsigned& exact) {
     const int4 qt = tri[f], gt = tri[g];

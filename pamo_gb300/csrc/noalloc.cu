@@ -58,7 +58,6 @@ size_t up256(size_t x) { return (x + 255) & ~size_t(255); }
 
 struct Layout {
     pamo::RoundCounters* rc;
-    int* scan_scratch;
     float4* pos;
     float4* orig_pos;
     int* occ;
@@ -79,7 +78,6 @@ Layout carve(unsigned char* base) {
         return p;
     };
     L.rc = (pamo::RoundCounters*)take(sizeof(pamo::RoundCounters));
-    L.scan_scratch = (int*)take(pamo::scan_scratch_ints() * sizeof(int));
     L.pos = (float4*)take((kNoAllocMaxPoints + 2) * sizeof(float4));
     L.orig_pos = (float4*)take((kNoAllocMaxPoints + 2) * sizeof(float4));
     L.occ = (int*)take((kNoAllocMaxPoints + 2) * sizeof(int));

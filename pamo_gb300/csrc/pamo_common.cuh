@@ -121,8 +121,8 @@ inline uint32_t collapse_threshold(float threshold) {
 // those of the kernel before it in the stream have ended, and wait in pdl_wait(), the first statement of every kernel,
 // until that kernel is complete and its writes are visible. Since every kernel waits, the completion of one is the
 // completion of all before it, and the order is a stream's usual one; what is saved is the launch between two kernels
-// (about 47 of them in a stage-2 round). Cooperative launches, memsets and copies stay ordinary.
-// Batch of 64 meshes 150.5 -> 134.4 ms, 5.24M faces 121.3 -> 120.6 ms, 20,480 faces 23.9 -> 22.5 ms, 1,280 faces 8.0 -> 7.3 ms,
+// (21 of them in a stage-2 round). Cooperative launches, memsets and copies stay ordinary.
+// Measured on rounds of 47 kernels: batch of 64 meshes 150.5 -> 134.4 ms, 5.24M faces 121.3 -> 120.6 ms, 20,480 faces 23.9 -> 22.5 ms, 1,280 faces 8.0 -> 7.3 ms,
 // one intersection check 0.81 -> 0.75 ms. Triggering the launch at a kernel's start instead (griddepcontrol.launch_dependents)
 // gains no more on small grids and loses on large ones (144.7 ms, 123.4 ms): the next kernel's blocks then sit beside the
 // running one.

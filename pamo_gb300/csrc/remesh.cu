@@ -167,6 +167,10 @@ __device__ __forceinline__ float box_sq(P3f p, float4 lo, float4 hi) {
 // about 140 M box tests and stays in L2 (the grid's 67 MB). The whole of stage 1, with the bit rows below: 14.8 -> 1.33
 // ms at 256^3 (327,680 faces), 2.58 -> 0.41 ms at 128^3 (20,480 faces); with four samples in flight, the fill's early end and
 // the spread of the cells over the warps 1.30 and 0.37 ms.
+// Measured on a whole call at 128^3, at 256^3 (the meshes above) and for 300 triangles across the whole grid at 256^3:
+// kSplatMax 1024, 2048, 4096: 0.38, 0.38, 0.38 / 1.31, 1.31, 1.31 / 8.9, 8.8, 8.6 ms; kSplatAhead 2, 4, 8: 0.37, 0.38, 0.39 / 1.27, 1.31,
+// 1.63 / 8.8, 8.8, 8.9 ms; kMaxChunks 256, 1024, 4096: 9.5, 8.8, 8.6 ms of the last, the others alike. Beyond the queue the
+// time grows: 1,500 such triangles 128 ms, 1,000 21 ms (918 and 811 ms with a tree walk per sample).
 constexpr int kSplatMax = 2048;      // samples of one warp's task
 constexpr int kSplatAhead = 4;       // samples of a lane whose values are loaded together
 constexpr int kMaxChunks = 1024;     // tasks of one triangle (larger boxes get larger chunks)
