@@ -40,8 +40,8 @@ CONFIGS = {
 STAGE3_STEPS = 5  # PaMO.run's process(..., 5) (simp_cuda/pamo/__init__.py:168-176)
 # DRAM bytes (read + write) per launch of the roofline kernel, from one ncu capture of the same workload
 # (dram__bytes_read.sum + dram__bytes_write.sum, a single-pass metric set, over all 101 launches of one job,
-# averaged); null where none was taken
-NCU_DRAM_BYTES_PER_LAUNCH = {"plain_large": {"edge_cost": 205320420.1}}
+# averaged: 61 launches with a thread an edge and 40 with eight lanes); null where none was taken
+NCU_DRAM_BYTES_PER_LAUNCH = {"plain_large": {"edge_cost": 204866045.5}}
 THRESHOLD, TOLERANCE = 1e-3, 4
 L2_FLUSH_BYTES = 512 << 20
 
