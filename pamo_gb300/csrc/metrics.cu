@@ -166,12 +166,12 @@ __device__ __forceinline__ float tri_g(F3 c, F3 w, F3 a, F3 b, F3 d, float& err,
 }
 
 // A point farther from the mesh's box than kFar of its extents is left to the float64 walk at once, one with more than kMaxNear
-// triangles to evaluate when it has that many: from there on the float walk no longer tells what it is for (a flat mesh seen
+// triangles to evaluate, or kMaxNodes nodes in a walk, when it has that many: from there on the float walk no longer tells what it is for (a flat mesh seen
 // from very far: thousands of triangles within the rounding of a float). 2,000 points at 500 extents of a star-shaped mesh
 // take 16 ms by the float walk and 46 by the other, but 500 to 1,000 extents above a flat mesh 0.78 ms and 0.56, and that
 // gap grows. kMaxNear 256, 1,024 and 4,096 gave the same times in every case tried (the centre of a sphere among them).
 constexpr float kFar = 100.f;
-constexpr int kMaxNear = 1024;
+constexpr int kMaxNear = 1024, kMaxNodes = 1 << 20;
 
 // One walk per point in float64 with a float64 box bound took 1.97 ms for 20,000 points and 327,680 faces: the float64
 // pipes (1/64 of the float32 rate) and three dependent loads a node set its time. The whole call, with its copies from and
@@ -233,9 +233,10 @@ __global__ void __launch_bounds__(kQT) k_point_mesh(const double* __restrict__ p
             for (int pass = 0; pass < 2; ++pass) {
                 int sp = 0, node = on && !left ? 0 : -1, guard = 0, count = 0;
                 while (__any_sync(0xffffffffu, node >= 0)) {
-                    if (node >= 0 && ++guard > (1 << 22)) {
-                        atomicOr(status, kErrIterLimit);
+                    if (node >= 0 && ++guard > kMaxNodes) {
+                        left = true;
                         node = -1;
+                        sp = 0;
                     }
                     if (node >= 0) {
                         const float4* rec = packed + 4 * (size_t)node;

@@ -93,6 +93,21 @@ def test_points_without_a_distance(faces):
     assert np.isinf(d2[bad]).all() and (fi[bad] == -1).all()
 
 
+def test_a_mesh_that_float_sees_as_one_point():
+    """A flat mesh of 4.5M faces far below the points, which lie in the box that a far triangle spans: to float every face is
+    as near as any other, more than the nodes that a walk may take; the walk in float64 tells them apart."""
+    n = 1500
+    x, y = np.meshgrid(np.linspace(0, 1, n + 1), np.linspace(0, 1, n + 1), indexing="ij")
+    V = np.column_stack([x.ravel(), y.ravel(), np.zeros(x.size)])
+    k = np.arange((n + 1) * (n + 1)).reshape(n + 1, n + 1)
+    a, b, c, d = k[:-1, :-1].ravel(), k[1:, :-1].ravel(), k[1:, 1:].ravel(), k[:-1, 1:].ravel()
+    F = np.concatenate([np.stack([a, b, c], 1), np.stack([a, c, d], 1), len(V) + np.arange(3)[None]]).astype(np.int32)
+    V = np.vstack([V, [[4e7, 4e7, 1e7], [4e7 + 10, 4e7, 1e7], [4e7, 4e7 + 10, 1e7]]])
+    P = np.column_stack([np.linspace(0.1, 0.9, 9), np.linspace(0.9, 0.1, 9), np.linspace(2e6, 5e6, 9)])
+    d2, fi = metrics.point_mesh_sqdist(P, V, F)
+    assert np.allclose(d2, P[:, 2] ** 2, rtol=1e-9, atol=0) and (fi >= 0).all() and (fi < len(F) - 1).all()
+
+
 def _seconds(P, V, F):
     metrics.point_mesh_sqdist(P, V, F)
     best = np.inf
