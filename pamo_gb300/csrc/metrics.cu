@@ -100,18 +100,19 @@ __device__ __forceinline__ F3 fabs3(F3 a) { return {fabsf(a.x), fabsf(a.y), fabs
 // float's rounding of a value):
 //  * a term y (y / 2 - w) with y, w and each operation rounded is off by at most 6 u |y| (|y| + |w|), with the sum of the
 //    three terms: kTerm of the sum of |y| (|y| + |w|);
-//  * a box's coordinates are those of float copies, off by u of the larger of an axis's two: kBox of it, by which the box is
-//    widened;
+//  * a box's coordinates are those of float copies: no vertex lies farther out than u of the side's own coordinate (x - u |x|
+//    grows with x), and each side is moved out by kBox of it;
 //  * a point of a triangle is y = (a - c) + v ab + w ac, off by at most u (|a| + 10 side + 2 |y|) in an axis, vertices' copies
 //    included, which counts |r| times, r = y - w being the slope of g: kVert of |r| |a|, kSide of |r| side (side: the longer
 //    of |ab| and |ac|; its share of the corner test below included), and the square of both where r vanishes;
 //  * kTiny: products that underflow.
+//  * kTies: a squared distance in float64 is rounded by a few 2^-53 of itself.
+constexpr float kTies = 1e-14f;
 constexpr float kTerm = 1e-6f, kBox = 2.5e-7f, kVert = 1.5e-7f, kSide = 1.5e-6f, kTiny = 1e-36f;
 
 // g at its least in a box (the exact vertices'), less its margin
 __device__ __forceinline__ void box_axis(float c, float w, float lo, float hi, float& g, float& size) {
-    const float grow = kBox * fmaxf(fabsf(lo), fabsf(hi));
-    const float y = fminf(fmaxf(w, (lo - c) - grow), (hi - c) + grow), m = fabsf(y);
+    const float y = fminf(fmaxf(w, (lo - c) - kBox * fabsf(lo)), (hi - c) + kBox * fabsf(hi)), m = fabsf(y);
     g += y * (0.5f * y - w);
     size += m * (m + fabsf(w));
 }
@@ -205,6 +206,8 @@ __global__ void __launch_bounds__(kQT) k_point_mesh(const double* __restrict__ p
                       fminf(fmaxf((float)pd.z, ends[2]), ends[5])};
         const D3 wd = {pd.x - c.x, pd.y - c.y, pd.z - c.z};
         const F3 w = {(float)wd.x, (float)wd.y, (float)wd.z};
+        // what counts as equally near: also what float64 does not tell apart (g may be the finer from very far)
+        const float tie = kTies * fdot(w, w) + kTiny;
         bool left = nl >= 2 && fmaxf(fabsf(w.x), fmaxf(fabsf(w.y), fabsf(w.z))) > kFar * extent;
         int near = 0;
         float upper = INFINITY;
@@ -263,7 +266,7 @@ __global__ void __launch_bounds__(kQT) k_point_mesh(const double* __restrict__ p
                             const int4 t = tri[f];
                             float err, low = 0.f;
                             if (pass == 0) {
-                                const float u = tri_g<false>(c, w, f3(pos[t.x]), f3(pos[t.y]), f3(pos[t.z]), err, low) + err + kTiny;
+                                const float u = tri_g<false>(c, w, f3(pos[t.x]), f3(pos[t.y]), f3(pos[t.z]), err, low) + err + tie;
                                 if (u < upper) upper = u;
                                 continue;
                             }
@@ -355,7 +358,7 @@ __global__ void __launch_bounds__(kQT) k_point_mesh_wide(const double* __restric
 #pragma unroll
             for (int side = 0; side < 2; ++side) {
                 nd[side] = box_lower_bound(p, lo[side], hi[side]);
-                if (nd[side] > best) continue;
+                if (nd[side] > best * (1.0 + kTies)) continue;  // equally near ones are all visited
                 const int x = __float_as_int(lo[side].w);
                 if (x >= 0) {
                     n[side] = x;
@@ -385,7 +388,7 @@ __global__ void __launch_bounds__(kQT) k_point_mesh_wide(const double* __restric
             }
             while (node < 0 && sp > 0) {
                 --sp;
-                if (!(s_dist[sp][me] > best)) node = s_node[sp][me];
+                if (!(s_dist[sp][me] > best * (1.0 + kTies))) node = s_node[sp][me];
             }
         }
         out_d2[i] = bf >= 0 ? best : INFINITY;

@@ -108,6 +108,45 @@ def test_a_mesh_that_float_sees_as_one_point():
     assert np.allclose(d2, P[:, 2] ** 2, rtol=1e-9, atol=0) and (fi >= 0).all() and (fi < len(F) - 1).all()
 
 
+def _all_sqdist(p, V, F):
+    """Squared distances of p to every face by the kernel's operations (Ericson, Real-Time Collision Detection, 5.1.5) in
+    float64 and in its order."""
+    dot = lambda u, w: u[..., 0] * w[..., 0] + u[..., 1] * w[..., 1] + u[..., 2] * w[..., 2]
+    a, b, c = V[F[:, 0]], V[F[:, 1]], V[F[:, 2]]
+    ab, ac, ap, bp, cp = b - a, c - a, p - a, p - b, p - c
+    d1, d2, d3, d4, d5, d6 = dot(ab, ap), dot(ac, ap), dot(ab, bp), dot(ac, bp), dot(ab, cp), dot(ac, cp)
+    va, vb, vc = d3 * d6 - d5 * d4, d5 * d2 - d1 * d6, d1 * d4 - d3 * d2
+    with np.errstate(all="ignore"):
+        t, u, w, den = d1 / (d1 - d3), d2 / (d2 - d6), (d4 - d3) / ((d4 - d3) + (d5 - d6)), 1.0 / (va + vb + vc)
+        s, r = vb * den, vc * den
+        q = a + (ab * s[:, None] + ac * r[:, None])
+        q = np.where(((va <= 0) & (d4 - d3 >= 0) & (d5 - d6 >= 0))[:, None], b + w[:, None] * (c - b), q)
+        q = np.where(((vb <= 0) & (d2 >= 0) & (d6 <= 0))[:, None], a + u[:, None] * ac, q)
+        q = np.where(((d6 >= 0) & (d5 <= d6))[:, None], c, q)
+        q = np.where(((vc <= 0) & (d1 >= 0) & (d3 <= 0))[:, None], a + t[:, None] * ab, q)
+        q = np.where(((d3 >= 0) & (d4 <= d3))[:, None], b, q)
+        q = np.where(((d1 <= 0) & (d2 <= 0))[:, None], a, q)
+    return dot(q - p, q - p)
+
+
+@pytest.mark.parametrize("away", [0.0, 1e3, 1e12])
+@pytest.mark.parametrize("far", [1.0, 1e2, 1e6, 1e9, 1e12, 1e15, 1e18])
+def test_the_smallest_index_of_equally_near_faces(far, away):
+    """The face by trying all in float64, where from far away many are equally near after rounding; with a far face, whose
+    box the points lie near (then the float walk takes them), and without."""
+    V, F = meshes.sphere(9)
+    V = V.astype(np.float64)
+    if away:
+        F = np.vstack([F, len(V) + np.arange(3)[None]]).astype(np.int32)
+        V = np.vstack([V, away * np.array([[4, 4, 4], [4.25, 4, 4], [4, 4.25, 4]])])
+    rng = np.random.default_rng(12)
+    P = -far * np.abs(rng.normal(0, 1.0, (97, 3)))  # on the other side than the far face
+    d2, fi = metrics.point_mesh_sqdist(P, V, F)
+    for i, p in enumerate(P):
+        all_d2 = _all_sqdist(p, V, F)
+        assert d2[i] == all_d2.min() and fi[i] == np.flatnonzero(all_d2 == all_d2.min())[0], (far, away, i)
+
+
 def _seconds(P, V, F):
     metrics.point_mesh_sqdist(P, V, F)
     best = np.inf
