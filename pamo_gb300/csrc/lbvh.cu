@@ -291,10 +291,9 @@ __global__ void __launch_bounds__(kSortThreads) k_rs_pass(const unsigned* __rest
         const unsigned late = __ballot_sync(0xffffffffu, !there);
         if (threadIdx.x == 0) s_late = late;
     }
-    __syncthreads();
-    const unsigned late = s_late;
     int all;
-    int at = block_exclusive_scan(total[threadIdx.x], &all, sm);
+    int at = block_exclusive_scan(total[threadIdx.x], &all, sm);  // its barriers follow the waits
+    const unsigned late = s_late;
     if (late == 0u) {
 #pragma unroll 8
         for (int k = 0; k < tile; ++k) at += __ldcg(&hist[256 * k + threadIdx.x]);
